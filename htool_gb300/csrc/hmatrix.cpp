@@ -911,6 +911,9 @@ void HMatrix::finalize(const std::vector<const double *> &bufs, const std::vecto
     c_h.assign((std::size_t)g_c[ng], P2Contrib{});
     c_leaf.assign((std::size_t)g_c[ng], 0);
     cidx_h.assign((std::size_t)g_q[ng], 0);
+    p2grp_h.assign(ng, int2{0, 0});
+    for (std::size_t gi = 0; gi < ng; gi++)
+        p2grp_h[gi] = make_int2((int)g_p[gi], groups[gorder[gi]].second);
     const long long off_p2 = off;
     constexpr long long kGroupGrain = 512;
     const long long nranges = ((long long)ng + kGroupGrain - 1) / kGroupGrain;
@@ -1072,7 +1075,8 @@ void HMatrix::finalize(const std::vector<const double *> &bufs, const std::vecto
     const double tl2 = now();
     assign_phase1_modes();
     emu_fresh_ = false; // fac was rewritten
-    upload_phase1_lists();
+    precision_ = 0;
+    upload_fp64_lists();
     lr_d.upload(lr_h, stream_);
     rot_d.upload(rot_h, stream_);
     {
@@ -1091,7 +1095,6 @@ void HMatrix::finalize(const std::vector<const double *> &bufs, const std::vecto
     st_.layout_device_seconds = tl2 - tl1;
     st_.layout_lists_seconds  = now() - tl2;
     mu_cap     = 0;
-    precision_ = 0;
     build_oz_arena(); // the digit planes follow new factors (none while off)
 }
 
@@ -1099,10 +1102,12 @@ void HMatrix::ensure_work(int mu) {
     if (mu <= mu_cap)
         return;
     layout_gen_++; // work buffers move: captured products are stale
+    // paired panels run an odd number of right-hand sides padded by one
+    const std::size_t even = mu > 1 ? (std::size_t)(mu + 1) & ~(std::size_t)1 : 1;
     xp.alloc((std::size_t)nc * mu + 1);
-    xs.alloc((std::size_t)nc * mu + 1);
+    xs.alloc((std::size_t)nc * even + 1);
     xexp.alloc(1);
-    A.alloc((std::size_t)std::max<long long>(a_slots, 1) * mu);
+    A.alloc((std::size_t)std::max<long long>(a_slots, 1) * even);
     z.alloc((std::size_t)std::max<long long>(zlen_, 1) * mu);
     xstage.alloc((std::size_t)nc * mu);
     ystage.alloc((std::size_t)nr * mu);
@@ -1332,12 +1337,178 @@ void HMatrix::upload_phase1_lists() {
     sc_d.upload(ch, stream_);
     if (ch.empty())
         sc_d.alloc(1);
-    if (!status_d.p) {
-        status_d.alloc(1);
-        HTGPU_CUDA(cudaMemsetAsync(status_d.p, 0, sizeof(int), stream_));
-        tickets_d.alloc(16); // phase 2: 0..7, phase 1: 8
-    }
+    ensure_status();
     HTGPU_CUDA(cudaStreamSynchronize(stream_));
+}
+
+void HMatrix::release_pair() {
+    pair_ready_ = false;
+    pair_d.release();
+    pair1_d.release();
+    pair2_d.release();
+    pairo_d.release();
+    n_pair1_ = n_pair2_ = 0;
+}
+
+// The paired panels of both phases (pair.cu). Phase 1: the Vt columns of
+// the leaves on one source cluster stacked, 32 to a panel, tile by tile.
+// Phase 2: every target cluster's rows cut at 32 (a full panel keeps every
+// lane busy; balanced cuts of 24 or 25 rows would leave a quarter idle), the
+// columns those of its row chunks. False when the mirror does not fit.
+bool HMatrix::build_pair() {
+    release_pair();
+    struct Tile { // one source tile: the sorted leaves [l0, l1), its outputs
+        int l0, l1, ch, jlen, xrow, nout;
+        long long out0, src;
+    };
+    // leaves by source cluster: counting sort on the first column, then by size
+    std::vector<int> first(lr_h.size(), 0), order, start((std::size_t)nc + 1, 0);
+    for (std::size_t i = 0; i < p1_h.size(); i++)
+        if ((p1_h[i].chunk & ~kEmuBit) == 0)
+            first[p1_h[i].leaf] = (int)i;
+    int nlr = 0;
+    for (const LrLeaf &L : lr_h)
+        if (L.r > 0) {
+            start[L.oj + 1]++;
+            nlr++;
+        }
+    for (int j = 0; j < nc; j++)
+        start[j + 1] += start[j];
+    order.resize(nlr);
+    {
+        std::vector<int> at(start.begin(), start.end() - 1);
+        for (int l = 0; l < (int)lr_h.size(); l++)
+            if (lr_h[l].r > 0)
+                order[at[lr_h[l].oj]++] = l;
+    }
+    host_parallel_chunks(nc, 4096, [&](long long lo, long long hi) {
+        for (long long j = lo; j < hi; j++)
+            if (start[j + 1] - start[j] > 1)
+                std::stable_sort(order.begin() + start[j], order.begin() + start[j + 1], [&](int a, int b) { return lr_h[a].n > lr_h[b].n; });
+    });
+    std::vector<Tile> tiles;
+    long long nout = 0, off = 0, np1 = 0;
+    for (int a = 0; a < nlr;) {
+        const LrLeaf &L = lr_h[order[a]];
+        int b = a, r = 0;
+        for (; b < nlr && lr_h[order[b]].oj == L.oj && lr_h[order[b]].n == L.n; b++)
+            r += lr_h[order[b]].r;
+        for (int ch = 0; ch < L.nch; ch++) {
+            const int j0 = ch * kPhase1Chunk, jlen = std::min(kPhase1Chunk, L.n - j0);
+            tiles.push_back({a, b, ch, jlen, L.oj + j0, r, nout, off});
+            nout += r;
+            np1 += (r + kPairRows - 1) / kPairRows;
+            off += 16LL * jlen * (r / kPairRows * (kPairRows / 2) + (r % kPairRows + 1) / 2);
+        }
+        a = b;
+    }
+    std::vector<int> oslot((std::size_t)nout);
+    std::vector<long long> osrc((std::size_t)nout);
+    std::vector<PairPanel> pan1((std::size_t)np1), pan2;
+    std::vector<long long> tp(tiles.size() + 1, 0);
+    for (std::size_t t = 0; t < tiles.size(); t++)
+        tp[t + 1] = tp[t] + (tiles[t].nout + kPairRows - 1) / kPairRows;
+    host_parallel_chunks((long long)tiles.size(), 256, [&](long long lo, long long hi) {
+        for (long long t = lo; t < hi; t++) {
+            const Tile &tl = tiles[(std::size_t)t];
+            std::size_t o  = (std::size_t)tl.out0;
+            for (int a = tl.l0; a < tl.l1; a++) {
+                const LrLeaf &L      = lr_h[order[a]];
+                const long long base = p1_h[first[order[a]] + tl.ch].off;
+                for (int k = 0; k < L.r; k++, o++) {
+                    oslot[o] = (int)(L.a_off + (long long)tl.ch * L.r + k);
+                    osrc[o]  = base + (long long)k * tl.jlen;
+                }
+            }
+            long long src = tl.src;
+            for (int c = 0; c * kPairRows < tl.nout; c++) {
+                const int h                  = std::min(kPairRows, tl.nout - c * kPairRows);
+                pan1[(std::size_t)(tp[t] + c)] = {src, tl.jlen, h, tl.xrow, (int)(tl.out0 + c * kPairRows)};
+                src += 16LL * tl.jlen * ((h + 1) / 2);
+            }
+        }
+    });
+    std::vector<PairSource> src2;
+    for (const int2 &g : p2grp_h) {
+        const PanelItem &pi = pan_h[g.x];
+        for (int lo = 0; lo < g.y; lo += kPairRows) {
+            const int h = std::min(kPairRows, g.y - lo);
+            pan2.push_back({off, pi.ncol, h, pi.q0, pi.row0 + lo});
+            src2.push_back({g.x, g.y, lo});
+            off += 16LL * pi.ncol * ((h + 1) / 2);
+        }
+    }
+    std::size_t fr = 0, tot = 0;
+    HTGPU_CUDA(cudaMemGetInfo(&fr, &tot));
+    if (nout >= (1LL << 31) || (std::size_t)off > fr / 4 * 3)
+        return false;
+    pair_d.alloc((std::size_t)std::max<long long>(off, 16));
+    pair1_d.upload(pan1, stream_);
+    pair2_d.upload(pan2, stream_);
+    pairo_d.upload(oslot, stream_);
+    n_pair1_ = (int)pan1.size();
+    n_pair2_ = (int)pan2.size();
+    {
+        DevBuf<long long> so;
+        DevBuf<PairSource> s2;
+        DevBuf<PanelItem> pd;
+        so.upload(osrc, stream_);
+        s2.upload(src2, stream_);
+        pd.upload(pan_h, stream_);
+        launch_pair_pack(pair1_d.p, n_pair1_, so.p, pair2_d.p, s2.p, n_pair2_, pd.p, fac.p, pair_d.p, stream_);
+        HTGPU_CUDA(cudaStreamSynchronize(stream_));
+    }
+    pair_ready_ = true;
+    return true;
+}
+
+// the FP64 products' launch lists: paired panels, or the chunk lists and
+// pre-split mirrors of the other kernels
+void HMatrix::upload_fp64_lists() {
+    if (!(pair_auto_ && presplit_on_ && emu_ok_ && precision_ == 0 && build_pair())) {
+        release_pair();
+        upload_phase1_lists();
+        return;
+    }
+    layout_gen_++; // buffers or launch lists change: captured products are stale
+    emu_.release();
+    emu2_.release();
+    emu_fresh_        = false;
+    fp64_lists_stale_ = false;
+    p1_bytes_ = p2_bytes_ = n_cols_ = 0;
+    for (auto &it : p1_h)
+        p1_bytes_ += 8LL * it.jlen * lr_h[it.leaf].r;
+    for (auto &pi : pan_h) {
+        p2_bytes_ += 8LL * pi.h * pi.ncol;
+        n_cols_ += pi.ncol;
+    }
+    n_sctas_  = stream_ctas() * kStreamWarpsPerCta * 8;
+    n_chunks_ = n_ranges_ = n_pair2_;
+    ensure_status();
+    HTGPU_CUDA(cudaStreamSynchronize(stream_));
+}
+
+// the caller chose a kernel or a split: FP64 products leave the paired panels
+void HMatrix::leave_pair() {
+    if (!pair_auto_)
+        return;
+    pair_auto_ = false;
+    if (!fac.p)
+        return;
+    if (precision_ != 0) { // the FP64 policy brings the lists
+        fp64_lists_stale_ = true;
+        return;
+    }
+    HTGPU_CUDA(cudaSetDevice(device_));
+    upload_fp64_lists();
+}
+
+void HMatrix::ensure_status() {
+    if (status_d.p)
+        return;
+    status_d.alloc(1);
+    HTGPU_CUDA(cudaMemsetAsync(status_d.p, 0, sizeof(int), stream_));
+    tickets_d.alloc(16); // phase 2: 0..7, phase 1: 8, paired panels: 10, 11
 }
 
 int HMatrix::device_status() {
@@ -1473,10 +1644,15 @@ void HMatrix::set_fp64_split(int p1, int n64) {
         upload_mixed_phase2();
         return;
     }
+    pair_auto_ = false;
+    apply_fp64_split(p1, n64);
+}
+
+void HMatrix::apply_fp64_split(int p1, int n64) {
     p1_permille_ = p1;
     p2_n64_      = n64;
     assign_phase1_modes();
-    upload_phase1_lists();
+    upload_fp64_lists();
 }
 
 void HMatrix::get_fp64_split(int *p1, int *n64) const {
@@ -1516,11 +1692,15 @@ void HMatrix::set_precision(int policy, double tau) {
         emu3_.release(); // the reduced-precision products' mirror
         tca_d.release();  // and the tensor cores' copy of the factors
         tcoff_d.release();
-        if (fp64_lists_stale_) // FP64 chunk lists and pre-split mirrors back
-            upload_phase1_lists();
+        if (fp64_lists_stale_) // the FP64 products' lists and mirrors back
+            upload_fp64_lists();
         if (oz_on_)
             build_oz_arena(); // the FP64 planes
         return;
+    }
+    if (pair_ready_) {
+        release_pair();
+        fp64_lists_stale_ = true;
     }
     if (emu_.p || emu2_.p) { // the reduced-precision products need no FP64 mirrors
         emu_.release();
@@ -1918,6 +2098,12 @@ void HMatrix::launch_product_with(const double *x, double *y, int mu_out, int nu
     // ones past mu_out zero, and writes mu_out
     const int mu     = std::max(mu_out, mu_run);
     const int groups = rhs_groups(mu);
+    // FP64 on paired panels, but many right-hand sides on the digit planes
+    // where they are
+    if (pair_ready_ && precision_ == 0 && !(mu >= kDfMinRhs && oz_S_ == 8 && w_oz && n_ozblk64_ > 0 && n_ozpan_ > 0)) {
+        launch_pair_product(x, y, mu_out, numbering, st, w_xs, w_xexp, w_A, w_z, marks, w_A != A.p);
+        return;
+    }
     launches_        = 0;
     launch_xexp(x, (long long)nc * mu_out, w_xexp, st);
     launch_gather_split(x, nc, numbering == kUserNumbering ? perm_s.p : nullptr, nc, mu, w_xexp, w_xp, w_xs, st, mu_out);
@@ -2066,6 +2252,39 @@ void HMatrix::launch_product_with(const double *x, double *y, int mu_out, int nu
     launches_ += 1;
 }
 
+// A product on paired panels: passes of 8, 6, 4, 2 or 1 right-hand sides,
+// each its split input, both phases and the sums between them; exact: the
+// scratch holds mu right-hand sides and none of padding
+void HMatrix::launch_pair_product(const double *x, double *y, int mu, int numbering, cudaStream_t st, F2 *w_xs, int *w_xexp, double *w_A, double *w_z, cudaEvent_t *marks, bool exact) {
+    float *X = reinterpret_cast<float *>(w_xs), *Af = reinterpret_cast<float *>(w_A);
+    float2 *zf   = reinterpret_cast<float2 *>(w_z);
+    int *tickets = tickets_d.p + 10;
+    launch_xexp(x, (long long)nc * mu, w_xexp, st);
+    launches_ = 1;
+    for (int c0 = 0; c0 < mu;) {
+        const int w = pair_pass_width(mu - c0, exact), n = std::min(w, mu - c0);
+        launch_pair_gather(x, nc, numbering == kUserNumbering ? perm_s.p : nullptr, nc, c0, w, mu, w_xexp, X, tickets, st);
+        if (marks && c0 == 0)
+            HTGPU_CUDA(cudaEventRecord(marks[0], st));
+        launch_pair_phase1(pair1_d.p, n_pair1_, tickets, pair_d.p, pairo_d.p, X, Af, w, status_d.p, st);
+        launch_pair_reduce(lr_d.p, multi_d.p, (int)multi_h.size(), w, Af, st);
+        if (!rot_h.empty())
+            launch_pair_rotate(rot_d.p, (long long)rot_h.size(), w, Af, st);
+        if (marks && c0 + n == mu)
+            HTGPU_CUDA(cudaEventRecord(marks[1], st));
+        launch_pair_phase2(pair2_d.p, n_pair2_, tickets, pair_d.p, cidx_d.p, X, Af, w, n, zf + (long long)c0 * zlen_, (int)zlen_, status_d.p, st);
+        launches_ += 2 + (n_pair1_ > 0) + !multi_h.empty() + !rot_h.empty();
+        c0 += n;
+    }
+    if (marks)
+        HTGPU_CUDA(cudaEventRecord(marks[2], st));
+    if (numbering == kGlobalToLocal)
+        launch_pair_zsum(zi_d.p + zloc0_, zloc1_ - zloc0_, zl_d.p, zf, (int)zlen_, mu, nullptr, w_xexp, y, local_row_count(), st, local_row_offset());
+    else
+        launch_pair_zsum(zi_d.p, (int)zi_h.size(), zl_d.p, zf, (int)zlen_, mu, numbering == kUserNumbering ? perm_t.p : nullptr, w_xexp, y, nr, st);
+    launches_ += 1;
+}
+
 // the per-cluster sums into y: every row in user or cluster numbering, or
 // (global-to-local products) the local rows only, at y[i - local offset]
 // the dense FP64 chunks of a reduced-precision product with many right-hand
@@ -2104,19 +2323,22 @@ void HMatrix::set_phase2_mode(int mode) {
     layout_gen_++; // captured products are stale
     require(mode == 0 || mode == 1, "phase-2 mode must be 0 (per-warp streams) or 1 (producer-fed)");
     p2_mode_ = mode;
+    leave_pair();
 }
 
 void HMatrix::set_phase1_mode(int mode) {
     layout_gen_++; // buffers or launch lists change: captured products are stale
     require(mode >= 0 && mode <= 2, "phase-1 mode must be 0 (tile kernels), 1 (streamed chunks) or 2 (tensor cores for reduced-precision products with 8 or more right-hand sides)");
     p1_mode_ = mode;
+    leave_pair();
 }
 
 void HMatrix::set_presplit(bool on) {
     HTGPU_CUDA(cudaSetDevice(device_));
     presplit_on_ = on;
+    pair_auto_   = false; // the kernels whose pre-split copies this switches
     if (fac.p) {
-        upload_phase1_lists();
+        upload_fp64_lists();
         if (precision_ != 0 && !ch2_h_.empty())
             upload_mixed_phase2();
     }
@@ -2215,6 +2437,16 @@ void HMatrix::autotune(int mu, int reps, float *best_ms) {
         }
         if (run >= kMmaMinRhs && n_tcblk_ > 0)
             try_digit_planes();
+    } else if (presplit_on_ && emu_ok_ && (pair_auto_ = true, upload_fp64_lists(), pair_ready_)) {
+        // paired panels, with many right-hand sides against the digit planes
+        best = timed();
+        if (mu >= kDfMinRhs)
+            try_digit_planes();
+        HTGPU_CUDA(cudaEventDestroy(e0));
+        HTGPU_CUDA(cudaEventDestroy(e1));
+        if (best_ms)
+            *best_ms = best;
+        return;
     } else {
         // every phase-1 mode with every DFMA/emulation split
         std::vector<std::pair<int, int>> splits;
@@ -2229,7 +2461,7 @@ void HMatrix::autotune(int mu, int reps, float *best_ms) {
         for (int mode : {0, 1})
             for (auto &c : splits) {
                 p1_mode_ = mode;
-                set_fp64_split(c.first, c.second);
+                apply_fp64_split(c.first, c.second);
                 const float ms = timed();
                 if (ms < best) {
                     best     = ms;
@@ -2238,7 +2470,7 @@ void HMatrix::autotune(int mu, int reps, float *best_ms) {
                 }
             }
         p1_mode_ = arg_mode;
-        set_fp64_split(arg.first, arg.second);
+        apply_fp64_split(arg.first, arg.second);
         if (rhs_run(mu) >= kDfMinRhs)
             try_digit_planes();
     }
@@ -2407,7 +2639,8 @@ void HMatrix::mvprod_transp(const double *in, double *out, int mu, bool host_ptr
             auto t = std::unique_ptr<HMatrix>(new HMatrix(Sz_, Tz_, eps_, eta_, device_, true));
             t->set_complex_layout(true);
             t->set_leaves(nl, lr.data(), uvt.data(), nd, dn.data(), ddt.data());
-            t->set_fp64_split(p1_permille_, p2_n64_);
+            if (!pair_auto_)
+                t->set_fp64_split(p1_permille_, p2_n64_);
             transp_ = std::move(t);
         }
         if (transp_->precision() != precision_ || (precision_ != 0 && transp_->tau_ != tau_))
@@ -2478,7 +2711,8 @@ void HMatrix::mvprod_transp(const double *in, double *out, int mu, bool host_ptr
         }
         auto t = std::unique_ptr<HMatrix>(new HMatrix(S, T, eps_, eta_, device_));
         t->set_leaves((int)lr_h.size(), lr.data(), uvt.data(), (int)dn_h.size(), dn.data(), ddt.data());
-        t->set_fp64_split(p1_permille_, p2_n64_);
+        if (!pair_auto_)
+            t->set_fp64_split(p1_permille_, p2_n64_);
         transp_ = std::move(t);
     }
     if (transp_->precision() != precision_ || (precision_ != 0 && transp_->tau_ != tau_))
@@ -2755,6 +2989,7 @@ std::map<std::string, std::string> HMatrix::infos() const {
     m["GPU_phase2_stream_ranges"]      = inum(precision_ ? n_ranges_m_ : n_ranges_);
     m["GPU_phase1_mode"]               = inum(p1_mode_);
     m["GPU_presplit_bytes"]            = inum(presplit_bytes());
+    m["GPU_paired_panels"]             = inum(pair_ready_ ? n_pair1_ + n_pair2_ : 0);
     return m;
 }
 

@@ -198,7 +198,7 @@ class HMatrix {
     int phase1_mode() const { return p1_mode_; }
     void set_presplit(bool on);
     bool presplit() const { return presplit_on_; }
-    long long presplit_bytes() const { return (long long)(((emu_fresh_ ? emu_.n : 0) + emu2_.n + emu3_.n) * sizeof(F2)); }
+    long long presplit_bytes() const { return (long long)(((emu_fresh_ ? emu_.n : 0) + emu2_.n + emu3_.n) * sizeof(F2) + pair_d.n); }
     void set_phase2_mode(int mode);
     int phase2_mode() const { return p2_mode_; }
     // tensor-core kernels of reduced-precision products with many
@@ -328,6 +328,23 @@ class HMatrix {
     const OzScratch *oz_scratch(int mu); // the H-matrix's own, when it holds mu right-hand sides
     void launch_sums(double *y, int mu, int numbering, const double *w_z, cudaStream_t st);
     void upload_phase1_lists();
+    // FP64 products on paired panels (pair.cu): the way they run unless the
+    // caller chose a DFMA split, a phase mode or no pre-split copies
+    // (pair_auto_), where every stored entry may be emulated and the mirror
+    // fits; upload_fp64_lists builds it or the lists of the other kernels
+    bool pair_auto_  = true;
+    bool pair_ready_ = false;
+    DevBuf<unsigned char> pair_d;
+    DevBuf<PairPanel> pair1_d, pair2_d;
+    DevBuf<int> pairo_d;
+    int n_pair1_ = 0, n_pair2_ = 0;
+    bool build_pair();
+    void release_pair();
+    void leave_pair();
+    void upload_fp64_lists();
+    void apply_fp64_split(int p1, int n64);
+    void ensure_status();
+    void launch_pair_product(const double *x, double *y, int mu, int numbering, cudaStream_t st, F2 *w_xs, int *w_xexp, double *w_A, double *w_z, cudaEvent_t *marks, bool exact);
     DevBuf<P1Item> p1e_d; // phase-1 tiles on the emulation (p1_d: on DFMA)
     DevBuf<F2> emu_;          // (hi, lo) split of the phase-1 region of fac, for an all-emulated streamed phase 1 (FP64 products)
     bool emu_fresh_ = false;  // emu_ matches fac
@@ -338,6 +355,7 @@ class HMatrix {
     bool fp64_lists_stale_ = false; // FP64 launch lists built while a reduced precision was set
     int n_p1_dfma_ = 0, n_p1_emu_ = 0;
     std::vector<PanelItem> pan_h; // phase-2 panels (one per P2Item)
+    std::vector<int2> p2grp_h;    // target clusters: (first panel, rows)
     std::vector<int> cidx_h;      // panel column coefficients
     DevBuf<int> cidx_d, cidxm_d;
     int n_p2_dfma_ = 0, n_p2_emu_ = 0; // phase-2 panels by kind of their first chunk

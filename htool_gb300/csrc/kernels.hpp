@@ -308,6 +308,43 @@ void launch_phase1_df_mrhs(const P1Item *items, int nitems, const LrLeaf *lr, co
 // part of a reduced-precision product) instead of writing it
 void launch_phase2_df_mrhs(const StreamChunk *chunks, const int *rc, int nrc, const unsigned char *fac, const unsigned char *pre, const int *cidx, const double *A, const F2 *xs, const int *xexp,
                            int mu, double *z, int zlen, bool add, cudaStream_t st);
+// ---- FP64 products on paired panels (pair.cu) ------------------------------
+// one panel: h <= 32 outputs x ncol inputs from byte src of the mirror on
+// (ceil(h / 2) 16-byte pairs {hi0, hi1, lo0, lo1} per input). Phase 1: the
+// inputs are the rows coef .. of x, the outputs the slots oslot[out ..];
+// phase 2: the inputs are cidx[coef ..], the outputs the z rows out ..
+struct PairPanel {
+    long long src;
+    int ncol, h, coef, out;
+};
+// where a phase-2 panel's rows lo .. of a target cluster of m rows sit in the
+// FP64 arena: the cluster's row-chunk panels pan0 ..
+struct PairSource {
+    int pan0, m, lo;
+};
+constexpr int kPairRows = 32; // outputs of a panel at most
+// right-hand sides of the next pass of a product with `left` to go: 8, 6, 4,
+// 2 or 1; an odd count above 1 runs padded by one, or (exact: scratch without
+// room for it) as an even pass and a single one
+int pair_pass_width(int left, bool exact);
+// the mirrors of both phases from the FP64 arena (osrc: the element offset of
+// every phase-1 output's column; s2: where the phase-2 panels' rows are)
+void launch_pair_pack(const PairPanel *p1, int np1, const long long *osrc, const PairPanel *p2, const PairSource *s2, int np2, const PanelItem *pan, const double *fac, unsigned char *mirror,
+                      cudaStream_t st);
+// one pass of w right-hand sides c0 .. (those from mu_src on zero): the split
+// input X (n x w pairs of floats; clears tickets[0..1]), the phase-1 sums A
+// (slots x w), the sums of multi-tile leaves, i times the sums (native complex
+// layout), the partial sums z of the first nrhs of them (zlen apart), and
+// the final sums over all mu
+void launch_pair_gather(const double *x, int ldx, const int *perm, int n, int c0, int w, int mu_src, const int *xexp, float *X, int *tickets, cudaStream_t st);
+void launch_pair_phase1(const PairPanel *panels, int npanels, int *tickets, const unsigned char *mirror, const int *oslot, const float *X, float *A, int w, int *status, cudaStream_t st);
+void launch_pair_reduce(const LrLeaf *lr, const int *multi, int nmulti, int w, float *A, cudaStream_t st);
+void launch_pair_rotate(const int2 *rows, long long nrows, int w, float *A, cudaStream_t st);
+void launch_pair_phase2(const PairPanel *panels, int npanels, int *tickets, const unsigned char *mirror, const int *cidx, const float *X, float *A, int w, int nrhs, float2 *z, int zlen, int *status,
+                        cudaStream_t st);
+void launch_pair_zsum(const ZItem *items, int nitems, const int *zl, const float2 *z, int zlen, int mu, const int *perm, const int *xexp, double *y, int ldy, cudaStream_t st, int shift = 0);
+// the limit of its waits and a panel whose first copy is left out (set_debug_waits)
+void set_pair_waits(long long cycles, long long skip);
 // ---- ACA rank predictor (mlp.cu) -------------------------------------------
 constexpr int kMlpIn = 10, kMlpHidden = 64;
 constexpr int kMlpParams = kMlpHidden * kMlpIn + kMlpHidden + kMlpHidden * kMlpHidden + kMlpHidden + kMlpHidden + 1;

@@ -1,0 +1,665 @@
+// FP64 products on paired panels: both phases of the product as one streaming
+// kernel in packed double-float arithmetic.
+//
+// The FP64 factors are laid out once per H-matrix as panels of at most 32
+// outputs x ncol inputs whose entries are already split into (hi, lo) floats
+// (split64_near), two neighbouring outputs side by side in 16 bytes:
+// {hi0, hi1, lo0, lo1}, an input's ceil(h / 2) pairs contiguous, inputs one
+// after the other.
+//   phase 1: the outputs are the phase-1 sums of the leaves on one source
+//            cluster tile (their Vt columns stacked, 32 at a time), the
+//            inputs the tile's rows of x: no sum crosses lanes, whatever the
+//            rank and the tile's height
+//   phase 2: the outputs are rows of a target cluster, the inputs the columns
+//            of every leaf on it (dense columns of x, phase-1 sums)
+// so one kernel serves both.  A warp owns a panel: lane = (pair of outputs,
+// slice of the inputs), the panel's bytes arrive by bulk copies in a ring of
+// shared-memory stages, the inputs' coefficients by 16-byte asynchronous
+// copies in the layout the arithmetic wants ({hi of two right-hand sides, lo
+// of two}).  Warps claim panels from a ticket, its next value and the next
+// panel's descriptor always requested a panel ahead.
+//
+// Arithmetic: fma / add / sub on float pairs (.f32x2), two right-hand
+// sides per instruction (one right-hand side: two outputs per instruction);
+// the multiply-add takes 10 instead of the 12 operations of df_fma, as
+//   t = s + p, p = RN(uh xh);  s + p = t + w exactly up to the rest
+//   l = fma(uh, xh, -(t - s)) = (p - (t - s)) + (uh xh - p)
+// gets the rounding errors of the product and of the sum in one operation.
+// The FP32 pipe takes 128 lane operations a clock and SM, so a product with
+// one right-hand side is bound by HBM, with four and more by that pipe.
+//
+// Measured against the tile and chunk kernels of stream.cu and
+// matvec_kernels.cu (which shuffle every coefficient, reduce every tile over
+// the warp and leave lanes idle on tiles of few rows), Laplace sphere, FP64:
+//   100 000 points  1 right-hand side 0.489 -> 0.381 ms, 2: 0.82 -> 0.44,
+//                   4: 1.79 -> 0.66, 8: 2.66 -> 1.10
+//   400 000 points  1: 2.11 -> 1.61 (6.6 TB/s in phase 1, 6.9 in phase 2, a
+//                   copy takes 6.8), 4: 7.94 -> 2.78
+// at no larger an error against the FP64 pipe (1.2e-14 .. 2.0e-14).
+//
+// Every wait is bounded; a warp whose wait ran out records status 2, lets its
+// copies in flight land (again bounded) and ends.
+#include "df64.cuh"
+#include "kernels.hpp"
+
+#include <algorithm>
+
+namespace htgpu {
+namespace {
+
+constexpr int kPairWarps = 4; // warps per CTA, each with its own panels and ring
+
+__device__ long long g_pair_wait = 4000000000ll; // SM clocks of a wait at most (about 2 s)
+__device__ long long g_pair_skip = -1;           // a panel whose first copy is left out (test support)
+
+typedef unsigned long long f2x; // two floats: low word first
+
+__device__ __forceinline__ f2x fx_fma(f2x a, f2x b, f2x c) {
+    f2x d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f2x fx_add(f2x a, f2x b) {
+    f2x d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f2x fx_sub(f2x a, f2x b) {
+    f2x d;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f2x fx(float lo, float hi) {
+    f2x d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ float2 fx2(f2x v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+
+struct DF2 { // two double-float accumulators
+    f2x s, c;
+};
+
+__device__ __forceinline__ void df2_fma(DF2 &a, f2x uh, f2x ul, f2x xh, f2x xl) {
+    // two scalar products: the assembler contracts mul.f32x2 and add.f32x2 to
+    // one fma in spite of their rounding modifiers, and t = RN(s + uh xh)
+    // would lose what TwoSum recovers (the product came out at 9e-9)
+    const float2 u = fx2(uh), v = fx2(xh);
+    const f2x p  = fx(__fmul_rn(u.x, v.x), __fmul_rn(u.y, v.y));
+    const f2x t  = fx_add(a.s, p);
+    const f2x nb = fx_sub(a.s, t);              // -(t - s)
+    const f2x w  = fx_sub(a.s, fx_add(t, nb)); // what s lost
+    f2x l        = fx_fma(uh, xh, nb);          // what the product lost, its own rounding included
+    l            = fx_fma(ul, xh, l);
+    l            = fx_fma(uh, xl, l);
+    a.c          = fx_add(a.c, fx_add(w, l)); // one rounding at c's size, the others at an ulp of s
+    a.s          = t;
+}
+
+__device__ __forceinline__ void df2_renorm(DF2 &a) {
+    const f2x s = fx_add(a.s, a.c);
+    a.c         = fx_add(a.c, fx_sub(a.s, s));
+    a.s         = s;
+}
+
+__device__ __forceinline__ DF2 df2_add(DF2 a, DF2 b) {
+    const f2x s  = fx_add(a.s, b.s);
+    const f2x nb = fx_sub(a.s, s);
+    const f2x w  = fx_sub(a.s, fx_add(s, nb));
+    const f2x v  = fx_add(b.s, nb);
+    DF2 r;
+    r.s = s;
+    r.c = fx_add(fx_add(a.c, b.c), fx_add(w, v));
+    return r;
+}
+
+__device__ __forceinline__ f2x shfl2(f2x v, int src) {
+    const float2 f = fx2(v);
+    return fx(__shfl_sync(0xffffffffu, f.x, src), __shfl_sync(0xffffffffu, f.y, src));
+}
+
+// a double as hi + lo, both rounded to nearest (|a - hi - lo| <= 2^-48 |a|; the
+// truncating split64 of the other kernels keeps 2^-46), by bit operations:
+// the conversions between double and float run on the FP64 pipe. |a| < 2^127;
+// below 2^-103 (and zero) gives 0, a value that is not finite NaN, so that it
+// reaches the outputs
+__device__ __forceinline__ F2 split64_near(double a) {
+    const long long b  = __double_as_longlong(a);
+    const int e        = (int)(b >> 52) & 0x7FF;
+    const long long m  = b + (1LL << 28);           // hi: 29 bits rounded off
+    const unsigned mh  = (unsigned)(m >> 32);
+    const unsigned hb  = (((unsigned)(m >> 29)) - 0xC0000000u) | (mh & 0x80000000u); // exponent 1023 -> 127 (mod 512), 23 fraction bits
+    const int r        = (int)(b - (m & ~((1LL << 29) - 1))); // a - hi in units of 2^(e - 1075), |r| <= 2^28
+    F2 f;
+    const float lo = (__int2float_rn(r) * 9.31322574615478515625e-10f) * __int_as_float((e - 918) << 23); // 2^-30, 2^(e - 1045)
+    const bool ok  = (unsigned)(e - 920) < 229u;
+    f.hi           = ok ? __uint_as_float(hb) : e == 0x7FF ? __int_as_float(0x7fffffff) : 0.f;
+    f.lo           = ok ? __int_as_float(__float_as_int(lo) ^ (int)((unsigned)(b >> 32) & 0x80000000u)) : 0.f;
+    return f;
+}
+
+__device__ __forceinline__ unsigned sa(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ bool mbar_try(unsigned long long *b, unsigned parity) {
+    unsigned ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(sa(b)), "r"(parity), "r"(20000u) : "memory");
+    return ok != 0;
+}
+
+// the whole warp waits for the phase; false when the wait ran out
+__device__ __forceinline__ bool pair_wait(unsigned long long *b, unsigned parity) {
+    bool ok = mbar_try(b, parity);
+    if (!__all_sync(0xffffffffu, ok)) {
+        const long long t0 = clock64();
+        while (true) {
+            ok = mbar_try(b, parity);
+            if (__all_sync(0xffffffffu, ok))
+                break;
+            if (__any_sync(0xffffffffu, clock64() - t0 > g_pair_wait))
+                return false;
+        }
+    }
+    return true;
+}
+
+// Per Q (pairs of right-hand sides; 0: one right-hand side): input columns
+// per stage, stages per warp, resident CTAs per SM.
+template <int Q>
+struct PairCfg {
+    static constexpr int kCols   = 16;
+    static constexpr int kStages = 3;
+    static constexpr int kCtas   = Q >= 3 ? 3 : 4;
+    static constexpr int kUnit   = Q ? 16 * Q : 8;              // bytes of an input's coefficients
+    static constexpr int kData   = 256 * kCols;                 // 16 pairs x 16 bytes a column
+    static constexpr int kCoef   = kData;                       // [q][column]
+    static constexpr int kDesc   = kCoef + kUnit * kCols;       // int4: h, columns, last chunk of its panel, output base
+    static constexpr int kStage  = (kDesc + 16 + 15) & ~15;
+    static constexpr int kBar    = kStages * kStage;
+    static constexpr int kWarp   = (kBar + 8 * kStages + 127) & ~127;
+    static constexpr int kSmem   = kPairWarps * kWarp;
+};
+
+// P1: coefficients are the rows of X from panel.coef on, sums go to the slots
+// oslot[panel.out ..] of A; else the coefficients cidx[panel.coef ..] name
+// slots of A (>= 0) or rows of X (~row), sums go to the rows panel.out .. of z
+template <int Q, bool P1>
+__global__ void __launch_bounds__(32 * kPairWarps, PairCfg<Q>::kCtas)
+    pair_kernel(const PairPanel *__restrict__ panels, int npanels, int *__restrict__ ticket, const unsigned char *__restrict__ mirror, const int *__restrict__ cidx, const int *__restrict__ oslot,
+                const float *__restrict__ X, float *__restrict__ A, float2 *__restrict__ z, int zlen, int nrhs, int *__restrict__ status) {
+    using C             = PairCfg<Q>;
+    constexpr int kCols = C::kCols, kStages = C::kStages, kUnit = C::kUnit;
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    unsigned char *wbase    = smem + (size_t)wid * C::kWarp;
+    unsigned long long *bar = reinterpret_cast<unsigned long long *>(wbase + C::kBar);
+    if (lane == 0)
+        for (int s = 0; s < kStages; s++)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sa(&bar[s])) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    __syncwarp();
+    unsigned long long pol;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
+    const long long skip = g_pair_skip;
+
+    // ---- panels: the current one (cur, from column jc on), the next one and
+    // the ticket after that (lane 0) in flight; the first two are the warp's
+    // own, the ticket counts the ones after every warp's first two
+    const int nwarps = gridDim.x * kPairWarps;
+    int icur = blockIdx.x * kPairWarps + wid, inxt = icur + nwarps, tk = 0;
+    PairPanel cur{}, nxt{};
+    if (icur < npanels)
+        cur = panels[icur];
+    if (inxt < npanels) {
+        nxt = panels[inxt];
+        if (lane == 0)
+            tk = 2 * nwarps + atomicAdd(ticket, 1);
+    }
+    int jc  = 0; // first column of cur not yet issued
+    int idx = 0; // the coefficient index of column jc + lane
+    auto load_idx = [&]() {
+        if constexpr (!P1)
+            idx = (icur < npanels && lane < kCols && jc + lane < cur.ncol) ? __ldg(cidx + cur.coef + jc + lane) : 0;
+    };
+    load_idx();
+    int issued = 0;
+    auto issue = [&]() { // the next chunk into stage issued % kStages; an empty copy group when none is left
+        if (icur < npanels) {
+            const int s  = issued % kStages;
+            const int hp = (cur.h + 1) >> 1;
+            const int nc = min(kCols, cur.ncol - jc);
+            unsigned char *st = wbase + (size_t)s * C::kStage;
+            if (lane == 0) {
+                *reinterpret_cast<int4 *>(st + C::kDesc) = make_int4(cur.h, nc, jc + nc == cur.ncol, cur.out);
+                const unsigned bytes                     = (unsigned)(16 * hp * nc);
+                if (!(icur == skip && jc == 0)) {
+                    asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(sa(&bar[s])), "r"(bytes) : "memory");
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(sa(st)),
+                                 "l"(mirror + cur.src + (long long)16 * hp * jc), "r"(bytes), "r"(sa(&bar[s])), "l"(pol)
+                                 : "memory");
+                }
+            }
+            if (lane < nc) {
+                const unsigned char *src;
+                if constexpr (P1)
+                    src = reinterpret_cast<const unsigned char *>(X) + (long long)kUnit * (cur.coef + jc + lane);
+                else
+                    src = idx >= 0 ? reinterpret_cast<const unsigned char *>(A) + (long long)kUnit * idx : reinterpret_cast<const unsigned char *>(X) + (long long)kUnit * (~idx);
+                if constexpr (Q == 0) {
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(sa(st + C::kCoef + 8 * lane)), "l"(src) : "memory");
+                } else {
+#pragma unroll
+                    for (int q = 0; q < Q; q++)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sa(st + C::kCoef + 16 * (q * kCols + lane))), "l"(src + 16 * q) : "memory");
+                }
+            }
+            issued++;
+            jc += nc;
+            if (jc == cur.ncol) {
+                jc   = 0;
+                cur  = nxt;
+                icur = inxt;
+                if (inxt < npanels) {
+                    inxt = __shfl_sync(0xffffffffu, tk, 0);
+                    if (inxt < npanels) {
+                        nxt = panels[inxt];
+                        if (lane == 0)
+                            tk = 2 * nwarps + atomicAdd(ticket, 1);
+                    }
+                }
+            }
+            load_idx();
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    constexpr int kAcc = Q ? 2 * Q : 1; // Q = 0: one, its two halves the two outputs; else [output][q]
+    DF2 acc[kAcc];
+#pragma unroll
+    for (int i = 0; i < kAcc; i++)
+        acc[i].s = acc[i].c = 0ull;
+
+#pragma unroll
+    for (int s = 0; s < kStages - 1; s++)
+        issue();
+    bool ok  = true;
+    int done = 0;
+    while (done < issued) {
+        const int s = done % kStages;
+        issue(); // into the stage the previous iteration read
+        asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 1) : "memory");
+        if (!pair_wait(&bar[s], (done / kStages) & 1)) {
+            ok = false;
+            break;
+        }
+        __syncwarp();
+        const unsigned char *st = wbase + (size_t)s * C::kStage;
+        const int4 d            = *reinterpret_cast<const int4 *>(st + C::kDesc);
+        const int h = d.x, nc = d.y, hp = (h + 1) >> 1;
+        const int S     = 32 / hp;
+        const int slice = lane / hp, pair = lane - slice * hp;
+        if (slice < S) {
+            const float4 *data = reinterpret_cast<const float4 *>(st) + pair;
+            if constexpr (Q == 0) {
+                const float2 *cf = reinterpret_cast<const float2 *>(st + C::kCoef);
+#pragma unroll 4
+                for (int t = slice; t < nc; t += S) {
+                    const float4 u = data[t * hp];
+                    const float2 x = cf[t];
+                    df2_fma(acc[0], fx(u.x, u.y), fx(u.z, u.w), fx(x.x, x.x), fx(x.y, x.y));
+                }
+            } else {
+                const float4 *cf = reinterpret_cast<const float4 *>(st + C::kCoef);
+#pragma unroll 2
+                for (int t = slice; t < nc; t += S) {
+                    const float4 u = data[t * hp];
+                    const f2x h0 = fx(u.x, u.x), h1 = fx(u.y, u.y), l0 = fx(u.z, u.z), l1 = fx(u.w, u.w);
+#pragma unroll
+                    for (int q = 0; q < Q; q++) {
+                        const float4 x = cf[q * kCols + t];
+                        const f2x xh = fx(x.x, x.y), xl = fx(x.z, x.w);
+                        df2_fma(acc[q], h0, l0, xh, xl);
+                        df2_fma(acc[Q + q], h1, l1, xh, xl);
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < kAcc; i++)
+            df2_renorm(acc[i]);
+        if (d.z) { // the panel's last chunk: slices summed in order, outputs written
+            for (int sl = 1; sl < S; sl++) {
+#pragma unroll
+                for (int i = 0; i < kAcc; i++) {
+                    const int src = (lane + sl * hp) & 31;
+                    DF2 o;
+                    o.s = shfl2(acc[i].s, src);
+                    o.c = shfl2(acc[i].c, src);
+                    if (slice == 0)
+                        acc[i] = df2_add(acc[i], o);
+                }
+            }
+            if (slice == 0) {
+#pragma unroll
+                for (int i = 0; i < kAcc; i++)
+                    df2_renorm(acc[i]);
+                if constexpr (Q == 0) {
+                    const float2 vs = fx2(acc[0].s), vc = fx2(acc[0].c);
+                    if constexpr (P1) {
+                        float2 *A2 = reinterpret_cast<float2 *>(A);
+                        A2[oslot[d.w + 2 * pair]] = make_float2(vs.x, vc.x);
+                        if (2 * pair + 1 < h)
+                            A2[oslot[d.w + 2 * pair + 1]] = make_float2(vs.y, vc.y);
+                    } else {
+                        z[d.w + 2 * pair] = make_float2(vs.x, vc.x);
+                        if (2 * pair + 1 < h)
+                            z[d.w + 2 * pair + 1] = make_float2(vs.y, vc.y);
+                    }
+                } else {
+#pragma unroll
+                    for (int o = 0; o < 2; o++) {
+                        if (2 * pair + o >= h)
+                            break;
+                        if constexpr (P1) {
+                            float4 *A4 = reinterpret_cast<float4 *>(A) + (long long)Q * oslot[d.w + 2 * pair + o];
+#pragma unroll
+                            for (int q = 0; q < Q; q++) {
+                                const float2 vs = fx2(acc[o * Q + q].s), vc = fx2(acc[o * Q + q].c);
+                                A4[q]           = make_float4(vs.x, vs.y, vc.x, vc.y);
+                            }
+                        } else {
+#pragma unroll
+                            for (int q = 0; q < Q; q++) {
+                                const float2 vs = fx2(acc[o * Q + q].s), vc = fx2(acc[o * Q + q].c);
+                                float2 *zr      = z + (long long)(2 * q) * zlen + d.w + 2 * pair + o;
+                                if (2 * q < nrhs)
+                                    zr[0] = make_float2(vs.x, vc.x);
+                                if (2 * q + 1 < nrhs)
+                                    zr[zlen] = make_float2(vs.y, vc.y);
+                            }
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < kAcc; i++)
+                acc[i].s = acc[i].c = 0ull;
+        }
+        __syncwarp(); // every lane is done with the stage before it is refilled
+        done++;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (!ok) {
+        if (lane == 0)
+            atomicExch(status, 2);
+        for (int p = done; p < issued; p++) // the copies in flight land before the warp leaves
+            if (!pair_wait(&bar[p % kStages], (p / kStages) & 1) && lane == 0)
+                atomicExch(status, 3);
+    }
+}
+
+// the gathered input of right-hand sides c0 .. c0 + w (those past mu_src
+// zero), split relative to the input's largest exponent: [row][q] of
+// {hi, hi, lo, lo}, w = 1: [row] of (hi, lo); also clears the two tickets
+__global__ void pair_gather_kernel(const double *__restrict__ x, int ldx, const int *__restrict__ perm, int n, int c0, int w, int mu_src, const int *__restrict__ xexp, float *__restrict__ X,
+                                   int *__restrict__ tickets) {
+    if (blockIdx.x == 0 && threadIdx.x < 2)
+        tickets[threadIdx.x] = 0;
+    const int shift = 1023 - max(*xexp, 1);
+    auto value      = [&](int src, int c) {
+        F2 r{0.f, 0.f};
+        if (c >= mu_src)
+            return r;
+        const double v = x[(long long)c * ldx + src];
+        const int ex   = (int)(((unsigned)__double2hiint(v) >> 20) & 0x7FFu);
+        if (ex == 0x7FF)
+            return split64_near(v);
+        return ex != 0 && ex + shift >= 1 ? split64_near(scale_pow2(v, shift)) : r;
+    };
+    const int Q           = w == 1 ? 1 : w >> 1;
+    const long long total = (long long)n * Q;
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
+        const int j = (int)(e / Q), q = (int)(e - (long long)j * Q);
+        const int src = perm ? perm[j] : j;
+        if (w == 1) {
+            const F2 a                          = value(src, c0);
+            reinterpret_cast<float2 *>(X)[j] = make_float2(a.hi, a.lo);
+        } else {
+            const F2 a = value(src, c0 + 2 * q), b = value(src, c0 + 2 * q + 1);
+            reinterpret_cast<float4 *>(X)[e] = make_float4(a.hi, b.hi, a.lo, b.lo);
+        }
+    }
+}
+
+// the tiles' sums of every multi-tile leaf into the first tile's slots
+__global__ void pair_reduce_kernel(const LrLeaf *__restrict__ lr, const int *__restrict__ multi, int w, float *__restrict__ A) {
+    const LrLeaf L = lr[multi[blockIdx.x]];
+    if (w == 1) {
+        float2 *base = reinterpret_cast<float2 *>(A) + L.a_off;
+        for (int e = threadIdx.x; e < L.r; e += blockDim.x) {
+            DF a{base[e].x, base[e].y};
+            for (int ch = 1; ch < L.nch; ch++) {
+                const float2 v = base[(long long)ch * L.r + e];
+                a              = df_add(a, DF{v.x, v.y});
+                df_renorm(a);
+            }
+            base[e] = make_float2(a.s, a.c);
+        }
+        return;
+    }
+    const int Q  = w >> 1;
+    float4 *base = reinterpret_cast<float4 *>(A) + L.a_off * Q;
+    for (int e = threadIdx.x; e < L.r * Q; e += blockDim.x) {
+        const float4 v = base[e];
+        DF2 a{fx(v.x, v.y), fx(v.z, v.w)};
+        for (int ch = 1; ch < L.nch; ch++) {
+            const float4 u = base[(long long)ch * L.r * Q + e];
+            a              = df2_add(a, DF2{fx(u.x, u.y), fx(u.z, u.w)});
+            df2_renorm(a);
+        }
+        const float2 s = fx2(a.s), c = fx2(a.c);
+        base[e] = make_float4(s.x, s.y, c.x, c.y);
+    }
+}
+
+// native complex layout: i times the sums (re, im) of every slot pair
+__global__ void pair_rotate_kernel(const int2 *__restrict__ rows, long long nrows, int Q, float4 *__restrict__ A) {
+    const long long total = nrows * Q;
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
+        const int2 p               = rows[e / Q];
+        const int q                = (int)(e % Q);
+        const float4 v             = A[(long long)p.x * Q + q];
+        A[(long long)p.y * Q + q] = make_float4(-v.y, v.x, -v.w, v.z);
+    }
+}
+
+// y[c * ldy + perm[i]] (no perm: i - shift) = sum over the covering clusters
+// (largest first) of z, brought back to the input's scale
+__global__ void pair_zsum_kernel(const ZItem *__restrict__ items, int nitems, const int *__restrict__ zl, const float2 *__restrict__ z, int zlen, int mu, const int *__restrict__ perm,
+                                 const int *__restrict__ xexp, double *__restrict__ y, int ldy, int shift) {
+    const int w    = blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (w >= nitems)
+        return;
+    const ZItem it = items[w];
+    const int xs   = max(*xexp, 1) - 1023;
+    const int n    = it.h * mu;
+    for (int e = lane; e < n; e += 32) {
+        const int c = e / it.h, i = it.row0 + e - c * it.h;
+        DF a{0.f, 0.f};
+        for (int l = it.lbeg; l < it.lend; l++) {
+            const float2 v = z[(long long)c * zlen + i + zl[l]];
+            a              = df_add(a, DF{v.x, v.y});
+            df_renorm(a);
+        }
+        const double v = df_to_double(a);
+        // NaN stays NaN through the scaling (an exponent field of 0x7FF has no room)
+        y[(long long)c * ldy + (perm ? perm[i] : i - shift)] = v == v ? scale_pow2_safe(v, xs) : v;
+    }
+}
+
+// ---- layout -----------------------------------------------------------------
+// phase 2: lane = output row of the panel; its FP64 row sits in one of the
+// target cluster's row-chunk panels (pan0 .. of m rows in all)
+__global__ void pair_pack2_kernel(const PairPanel *__restrict__ panels, const PairSource *__restrict__ srcs, int npanels, const PanelItem *__restrict__ pan, const double *__restrict__ fac,
+                                  unsigned char *__restrict__ mirror) {
+    const int lane = threadIdx.x & 31, nw = gridDim.x * (blockDim.x >> 5);
+    for (int p = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); p < npanels; p += nw) {
+        const PairPanel d  = panels[p];
+        const PairSource s = srcs[p];
+        const int hp       = (d.h + 1) >> 1;
+        if (lane >= 2 * hp)
+            continue;
+        const bool live = lane < d.h;
+        const long long i = s.lo + (live ? lane : 0), nchunk = (s.m + 31) / 32;
+        const long long q = ((i + 1) * nchunk - 1) / s.m; // the row chunk of row i: floor(m q / nchunk) <= i
+        const PanelItem pi = pan[s.pan0 + q];
+        const double *row  = fac + pi.off + (i - (long long)s.m * q / nchunk);
+        float *dst         = reinterpret_cast<float *>(mirror + d.src) + 4 * (lane >> 1) + (lane & 1);
+#pragma unroll 4
+        for (int k = 0; k < d.ncol; k++) {
+            const F2 f            = split64_near(live ? row[(long long)pi.h * k] : 0.);
+            dst[4LL * hp * k]     = f.hi;
+            dst[4LL * hp * k + 2] = f.lo;
+        }
+    }
+}
+
+// phase 1: outputs osrc[out ..] (FP64 element offsets of their columns),
+// inputs the column's rows; 32 x 32 tiles turned over in shared memory
+__global__ void __launch_bounds__(128) pair_pack1_kernel(const PairPanel *__restrict__ panels, int npanels, const long long *__restrict__ osrc, const double *__restrict__ fac,
+                                                         unsigned char *__restrict__ mirror) {
+    __shared__ float2 tile[4][32][33];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = gridDim.x * 4;
+    for (int p = blockIdx.x * 4 + wid; p < npanels; p += nw) {
+        const PairPanel d       = panels[p];
+        const int hp            = (d.h + 1) >> 1;
+        const long long my_src = lane < d.h ? osrc[d.out + lane] : 0;
+        for (int k0 = 0; k0 < d.ncol; k0 += 32) {
+            const int nk = min(32, d.ncol - k0);
+            __syncwarp();
+#pragma unroll 8
+            for (int o = 0; o < 32; o++) {
+                const long long so = __shfl_sync(0xffffffffu, my_src, o);
+                const F2 f         = split64_near(o < d.h && lane < nk ? fac[so + k0 + lane] : 0.);
+                tile[wid][lane][o] = make_float2(f.hi, f.lo);
+            }
+            __syncwarp();
+            if (lane < 2 * hp) {
+                float *dst = reinterpret_cast<float *>(mirror + d.src) + 4LL * hp * k0 + 4 * (lane >> 1) + (lane & 1);
+                for (int k = 0; k < nk; k++) {
+                    const float2 f        = tile[wid][k][lane];
+                    dst[4LL * hp * k]     = f.x;
+                    dst[4LL * hp * k + 2] = f.y;
+                }
+            }
+        }
+    }
+}
+
+int pair_sms() {
+    int dev = 0, sms = 0;
+    HTGPU_CUDA(cudaGetDevice(&dev));
+    HTGPU_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    return std::max(sms, 1);
+}
+
+template <int Q, bool P1>
+void launch_pair_q(const PairPanel *panels, int npanels, int *ticket, const unsigned char *mirror, const int *cidx, const int *oslot, const float *X, float *A, float2 *z, int zlen, int nrhs,
+                   int *status, cudaStream_t st) {
+    static unsigned long long done = 0; // devices whose shared-memory limit was raised
+    int dev = 0;
+    HTGPU_CUDA(cudaGetDevice(&dev));
+    if (dev >= 64 || !(done >> dev & 1)) {
+        HTGPU_CUDA(cudaFuncSetAttribute(pair_kernel<Q, P1>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<Q>::kSmem));
+        if (dev < 64)
+            done |= 1ull << dev;
+    }
+    const int nctas = std::min(PairCfg<Q>::kCtas * pair_sms(), (npanels + kPairWarps - 1) / kPairWarps);
+    pair_kernel<Q, P1><<<nctas, 32 * kPairWarps, PairCfg<Q>::kSmem, st>>>(panels, npanels, ticket, mirror, cidx, oslot, X, A, z, zlen, nrhs, status);
+    HTGPU_CUDA(cudaGetLastError());
+}
+
+template <bool P1>
+void launch_pair(const PairPanel *panels, int npanels, int *ticket, const unsigned char *mirror, const int *cidx, const int *oslot, const float *X, float *A, float2 *z, int zlen, int w, int nrhs,
+                 int *status, cudaStream_t st) {
+    if (npanels <= 0)
+        return;
+    switch (w) {
+    case 1: launch_pair_q<0, P1>(panels, npanels, ticket, mirror, cidx, oslot, X, A, z, zlen, nrhs, status, st); break;
+    case 2: launch_pair_q<1, P1>(panels, npanels, ticket, mirror, cidx, oslot, X, A, z, zlen, nrhs, status, st); break;
+    case 4: launch_pair_q<2, P1>(panels, npanels, ticket, mirror, cidx, oslot, X, A, z, zlen, nrhs, status, st); break;
+    case 6: launch_pair_q<3, P1>(panels, npanels, ticket, mirror, cidx, oslot, X, A, z, zlen, nrhs, status, st); break;
+    case 8: launch_pair_q<4, P1>(panels, npanels, ticket, mirror, cidx, oslot, X, A, z, zlen, nrhs, status, st); break;
+    default: require(false, "paired panels: 1, 2, 4, 6 or 8 right-hand sides a pass"); break;
+    }
+}
+
+} // namespace
+
+int pair_pass_width(int left, bool exact) {
+    if (left >= 8)
+        return 8;
+    if (left == 1)
+        return 1;
+    return (left & 1) && exact ? left - 1 : (left + 1) & ~1;
+}
+
+void launch_pair_gather(const double *x, int ldx, const int *perm, int n, int c0, int w, int mu_src, const int *xexp, float *X, int *tickets, cudaStream_t st) {
+    const long long total = (long long)n * (w == 1 ? 1 : w >> 1);
+    const int blocks      = (int)std::max<long long>(1, std::min<long long>((total + 255) / 256, 16LL * pair_sms()));
+    pair_gather_kernel<<<blocks, 256, 0, st>>>(x, ldx, perm, n, c0, w, mu_src, xexp, X, tickets);
+    HTGPU_CUDA(cudaGetLastError());
+}
+
+void launch_pair_phase1(const PairPanel *panels, int npanels, int *tickets, const unsigned char *mirror, const int *oslot, const float *X, float *A, int w, int *status, cudaStream_t st) {
+    launch_pair<true>(panels, npanels, tickets, mirror, nullptr, oslot, X, A, nullptr, 0, w, w, status, st);
+}
+
+void launch_pair_phase2(const PairPanel *panels, int npanels, int *tickets, const unsigned char *mirror, const int *cidx, const float *X, float *A, int w, int nrhs, float2 *z, int zlen, int *status,
+                        cudaStream_t st) {
+    launch_pair<false>(panels, npanels, tickets + 1, mirror, cidx, nullptr, X, A, z, zlen, w, nrhs, status, st);
+}
+
+void launch_pair_reduce(const LrLeaf *lr, const int *multi, int nmulti, int w, float *A, cudaStream_t st) {
+    if (nmulti <= 0)
+        return;
+    pair_reduce_kernel<<<nmulti, 128, 0, st>>>(lr, multi, w, A);
+    HTGPU_CUDA(cudaGetLastError());
+}
+
+void launch_pair_rotate(const int2 *rows, long long nrows, int w, float *A, cudaStream_t st) {
+    require(w >= 2, "complex sums come in pairs of right-hand sides");
+    const long long total = nrows * (w >> 1);
+    if (total <= 0)
+        return;
+    pair_rotate_kernel<<<(int)std::min<long long>((total + 255) / 256, 4096), 256, 0, st>>>(rows, nrows, w >> 1, reinterpret_cast<float4 *>(A));
+    HTGPU_CUDA(cudaGetLastError());
+}
+
+void launch_pair_zsum(const ZItem *items, int nitems, const int *zl, const float2 *z, int zlen, int mu, const int *perm, const int *xexp, double *y, int ldy, cudaStream_t st, int shift) {
+    if (nitems <= 0)
+        return;
+    pair_zsum_kernel<<<(nitems + 7) / 8, 256, 0, st>>>(items, nitems, zl, z, zlen, mu, perm, xexp, y, ldy, shift);
+    HTGPU_CUDA(cudaGetLastError());
+}
+
+void launch_pair_pack(const PairPanel *p1, int np1, const long long *osrc, const PairPanel *p2, const PairSource *s2, int np2, const PanelItem *pan, const double *fac, unsigned char *mirror,
+                      cudaStream_t st) {
+    const int most = 16 * pair_sms();
+    if (np1 > 0)
+        pair_pack1_kernel<<<std::min(most, (np1 + 3) / 4), 128, 0, st>>>(p1, np1, osrc, fac, mirror);
+    if (np2 > 0)
+        pair_pack2_kernel<<<std::min(most, (np2 + 7) / 8), 256, 0, st>>>(p2, s2, np2, pan, fac, mirror);
+    HTGPU_CUDA(cudaGetLastError());
+}
+
+void set_pair_waits(long long cycles, long long skip) {
+    HTGPU_CUDA(cudaMemcpyToSymbol(g_pair_wait, &cycles, sizeof(cycles)));
+    HTGPU_CUDA(cudaMemcpyToSymbol(g_pair_skip, &skip, sizeof(skip)));
+}
+
+} // namespace htgpu

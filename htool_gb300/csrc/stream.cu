@@ -1698,6 +1698,7 @@ int stream2_units_target() {
 void set_debug_waits(long long cycles, long long skip_chunk) {
     HTGPU_CUDA(cudaMemcpyToSymbol(g_wait_cycles, &cycles, sizeof(cycles)));
     HTGPU_CUDA(cudaMemcpyToSymbol(g_skip_chunk, &skip_chunk, sizeof(skip_chunk)));
+    set_pair_waits(cycles, skip_chunk);
     HTGPU_CUDA(cudaDeviceSynchronize());
 }
 

@@ -354,7 +354,15 @@ int htgpu_hmatrix_phase_bytes(htgpu_hmatrix h, int mu, long long *bytes);
  * phase-1 share is kept for the FP64 product).  Each precision keeps its own
  * split; defaults 0 / 350 (FP64) and 0 (reduced-precision dense blocks),
  * what the autotuner picks on Laplace spheres.  No counterpart in the
- * reference (its BLAS calls decide this, include/htool/types/matrix.hpp:320-383). */
+ * reference (its BLAS calls decide this, include/htool/types/matrix.hpp:320-383).
+ * FP64 products run on paired panels (every factor pre-split into (hi, lo)
+ * float pairs, both phases in double-float arithmetic, no FP64-pipe share)
+ * until a call of this function, htgpu_hmatrix_set_phase1_mode,
+ * htgpu_hmatrix_set_phase2_mode or htgpu_hmatrix_set_presplit chooses the
+ * kernels these functions configure; htgpu_hmatrix_autotune brings the
+ * panels back.  Where the panels do not fit in three quarters of the free
+ * memory, or a stored entry is too large for the emulation, those kernels
+ * run with the defaults. */
 int htgpu_hmatrix_set_fp64_split(htgpu_hmatrix h, int phase1_dfma_permille, int phase2_dfma_permille);
 int htgpu_hmatrix_get_fp64_split(htgpu_hmatrix h, int *phase1_dfma_permille, int *phase2_dfma_permille);
 
