@@ -103,21 +103,30 @@ __device__ __forceinline__ void oz_mma_i(unsigned tmem_d, unsigned long long a, 
 // The S (S + 1) / 2 plane products of one slab in few MMAs: A plane i times
 // the B planes j = 0 .. S - 1 - i side by side along N lands in the
 // accumulators of the diagonals i + j, which lie side by side in tensor
-// memory (plane rows nb each, at most 256 columns a MMA).  The instruction
+// memory (plane rows NB each, at most 256 columns a MMA).  The instruction
 // descriptor of tcgen05.mma kind::f16: FP32 accumulator (bits 4-5 = 1), A
 // and B BF16 (bits 7-9, 10-12 = 1), both K-major, N / 8 at bits 17-22,
-// M / 16 at bits 24-28.
-template <int S>
-__device__ __forceinline__ void oz_slab_mmas(unsigned tmem, unsigned a0, unsigned b0, int nb, bool first) {
-    const int per = 256 / nb; // B planes a MMA
+// M / 16 at bits 24-28.  Called by a whole warp, whose lane 0 issues: shapes
+// known at compile time and addresses uniform over the warp leave a few
+// instructions a MMA (one thread computing them at run time took 1 300
+// cycles a slab and bound both phases).
+template <int S, int NB>
+__device__ __forceinline__ void oz_slab_mmas(unsigned tmem, unsigned a0, unsigned b0, bool first, bool issue) {
+    constexpr int per = 256 / NB; // B planes a MMA
+    const unsigned long long da = oz_desc(a0), db = oz_desc(b0); // addresses below 2^18: the 14-bit field never carries
+    if (issue) {
 #pragma unroll
-    for (int i = 0; i < S; i++)
-        for (int j0 = 0; j0 < S - i; j0 += per) {
-            const int cnt        = min(per, S - i - j0);
-            const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)((cnt * nb) >> 3) << 17) | ((unsigned)(kOzM >> 4) << 24);
-            oz_mma_i(tmem + (unsigned)((i + j0) * nb), oz_desc(a0 + i * kOzPlaneA), oz_desc(b0 + j0 * nb * 32), idesc, !(first && i == 0));
-        }
+        for (int i = 0; i < S; i++)
+#pragma unroll
+            for (int j0 = 0; j0 < S - i; j0 += per) {
+                const int cnt        = S - i - j0 < per ? S - i - j0 : per;
+                const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)((cnt * NB) >> 3) << 17) | ((unsigned)(kOzM >> 4) << 24);
+                oz_mma_i(tmem + (unsigned)((i + j0) * NB), da + (unsigned)(i * kOzPlaneA / 16), db + (unsigned)(j0 * NB * 32 / 16), idesc, !(first && i == 0));
+            }
+    }
 }
+// the whole warp waits for a phase; false (on every lane) when it ran out
+__device__ __forceinline__ bool oz_warp_wait(unsigned long long *b, unsigned parity) { return __all_sync(0xffffffffu, bar_wait(b, parity)); }
 
 // biased exponent field of |v| (0 for zero and subnormals)
 __device__ __forceinline__ int oz_ebits(double v) { return (int)(((unsigned long long)__double_as_longlong(v) >> 52) & 0x7FF); }
@@ -142,28 +151,34 @@ __device__ __forceinline__ long long oz_fixed(double v, int emax) {
     return (b >> 63) ? -q : q;
 }
 
-// balanced base-128 digits of q, d[0] the top one, without a carry chain:
-// adding 64 to every lower digit position (the constant 64 * (1 + 128 +
-// ... + 128^(S-2))) turns the balanced digits d in [-64, 63] into the plain
-// 7-bit fields d + 64 of q + bias, and the top digit into its arithmetic
-// shift -- the same digits as the sequential split, a shift, a mask and a
-// subtraction each
+// The balanced base-128 digits of q (d_0 the top one) as 7-bit fields, without
+// a carry chain: adding 64 at every digit position (the constant 64 * (1 + 128
+// + ... + 128^(S-1))) turns the digits d in [-64, 63] into the plain fields
+// d + 64 of q + bias (|d_0| <= 33, so the top field is one too).  lo holds the
+// fields of the digits S - 4 .. S - 1, hi those above.
+struct OzFields {
+    unsigned hi, lo;
+};
 template <int S>
-__device__ __forceinline__ void oz_digits(long long q, int (&d)[S]) {
-    long long bias = 0;
+__device__ __forceinline__ OzFields oz_fields(long long q) {
+    static_assert(S == 4 || S == 8, "four fields a word");
+    unsigned long long bias = 0;
 #pragma unroll
-    for (int i = 0; i < S - 1; i++)
-        bias |= 64ll << (7 * i);
-    const long long u = q + bias;
-    d[0]              = (int)(u >> (7 * (S - 1)));
-#pragma unroll
-    for (int i = 1; i < S; i++)
-        d[i] = (int)((u >> (7 * (S - 1 - i))) & 127) - 64;
+    for (int i = 0; i < S; i++)
+        bias |= 64ull << (7 * i);
+    const unsigned long long u = (unsigned long long)q + bias;
+    return {(unsigned)(u >> 28), (unsigned)u & 0x0FFFFFFFu};
 }
-
-__device__ __forceinline__ unsigned oz_bf2(int a, int b) { // two small integers as BF16 (exact)
+// digit s of two values as BF16, exact: 0x4300 + f is 128 + f for a 7-bit
+// field f, and 128 + f - 192 the digit (the conversions from integers, eight a
+// value, held the cutting threads to 16 a clock)
+template <int S>
+__device__ __forceinline__ unsigned oz_digit2(const OzFields &a, const OzFields &b, int s) {
+    const int sh     = 7 * ((S - 1 - s) & 3);
+    const unsigned x = s < S - 4 ? a.hi : a.lo, y = s < S - 4 ? b.hi : b.lo;
+    const unsigned w = 0x43004300u + ((x >> sh) & 127u) + (((y >> sh) & 127u) << 16);
     unsigned r;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"((float)b), "f"((float)a));
+    asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(w), "r"(0x43404340u));
     return r;
 }
 
@@ -171,47 +186,76 @@ __device__ __forceinline__ unsigned oz_bf2(int a, int b) { // two small integers
 // 16-byte store per plane
 template <int S, int T>
 __device__ __forceinline__ void oz_put8(unsigned char *planes, int plane_bytes, int row, int k, const double (&v)[8], int emax) {
-    int d[8][S];
+    OzFields d[8];
 #pragma unroll
     for (int q = 0; q < 8; q++)
-        oz_digits<S>(oz_fixed<T>(v[q], emax), d[q]);
+        d[q] = oz_fields<S>(oz_fixed<T>(v[q], emax));
 #pragma unroll
     for (int s = 0; s < S; s++) {
         uint4 w;
-        w.x = oz_bf2(d[0][s], d[1][s]);
-        w.y = oz_bf2(d[2][s], d[3][s]);
-        w.z = oz_bf2(d[4][s], d[5][s]);
-        w.w = oz_bf2(d[6][s], d[7][s]);
+        w.x = oz_digit2<S>(d[0], d[1], s);
+        w.y = oz_digit2<S>(d[2], d[3], s);
+        w.z = oz_digit2<S>(d[4], d[5], s);
+        w.w = oz_digit2<S>(d[6], d[7], s);
         *reinterpret_cast<uint4 *>(planes + (size_t)s * plane_bytes + oz_off(row, k)) = w;
     }
 }
 
-// two consecutive K values (k even), one 4-byte store per plane
-template <int S, int T>
-__device__ __forceinline__ void oz_put2(unsigned char *planes, int plane_bytes, int row, int k, const double (&v)[2], int emax) {
-    int d[2][S];
-    oz_digits<S>(oz_fixed<T>(v[0], emax), d[0]);
-    oz_digits<S>(oz_fixed<T>(v[1], emax), d[1]);
+// The same eight digit planes of eight consecutive K values in fewer
+// operations (phase 2 cuts every coefficient anew for each row chunk that uses
+// it, and its instructions bound it): |v| 2^(T + 1024 - emax) by one funnel
+// shift, the rounding, the sign's two's complement and the digits' bias in one
+// 64-bit addition (ties round up instead of away from zero), then the fields of
+// two neighbouring values side by side, two digits to a word.
+// (Two's-complement 7-bit fields would need no bias and no subtraction, but
+// their products are all of one sign and up to 33 * 127: the MMA sums then
+// grow past 2^23, where the measured products lost bits.)
+__device__ __forceinline__ unsigned long long oz_fields2x(double v, int emax) { // 2 (q + bias), rounded in its lowest bit
+    constexpr unsigned long long kBias = 64ull * ((1ull << 56) - 1) / 127; // 64 at each of the eight positions
+    const unsigned vh = (unsigned)__double2hiint(v), vl = (unsigned)__double2loint(v);
+    const int r       = min(emax - (int)((vh >> 20) & 0x7FFu), 63); // a zero or subnormal shifts out
+    const unsigned mh = (vh & 0xFFFFFu) | 0x100000u;
+    unsigned h = __funnelshift_l(vl, mh, 2), l = vl << 2;
+    if (r >= 32) {
+        l = h;
+        h = 0u;
+    }
+    l                = __funnelshift_r(l, h, r & 31);
+    h                = h >> (r & 31);
+    const unsigned s = (unsigned)((int)vh >> 31);
+    return (((unsigned long long)(h ^ s) << 32) | (l ^ s)) + (2ull * kBias + 1ull) + (unsigned long long)(s & 1u);
+}
+template <int T>
+__device__ __forceinline__ void oz_put8_fast(unsigned char *planes, int plane_bytes, int row, int k, const double (&v)[8], int emax) {
+    static_assert(T == 54, "eight digits");
+    unsigned w[8][4]; // [digit][pair of values]
 #pragma unroll
-    for (int s = 0; s < S; s++)
-        *reinterpret_cast<unsigned *>(planes + (size_t)s * plane_bytes + oz_off(row, k)) = oz_bf2(d[0][s], d[1][s]);
+    for (int q = 0; q < 4; q++) {
+        const unsigned long long a = oz_fields2x(v[2 * q], emax), b = oz_fields2x(v[2 * q + 1], emax);
+#pragma unroll
+        for (int p = 0; p < 4; p++) { // digits 7 - 2p (low field) and 6 - 2p of both values
+            const unsigned c = __byte_perm((unsigned)(a >> (14 * p + 1)), (unsigned)(b >> (14 * p + 1)), 0x5410);
+            w[7 - 2 * p][q]  = (c & 0x007F007Fu) | 0x43004300u;
+            w[6 - 2 * p][q]  = ((c >> 7) & 0x007F007Fu) | 0x43004300u;
+        }
+    }
+#pragma unroll
+    for (int s = 0; s < 8; s++) {
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            asm("sub.rn.bf16x2 %0, %0, %1;" : "+r"(w[s][q]) : "r"(0x43404340u));
+        *reinterpret_cast<uint4 *>(planes + (size_t)s * plane_bytes + oz_off(row, k)) = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
+    }
 }
 
-// four consecutive K values (k a multiple of 4), one 8-byte store per plane.
-// (Two's-complement 7-bit fields would take fewer operations than the
-// balanced digits, but their products are all of one sign and up to
-// 33 * 127: the MMA sums then grow past 2^23, where the measured products
-// lost bits.)
-template <int S, int T>
-__device__ __forceinline__ void oz_put4(unsigned char *planes, int plane_bytes, int row, int k, const double (&v)[4], const int (&emax)[4]) {
-    int d[4][S];
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-        oz_digits<S>(oz_fixed<T>(v[q], emax[q]), d[q]);
-#pragma unroll
-    for (int s = 0; s < S; s++)
-        *reinterpret_cast<uint2 *>(planes + (size_t)s * plane_bytes + oz_off(row, k)) = make_uint2(oz_bf2(d[0][s], d[1][s]), oz_bf2(d[2][s], d[3][s]));
-}
+// the sums of the S = 8 diagonals of one column (exact integers below 2^23
+// in FP32) as two words 28 bits apart: neighbouring diagonals fit 32 bits
+struct OzQuad {
+    int c[4]; // diagonals 2p, 2p + 1
+};
+__device__ __forceinline__ int oz_duo(unsigned hi, unsigned lo) { return __float2int_rn(__uint_as_float(hi)) * 128 + __float2int_rn(__uint_as_float(lo)); }
+__device__ __forceinline__ long long oz_high(const OzQuad &q) { return (long long)q.c[0] * 16384 + q.c[1]; }
+__device__ __forceinline__ long long oz_low(const OzQuad &q) { return (long long)q.c[2] * 16384 + q.c[3]; }
 
 // |I| normalised: the leading bit at 127, its position, the sign
 struct OzNorm {
@@ -249,6 +293,37 @@ __device__ __forceinline__ double oz_i2d(__int128 I, int k) {
     if (ex <= 0)
         return 0.;
     return __longlong_as_double((long long)((n.neg ? 1ull << 63 : 0ull) | ((unsigned long long)ex << 52) | (m & 0xFFFFFFFFFFFFFull)));
+}
+
+// (hi 2^28 + lo) 2^k as a double, |hi|, |lo| < 2^47: the same rounding on
+// 64-bit words
+__device__ __forceinline__ double oz_pair2d(long long hi, long long lo, int k) {
+    long long t   = hi + (lo >> 28);
+    unsigned r    = (unsigned)lo & 0x0FFFFFFFu; // I = t 2^28 + r, 0 <= r < 2^28
+    const bool ng = t < 0;
+    if (ng) {
+        t = -t - (r != 0);
+        r = r ? 0x10000000u - r : 0u;
+    }
+    if (t == 0) {
+        t = r;
+        r = 0;
+        k -= 28;
+    }
+    if (t == 0)
+        return 0.;
+    const int lz                  = __clzll(t); // at least 16: t < 2^48
+    const unsigned long long rest = (unsigned long long)r << 36;
+    const unsigned long long w    = ((unsigned long long)t << lz) | (rest >> (64 - lz));
+    unsigned long long m          = w >> 11; // 53 bits
+    const unsigned rem            = (unsigned)w & 0x7FFu;
+    int ex                        = 1023 + 91 - lz + k;
+    if (rem > 0x400u || (rem == 0x400u && ((rest << lz) != 0 || (m & 1))))
+        m++;
+    ex += (int)(m >> 53); // a carry leaves a zero fraction
+    if (ex <= 0)
+        return 0.;
+    return __longlong_as_double((long long)((ng ? 1ull << 63 : 0ull) | ((unsigned long long)ex << 52) | (m & 0xFFFFFFFFFFFFFull)));
 }
 
 // I 2^k as a float (round to nearest even)
@@ -430,14 +505,18 @@ __global__ void __launch_bounds__(128) oz_xplanes_kernel(const double *__restric
     oz_put8<S, OzCfg<S>::kT>(xplanes + ((long long)g * npass + p) * OzCfg<S>::kBslab, kOzPlaneB, n, k0, v, e);
 }
 
-// Warp-specialised phase 1 for inputs cut into planes once.  One thread of
-// warp 0 runs ahead issuing, per 16-row slab, the bulk copies of the block's
-// A planes and of the input group's B planes into a ring of four stages,
-// and, as the slabs land, their MMAs; warps 1-8 read the accumulators out
+// Warp-specialised phase 1 for inputs cut into planes once.  Warp 17 runs
+// ahead issuing, per 16-row slab, the bulk copies of the block's A planes and
+// of the input group's B planes into a ring of four stages, warp 0 the MMAs
+// of the slabs as they land; warps 1-16 read the accumulators out
 // after the last slab of each block and pass (tensor-memory lanes 32 (warp
-// mod 4) .., warps 1-4 the first 32 right-hand sides, 5-8 the last 32),
-// while the next block's copies already fly.
-constexpr int kOzFastThreads = 288;
+// mod 4) .., warps 1-4 the first 16 right-hand sides, 5-8 the next 16, ..),
+// while the next block's copies already fly.  Bound by the hand-over of the
+// one set of accumulators tensor memory holds (40% of the MMA warp's time it
+// waits for the read-out, 50% it issues); 64 right-hand sides of a 100 000-point
+// sphere 1.13 -> 0.98 ms with a warp that issues at compile-time shapes and
+// twice the read-out warps, which take 32-bit words out before they convert.
+constexpr int kOzFastThreads = 576;
 
 template <int S, bool OUT64>
 __global__ void __launch_bounds__(kOzFastThreads, 1) phase1_ozb_kernel(const TcBlock *__restrict__ blocks, int nblocks, const TcSeg *__restrict__ segs,
@@ -455,7 +534,7 @@ __global__ void __launch_bounds__(kOzFastThreads, 1) phase1_ozb_kernel(const TcB
     unsigned long long *accf  = full + 2 * NST;                                               // a pass's accumulators complete
     unsigned long long *acce  = accf + 1;                                                     // and read out
     unsigned *tslot           = reinterpret_cast<unsigned *>(smem + NST * C::kBuf + 96);
-    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, wid = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int npass = (mu + kOzN - 1) / kOzN;
     if (tid == 0) {
         for (int k = 0; k < NST; k++) {
@@ -463,7 +542,7 @@ __global__ void __launch_bounds__(kOzFastThreads, 1) phase1_ozb_kernel(const TcB
             bar_init(&empty[k]);
         }
         bar_init(accf);
-        bar_init_n(acce, 8); // one arrival per read-out warp
+        bar_init_n(acce, 16); // one arrival per read-out warp
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (wid == 0)
@@ -473,82 +552,81 @@ __global__ void __launch_bounds__(kOzFastThreads, 1) phase1_ozb_kernel(const TcB
     fence_after();
     const unsigned tmem = *tslot;
     bool fail           = false;
-    if (wid == 0) {
-        if (lane == 0) {
-            // two cursors over (block, pass, slab): copies run up to NST
-            // slabs ahead of the MMAs
-            struct Cursor {
-                int bi, p, s, nsl, g0;
-                long long aoff;
-            };
-            auto load = [&](Cursor &c) {
-                if (c.bi < nblocks) {
-                    const TcBlock B = blocks[c.bi];
-                    c.nsl           = ((B.xrow & (kOzK - 1)) + B.jlen + kOzK - 1) / kOzK;
-                    c.g0            = B.xrow / kOzK;
-                    c.aoff          = ozoff[c.bi];
-                }
-            };
-            auto advance = [&](Cursor &c) {
-                if (++c.s == c.nsl) {
-                    c.s = 0;
-                    if (++c.p == npass) {
-                        c.p = 0;
-                        c.bi += gridDim.x;
-                        load(c);
-                    }
-                }
-            };
-            Cursor cc{(int)blockIdx.x, 0, 0, 0, 0, 0};
-            load(cc);
-            Cursor mc = cc;
-            int ci = 0, mi = 0, np = 0; // copies issued, slabs multiplied, passes completed
-            while (mc.bi < nblocks && !fail) {
-                while (cc.bi < nblocks && ci < mi + NST) {
-                    const int stg = ci % NST, use = ci / NST;
-                    if (use > 0 && !bar_wait(&empty[stg], (use - 1) & 1)) { // the MMAs of slab ci - NST read this stage
-                        fail = true;
-                        break;
-                    }
-                    unsigned char *stage = smem + (size_t)stg * C::kBuf;
-                    bar_expect_tx(&full[stg], C::kBuf);
-                    bulk_g2s(stage, arena + cc.aoff + (long long)cc.s * C::kSlab, C::kSlab, &full[stg]);
-                    bulk_g2s(stage + C::kSlab, xplanes + ((long long)(cc.g0 + cc.s) * npass + cc.p) * C::kBslab, C::kBslab, &full[stg]);
-                    ci++;
-                    advance(cc);
-                }
-                if (fail)
-                    break;
-                const int stg = mi % NST, use = mi / NST;
-                // the read-out of the previous pass is done with the accumulators
-                if (mc.s == 0 && np > 0 && !bar_wait(acce, (np - 1) & 1)) {
-                    fail = true;
-                    break;
-                }
-                if (!bar_wait(&full[stg], use & 1)) {
-                    fail = true;
-                    break;
-                }
-                fence_after();
-                const unsigned a0 = smem_u32(smem + (size_t)stg * C::kBuf), b0 = a0 + C::kSlab;
-                oz_slab_mmas<S>(tmem, a0, b0, kOzN, mc.s == 0);
-                commit(&empty[stg]);
-                mi++;
-                const bool last = mc.s == mc.nsl - 1;
-                advance(mc);
-                if (last) {
-                    commit(accf);
-                    np++;
-                }
-            }
-            if (fail) {
-                atomicExch(status, 4);
-                for (int k = mi; k < ci; k++) // the copies in flight land before the CTA leaves
-                    bar_wait(&full[k % NST], (k / NST) & 1);
+    // a cursor over (block, pass, slab)
+    struct Cursor {
+        int bi, p, s, nsl, g0;
+        long long aoff;
+    };
+    auto load = [&](Cursor &c) {
+        if (c.bi < nblocks) {
+            const TcBlock B = blocks[c.bi];
+            c.nsl           = ((B.xrow & (kOzK - 1)) + B.jlen + kOzK - 1) / kOzK;
+            c.g0            = B.xrow / kOzK;
+            c.aoff          = ozoff[c.bi];
+        }
+    };
+    auto advance = [&](Cursor &c) {
+        if (++c.s == c.nsl) {
+            c.s = 0;
+            if (++c.p == npass) {
+                c.p = 0;
+                c.bi += gridDim.x;
+                load(c);
             }
         }
+    };
+    if (wid == 17) { // copies
+        Cursor c{(int)blockIdx.x, 0, 0, 0, 0, 0};
+        load(c);
+        int n = 0;
+        for (; c.bi < nblocks; n++) {
+            const int stg = n % NST, use = n / NST;
+            if (use > 0 && !oz_warp_wait(&empty[stg], (use - 1) & 1)) { // the MMAs of slab n - NST read this stage
+                fail = true;
+                break;
+            }
+            if (lane == 0) {
+                unsigned char *stage = smem + (size_t)stg * C::kBuf;
+                bar_expect_tx(&full[stg], C::kBuf);
+                bulk_g2s(stage, arena + c.aoff + (long long)c.s * C::kSlab, C::kSlab, &full[stg]);
+                bulk_g2s(stage + C::kSlab, xplanes + ((long long)(c.g0 + c.s) * npass + c.p) * C::kBslab, C::kBslab, &full[stg]);
+            }
+            advance(c);
+        }
+        if (fail) {
+            if (lane == 0)
+                atomicExch(status, 4);
+            for (int k = max(0, n - NST); k < n; k++) // the copies in flight land before the CTA leaves
+                bar_wait(&full[k % NST], (k / NST) & 1);
+        }
+    } else if (wid == 0) { // MMAs
+        Cursor c{(int)blockIdx.x, 0, 0, 0, 0, 0};
+        load(c);
+        int np = 0; // passes completed
+        for (int n = 0; c.bi < nblocks; n++) {
+            const int stg = n % NST, use = n / NST;
+            // the read-out of the previous pass is done with the accumulators
+            if ((c.s == 0 && np > 0 && !oz_warp_wait(acce, (np - 1) & 1)) || !oz_warp_wait(&full[stg], use & 1)) {
+                fail = true;
+                break;
+            }
+            fence_after();
+            const unsigned a0 = smem_u32(smem) + (unsigned)stg * C::kBuf;
+            oz_slab_mmas<S, kOzN>(tmem, a0, a0 + C::kSlab, c.s == 0, lane == 0);
+            __syncwarp();
+            const bool last = c.s == c.nsl - 1;
+            if (lane == 0) {
+                commit(&empty[stg]);
+                if (last)
+                    commit(accf);
+            }
+            np += last;
+            advance(c);
+        }
+        if (fail && lane == 0)
+            atomicExch(status, 4);
     } else {
-        const int orow = 32 * (wid & 3) + lane, c0 = 32 * ((wid - 1) >> 2);
+        const int orow = 32 * (wid & 3) + lane, c0 = 16 * ((wid - 1) >> 2);
         const int kunits = OUT64 ? 0 : 1023 - max(*xexp, 1); // FP32 sums in the units of the split input
         int np = 0;
         for (int bi = blockIdx.x; bi < nblocks && !fail; bi += gridDim.x) {
@@ -571,50 +649,77 @@ __global__ void __launch_bounds__(kOzFastThreads, 1) phase1_ozb_kernel(const TcB
             }
             const int kr = 7 * (S - 1) + rexp[(long long)bi * kOzM + orow] - 2044 - 2 * T + kunits;
             for (int p = 0; p < npass; p++) {
-                if (!bar_wait(accf, np & 1)) {
+                if (!__all_sync(0xffffffffu, bar_wait(accf, np & 1))) {
                     fail = true;
                     break;
                 }
                 fence_after();
-                // the accumulators out of tensor memory first, into two exact
-                // 64-bit partial sums per column (diagonals D < S/2 and the
-                // rest: I = hi 2^(7 S/2) + lo); tensor memory is released
-                // before the conversions, so the next block's MMAs overlap them
-                long long hi[32], lo[32];
+                // the accumulators out of tensor memory first, neighbouring
+                // diagonals in one exact 32-bit word; tensor memory is
+                // released before the conversions, so the next block's MMAs
+                // overlap them
+                int x[16][S / 2];
+                const unsigned tacc = tmem + ((unsigned)(32 * (wid & 3)) << 16) + (unsigned)c0;
 #pragma unroll
-                for (int q = 0; q < 32; q++)
-                    hi[q] = lo[q] = 0;
+                for (int d = 0; d < S / 2; d++) {
+                    unsigned r0[16], r1[16];
+                    tmem_ld16(tacc + (unsigned)(2 * d * kOzN), r0);
+                    tmem_ld16(tacc + (unsigned)((2 * d + 1) * kOzN), r1);
 #pragma unroll
-                for (int D = 0; D < S; D++)
-#pragma unroll
-                    for (int c16 = 0; c16 < 2; c16++) {
-                        unsigned r[16];
-                        tmem_ld16(tmem + ((unsigned)(32 * (wid & 3)) << 16) + (unsigned)(D * kOzN + c0 + 16 * c16), r);
-#pragma unroll
-                        for (int q = 0; q < 16; q++) {
-                            const long long a = (long long)__float2int_rn(__uint_as_float(r[q]));
-                            if (D < S / 2)
-                                hi[16 * c16 + q] += a << (7 * (S / 2 - 1 - D));
-                            else
-                                lo[16 * c16 + q] += a << (7 * (S - 1 - D));
-                        }
-                    }
+                    for (int q = 0; q < 16; q++)
+                        x[q][d] = oz_duo(r0[q], r1[q]);
+                }
                 fence_before();
                 __syncwarp();
                 if (lane == 0)
                     bar_arrive(acce);
-                if (osg >= 0)
+                if (osg >= 0) {
+                    const bool two = (mu & 1) == 0; // rows of A are 16-byte aligned (8 bytes of FP32)
 #pragma unroll
-                    for (int q = 0; q < 32; q++) {
+                    for (int q = 0; q < 16; q += 2) {
                         const int c = kOzN * p + c0 + q;
-                        if (c < mu) {
-                            const __int128 I = ((__int128)hi[q] << (7 * (S / 2))) + lo[q];
-                            if (OUT64)
-                                reinterpret_cast<double *>(Aout)[oo + c] = oz_i2d(I, kr + __ldg(ecol + c));
-                            else
-                                reinterpret_cast<float *>(Aout)[oo + c] = oz_i2f(I, kr + __ldg(ecol + c)) * osc;
+                        if (c >= mu)
+                            break;
+                        double v[2];
+                        float f[2];
+#pragma unroll
+                        for (int u = 0; u < 2; u++) {
+                            const int k = kr + (c + u < mu ? __ldg(ecol + c + u) : 0);
+                            if constexpr (S == 8) {
+                                const long long hi = (long long)x[q + u][0] * 16384 + x[q + u][1], lo = (long long)x[q + u][2] * 16384 + x[q + u][3];
+                                if (OUT64)
+                                    v[u] = oz_pair2d(hi, lo, k);
+                                else
+                                    f[u] = oz_i2f(((__int128)hi << 28) + lo, k) * osc;
+                            } else {
+                                const __int128 I = (__int128)((long long)x[q + u][0] * 16384 + x[q + u][1]);
+                                if (OUT64)
+                                    v[u] = oz_i2d(I, k);
+                                else
+                                    f[u] = oz_i2f(I, k) * osc;
+                            }
+                        }
+                        if (OUT64) {
+                            double *o = reinterpret_cast<double *>(Aout) + oo + c;
+                            if (two) {
+                                *reinterpret_cast<double2 *>(o) = make_double2(v[0], v[1]);
+                            } else {
+                                o[0] = v[0];
+                                if (c + 1 < mu)
+                                    o[1] = v[1];
+                            }
+                        } else {
+                            float *o = reinterpret_cast<float *>(Aout) + oo + c;
+                            if (two) {
+                                *reinterpret_cast<float2 *>(o) = make_float2(f[0], f[1]);
+                            } else {
+                                o[0] = f[0];
+                                if (c + 1 < mu)
+                                    o[1] = f[1];
+                            }
                         }
                     }
+                }
                 np++;
             }
         }
@@ -716,7 +821,7 @@ __global__ void __launch_bounds__(kOzThreads, S <= 4 ? 2 : 1) phase1_oz_kernel(c
                     if (bar_wait(&fulls[buf], use & 1)) {
                         fence_after();
                         const unsigned a0 = smem_u32(stage), b0 = a0 + S * kOzPlaneA;
-                        oz_slab_mmas<S>(tmem, a0, b0, kOzN, ks == 0);
+                        oz_slab_mmas<S, kOzN>(tmem, a0, b0, ks == 0, true);
                         commit(&bars[buf]);
                     } else {
                         fail = true; // spreads at the next barrier
@@ -894,59 +999,88 @@ __global__ void oz_panel_exp_kernel(const OzPanel *__restrict__ panels, int npan
         pexp[(long long)q * mu + rhs] = oz_panel_exp(panels[q], groups, gexp, agexp, mu, rhs);
 }
 
-template <int S>
 struct Oz2Cfg {
-    static constexpr int kA      = S * kOzPlaneA;   // 128 x 16 per plane (rows 64-127 zero)
-    static constexpr int kB      = S * 32 * 32;     // N <= 32 rows x 16 per plane
+    static constexpr int kS      = 8;               // digit planes
+    static constexpr int kA      = kS * 64 * 32;     // 64 right-hand sides x 16 columns per plane, two planes to one 128-row operand
+    static constexpr int kB      = kS * 32 * 32;     // N <= 32 rows x 16 per plane
     static constexpr int kStage  = kA + kB;
     static constexpr int kStages = 4;
-    static constexpr int kAcc    = 4 * 16 * 32 * 16; // the readers' 64-bit partial sums (hi, lo) between rounds
-    static constexpr int kSmem   = kStages * kStage + 256 + kAcc;
-    static constexpr unsigned kCols = S * 32 <= 128 ? 128u : 256u;
+    static constexpr int kBars   = kStages * kStage;
+    static constexpr int kAcc    = kBars + 256;           // the readers' 64-bit partial sums between rounds (8 warps x 16 rows x 32 lanes x 16 B)
+    static constexpr int kXch    = kAcc + 8 * 16 * 32 * 16; // the sums of 8 rows on their way to the warp that converts them
+    static constexpr int kOut    = kXch + 8 * 8 * 32 * 16;  // its 8 rows' values on the way to z
+    static constexpr int kSmem   = kOut + 8 * 8 * 32 * 8;
+    static constexpr unsigned kBuf  = kS * 32;   // tensor-memory columns of one set of accumulators
+    static constexpr unsigned kCols = 2 * kBuf;  // two sets: a round's MMAs run while the round before is read out
 };
+static_assert(Oz2Cfg::kSmem <= 227 * 1024, "shared memory of a CTA");
 
-// Twenty-one warps in three roles over the same sequence of (panel, pass of
-// 64 right-hand sides, 16-column slab): warps 2 and 6-20 cut each slab's
-// coefficients into planes (thread t: right-hand side t mod 64, 2 columns;
-// the next slab's coefficients loaded while the current one is cut) into a
-// ring of four stages -- many warps, few registers each, to hide the
-// latency of the gathered coefficients; lane 0 of warp 3 copies the panel's
-// planes in and issues the MMAs as both halves of a stage are ready; warps
-// 0, 1, 4, 5 (tensor-memory lanes 0-63: the right-hand sides) add each
-// round's accumulators into exact 64-bit sums kept in shared memory and
-// write the z rows at the end of a pass.  The exponent bounds come from
-// pexp (oz_panel_exp_kernel).
-constexpr int kOz2Threads = 672;
+// One slab: the coefficient planes 2 jj and 2 jj + 1 of the 64 right-hand
+// sides are the rows 0-63 and 64-127 of one operand, the panel's planes i lie
+// side by side along N: slot i + 2 jj of tensor memory takes the diagonal
+// i + 2 jj in the lanes 0-63 and i + 2 jj + 1 in the lanes 64-127 (so there
+// slot 7 holds only pairs to be dropped).  Four MMAs of 640 columns in all
+// for 32 rows, where eight with one plane and 64 empty rows each took 1 152.
+template <int NB>
+__device__ __forceinline__ void oz2_slab_mmas(unsigned tmem, unsigned a0, unsigned b0, bool first) {
+    const unsigned long long da = oz_desc(a0), db = oz_desc(b0);
+#pragma unroll
+    for (int jj = 0; jj < 4; jj++) {
+        const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(((8 - 2 * jj) * NB) >> 3) << 17) | ((unsigned)(kOzM >> 4) << 24);
+        oz_mma_i(tmem + (unsigned)(2 * jj * NB), da + (unsigned)(jj * kOzPlaneA / 16), db, idesc, !(first && jj == 0));
+    }
+}
 
-template <int S>
-__global__ void __launch_bounds__(kOz2Threads, 1) phase2_oz_kernel(const OzPanel *__restrict__ panels, int npanels, const int *__restrict__ groups, const unsigned char *__restrict__ parena,
-                                                                   const int *__restrict__ prexp, const int *__restrict__ cidx, const double *__restrict__ A, const double *__restrict__ xp,
-                                                                   const int *__restrict__ pexp, int mu, double *__restrict__ z, int zlen, int add, int *__restrict__ status) {
-    using C           = Oz2Cfg<S>;
-    constexpr int T   = OzCfg<S>::kT;
+// Twenty-six warps in four roles over the same sequence of (panel, pass of
+// 64 right-hand sides, 16-column slab).  Warp 9 copies the panel's planes into
+// a ring of four stages.  Warps 10-25, four to a stage, cut every fourth
+// slab's coefficients into planes (thread t: right-hand side t mod 64, 8
+// columns, so each plane takes one 16-byte store without bank conflicts; the
+// values of the group's next slab and the indices of the one after that are
+// requested before a slab is cut).  Warp 8 issues the MMAs as both halves of
+// a stage are ready, rounds alternating between two sets of accumulators.
+// Warps 0-7 (tensor-memory lanes 32 (warp mod 4) .., the first or last 16
+// rows) turn each round's accumulators into exact 64-bit sums, kept in shared
+// memory between the rounds of a pass; at its end the warps of a right-hand
+// side's even and odd planes exchange half their rows, convert and write z.
+// The exponent bounds come from pexp (oz_panel_exp_kernel).
+//
+// Bound by the integer operations of the cutting and of the read-out (4 400
+// instructions a slab and SM, the ALU pipe 66% busy; DRAM 24%).  64 right-hand
+// sides of a 100 000-point sphere: 2.70 -> 2.04 ms, most of it from the MMA
+// warp, whose single issuing thread had bound the kernel, then from the cutting
+// in 16-byte stores and the second set of accumulators.
+constexpr int kOz2Threads = 832;
+
+__global__ void __launch_bounds__(kOz2Threads, 1) phase2_oz_kernel(const OzPanel *__restrict__ panels, int npanels, const unsigned char *__restrict__ parena, const int *__restrict__ prexp,
+                                                                   const int *__restrict__ cidx, const double *__restrict__ A, const double *__restrict__ xp, const int *__restrict__ pexp, int mu,
+                                                                   double *__restrict__ z, int zlen, int add, int *__restrict__ status) {
+    using C           = Oz2Cfg;
+    constexpr int T   = OzCfg<8>::kT;
     constexpr int NST = C::kStages;
     extern __shared__ __align__(1024) unsigned char smem[];
-    unsigned long long *fulla = reinterpret_cast<unsigned long long *>(smem + NST * C::kStage); // [NST] coefficients cut (512 arrivals)
-    unsigned long long *fullb = fulla + NST;                                                    // [NST] panel planes landed
-    unsigned long long *empty = fulla + 2 * NST;                                                // [NST] a stage's MMAs done
-    unsigned long long *accf  = fulla + 3 * NST;                                                // a round's accumulators complete
-    unsigned long long *acce  = accf + 1;                                                       // and added up by the readers (4 arrivals)
-    unsigned *tslot           = reinterpret_cast<unsigned *>(smem + NST * C::kStage + 128);
-    const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
+    unsigned long long *fulla = reinterpret_cast<unsigned long long *>(smem + C::kBars); // [NST] coefficients cut (4 arrivals)
+    unsigned long long *fullb = fulla + NST;                                             // [NST] panel planes landed
+    unsigned long long *empty = fulla + 2 * NST;                                         // [NST] a stage's MMAs done
+    unsigned long long *accf  = fulla + 3 * NST;                                         // [2] a round's accumulators complete
+    unsigned long long *acce  = accf + 2;                                                // [2] and added up by the readers (8 arrivals)
+    unsigned long long *pairb = accf + 4;                                                // [4] the two warps of an exchange
+    unsigned *tslot           = reinterpret_cast<unsigned *>(accf + 8);
+    static_assert(8 * (3 * NST + 8) + 4 <= 256, "the barriers' block");
+    const int tid = threadIdx.x, wid = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int npass = (mu + kOzN - 1) / kOzN;
-    for (int i = tid; i < NST * C::kA / 16; i += blockDim.x) { // the A planes' rows 64-127 stay zero
-        const int st = i / (C::kA / 16), w = i - st * (C::kA / 16);
-        reinterpret_cast<uint4 *>(smem + (size_t)st * C::kStage)[w] = make_uint4(0u, 0u, 0u, 0u);
-    }
-    proxy_fence();
     if (tid == 0) {
         for (int k = 0; k < NST; k++) {
-            bar_init_n(&fulla[k], 512);
+            bar_init_n(&fulla[k], 4); // one arrival per warp of the stage's stagers
             bar_init(&fullb[k]);
             bar_init(&empty[k]);
         }
-        bar_init(accf);
-        bar_init_n(acce, 4);
+        for (int k = 0; k < 2; k++) {
+            bar_init(&accf[k]);
+            bar_init_n(&acce[k], 8);
+        }
+        for (int k = 0; k < 4; k++)
+            bar_init_n(&pairb[k], 2);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (wid == 0)
@@ -958,11 +1092,18 @@ __global__ void __launch_bounds__(kOz2Threads, 1) phase2_oz_kernel(const OzPanel
     bool fail           = false;
     // a cursor over (panel, pass, slab)
     struct Cur {
-        int bi, p, s, nsl;
+        int bi, p, s, nsl, q0, ncol, nb;
+        long long poff;
     };
     auto load = [&](Cur &c) {
-        if (c.bi < npanels)
-            c.nsl = (panels[c.bi].ncol + kOzK - 1) / kOzK;
+        if (c.bi < npanels) {
+            const OzPanel P = panels[c.bi];
+            c.ncol          = P.ncol;
+            c.q0            = P.q0;
+            c.nsl           = (P.ncol + kOzK - 1) / kOzK;
+            c.nb            = P.h <= 16 ? 16 : 32;
+            c.poff          = P.poff;
+        }
     };
     auto advance = [&](Cur &c) {
         if (++c.s == c.nsl) {
@@ -974,182 +1115,221 @@ __global__ void __launch_bounds__(kOz2Threads, 1) phase2_oz_kernel(const OzPanel
             }
         }
     };
-    if (wid == 3) {
-        if (lane == 0) { // copies and MMAs
-            Cur cc{(int)blockIdx.x, 0, 0, 0};
-            load(cc);
-            Cur mc = cc;
-            int ci = 0, mi = 0, rounds = 0, inround = 0;
-            while (mc.bi < npanels && !fail) {
-                while (cc.bi < npanels && ci < mi + NST) {
-                    const int stg = ci % NST, use = ci / NST;
-                    if (use > 0 && !bar_wait(&empty[stg], (use - 1) & 1)) {
-                        fail = true;
-                        break;
-                    }
-                    const OzPanel P = panels[cc.bi];
-                    const int bytes = S * 32 * (P.h <= 16 ? 16 : 32);
-                    bar_expect_tx(&fullb[stg], bytes);
-                    bulk_g2s(smem + (size_t)stg * C::kStage + C::kA, parena + P.poff + (long long)cc.s * bytes, bytes, &fullb[stg]);
-                    ci++;
-                    advance(cc);
-                }
-                if (fail)
-                    break;
-                const int stg = mi % NST, use = mi / NST;
-                if (inround == 0 && rounds > 0 && !bar_wait(acce, (rounds - 1) & 1)) { // the readers hold the last round
-                    fail = true;
-                    break;
-                }
-                if (!bar_wait(&fullb[stg], use & 1) || !bar_wait(&fulla[stg], use & 1)) {
-                    fail = true;
-                    break;
-                }
-                fence_after();
-                const int N       = panels[mc.bi].h <= 16 ? 16 : 32;
-                const unsigned a0 = smem_u32(smem + (size_t)stg * C::kStage), b0 = a0 + C::kA;
-                oz_slab_mmas<S>(tmem, a0, b0, N, inround == 0);
-                commit(&empty[stg]);
-                mi++;
-                const bool end = mc.s == mc.nsl - 1 || inround == kOzRound - 1;
-                advance(mc);
-                inround++;
-                if (end) {
-                    commit(accf);
-                    rounds++;
-                    inround = 0;
-                }
-            }
-            if (fail) {
-                atomicExch(status, 4);
-                for (int k = mi; k < ci; k++) // the copies in flight land before the CTA leaves
-                    bar_wait(&fullb[k % NST], (k / NST) & 1);
-            }
-        }
-    } else if (wid == 2 || wid >= 6) { // coefficient stagers
-        const int t = 32 * (wid == 2 ? 0 : wid - 5) + lane, n = t & 63, k0 = (t >> 6) * 2;
-        Cur c{(int)blockIdx.x, 0, 0, 0};
+    auto start = [&]() {
+        Cur c{(int)blockIdx.x, 0, 0, 0, 0, 0, 0, 0};
         load(c);
-        double v[2];
-        int ve = 0; // the slab's exponent bound, loaded with its coefficients
-        auto loadc = [&](const Cur &k) {
-#pragma unroll
-            for (int q = 0; q < 2; q++)
-                v[q] = 0.;
-            ve = 0;
-            if (k.bi >= npanels)
-                return;
-            const OzPanel P = panels[k.bi];
-            const int rhs   = kOzN * k.p + n;
-            if (rhs >= mu)
-                return;
-            ve = __ldg(pexp + (long long)k.bi * mu + rhs);
-#pragma unroll
-            for (int q = 0; q < 2; q++) {
-                const int col = kOzK * k.s + k0 + q;
-                if (col < P.ncol) {
-                    const int kx = __ldg(cidx + P.q0 + col);
-                    v[q]         = kx >= 0 ? __ldg(A + (long long)kx * mu + rhs) : __ldg(xp + (long long)(~kx) * mu + rhs);
-                }
-            }
-        };
-        loadc(c);
-        int it = 0;
-        while (c.bi < npanels && !fail) {
-            const int stg = it % NST, use = it / NST;
-            if (use > 0 && !bar_wait(&empty[stg], (use - 1) & 1)) {
+        return c;
+    };
+    if (wid == 9) { // copies of the panel's planes
+        Cur c = start();
+        int n = 0;
+        for (; c.bi < npanels; n++) {
+            const int stg = n % NST, use = n / NST;
+            if (use > 0 && !oz_warp_wait(&empty[stg], (use - 1) & 1)) {
                 fail = true;
                 break;
             }
-            const int e   = ve;
-            double cur[2] = {v[0], v[1]};
-            Cur nx        = c;
-            advance(nx);
-            loadc(nx); // the next slab's coefficients fly while this one is cut
-            oz_put2<S, T>(smem + (size_t)stg * C::kStage, kOzPlaneA, n, k0, cur, e);
-            proxy_fence();
-            bar_arrive(&fulla[stg]);
-            c = nx;
-            it++;
+            if (lane == 0) {
+                const int bytes = C::kS * 32 * c.nb;
+                bar_expect_tx(&fullb[stg], bytes);
+                bulk_g2s(smem + (size_t)stg * C::kStage + C::kA, parena + c.poff + (long long)c.s * bytes, bytes, &fullb[stg]);
+            }
+            advance(c);
         }
-        if (fail && lane == 0)
-            atomicExch(status, 4);
-    } else { // readers: warps 0, 1 (columns 0-15), 4, 5 (16-31)
-        const int m = 32 * (wid & 3) + lane, ch = wid >> 2, rw = 2 * ch + (wid & 3);
-        // this thread's 64-bit partial sums: hi of column q at sacc[q][lane],
-        // lo at sacc[16 + q][lane], in its warp's block
-        long long *sacc = reinterpret_cast<long long *>(smem + NST * C::kStage + 256) + (size_t)rw * 32 * 32;
-#pragma unroll
-        for (int q = 0; q < 32; q++)
-            sacc[q * 32 + lane] = 0;
-        Cur c{(int)blockIdx.x, 0, 0, 0};
-        load(c);
-        int rounds = 0;
-        while (c.bi < npanels && !fail) {
-            const OzPanel P = panels[c.bi];
-            const int N     = P.h <= 16 ? 16 : 32;
-            // this round: slabs c.s .. end of round or of the pass
-            const int last = min(c.nsl - 1, c.s + kOzRound - 1);
-            if (!bar_wait(accf, rounds & 1)) {
+        if (fail) {
+            if (lane == 0)
+                atomicExch(status, 4);
+            for (int k = max(0, n - NST); k < n; k++) // the copies in flight land before the CTA leaves
+                bar_wait(&fullb[k % NST], (k / NST) & 1);
+        }
+    } else if (wid == 8) { // MMAs
+        Cur c      = start();
+        int rounds = 0, inround = 0;
+        for (int n = 0; c.bi < npanels; n++) {
+            const int stg = n % NST, use = n / NST;
+            // the readers are done with this set's round before last
+            if ((inround == 0 && rounds > 1 && !oz_warp_wait(&acce[rounds & 1], ((rounds >> 1) - 1) & 1)) || !oz_warp_wait(&fullb[stg], use & 1) || !oz_warp_wait(&fulla[stg], use & 1)) {
                 fail = true;
                 break;
             }
             fence_after();
-            if (16 * ch < N) {
+            const unsigned a0 = smem_u32(smem) + (unsigned)stg * C::kStage, acc = tmem + (unsigned)(rounds & 1) * C::kBuf;
+            const bool end    = c.s == c.nsl - 1 || inround == kOzRound - 1;
+            if (lane == 0) {
+                if (c.nb == 16)
+                    oz2_slab_mmas<16>(acc, a0, a0 + C::kA, inround == 0);
+                else
+                    oz2_slab_mmas<32>(acc, a0, a0 + C::kA, inround == 0);
+                commit(&empty[stg]);
+                if (end)
+                    commit(&accf[rounds & 1]);
+            }
+            __syncwarp();
+            rounds += end;
+            inround = end ? 0 : inround + 1;
+            advance(c);
+        }
+        if (fail && lane == 0)
+            atomicExch(status, 4);
+    } else if (wid >= 10) { // coefficient stagers
+        const int sw = wid - 10, grp = sw >> 2, t = 32 * (sw & 3) + lane, n = t & 63, k0 = (t >> 6) * 8;
+        constexpr int kNone = -2147483647 - 1; // no column there (as a row of x: one past any)
+        Cur f = start();
+        auto skip = [&](int k) {
+            for (int q = 0; q < k && f.bi < npanels; q++)
+                advance(f);
+        };
+        skip(grp);
+        int ix[8], rx = 0, ex = 0; // the group's slab after next: indices, right-hand side, exponent bound
+        bool live = false;
+        auto request = [&]() {
+            live = f.bi < npanels;
+            rx   = kOzN * f.p + n;
+            ex   = live && rx < mu ? __ldg(pexp + (long long)f.bi * mu + rx) : 0;
 #pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const int col = kOzK * f.s + k0 + q;
+                ix[q]         = live && rx < mu && col < f.ncol ? __ldg(cidx + f.q0 + col) : kNone;
+            }
+            skip(NST);
+        };
+        double v[8], w[8];
+        auto values = [&]() {
+#pragma unroll
+            for (int q = 0; q < 8; q++)
+                w[q] = ix[q] == kNone ? 0. : ix[q] >= 0 ? __ldg(A + (long long)ix[q] * mu + rx) : __ldg(xp + (long long)(~ix[q]) * mu + rx);
+        };
+        request();
+        bool more = live;
+        int e     = ex;
+        values();
+        request();
+        int use = 0;
+        while (more && !fail) {
+#pragma unroll
+            for (int q = 0; q < 8; q++)
+                v[q] = w[q];
+            const int ecur  = e;
+            const bool next = live;
+            e               = ex;
+            values();  // of the group's next slab
+            request(); // indices of the one after that
+            if (!__all_sync(0xffffffffu, use == 0 || bar_wait(&empty[grp], (use - 1) & 1))) {
+                fail = true;
+                break;
+            }
+            oz_put8_fast<T>(smem + (size_t)grp * C::kStage, 64 * 32, n, k0, v, ecur); // plane s at 2 KB s: rows 64 (s mod 2) .. of operand s / 2
+            proxy_fence();
+            __syncwarp();
+            if (lane == 0)
+                bar_arrive(&fulla[grp]);
+            use++;
+            more = next;
+        }
+        if (fail && lane == 0)
+            atomicExch(status, 4);
+    } else { // readers: right-hand sides 32 (wid mod 2) .., even (wid mod 4 < 2) or odd planes, rows 16 (wid / 4) ..
+        const int quad = wid & 3, ch = wid >> 2, odd = quad >> 1, m = 32 * (quad & 1) + lane;
+        long long *sacc = reinterpret_cast<long long *>(smem + C::kAcc) + (size_t)wid * 16 * 32 * 2;
+        long long *give = reinterpret_cast<long long *>(smem + C::kXch) + (size_t)wid * 8 * 32 * 2;
+        const long long *take = reinterpret_cast<long long *>(smem + C::kXch) + (size_t)(wid ^ 2) * 8 * 32 * 2;
+        double *sz               = reinterpret_cast<double *>(smem + C::kOut) + (size_t)wid * 8 * 32;
+        unsigned long long *mate = &pairb[2 * ch + (quad & 1)];
+        int phase                = 0;
+        auto meet = [&]() { // both warps of the exchange have come here
+            __syncwarp();
+            if (lane == 0)
+                bar_arrive(mate);
+            return oz_warp_wait(mate, phase++ & 1);
+        };
+        Cur c      = start();
+        int rounds = 0;
+        while (c.bi < npanels) {
+            const OzPanel P = panels[c.bi];
+            const int N     = P.h <= 16 ? 16 : 32;
+            // this round: slabs c.s .. end of round or of the pass
+            const int last   = min(c.nsl - 1, c.s + kOzRound - 1);
+            const bool first = c.s == 0, pass_end = last == c.nsl - 1, on = 16 * ch < N;
+            const int p = c.p, rhs = kOzN * p + m;
+            // the exponents of this lane's right-hand side and of row `lane`
+            const int kx = (pass_end && on && rhs < mu) ? 7 * (C::kS - 1) + __ldg(pexp + (long long)c.bi * mu + rhs) - 2044 - 2 * T : 0;
+            const int kr = (pass_end && on) ? __ldg(prexp + (long long)c.bi * 32 + lane) : 0;
+            if (!oz_warp_wait(&accf[rounds & 1], (rounds >> 1) & 1)) {
+                fail = true;
+                break;
+            }
+            fence_after();
+            const unsigned tacc = tmem + (unsigned)(rounds & 1) * C::kBuf + ((unsigned)(32 * quad) << 16) + (unsigned)(16 * ch);
+            // the 16 rows' sums as two words 28 bits apart (those of the odd
+            // planes one slot down), kept or, at the end of the pass, given
+            // where the other warp converts the row
+            if (on) {
+#pragma unroll 1
                 for (int h8 = 0; h8 < 2; h8++) {
-                    long long hi[8], lo[8];
+                    OzQuad x[8];
 #pragma unroll
-                    for (int q = 0; q < 8; q++)
-                        hi[q] = lo[q] = 0;
+                    for (int d = 0; d < 4; d++) {
+                        unsigned r0[8], r1[8];
+                        const int s0 = 2 * d - odd; // slots s0, s0 + 1
+                        tmem_ld8x2(tacc + (unsigned)(max(s0, 0) * N + 8 * h8), tacc + (unsigned)((s0 + 1) * N + 8 * h8), r0, r1);
 #pragma unroll
-                    for (int D = 0; D < S; D++) {
-                        unsigned r[8];
-                        tmem_ld8(tmem + ((unsigned)(32 * (wid & 3)) << 16) + (unsigned)(D * N + 16 * ch + 8 * h8), r);
-#pragma unroll
-                        for (int q = 0; q < 8; q++) {
-                            const long long a = (long long)__float2int_rn(__uint_as_float(r[q]));
-                            if (D < S / 2)
-                                hi[q] += a << (7 * (S / 2 - 1 - D));
-                            else
-                                lo[q] += a << (7 * (S - 1 - D));
-                        }
+                        for (int q = 0; q < 8; q++)
+                            x[q].c[d] = oz_duo(d == 0 && odd ? 0u : r0[q], r1[q]);
+                    }
+                    long long *hs = sacc + 8 * 32 * h8 + lane, *hd = hs, *ld = hs + 16 * 32;
+                    if (pass_end && h8 != odd) {
+                        hd = give + lane;
+                        ld = give + 8 * 32 + lane;
                     }
 #pragma unroll
                     for (int q = 0; q < 8; q++) {
-                        sacc[(8 * h8 + q) * 32 + lane] += hi[q];
-                        sacc[(16 + 8 * h8 + q) * 32 + lane] += lo[q];
+                        long long hi = oz_high(x[q]), lo = oz_low(x[q]);
+                        if (!first) {
+                            hi += hs[q * 32];
+                            lo += hs[(16 + q) * 32];
+                        }
+                        hd[q * 32] = hi;
+                        ld[q * 32] = lo;
                     }
                 }
             }
             fence_before();
             __syncwarp();
             if (lane == 0)
-                bar_arrive(acce);
+                bar_arrive(&acce[rounds & 1]);
             rounds++;
-            const bool pass_end = last == c.nsl - 1;
-            const int bi = c.bi, p = c.p;
-            c.s = last; // the cursor past this round
-            advance(c);
-            if (pass_end) {
-                const int rhs = kOzN * p + m;
-                if (16 * ch < N && rhs < mu) {
-                    const int k = 7 * (S - 1) + __ldg(pexp + (long long)bi * mu + rhs) - 2044 - 2 * T;
-                    double *zc  = z + (long long)rhs * zlen + P.row0;
+            if (pass_end && on) {
+                if (!meet()) {
+                    fail = true;
+                    break;
+                }
+                const long long *keep = sacc + 8 * 32 * odd;
 #pragma unroll 4
-                    for (int q = 0; q < 16; q++) {
-                        const int r = 16 * ch + q;
-                        if (r < P.h) {
-                            const __int128 I = ((__int128)sacc[q * 32 + lane] << (7 * (S / 2))) + sacc[(16 + q) * 32 + lane];
-                            const double v   = oz_i2d(I, k + __ldg(prexp + (long long)bi * 32 + r));
-                            zc[r]            = add ? zc[r] + v : v;
+                for (int q = 0; q < 8; q++) {
+                    const int row = 16 * ch + 8 * odd + q; // value of (row, lane) at column (lane + 4 q) mod 32
+                    const long long hi = keep[q * 32 + lane] + take[q * 32 + lane], lo = keep[(16 + q) * 32 + lane] + take[(8 + q) * 32 + lane];
+                    sz[q * 32 + ((lane + 4 * q) & 31)] = oz_pair2d(hi, lo, kx + __shfl_sync(0xffffffffu, kr, row));
+                }
+                if (!meet()) { // taken: the next pass may give again
+                    fail = true;
+                    break;
+                }
+                // lanes over the rows: four right-hand sides a store
+                const int q = lane & 7, row = 16 * ch + 8 * odd + q;
+                if (row < P.h)
+#pragma unroll 4
+                    for (int u = lane >> 3; u < 32; u += 4) {
+                        const int cz = kOzN * p + 32 * (quad & 1) + u;
+                        if (cz < mu) {
+                            double *zc     = z + (long long)cz * zlen + P.row0 + row;
+                            const double v = sz[q * 32 + ((u + 4 * q) & 31)];
+                            *zc            = add ? *zc + v : v;
                         }
                     }
-                }
-#pragma unroll
-                for (int q = 0; q < 32; q++)
-                    sacc[q * 32 + lane] = 0;
+                __syncwarp();
             }
+            c.s = last; // the cursor past this round
+            advance(c);
         }
         if (fail && lane == 0)
             atomicExch(status, 4);
@@ -1290,12 +1470,12 @@ void launch_phase2_oz(const OzPanel *panels, int npanels, const int *groups, con
     int dev = 0, sms = 0;
     HTGPU_CUDA(cudaGetDevice(&dev));
     if (dev >= 64 || !(done >> dev & 1)) {
-        oz_smem_attr(phase2_oz_kernel<8>, Oz2Cfg<8>::kSmem);
+        oz_smem_attr(phase2_oz_kernel, Oz2Cfg::kSmem);
         if (dev < 64)
             done |= 1ull << dev;
     }
     HTGPU_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    phase2_oz_kernel<8><<<std::min(npanels, sms), kOz2Threads, Oz2Cfg<8>::kSmem, st>>>(panels, npanels, groups, parena, prexp, cidx, A, xp, sc.pexp, mu, z, zlen, add ? 1 : 0, status);
+    phase2_oz_kernel<<<std::min(npanels, sms), kOz2Threads, Oz2Cfg::kSmem, st>>>(panels, npanels, parena, prexp, cidx, A, xp, sc.pexp, mu, z, zlen, add ? 1 : 0, status);
     HTGPU_CUDA(cudaGetLastError());
 }
 
