@@ -1104,7 +1104,7 @@ void HMatrix::ensure_work(int mu) {
     layout_gen_++; // work buffers move: captured products are stale
     // paired panels run an odd number of right-hand sides padded by one
     const std::size_t even = mu > 1 ? (std::size_t)(mu + 1) & ~(std::size_t)1 : 1;
-    xp.alloc((std::size_t)nc * mu + 1);
+    xp.alloc((std::size_t)nc * even + 1);
     xs.alloc((std::size_t)nc * even + 1);
     xexp.alloc(1);
     A.alloc((std::size_t)std::max<long long>(a_slots, 1) * even);
@@ -1355,14 +1355,99 @@ void HMatrix::release_pair() {
 // Phase 2: every target cluster's rows cut at 32 (a full panel keeps every
 // lane busy; balanced cuts of 24 or 25 rows would leave a quarter idle), the
 // columns those of its row chunks. False when the mirror does not fit.
-bool HMatrix::build_pair() {
+bool HMatrix::build_pair(bool dense_only) {
     release_pair();
-    struct Tile { // one source tile: the sorted leaves [l0, l1), its outputs
-        int l0, l1, ch, jlen, xrow, nout;
-        long long out0, src;
+    struct Tile { // outputs of a source tile, the first one's index, bytes before it, panels before it
+        int nout;
+        long long out0, src, pan0;
     };
-    // leaves by source cluster: counting sort on the first column, then by size
-    std::vector<int> first(lr_h.size(), 0), order, start((std::size_t)nc + 1, 0);
+    std::vector<int> order, first;
+    std::vector<SourceTile> tiles;
+    if (!dense_only)
+        source_tiles(order, first, tiles);
+    std::vector<Tile> at(tiles.size());
+    long long nout = 0, off = 0, np1 = 0;
+    for (std::size_t t = 0; t < tiles.size(); t++) {
+        int r = 0;
+        for (int a = tiles[t].l0; a < tiles[t].l1; a++)
+            r += lr_h[order[a]].r;
+        at[t] = {r, nout, off, np1};
+        nout += r;
+        np1 += (r + kPairRows - 1) / kPairRows;
+        off += 16LL * tiles[t].jlen * (r / kPairRows * (kPairRows / 2) + (r % kPairRows + 1) / 2);
+    }
+    std::vector<int> oslot((std::size_t)nout);
+    std::vector<long long> osrc((std::size_t)nout);
+    std::vector<PairPanel> pan1((std::size_t)np1), pan2;
+    host_parallel_chunks((long long)tiles.size(), 256, [&](long long lo, long long hi) {
+        for (long long t = lo; t < hi; t++) {
+            const SourceTile &tl = tiles[(std::size_t)t];
+            const Tile &o        = at[(std::size_t)t];
+            std::size_t q        = (std::size_t)o.out0;
+            for (int a = tl.l0; a < tl.l1; a++) {
+                const LrLeaf &L      = lr_h[order[a]];
+                const long long base = p1_h[first[order[a]] + tl.ch].off;
+                for (int k = 0; k < L.r; k++, q++) {
+                    oslot[q] = (int)(L.a_off + (long long)tl.ch * L.r + k);
+                    osrc[q]  = base + (long long)k * tl.jlen;
+                }
+            }
+            long long src = o.src;
+            for (int c = 0; c * kPairRows < o.nout; c++) {
+                const int h                      = std::min(kPairRows, o.nout - c * kPairRows);
+                pan1[(std::size_t)(o.pan0 + c)] = {src, tl.jlen, h, tl.xrow, (int)(o.out0 + c * kPairRows)};
+                src += 16LL * tl.jlen * ((h + 1) / 2);
+            }
+        }
+    });
+    std::vector<PairSource> src2;
+    for (const int2 &g : p2grp_h) {
+        const PanelItem &pi = pan_h[g.x];
+        int ncol            = pi.ncol;
+        if (dense_only) { // the dense columns come first
+            ncol = 0;
+            for (int c = p2_h[g.x].cbeg; c < p2_h[g.x].cend; c++)
+                ncol += c_leaf[c] < 0 ? c_h[c].w : 0;
+            if (ncol == 0)
+                continue;
+        }
+        for (int lo = 0; lo < g.y; lo += kPairRows) {
+            const int h = std::min(kPairRows, g.y - lo);
+            pan2.push_back({off, ncol, h, pi.q0, pi.row0 + lo});
+            src2.push_back({g.x, g.y, lo});
+            off += 16LL * ncol * ((h + 1) / 2);
+        }
+    }
+    std::size_t fr = 0, tot = 0;
+    HTGPU_CUDA(cudaMemGetInfo(&fr, &tot));
+    if (nout >= (1LL << 31) || (std::size_t)off > fr / 4 * 3)
+        return false;
+    pair_d.alloc((std::size_t)std::max<long long>(off, 16));
+    pair1_d.upload(pan1, stream_);
+    pair2_d.upload(pan2, stream_);
+    pairo_d.upload(oslot, stream_);
+    n_pair1_ = (int)pan1.size();
+    n_pair2_ = (int)pan2.size();
+    {
+        DevBuf<long long> so;
+        DevBuf<PairSource> s2;
+        DevBuf<PanelItem> pd;
+        so.upload(osrc, stream_);
+        s2.upload(src2, stream_);
+        pd.upload(pan_h, stream_);
+        launch_pair_pack(pair1_d.p, n_pair1_, so.p, pair2_d.p, s2.p, n_pair2_, pd.p, fac.p, pair_d.p, stream_);
+        HTGPU_CUDA(cudaStreamSynchronize(stream_));
+    }
+    pair_ready_ = !dense_only;
+    return true;
+}
+
+// The leaves by source cluster (counting sort on the first column, larger
+// clusters first), every cluster's columns cut into the tiles of p1_h;
+// first: each leaf's first tile there.
+void HMatrix::source_tiles(std::vector<int> &order, std::vector<int> &first, std::vector<SourceTile> &tiles) const {
+    std::vector<int> start((std::size_t)nc + 1, 0);
+    first.assign(lr_h.size(), 0);
     for (std::size_t i = 0; i < p1_h.size(); i++)
         if ((p1_h[i].chunk & ~kEmuBit) == 0)
             first[p1_h[i].leaf] = (int)i;
@@ -1386,80 +1471,88 @@ bool HMatrix::build_pair() {
             if (start[j + 1] - start[j] > 1)
                 std::stable_sort(order.begin() + start[j], order.begin() + start[j + 1], [&](int a, int b) { return lr_h[a].n > lr_h[b].n; });
     });
-    std::vector<Tile> tiles;
-    long long nout = 0, off = 0, np1 = 0;
     for (int a = 0; a < nlr;) {
         const LrLeaf &L = lr_h[order[a]];
-        int b = a, r = 0;
-        for (; b < nlr && lr_h[order[b]].oj == L.oj && lr_h[order[b]].n == L.n; b++)
-            r += lr_h[order[b]].r;
-        for (int ch = 0; ch < L.nch; ch++) {
-            const int j0 = ch * kPhase1Chunk, jlen = std::min(kPhase1Chunk, L.n - j0);
-            tiles.push_back({a, b, ch, jlen, L.oj + j0, r, nout, off});
-            nout += r;
-            np1 += (r + kPairRows - 1) / kPairRows;
-            off += 16LL * jlen * (r / kPairRows * (kPairRows / 2) + (r % kPairRows + 1) / 2);
-        }
+        int b           = a;
+        while (b < nlr && lr_h[order[b]].oj == L.oj && lr_h[order[b]].n == L.n)
+            b++;
+        for (int ch = 0; ch < L.nch; ch++)
+            tiles.push_back({a, b, ch, std::min(kPhase1Chunk, L.n - ch * kPhase1Chunk), L.oj + ch * kPhase1Chunk});
         a = b;
     }
-    std::vector<int> oslot((std::size_t)nout);
-    std::vector<long long> osrc((std::size_t)nout);
-    std::vector<PairPanel> pan1((std::size_t)np1), pan2;
-    std::vector<long long> tp(tiles.size() + 1, 0);
-    for (std::size_t t = 0; t < tiles.size(); t++)
-        tp[t + 1] = tp[t] + (tiles[t].nout + kPairRows - 1) / kPairRows;
-    host_parallel_chunks((long long)tiles.size(), 256, [&](long long lo, long long hi) {
-        for (long long t = lo; t < hi; t++) {
-            const Tile &tl = tiles[(std::size_t)t];
-            std::size_t o  = (std::size_t)tl.out0;
-            for (int a = tl.l0; a < tl.l1; a++) {
-                const LrLeaf &L      = lr_h[order[a]];
-                const long long base = p1_h[first[order[a]] + tl.ch].off;
-                for (int k = 0; k < L.r; k++, o++) {
-                    oslot[o] = (int)(L.a_off + (long long)tl.ch * L.r + k);
-                    osrc[o]  = base + (long long)k * tl.jlen;
+}
+
+void HMatrix::release_red() {
+    red_ready_ = false;
+    red_d.release();
+    red1_d.release();
+    redo_d.release();
+    n_red1_ = 0;
+}
+
+// The streams of reduced-precision products (red.cu): the dense blocks as
+// paired panels, and the reduced tiles p1m (their FP32 columns in pad) stacked
+// by kind, 64 columns to a phase-1 panel.
+void HMatrix::build_red(const std::vector<P1Item> &p1m) {
+    release_red();
+    if (!(red_auto_ && emu_ok_ && presplit_on_) || !build_pair(true))
+        return;
+    std::vector<int> order, first;
+    std::vector<SourceTile> tiles;
+    source_tiles(order, first, tiles);
+    std::vector<RedPanel> pan;
+    std::vector<int2> outs;
+    std::vector<long long> osrc;
+    long long off = 0;
+    for (const SourceTile &t : tiles) {
+        const long long l32 = ld_f32(t.jlen), l16 = ld_bf16(t.jlen);
+        for (int kind : {(int)kStreamF32, (int)kStreamBf16}) {
+            const bool f       = kind == kStreamF32;
+            const std::size_t o0 = outs.size();
+            for (int a = t.l0; a < t.l1; a++) {
+                const LrLeaf &L = lr_h[order[a]];
+                const P1Item &m = p1m[(std::size_t)(first[order[a]] + t.ch)];
+                const int c32   = m.pad;
+                for (int k = f ? 0 : c32; k < (f ? c32 : L.r); k++) {
+                    outs.push_back(make_int2((int)(L.a_off + (long long)t.ch * L.r + k), (int)L.a_off + k));
+                    osrc.push_back(m.off + (f ? 4 * l32 * k : 4 * l32 * c32 + 2 * l16 * (k - c32)));
                 }
             }
-            long long src = tl.src;
-            for (int c = 0; c * kPairRows < tl.nout; c++) {
-                const int h                  = std::min(kPairRows, tl.nout - c * kPairRows);
-                pan1[(std::size_t)(tp[t] + c)] = {src, tl.jlen, h, tl.xrow, (int)(tl.out0 + c * kPairRows)};
-                src += 16LL * tl.jlen * ((h + 1) / 2);
+            for (std::size_t o = o0; o < outs.size(); o += kRedOuts) {
+                const int h = (int)std::min<std::size_t>(kRedOuts, outs.size() - o);
+                pan.push_back({off, t.jlen, h, t.xrow, (int)o, kind, 0});
+                off += (long long)t.jlen * (f ? 16 * ((h + 3) / 4) : 16 * ((h + 7) / 8));
             }
-        }
-    });
-    std::vector<PairSource> src2;
-    for (const int2 &g : p2grp_h) {
-        const PanelItem &pi = pan_h[g.x];
-        for (int lo = 0; lo < g.y; lo += kPairRows) {
-            const int h = std::min(kPairRows, g.y - lo);
-            pan2.push_back({off, pi.ncol, h, pi.q0, pi.row0 + lo});
-            src2.push_back({g.x, g.y, lo});
-            off += 16LL * pi.ncol * ((h + 1) / 2);
         }
     }
     std::size_t fr = 0, tot = 0;
     HTGPU_CUDA(cudaMemGetInfo(&fr, &tot));
-    if (nout >= (1LL << 31) || (std::size_t)off > fr / 4 * 3)
-        return false;
-    pair_d.alloc((std::size_t)std::max<long long>(off, 16));
-    pair1_d.upload(pan1, stream_);
-    pair2_d.upload(pan2, stream_);
-    pairo_d.upload(oslot, stream_);
-    n_pair1_ = (int)pan1.size();
-    n_pair2_ = (int)pan2.size();
-    {
-        DevBuf<long long> so;
-        DevBuf<PairSource> s2;
-        DevBuf<PanelItem> pd;
-        so.upload(osrc, stream_);
-        s2.upload(src2, stream_);
-        pd.upload(pan_h, stream_);
-        launch_pair_pack(pair1_d.p, n_pair1_, so.p, pair2_d.p, s2.p, n_pair2_, pd.p, fac.p, pair_d.p, stream_);
-        HTGPU_CUDA(cudaStreamSynchronize(stream_));
-    }
-    pair_ready_ = true;
-    return true;
+    if (outs.size() >= (1ULL << 31) || (std::size_t)off > fr / 4 * 3)
+        return;
+    red_d.alloc((std::size_t)std::max<long long>(off, 16));
+    red1_d.upload(pan, stream_);
+    redo_d.upload(outs, stream_);
+    n_red1_ = (int)pan.size();
+    DevBuf<long long> so;
+    so.upload(osrc, stream_);
+    launch_red_pack(red1_d.p, n_red1_, so.p, mix_.p, red_d.p, stream_);
+    HTGPU_CUDA(cudaStreamSynchronize(stream_));
+    red_ready_ = true;
+}
+
+// the caller chose a kernel or a split: reduced-precision products leave the
+// warp-fed streams
+void HMatrix::leave_red() {
+    if (!red_auto_)
+        return;
+    red_auto_ = false;
+    if (!red_ready_)
+        return;
+    layout_gen_++;
+    HTGPU_CUDA(cudaSetDevice(device_));
+    HTGPU_CUDA(cudaStreamSynchronize(stream_));
+    release_red();
+    release_pair();
 }
 
 // the FP64 products' launch lists: paired panels, or the chunk lists and
@@ -1508,7 +1601,7 @@ void HMatrix::ensure_status() {
         return;
     status_d.alloc(1);
     HTGPU_CUDA(cudaMemsetAsync(status_d.p, 0, sizeof(int), stream_));
-    tickets_d.alloc(16); // phase 2: 0..7, phase 1: 8, paired panels: 10, 11
+    tickets_d.alloc(16); // phase 2: 0..7, phase 1: 8, warp-fed streams: 10..12
 }
 
 int HMatrix::device_status() {
@@ -1596,6 +1689,20 @@ void HMatrix::upload_mixed_phase2() {
         scr_d.upload(red, stream_);
         if (red.empty())
             scr_d.alloc(1);
+        { // the same where the dense chunks' sums come first only in the row chunks that have any
+            std::vector<StreamChunk> redp = red;
+            std::size_t k                 = 0;
+            for (int w = 0; w < n_p2rc_m_; w++) {
+                const bool dense = ch2[rc[w]].kind == kStreamDfma || ch2[rc[w]].kind == kStreamEmu;
+                int n            = 0;
+                for (int c = rc[w]; c < rc[w + 1]; c++)
+                    n += ch2[c].kind == kStreamF32 || ch2[c].kind == kStreamBf16;
+                k += n;
+                if (n > 0 && !dense)
+                    redp[k - 1].flags &= (unsigned char)~kStreamAdd;
+            }
+            redp_d.upload(redp, stream_);
+        }
         const std::vector<int> rr = stream_ranges(red, n_sctas_);
         n_ranges_r_               = (int)rr.size() - 1;
         srr_d.upload(rr, stream_);
@@ -1640,6 +1747,7 @@ void HMatrix::upload_mixed_phase2() {
 void HMatrix::set_fp64_split(int p1, int n64) {
     require(p1 >= 0 && p1 <= 1000 && n64 >= 0 && n64 <= 1000, "FP64 split: phase-1 and phase-2 DFMA shares in [0, 1000] per mille");
     if (precision_ != 0) { // the dense blocks of a reduced-precision product
+        leave_red();
         p2m_n64_ = n64;
         upload_mixed_phase2();
         return;
@@ -1689,6 +1797,9 @@ void HMatrix::set_precision(int policy, double tau) {
     precision_ = policy;
     tau_       = tau;
     if (policy == 0) {
+        release_red();
+        if (!pair_ready_)
+            release_pair();
         emu3_.release(); // the reduced-precision products' mirror
         tca_d.release();  // and the tensor cores' copy of the factors
         tcoff_d.release();
@@ -1910,6 +2021,7 @@ void HMatrix::set_precision(int policy, double tau) {
         launch_swizzle(dz.p, (int)swz.size(), fac.p, dso.p, cidxm_d.p, cmax.p, mix_.p, stream_);
         HTGPU_CUDA(cudaStreamSynchronize(stream_));
     }
+    build_red(p1m);
     build_tc_arena();
     build_oz_arena();
 }
@@ -2105,13 +2217,19 @@ void HMatrix::launch_product_with(const double *x, double *y, int mu_out, int nu
         return;
     }
     launches_        = 0;
+    // many right-hand sides on the tensor cores when epsilon leaves room for their FP32 sums
+    const bool mma = mu >= kMmaMinRhs && eps_ >= kMmaMinEps;
+    // (one right-hand side stays on the producer-fed chunks: their bookkeeping
+    // runs on a warp of its own; 200 000 points 0.505 ms against 0.565 ms)
+    if (red_ready_ && precision_ != 0 && mu >= 2 && !mma && !(mu >= kMmaMinRhs && oz_S_ == 4 && w_oz && n_tcblk_ > 0)) {
+        launch_red_product(x, y, mu_out, numbering, st, w_xp, w_xs, w_xexp, w_A, w_z, marks, w_A != A.p);
+        return;
+    }
     launch_xexp(x, (long long)nc * mu_out, w_xexp, st);
     launch_gather_split(x, nc, numbering == kUserNumbering ? perm_s.p : nullptr, nc, mu, w_xexp, w_xp, w_xs, st, mu_out);
     launches_ += 2;
     if (marks)
         HTGPU_CUDA(cudaEventRecord(marks[0], st));
-    // many right-hand sides on the tensor cores when epsilon leaves room for their FP32 sums
-    const bool mma = mu >= kMmaMinRhs && eps_ >= kMmaMinEps;
     if (precision_ != 0) {
         if (n_p1m_ && mu <= 2 && p1_mode_ >= 1) {
             launch_phase1_stream(p1rm_d.p, n_p1m_ranges_, p1cm_d.p, p1m_kinds_, mix_.p, w_xp, w_xs, scalef_d.p, w_xexp, mu, w_A, status_d.p, st);
@@ -2278,10 +2396,55 @@ void HMatrix::launch_pair_product(const double *x, double *y, int mu, int number
     }
     if (marks)
         HTGPU_CUDA(cudaEventRecord(marks[2], st));
+    launch_pair_sums(y, mu, numbering, w_z, w_xexp, st);
+    launches_ += 1;
+}
+
+void HMatrix::launch_pair_sums(double *y, int mu, int numbering, const double *w_z, const int *w_xexp, cudaStream_t st) {
+    const float2 *zf = reinterpret_cast<const float2 *>(w_z);
     if (numbering == kGlobalToLocal)
         launch_pair_zsum(zi_d.p + zloc0_, zloc1_ - zloc0_, zl_d.p, zf, (int)zlen_, mu, nullptr, w_xexp, y, local_row_count(), st, local_row_offset());
     else
         launch_pair_zsum(zi_d.p, (int)zi_h.size(), zl_d.p, zf, (int)zlen_, mu, numbering == kUserNumbering ? perm_t.p : nullptr, w_xexp, y, nr, st);
+}
+
+// A reduced-precision product on the warp-fed streams: per pass the split
+// input for the dense blocks (w_xp) and for the reduced columns (w_xs), the
+// reduced phase 1 (one or two right-hand sides: the staged tiles of stream.cu,
+// whose FP32 sums run over lanes; more: the stacked panels), the dense blocks'
+// sums and the reduced columns' onto them
+void HMatrix::launch_red_product(const double *x, double *y, int mu, int numbering, cudaStream_t st, double *w_xp, F2 *w_xs, int *w_xexp, double *w_A, double *w_z, cudaEvent_t *marks, bool exact) {
+    float *X = reinterpret_cast<float *>(w_xp), *Xr = reinterpret_cast<float *>(w_xs), *Af = reinterpret_cast<float *>(w_A);
+    float2 *zf        = reinterpret_cast<float2 *>(w_z);
+    int *tickets      = tickets_d.p + 10;
+    const int *perm   = numbering == kUserNumbering ? perm_s.p : nullptr;
+    const bool stack  = mu >= 3;
+    launch_xexp(x, (long long)nc * mu, w_xexp, st);
+    launches_ = 1;
+    for (int c0 = 0; c0 < mu;) {
+        const int w = pair_pass_width(mu - c0, exact), n = std::min(w, mu - c0);
+        launch_pair_gather(x, nc, perm, nc, c0, w, mu, w_xexp, X, tickets, st);
+        launch_red_gather(x, nc, perm, nc, c0, w, mu, w_xexp, stack, Xr, st);
+        if (marks && c0 == 0)
+            HTGPU_CUDA(cudaEventRecord(marks[0], st));
+        if (stack)
+            launch_red_phase1(red1_d.p, n_red1_, tickets, red_d.p, redo_d.p, scalef_d.p, Xr, Af, w, status_d.p, st);
+        else if (n_p1m_)
+            launch_phase1_stream(p1rm_d.p, n_p1m_ranges_, p1cm_d.p, p1m_kinds_, mix_.p, nullptr, w_xs, scalef_d.p, w_xexp, w, w_A, status_d.p, st);
+        if (!multi_h.empty())
+            launch_reduce_tiles_f(lr_d.p, multi_d.p, (int)multi_h.size(), w, Af, st);
+        if (!rot_h.empty())
+            launch_rotate_slots_f(rot_d.p, (long long)rot_h.size(), w, Af, st);
+        if (marks && c0 + n == mu)
+            HTGPU_CUDA(cudaEventRecord(marks[1], st));
+        launch_pair_phase2(pair2_d.p, n_pair2_, tickets, pair_d.p, cidx_d.p, X, nullptr, w, n, zf + (long long)c0 * zlen_, (int)zlen_, status_d.p, st);
+        launch_red_phase2(redp_d.p, srr_d.p, n_ranges_r_, tickets + 2, mix_.p, cidxm_d.p, Af, w, n, zf + (long long)c0 * zlen_, (int)zlen_, status_d.p, st);
+        launches_ += 2 + (n_p1m_ > 0) + !multi_h.empty() + !rot_h.empty() + (n_pair2_ > 0) + (n_ranges_r_ > 0);
+        c0 += n;
+    }
+    if (marks)
+        HTGPU_CUDA(cudaEventRecord(marks[2], st));
+    launch_pair_sums(y, mu, numbering, w_z, w_xexp, st);
     launches_ += 1;
 }
 
@@ -2323,6 +2486,7 @@ void HMatrix::set_phase2_mode(int mode) {
     layout_gen_++; // captured products are stale
     require(mode == 0 || mode == 1, "phase-2 mode must be 0 (per-warp streams) or 1 (producer-fed)");
     p2_mode_ = mode;
+    leave_red();
     leave_pair();
 }
 
@@ -2330,11 +2494,13 @@ void HMatrix::set_phase1_mode(int mode) {
     layout_gen_++; // buffers or launch lists change: captured products are stale
     require(mode >= 0 && mode <= 2, "phase-1 mode must be 0 (tile kernels), 1 (streamed chunks) or 2 (tensor cores for reduced-precision products with 8 or more right-hand sides)");
     p1_mode_ = mode;
+    leave_red();
     leave_pair();
 }
 
 void HMatrix::set_presplit(bool on) {
     HTGPU_CUDA(cudaSetDevice(device_));
+    leave_red();
     presplit_on_ = on;
     pair_auto_   = false; // the kernels whose pre-split copies this switches
     if (fac.p) {
@@ -2390,6 +2556,21 @@ void HMatrix::autotune(int mu, int reps, float *best_ms) {
         else
             set_digit_planes(was);
     };
+    if (precision_ != 0 && !red_ready_ && emu_ok_ && presplit_on_ && mu >= 2 && !(mu >= kMmaMinRhs && eps_ >= kMmaMinEps)) {
+        red_auto_ = true; // back from a caller's choice
+        set_precision(precision_, tau_);
+    }
+    if (red_ready_ && precision_ != 0 && mu >= 2 && !(mu >= kMmaMinRhs && eps_ >= kMmaMinEps)) {
+        // the warp-fed streams, with many right-hand sides against the digit planes
+        best = timed();
+        if (mu >= kMmaMinRhs && n_tcblk_ > 0)
+            try_digit_planes();
+        HTGPU_CUDA(cudaEventDestroy(e0));
+        HTGPU_CUDA(cudaEventDestroy(e1));
+        if (best_ms)
+            *best_ms = best;
+        return;
+    }
     if (precision_ != 0) {
         // phase-1 modes with the dense blocks' DFMA / emulation split
         int arg_mode = p1_mode_, arg_split = p2m_n64_;

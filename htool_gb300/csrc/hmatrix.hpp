@@ -198,7 +198,7 @@ class HMatrix {
     int phase1_mode() const { return p1_mode_; }
     void set_presplit(bool on);
     bool presplit() const { return presplit_on_; }
-    long long presplit_bytes() const { return (long long)(((emu_fresh_ ? emu_.n : 0) + emu2_.n + emu3_.n) * sizeof(F2) + pair_d.n); }
+    long long presplit_bytes() const { return (long long)(((emu_fresh_ ? emu_.n : 0) + emu2_.n + emu3_.n) * sizeof(F2) + pair_d.n); } // and the paired panels
     void set_phase2_mode(int mode);
     int phase2_mode() const { return p2_mode_; }
     // tensor-core kernels of reduced-precision products with many
@@ -235,6 +235,7 @@ class HMatrix {
     void set_phase2_dense_split(bool on) {
         split_dense_ = on;
         layout_gen_++;
+        leave_red();
     }
     bool phase2_dense_split() const { return split_dense_; }
     bool emulation_allowed() const { return emu_ok_; }
@@ -338,8 +339,29 @@ class HMatrix {
     DevBuf<PairPanel> pair1_d, pair2_d;
     DevBuf<int> pairo_d;
     int n_pair1_ = 0, n_pair2_ = 0;
-    bool build_pair();
+    bool build_pair(bool dense_only = false);
     void release_pair();
+    // the source tiles of phase 1 with the leaves on each: leaves
+    // order[l0 .. l1) have the tile ch of the same columns (x rows xrow ..)
+    struct SourceTile {
+        int l0, l1, ch, jlen, xrow;
+    };
+    void source_tiles(std::vector<int> &order, std::vector<int> &first, std::vector<SourceTile> &tiles) const;
+    // reduced-precision products off the tensor cores on warp-fed streams
+    // (red.cu), their dense blocks on paired panels (pair_d then holds
+    // those): likewise unless the caller chose a kernel or a split
+    bool red_auto_  = true;
+    bool red_ready_ = false;
+    DevBuf<unsigned char> red_d;
+    DevBuf<RedPanel> red1_d;
+    DevBuf<int2> redo_d;
+    DevBuf<StreamChunk> redp_d; // the reduced chunks, adding onto z where the row chunk has dense columns
+    int n_red1_ = 0;
+    void build_red(const std::vector<P1Item> &p1m);
+    void release_red();
+    void leave_red();
+    void launch_red_product(const double *x, double *y, int mu, int numbering, cudaStream_t st, double *w_xp, F2 *w_xs, int *w_xexp, double *w_A, double *w_z, cudaEvent_t *marks, bool exact);
+    void launch_pair_sums(double *y, int mu, int numbering, const double *w_z, const int *w_xexp, cudaStream_t st);
     void leave_pair();
     void upload_fp64_lists();
     void apply_fp64_split(int p1, int n64);

@@ -332,7 +332,7 @@ int pair_pass_width(int left, bool exact);
 void launch_pair_pack(const PairPanel *p1, int np1, const long long *osrc, const PairPanel *p2, const PairSource *s2, int np2, const PanelItem *pan, const double *fac, unsigned char *mirror,
                       cudaStream_t st);
 // one pass of w right-hand sides c0 .. (those from mu_src on zero): the split
-// input X (n x w pairs of floats; clears tickets[0..1]), the phase-1 sums A
+// input X (n x w pairs of floats; clears tickets[0..2]), the phase-1 sums A
 // (slots x w), the sums of multi-tile leaves, i times the sums (native complex
 // layout), the partial sums z of the first nrhs of them (zlen apart), and
 // the final sums over all mu
@@ -345,6 +345,27 @@ void launch_pair_phase2(const PairPanel *panels, int npanels, int *tickets, cons
 void launch_pair_zsum(const ZItem *items, int nitems, const int *zl, const float2 *z, int zlen, int mu, const int *perm, const int *xexp, double *y, int ldy, cudaStream_t st, int shift = 0);
 // the limit of its waits and a panel whose first copy is left out (set_debug_waits)
 void set_pair_waits(long long cycles, long long skip);
+// ---- reduced-precision products off the tensor cores (red.cu) --------------
+// one phase-1 panel: h <= 64 outputs of one kind (kStreamF32 / kStreamBf16)
+// x nk rows of x from xrow on, from byte src of the mirror on (rows of h
+// elements padded to 16 bytes); its sums times scale[outs.y] go to the slots
+// outs.x of outs[out ..]
+struct RedPanel {
+    long long src;
+    int nk, h, xrow, out, kind, pad;
+};
+constexpr int kRedOuts = 64; // outputs of a phase-1 panel at most
+// one pass of w right-hand sides: the leading floats of the split input
+// (hi_only, n x w floats) or its (hi, lo) pairs; the float phase-1 sums (slots
+// x w); the chunks' sums into z (double-float rows; kStreamAdd on a row
+// chunk's last chunk: onto the dense part that is there)
+void launch_red_gather(const double *x, int ldx, const int *perm, int n, int c0, int w, int mu_src, const int *xexp, bool hi_only, float *out, cudaStream_t st);
+void launch_red_phase1(const RedPanel *panels, int npanels, int *ticket, const unsigned char *mirror, const int2 *outs, const float *scale, const float *X, float *A, int w, int *status, cudaStream_t st);
+void launch_red_phase2(const StreamChunk *chunks, const int *rbeg, int nranges, int *ticket, const unsigned char *mix, const int *cidx, const float *A, int w, int nrhs, float2 *z, int zlen, int *status,
+                       cudaStream_t st);
+// the phase-1 panels from the reduced tiles (osrc: byte offset of every output's column)
+void launch_red_pack(const RedPanel *panels, int npanels, const long long *osrc, const unsigned char *mix, unsigned char *mirror, cudaStream_t st);
+void set_red_waits(long long cycles);
 // ---- ACA rank predictor (mlp.cu) -------------------------------------------
 constexpr int kMlpIn = 10, kMlpHidden = 64;
 constexpr int kMlpParams = kMlpHidden * kMlpIn + kMlpHidden + kMlpHidden * kMlpHidden + kMlpHidden + kMlpHidden + 1;

@@ -39,7 +39,7 @@
 //
 // Every wait is bounded; a warp whose wait ran out records status 2, lets its
 // copies in flight land (again bounded) and ends.
-#include "df64.cuh"
+#include "f32x2.cuh"
 #include "kernels.hpp"
 
 #include <algorithm>
@@ -49,78 +49,7 @@ namespace {
 
 constexpr int kPairWarps = 4; // warps per CTA, each with its own panels and ring
 
-__device__ long long g_pair_wait = 4000000000ll; // SM clocks of a wait at most (about 2 s)
-__device__ long long g_pair_skip = -1;           // a panel whose first copy is left out (test support)
-
-typedef unsigned long long f2x; // two floats: low word first
-
-__device__ __forceinline__ f2x fx_fma(f2x a, f2x b, f2x c) {
-    f2x d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ f2x fx_add(f2x a, f2x b) {
-    f2x d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f2x fx_sub(f2x a, f2x b) {
-    f2x d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f2x fx(float lo, float hi) {
-    f2x d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-    return d;
-}
-__device__ __forceinline__ float2 fx2(f2x v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-
-struct DF2 { // two double-float accumulators
-    f2x s, c;
-};
-
-__device__ __forceinline__ void df2_fma(DF2 &a, f2x uh, f2x ul, f2x xh, f2x xl) {
-    // two scalar products: the assembler contracts mul.f32x2 and add.f32x2 to
-    // one fma in spite of their rounding modifiers, and t = RN(s + uh xh)
-    // would lose what TwoSum recovers (the product came out at 9e-9)
-    const float2 u = fx2(uh), v = fx2(xh);
-    const f2x p  = fx(__fmul_rn(u.x, v.x), __fmul_rn(u.y, v.y));
-    const f2x t  = fx_add(a.s, p);
-    const f2x nb = fx_sub(a.s, t);              // -(t - s)
-    const f2x w  = fx_sub(a.s, fx_add(t, nb)); // what s lost
-    f2x l        = fx_fma(uh, xh, nb);          // what the product lost, its own rounding included
-    l            = fx_fma(ul, xh, l);
-    l            = fx_fma(uh, xl, l);
-    a.c          = fx_add(a.c, fx_add(w, l)); // one rounding at c's size, the others at an ulp of s
-    a.s          = t;
-}
-
-__device__ __forceinline__ void df2_renorm(DF2 &a) {
-    const f2x s = fx_add(a.s, a.c);
-    a.c         = fx_add(a.c, fx_sub(a.s, s));
-    a.s         = s;
-}
-
-__device__ __forceinline__ DF2 df2_add(DF2 a, DF2 b) {
-    const f2x s  = fx_add(a.s, b.s);
-    const f2x nb = fx_sub(a.s, s);
-    const f2x w  = fx_sub(a.s, fx_add(s, nb));
-    const f2x v  = fx_add(b.s, nb);
-    DF2 r;
-    r.s = s;
-    r.c = fx_add(fx_add(a.c, b.c), fx_add(w, v));
-    return r;
-}
-
-__device__ __forceinline__ f2x shfl2(f2x v, int src) {
-    const float2 f = fx2(v);
-    return fx(__shfl_sync(0xffffffffu, f.x, src), __shfl_sync(0xffffffffu, f.y, src));
-}
+__device__ long long g_pair_skip = -1; // a panel whose first copy is left out (test support)
 
 // a double as hi + lo, both rounded to nearest (|a - hi - lo| <= 2^-48 |a|; the
 // truncating split64 of the other kernels keeps 2^-46), by bit operations:
@@ -140,30 +69,6 @@ __device__ __forceinline__ F2 split64_near(double a) {
     f.hi           = ok ? __uint_as_float(hb) : e == 0x7FF ? __int_as_float(0x7fffffff) : 0.f;
     f.lo           = ok ? __int_as_float(__float_as_int(lo) ^ (int)((unsigned)(b >> 32) & 0x80000000u)) : 0.f;
     return f;
-}
-
-__device__ __forceinline__ unsigned sa(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ bool mbar_try(unsigned long long *b, unsigned parity) {
-    unsigned ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(sa(b)), "r"(parity), "r"(20000u) : "memory");
-    return ok != 0;
-}
-
-// the whole warp waits for the phase; false when the wait ran out
-__device__ __forceinline__ bool pair_wait(unsigned long long *b, unsigned parity) {
-    bool ok = mbar_try(b, parity);
-    if (!__all_sync(0xffffffffu, ok)) {
-        const long long t0 = clock64();
-        while (true) {
-            ok = mbar_try(b, parity);
-            if (__all_sync(0xffffffffu, ok))
-                break;
-            if (__any_sync(0xffffffffu, clock64() - t0 > g_pair_wait))
-                return false;
-        }
-    }
-    return true;
 }
 
 // Per Q (pairs of right-hand sides; 0: one right-hand side): input columns
@@ -197,13 +102,11 @@ __global__ void __launch_bounds__(32 * kPairWarps, PairCfg<Q>::kCtas)
     unsigned char *wbase    = smem + (size_t)wid * C::kWarp;
     unsigned long long *bar = reinterpret_cast<unsigned long long *>(wbase + C::kBar);
     if (lane == 0)
-        for (int s = 0; s < kStages; s++)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sa(&bar[s])) : "memory");
+        ring_init(bar, kStages);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncwarp();
-    unsigned long long pol;
-    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
-    const long long skip = g_pair_skip;
+    const unsigned long long pol = stream_policy();
+    const long long skip         = g_pair_skip;
 
     // ---- panels: the current one (cur, from column jc on), the next one and
     // the ticket after that (lane 0) in flight; the first two are the warp's
@@ -235,12 +138,8 @@ __global__ void __launch_bounds__(32 * kPairWarps, PairCfg<Q>::kCtas)
             if (lane == 0) {
                 *reinterpret_cast<int4 *>(st + C::kDesc) = make_int4(cur.h, nc, jc + nc == cur.ncol, cur.out);
                 const unsigned bytes                     = (unsigned)(16 * hp * nc);
-                if (!(icur == skip && jc == 0)) {
-                    asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}" ::"r"(sa(&bar[s])), "r"(bytes) : "memory");
-                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(sa(st)),
-                                 "l"(mirror + cur.src + (long long)16 * hp * jc), "r"(bytes), "r"(sa(&bar[s])), "l"(pol)
-                                 : "memory");
-                }
+                if (!(icur == skip && jc == 0))
+                    ring_copy(st, mirror + cur.src + (long long)16 * hp * jc, bytes, &bar[s], pol);
             }
             if (lane < nc) {
                 const unsigned char *src;
@@ -249,11 +148,11 @@ __global__ void __launch_bounds__(32 * kPairWarps, PairCfg<Q>::kCtas)
                 else
                     src = idx >= 0 ? reinterpret_cast<const unsigned char *>(A) + (long long)kUnit * idx : reinterpret_cast<const unsigned char *>(X) + (long long)kUnit * (~idx);
                 if constexpr (Q == 0) {
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(sa(st + C::kCoef + 8 * lane)), "l"(src) : "memory");
+                    copy_async<8>(st + C::kCoef + 8 * lane, src);
                 } else {
 #pragma unroll
                     for (int q = 0; q < Q; q++)
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sa(st + C::kCoef + 16 * (q * kCols + lane))), "l"(src + 16 * q) : "memory");
+                        copy_async<16>(st + C::kCoef + 16 * (q * kCols + lane), src + 16 * q);
                 }
             }
             issued++;
@@ -273,7 +172,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, PairCfg<Q>::kCtas)
             }
             load_idx();
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        copies_commit();
     };
 
     constexpr int kAcc = Q ? 2 * Q : 1; // Q = 0: one, its two halves the two outputs; else [output][q]
@@ -290,8 +189,8 @@ __global__ void __launch_bounds__(32 * kPairWarps, PairCfg<Q>::kCtas)
     while (done < issued) {
         const int s = done % kStages;
         issue(); // into the stage the previous iteration read
-        asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 1) : "memory");
-        if (!pair_wait(&bar[s], (done / kStages) & 1)) {
+        copies_wait<kStages - 1>();
+        if (!warp_wait_phase(&bar[s], (done / kStages) & 1)) {
             ok = false;
             break;
         }
@@ -391,22 +290,22 @@ __global__ void __launch_bounds__(32 * kPairWarps, PairCfg<Q>::kCtas)
         __syncwarp(); // every lane is done with the stage before it is refilled
         done++;
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
+    copies_wait<0>();
     if (!ok) {
         if (lane == 0)
             atomicExch(status, 2);
         for (int p = done; p < issued; p++) // the copies in flight land before the warp leaves
-            if (!pair_wait(&bar[p % kStages], (p / kStages) & 1) && lane == 0)
+            if (!warp_wait_phase(&bar[p % kStages], (p / kStages) & 1) && lane == 0)
                 atomicExch(status, 3);
     }
 }
 
 // the gathered input of right-hand sides c0 .. c0 + w (those past mu_src
 // zero), split relative to the input's largest exponent: [row][q] of
-// {hi, hi, lo, lo}, w = 1: [row] of (hi, lo); also clears the two tickets
+// {hi, hi, lo, lo}, w = 1: [row] of (hi, lo); also clears the three tickets
 __global__ void pair_gather_kernel(const double *__restrict__ x, int ldx, const int *__restrict__ perm, int n, int c0, int w, int mu_src, const int *__restrict__ xexp, float *__restrict__ X,
                                    int *__restrict__ tickets) {
-    if (blockIdx.x == 0 && threadIdx.x < 2)
+    if (blockIdx.x == 0 && threadIdx.x < 3)
         tickets[threadIdx.x] = 0;
     const int shift = 1023 - max(*xexp, 1);
     auto value      = [&](int src, int c) {
@@ -658,8 +557,9 @@ void launch_pair_pack(const PairPanel *p1, int np1, const long long *osrc, const
 }
 
 void set_pair_waits(long long cycles, long long skip) {
-    HTGPU_CUDA(cudaMemcpyToSymbol(g_pair_wait, &cycles, sizeof(cycles)));
+    HTGPU_CUDA(cudaMemcpyToSymbol(g_wait_limit, &cycles, sizeof(cycles)));
     HTGPU_CUDA(cudaMemcpyToSymbol(g_pair_skip, &skip, sizeof(skip)));
+    set_red_waits(cycles);
 }
 
 } // namespace htgpu

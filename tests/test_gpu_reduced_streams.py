@@ -1,0 +1,61 @@
+"""Reduced-precision products off the tensor cores on the warp-fed streams
+(red.cu) against the chunk and tile kernels that a choice of phase-2 mode keeps.
+
+Both take the same FP32 sums in the same order (every FMA rounds once), so
+they differ only in how those sums and the dense FP64 blocks are added up in
+double-float arithmetic: by less than the 4e-13 of two FP64 products."""
+import numpy as np
+import pytest
+
+import htool_gb300 as H
+from htool_gb300 import geometry as G
+
+pytestmark = pytest.mark.gpu
+
+TOL = 4e-13
+
+
+def rel(a, b):
+    return np.linalg.norm(a - b) / np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("n", [31, 513, 3000])
+@pytest.mark.parametrize("policy", ["fp32", "mixed", "bf16"])
+def test_streams_match_the_chunk_kernels(n, policy):
+    pts = G.ellipsoid(n, (1.0, 0.7, 1.3), seed=n)
+    t = H.Cluster().build(n, pts)
+    hm = H.HMatrix(t, t, 1e-6, 10.0).build(H.LAPLACE, pts).set_precision(policy, 1.0)
+    mus = (1, 2, 3, 5, 8, 9, 14)
+    xs = {mu: G.rhs(n, mu, seed=mu) for mu in mus}
+    ys = {mu: hm.mvprod_global_to_global(xs[mu], mu) for mu in mus}
+    assert all(np.array_equal(ys[mu], hm.mvprod_global_to_global(xs[mu], mu)) for mu in mus)
+    hm.set_phase2_mode("producer")
+    for mu in mus:
+        assert rel(ys[mu], hm.mvprod_global_to_global(xs[mu], mu)) < TOL, mu
+    assert hm.autotune(3, 2) > 0  # back on the streams
+    assert np.array_equal(ys[3], hm.mvprod_global_to_global(xs[3], 3))
+    assert hm.device_status() == 0
+
+
+@pytest.mark.parametrize("layout", ["real", "native"])
+def test_complex_streams_match_the_chunk_kernels(layout):
+    n = 3000
+    pts = G.cube_surface(n, seed=5)
+    t = H.Cluster().build(n, pts)
+    hm = H.HMatrix(t, t, 1e-5, 3.0, dtype=np.complex128, complex_layout=layout).build(H.HELMHOLTZ, pts, kernel_param=20.0).set_precision("mixed", 1.0)
+    ys = {mu: hm.mvprod_global_to_global(G.rhs(n, mu, seed=mu, dtype=np.complex128), mu) for mu in (1, 2, 3)}
+    hm.set_phase2_mode("producer")
+    for mu, y in ys.items():
+        assert rel(y, hm.mvprod_global_to_global(G.rhs(n, mu, seed=mu, dtype=np.complex128), mu)) < TOL, mu
+
+
+def test_rows_without_dense_leaves_and_rectangles():
+    """targets far from the sources: no dense leaf, every row from reduced columns alone"""
+    xt, xs = G.sphere(900, seed=1) + 4.0, G.sphere(2100, seed=2)
+    t, s = H.Cluster().build(900, xt), H.Cluster().build(2100, xs)
+    hm = H.HMatrix(t, s, 1e-6, 10.0).build(H.LAPLACE, xt, xs).set_precision("mixed", 1.0)
+    assert hm.get_ndmat() == 0
+    x = G.rhs(2100, 4, seed=3)
+    y = hm.mvprod_global_to_global(x, 4)
+    hm.set_phase2_mode("warp")
+    assert rel(y, hm.mvprod_global_to_global(x, 4)) < TOL
