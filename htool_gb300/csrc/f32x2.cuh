@@ -125,6 +125,28 @@ __device__ __forceinline__ void ring_copy(void *dst, const void *src, unsigned b
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(sa(dst)), "l"(src), "r"(bytes), "r"(sa(bar)), "l"(pol) : "memory");
 }
 
+// Programmatic dependent launch: the kernels of a product follow each other on
+// one stream, and each may start (set up its rings, read its descriptors)
+// while the one before it ends.  pdl_wait returns when that one has completed
+// and its writes are visible; pdl_next lets the next one be launched.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+void pdl_launch(void (*kernel)(P...), int grid, int block, int smem, cudaStream_t st, A... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c                             = {};
+    c.gridDim                                        = dim3((unsigned)grid);
+    c.blockDim                                       = dim3((unsigned)block);
+    c.dynamicSmemBytes                               = (size_t)smem;
+    c.stream                                         = st;
+    c.attrs                                          = at;
+    c.numAttrs                                       = 1;
+    HTGPU_CUDA(cudaLaunchKernelEx(&c, kernel, P(args)...));
+}
+
 template <int B>
 __device__ __forceinline__ void copy_async(void *dst, const void *src) {
     if constexpr (B == 16)

@@ -61,6 +61,37 @@ void stack_tiles(const std::vector<P1Item> &items, const std::vector<LrLeaf> &lr
     std::stable_sort(blks.begin(), blks.end(), [](const TcBlock &a, const TcBlock &b) { return a.jlen > b.jlen; });
 }
 
+// The order in which warps claim panels, as their indices.  Up to some 18
+// panels a warp: most work first, so that the last ones claimed are short
+// (20 000 points 0.105 -> 0.093 ms, 50 000 with 8 right-hand sides 0.53 ->
+// 0.48).  More: as they lie, so that long panels, bound by HBM, run beside short
+// ones, bound by their set-up (400 000 points: 1.58 ms, the short ones last
+// 1.63).  A stable counting sort.
+std::vector<int> claim_order(const std::vector<PairPanel> &pan) {
+    constexpr int kKeys        = 4096;
+    constexpr std::size_t kFew = 24576;
+    std::vector<int> by(pan.size());
+    std::iota(by.begin(), by.end(), 0);
+    if (pan.size() >= kFew)
+        return by;
+    auto key = [&](const PairPanel &p) { return kKeys - 1 - std::min<long long>(kKeys - 1, (long long)p.ncol * ((p.h + 1) / 2) / 64); };
+    std::vector<int> at(kKeys + 1, 0);
+    for (const PairPanel &p : pan)
+        at[(std::size_t)key(p) + 1]++;
+    for (int k = 0; k < kKeys; k++)
+        at[k + 1] += at[k];
+    for (std::size_t i = 0; i < pan.size(); i++)
+        by[at[(std::size_t)key(pan[i])]++] = (int)i;
+    return by;
+}
+template <typename T>
+void permute(std::vector<T> &v, const std::vector<int> &by) {
+    std::vector<T> w(v.size());
+    for (std::size_t i = 0; i < v.size(); i++)
+        w[i] = v[(std::size_t)by[i]];
+    v.swap(w);
+}
+
 double now() { return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count(); }
 
 // largest q with q * (M + N) <= M * N in htool's 32-bit int arithmetic
@@ -1418,6 +1449,10 @@ bool HMatrix::build_pair(bool dense_only) {
             off += 16LL * ncol * ((h + 1) / 2);
         }
     }
+    const std::vector<int> by1 = claim_order(pan1), by2 = claim_order(pan2);
+    permute(pan1, by1);
+    permute(pan2, by2);
+    permute(src2, by2);
     std::size_t fr = 0, tot = 0;
     HTGPU_CUDA(cudaMemGetInfo(&fr, &tot));
     if (nout >= (1LL << 31) || (std::size_t)off > fr / 4 * 3)

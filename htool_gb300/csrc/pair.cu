@@ -31,10 +31,10 @@
 // Measured against the tile and chunk kernels of stream.cu and
 // matvec_kernels.cu (which shuffle every coefficient, reduce every tile over
 // the warp and leave lanes idle on tiles of few rows), Laplace sphere, FP64:
-//   100 000 points  1 right-hand side 0.489 -> 0.381 ms, 2: 0.82 -> 0.44,
-//                   4: 1.79 -> 0.66, 8: 2.66 -> 1.10
-//   400 000 points  1: 2.11 -> 1.61 (6.6 TB/s in phase 1, 6.9 in phase 2, a
-//                   copy takes 6.8), 4: 7.94 -> 2.78
+//   100 000 points  1 right-hand side 0.489 -> 0.356 ms, 2: 0.82 -> 0.40,
+//                   4: 1.79 -> 0.57, 8: 2.66 -> 1.01
+//   400 000 points  1: 2.11 -> 1.58 (6.7 TB/s in phase 1, 7.0 in phase 2, a
+//                   copy takes 6.8), 4: 7.94 -> 2.42
 // at no larger an error against the FP64 pipe (1.2e-14 .. 2.0e-14).
 //
 // Every wait is bounded; a warp whose wait ran out records status 2, lets its
@@ -72,12 +72,15 @@ __device__ __forceinline__ F2 split64_near(double a) {
 }
 
 // Per Q (pairs of right-hand sides; 0: one right-hand side): input columns
-// per stage, stages per warp, resident CTAs per SM.
+// per stage, stages per warp, resident CTAs per SM.  Two long stages and twelve
+// warps an SM beat three of 16 columns and sixteen warps (the bookkeeping of a
+// stage against 4 or 8 KB of data; 100 000 points, 4 right-hand sides 0.66 ->
+// 0.58 ms); 24 columns keep the three CTAs in shared memory with 6 and 8.
 template <int Q>
 struct PairCfg {
-    static constexpr int kCols   = 16;
-    static constexpr int kStages = 3;
-    static constexpr int kCtas   = Q >= 3 ? 3 : 4;
+    static constexpr int kCols   = Q >= 3 ? 24 : 32;
+    static constexpr int kStages = 2;
+    static constexpr int kCtas   = 3;
     static constexpr int kUnit   = Q ? 16 * Q : 8;              // bytes of an input's coefficients
     static constexpr int kData   = 256 * kCols;                 // 16 pairs x 16 bytes a column
     static constexpr int kCoef   = kData;                       // [q][column]
@@ -88,6 +91,121 @@ struct PairCfg {
     static constexpr int kSmem   = kPairWarps * kWarp;
 };
 
+template <int Q>
+constexpr int kPairAcc = Q ? 2 * Q : 1; // Q = 0: one, its two halves the two outputs; else [output][q]
+
+// one landed chunk (h outputs, nc inputs) into the lane's accumulators
+template <int Q>
+__device__ __forceinline__ void pair_chunk(const unsigned char *st, int h, int nc, int lane, DF2 (&acc)[kPairAcc<Q>]) {
+    using C      = PairCfg<Q>;
+    const int hp = (h + 1) >> 1, S = 32 / hp, slice = lane / hp;
+    if (slice < S) {
+        const float4 *data = reinterpret_cast<const float4 *>(st) + lane - slice * hp;
+        if constexpr (Q == 0) {
+            const float2 *cf = reinterpret_cast<const float2 *>(st + C::kCoef);
+#pragma unroll 4
+            for (int t = slice; t < nc; t += S) {
+                const float4 u = data[t * hp];
+                const float2 x = cf[t];
+                df2_fma(acc[0], fx(u.x, u.y), fx(u.z, u.w), fx(x.x, x.x), fx(x.y, x.y));
+            }
+        } else {
+            const float4 *cf = reinterpret_cast<const float4 *>(st + C::kCoef);
+#pragma unroll 2
+            for (int t = slice; t < nc; t += S) {
+                const float4 u = data[t * hp];
+                const f2x h0 = fx(u.x, u.x), h1 = fx(u.y, u.y), l0 = fx(u.z, u.z), l1 = fx(u.w, u.w);
+#pragma unroll
+                for (int q = 0; q < Q; q++) {
+                    const float4 x = cf[q * C::kCols + t];
+                    const f2x xh = fx(x.x, x.y), xl = fx(x.z, x.w);
+                    df2_fma(acc[q], h0, l0, xh, xl);
+                    df2_fma(acc[Q + q], h1, l1, xh, xl);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kPairAcc<Q>; i++)
+        df2_renorm(acc[i]);
+}
+
+// the slices' sums, in order, to the lanes of slice 0
+template <int Q>
+__device__ __forceinline__ void pair_slices(int h, int lane, DF2 (&acc)[kPairAcc<Q>]) {
+    const int hp = (h + 1) >> 1, S = 32 / hp;
+    for (int sl = 1; sl < S; sl++) {
+#pragma unroll
+        for (int i = 0; i < kPairAcc<Q>; i++) {
+            const int src = (lane + sl * hp) & 31;
+            DF2 o;
+            o.s = shfl2(acc[i].s, src);
+            o.c = shfl2(acc[i].c, src);
+            if (lane < hp)
+                acc[i] = df2_add(acc[i], o);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kPairAcc<Q>; i++)
+        df2_renorm(acc[i]);
+}
+
+// the sums of the outputs 2 pair, 2 pair + 1 of a panel to A (P1) or z
+template <int Q, bool P1>
+__device__ __forceinline__ void pair_store(int h, int out, int pair, const DF2 (&acc)[kPairAcc<Q>], const int *__restrict__ oslot, float *__restrict__ A, float2 *__restrict__ z, int zlen, int nrhs) {
+#pragma unroll
+    for (int o = 0; o < 2; o++) {
+        if (2 * pair + o >= h)
+            break;
+        if constexpr (Q == 0) {
+            const float2 vs = fx2(acc[0].s), vc = fx2(acc[0].c);
+            (P1 ? reinterpret_cast<float2 *>(A) + oslot[out + 2 * pair + o] : z + out + 2 * pair + o)[0] = o ? make_float2(vs.y, vc.y) : make_float2(vs.x, vc.x);
+        } else if constexpr (P1) {
+            float4 *A4 = reinterpret_cast<float4 *>(A) + (long long)Q * oslot[out + 2 * pair + o];
+#pragma unroll
+            for (int q = 0; q < Q; q++) {
+                const float2 vs = fx2(acc[o * Q + q].s), vc = fx2(acc[o * Q + q].c);
+                A4[q]           = make_float4(vs.x, vs.y, vc.x, vc.y);
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < Q; q++) {
+                const float2 vs = fx2(acc[o * Q + q].s), vc = fx2(acc[o * Q + q].c);
+                float2 *zr      = z + (long long)(2 * q) * zlen + out + 2 * pair + o;
+                if (2 * q < nrhs)
+                    zr[0] = make_float2(vs.x, vc.x);
+                if (2 * q + 1 < nrhs)
+                    zr[zlen] = make_float2(vs.y, vc.y);
+            }
+        }
+    }
+}
+
+// the copies of one chunk: columns jc .. jc + nc of panel p into stage st,
+// idx the coefficient index of this lane's column (phase 2)
+template <int Q, bool P1>
+__device__ __forceinline__ void pair_copies(const PairPanel &p, int jc, int nc, int idx, bool data, unsigned char *st, unsigned long long *bar, const unsigned char *mirror, const float *X,
+                                            const float *A, unsigned long long pol, int lane) {
+    using C      = PairCfg<Q>;
+    const int hp = (p.h + 1) >> 1;
+    if (lane == 0 && data)
+        ring_copy(st, mirror + p.src + (long long)16 * hp * jc, (unsigned)(16 * hp * nc), bar, pol);
+    if (lane < nc) {
+        const unsigned char *src;
+        if constexpr (P1)
+            src = reinterpret_cast<const unsigned char *>(X) + (long long)C::kUnit * (p.coef + jc + lane);
+        else
+            src = idx >= 0 ? reinterpret_cast<const unsigned char *>(A) + (long long)C::kUnit * idx : reinterpret_cast<const unsigned char *>(X) + (long long)C::kUnit * (~idx);
+        if constexpr (Q == 0) {
+            copy_async<8>(st + C::kCoef + 8 * lane, src);
+        } else {
+#pragma unroll
+            for (int q = 0; q < Q; q++)
+                copy_async<16>(st + C::kCoef + 16 * (q * C::kCols + lane), src + 16 * q);
+        }
+    }
+}
+
 // P1: coefficients are the rows of X from panel.coef on, sums go to the slots
 // oslot[panel.out ..] of A; else the coefficients cidx[panel.coef ..] name
 // slots of A (>= 0) or rows of X (~row), sums go to the rows panel.out .. of z
@@ -96,7 +214,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, PairCfg<Q>::kCtas)
     pair_kernel(const PairPanel *__restrict__ panels, int npanels, int *__restrict__ ticket, const unsigned char *__restrict__ mirror, const int *__restrict__ cidx, const int *__restrict__ oslot,
                 const float *__restrict__ X, float *__restrict__ A, float2 *__restrict__ z, int zlen, int nrhs, int *__restrict__ status) {
     using C             = PairCfg<Q>;
-    constexpr int kCols = C::kCols, kStages = C::kStages, kUnit = C::kUnit;
+    constexpr int kCols = C::kCols, kStages = C::kStages;
     extern __shared__ __align__(128) unsigned char smem[];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned char *wbase    = smem + (size_t)wid * C::kWarp;
@@ -116,11 +234,8 @@ __global__ void __launch_bounds__(32 * kPairWarps, PairCfg<Q>::kCtas)
     PairPanel cur{}, nxt{};
     if (icur < npanels)
         cur = panels[icur];
-    if (inxt < npanels) {
+    if (inxt < npanels)
         nxt = panels[inxt];
-        if (lane == 0)
-            tk = 2 * nwarps + atomicAdd(ticket, 1);
-    }
     int jc  = 0; // first column of cur not yet issued
     int idx = 0; // the coefficient index of column jc + lane
     auto load_idx = [&]() {
@@ -128,33 +243,19 @@ __global__ void __launch_bounds__(32 * kPairWarps, PairCfg<Q>::kCtas)
             idx = (icur < npanels && lane < kCols && jc + lane < cur.ncol) ? __ldg(cidx + cur.coef + jc + lane) : 0;
     };
     load_idx();
+    pdl_next();
+    pdl_wait(); // X, A and the ticket are the previous kernels'
+    if (inxt < npanels && lane == 0)
+        tk = 2 * nwarps + atomicAdd(ticket, 1);
     int issued = 0;
     auto issue = [&]() { // the next chunk into stage issued % kStages; an empty copy group when none is left
         if (icur < npanels) {
-            const int s  = issued % kStages;
-            const int hp = (cur.h + 1) >> 1;
-            const int nc = min(kCols, cur.ncol - jc);
+            const int s       = issued % kStages;
+            const int nc      = min(kCols, cur.ncol - jc);
             unsigned char *st = wbase + (size_t)s * C::kStage;
-            if (lane == 0) {
+            if (lane == 0)
                 *reinterpret_cast<int4 *>(st + C::kDesc) = make_int4(cur.h, nc, jc + nc == cur.ncol, cur.out);
-                const unsigned bytes                     = (unsigned)(16 * hp * nc);
-                if (!(icur == skip && jc == 0))
-                    ring_copy(st, mirror + cur.src + (long long)16 * hp * jc, bytes, &bar[s], pol);
-            }
-            if (lane < nc) {
-                const unsigned char *src;
-                if constexpr (P1)
-                    src = reinterpret_cast<const unsigned char *>(X) + (long long)kUnit * (cur.coef + jc + lane);
-                else
-                    src = idx >= 0 ? reinterpret_cast<const unsigned char *>(A) + (long long)kUnit * idx : reinterpret_cast<const unsigned char *>(X) + (long long)kUnit * (~idx);
-                if constexpr (Q == 0) {
-                    copy_async<8>(st + C::kCoef + 8 * lane, src);
-                } else {
-#pragma unroll
-                    for (int q = 0; q < Q; q++)
-                        copy_async<16>(st + C::kCoef + 16 * (q * kCols + lane), src + 16 * q);
-                }
-            }
+            pair_copies<Q, P1>(cur, jc, nc, idx, !(icur == skip && jc == 0), st, &bar[s], mirror, X, A, pol, lane);
             issued++;
             jc += nc;
             if (jc == cur.ncol) {
@@ -175,10 +276,9 @@ __global__ void __launch_bounds__(32 * kPairWarps, PairCfg<Q>::kCtas)
         copies_commit();
     };
 
-    constexpr int kAcc = Q ? 2 * Q : 1; // Q = 0: one, its two halves the two outputs; else [output][q]
-    DF2 acc[kAcc];
+    DF2 acc[kPairAcc<Q>];
 #pragma unroll
-    for (int i = 0; i < kAcc; i++)
+    for (int i = 0; i < kPairAcc<Q>; i++)
         acc[i].s = acc[i].c = 0ull;
 
 #pragma unroll
@@ -197,94 +297,13 @@ __global__ void __launch_bounds__(32 * kPairWarps, PairCfg<Q>::kCtas)
         __syncwarp();
         const unsigned char *st = wbase + (size_t)s * C::kStage;
         const int4 d            = *reinterpret_cast<const int4 *>(st + C::kDesc);
-        const int h = d.x, nc = d.y, hp = (h + 1) >> 1;
-        const int S     = 32 / hp;
-        const int slice = lane / hp, pair = lane - slice * hp;
-        if (slice < S) {
-            const float4 *data = reinterpret_cast<const float4 *>(st) + pair;
-            if constexpr (Q == 0) {
-                const float2 *cf = reinterpret_cast<const float2 *>(st + C::kCoef);
-#pragma unroll 4
-                for (int t = slice; t < nc; t += S) {
-                    const float4 u = data[t * hp];
-                    const float2 x = cf[t];
-                    df2_fma(acc[0], fx(u.x, u.y), fx(u.z, u.w), fx(x.x, x.x), fx(x.y, x.y));
-                }
-            } else {
-                const float4 *cf = reinterpret_cast<const float4 *>(st + C::kCoef);
-#pragma unroll 2
-                for (int t = slice; t < nc; t += S) {
-                    const float4 u = data[t * hp];
-                    const f2x h0 = fx(u.x, u.x), h1 = fx(u.y, u.y), l0 = fx(u.z, u.z), l1 = fx(u.w, u.w);
+        pair_chunk<Q>(st, d.x, d.y, lane, acc);
+        if (d.z) { // the panel's last chunk
+            pair_slices<Q>(d.x, lane, acc);
+            if (2 * lane < d.x)
+                pair_store<Q, P1>(d.x, d.w, lane, acc, oslot, A, z, zlen, nrhs);
 #pragma unroll
-                    for (int q = 0; q < Q; q++) {
-                        const float4 x = cf[q * kCols + t];
-                        const f2x xh = fx(x.x, x.y), xl = fx(x.z, x.w);
-                        df2_fma(acc[q], h0, l0, xh, xl);
-                        df2_fma(acc[Q + q], h1, l1, xh, xl);
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < kAcc; i++)
-            df2_renorm(acc[i]);
-        if (d.z) { // the panel's last chunk: slices summed in order, outputs written
-            for (int sl = 1; sl < S; sl++) {
-#pragma unroll
-                for (int i = 0; i < kAcc; i++) {
-                    const int src = (lane + sl * hp) & 31;
-                    DF2 o;
-                    o.s = shfl2(acc[i].s, src);
-                    o.c = shfl2(acc[i].c, src);
-                    if (slice == 0)
-                        acc[i] = df2_add(acc[i], o);
-                }
-            }
-            if (slice == 0) {
-#pragma unroll
-                for (int i = 0; i < kAcc; i++)
-                    df2_renorm(acc[i]);
-                if constexpr (Q == 0) {
-                    const float2 vs = fx2(acc[0].s), vc = fx2(acc[0].c);
-                    if constexpr (P1) {
-                        float2 *A2 = reinterpret_cast<float2 *>(A);
-                        A2[oslot[d.w + 2 * pair]] = make_float2(vs.x, vc.x);
-                        if (2 * pair + 1 < h)
-                            A2[oslot[d.w + 2 * pair + 1]] = make_float2(vs.y, vc.y);
-                    } else {
-                        z[d.w + 2 * pair] = make_float2(vs.x, vc.x);
-                        if (2 * pair + 1 < h)
-                            z[d.w + 2 * pair + 1] = make_float2(vs.y, vc.y);
-                    }
-                } else {
-#pragma unroll
-                    for (int o = 0; o < 2; o++) {
-                        if (2 * pair + o >= h)
-                            break;
-                        if constexpr (P1) {
-                            float4 *A4 = reinterpret_cast<float4 *>(A) + (long long)Q * oslot[d.w + 2 * pair + o];
-#pragma unroll
-                            for (int q = 0; q < Q; q++) {
-                                const float2 vs = fx2(acc[o * Q + q].s), vc = fx2(acc[o * Q + q].c);
-                                A4[q]           = make_float4(vs.x, vs.y, vc.x, vc.y);
-                            }
-                        } else {
-#pragma unroll
-                            for (int q = 0; q < Q; q++) {
-                                const float2 vs = fx2(acc[o * Q + q].s), vc = fx2(acc[o * Q + q].c);
-                                float2 *zr      = z + (long long)(2 * q) * zlen + d.w + 2 * pair + o;
-                                if (2 * q < nrhs)
-                                    zr[0] = make_float2(vs.x, vc.x);
-                                if (2 * q + 1 < nrhs)
-                                    zr[zlen] = make_float2(vs.y, vc.y);
-                            }
-                        }
-                    }
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < kAcc; i++)
+            for (int i = 0; i < kPairAcc<Q>; i++)
                 acc[i].s = acc[i].c = 0ull;
         }
         __syncwarp(); // every lane is done with the stage before it is refilled
@@ -300,11 +319,122 @@ __global__ void __launch_bounds__(32 * kPairWarps, PairCfg<Q>::kCtas)
     }
 }
 
+// The same sums with the four warps of a CTA on one panel: warp w takes the
+// chunks w, w + 4, .., its partial sums meet in shared memory, and the warps in
+// turn add a panel's four up and write them while the others go on.  For
+// products with so few panels that whole warps would wait on a few long ones.
+template <bool P1>
+__global__ void __launch_bounds__(32 * kPairWarps, PairCfg<0>::kCtas)
+    pair_coop_kernel(const PairPanel *__restrict__ panels, int npanels, const unsigned char *__restrict__ mirror, const int *__restrict__ cidx, const int *__restrict__ oslot,
+                     const float *__restrict__ X, float *__restrict__ A, float2 *__restrict__ z, int zlen, int nrhs, int *__restrict__ status) {
+    constexpr int Q     = 0; // one right-hand side
+    using C             = PairCfg<Q>;
+    constexpr int kCols = C::kCols, kStages = C::kStages;
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ DF2 part[2][kPairWarps][16][kPairAcc<Q>];
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    unsigned char *wbase    = smem + (size_t)wid * C::kWarp;
+    unsigned long long *bar = reinterpret_cast<unsigned long long *>(wbase + C::kBar);
+    if (lane == 0)
+        ring_init(bar, kStages);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    __syncwarp();
+    const unsigned long long pol = stream_policy();
+    const long long skip         = g_pair_skip;
+    // the next chunk to issue: columns jc .. of panel icur
+    int icur = blockIdx.x, jc = wid * kCols, idx = 0, issued = 0;
+    PairPanel cur{};
+    auto seek = [&]() { // to the first panel from icur on with a chunk for this warp
+        while (icur < npanels) {
+            cur = panels[icur];
+            if (jc < cur.ncol)
+                break;
+            icur += gridDim.x;
+            jc = wid * kCols;
+        }
+        if constexpr (!P1)
+            idx = (icur < npanels && lane < kCols && jc + lane < cur.ncol) ? __ldg(cidx + cur.coef + jc + lane) : 0;
+    };
+    seek();
+    pdl_next();
+    pdl_wait(); // X and A are the previous kernels'
+    auto issue = [&]() {
+        if (icur < npanels) {
+            const int s  = issued % kStages;
+            const int nc = min(kCols, cur.ncol - jc);
+            pair_copies<Q, P1>(cur, jc, nc, idx, !(icur == skip && jc == 0), wbase + (size_t)s * C::kStage, &bar[s], mirror, X, A, pol, lane);
+            issued++;
+            jc += kPairWarps * kCols;
+            if (jc < cur.ncol) {
+                if constexpr (!P1)
+                    idx = (lane < kCols && jc + lane < cur.ncol) ? __ldg(cidx + cur.coef + jc + lane) : 0;
+            } else {
+                icur += gridDim.x;
+                jc = wid * kCols;
+                seek();
+            }
+        }
+        copies_commit();
+    };
+#pragma unroll
+    for (int s = 0; s < kStages - 1; s++)
+        issue();
+    bool ok  = true;
+    int done = 0, turn = 0;
+    for (int p = blockIdx.x; p < npanels; p += gridDim.x, turn++) {
+        const PairPanel d = panels[p];
+        DF2 acc[kPairAcc<Q>];
+#pragma unroll
+        for (int i = 0; i < kPairAcc<Q>; i++)
+            acc[i].s = acc[i].c = 0ull;
+        for (int j = wid * kCols; j < d.ncol && ok; j += kPairWarps * kCols) {
+            const int s = done % kStages;
+            issue();
+            copies_wait<kStages - 1>();
+            if (!warp_wait_phase(&bar[s], (done / kStages) & 1)) { // the warp goes on to every barrier of the CTA, without its chunks
+                ok = false;
+                break;
+            }
+            __syncwarp();
+            pair_chunk<Q>(wbase + (size_t)s * C::kStage, d.h, min(kCols, d.ncol - j), lane, acc);
+            __syncwarp();
+            done++;
+        }
+        pair_slices<Q>(d.h, lane, acc);
+        if (2 * lane < d.h)
+#pragma unroll
+            for (int i = 0; i < kPairAcc<Q>; i++)
+                part[turn & 1][wid][lane][i] = acc[i];
+        __syncthreads();
+        if ((turn & 3) == wid && 2 * lane < d.h) {
+#pragma unroll
+            for (int i = 0; i < kPairAcc<Q>; i++) {
+                acc[i] = part[turn & 1][0][lane][i];
+#pragma unroll
+                for (int w = 1; w < kPairWarps; w++)
+                    acc[i] = df2_add(acc[i], part[turn & 1][w][lane][i]);
+                df2_renorm(acc[i]);
+            }
+            pair_store<Q, P1>(d.h, d.out, lane, acc, oslot, A, z, zlen, nrhs);
+        }
+    }
+    copies_wait<0>();
+    if (!ok) {
+        if (lane == 0)
+            atomicExch(status, 2);
+        for (int p = done; p < issued; p++)
+            if (!warp_wait_phase(&bar[p % kStages], (p / kStages) & 1) && lane == 0)
+                atomicExch(status, 3);
+    }
+}
+
 // the gathered input of right-hand sides c0 .. c0 + w (those past mu_src
 // zero), split relative to the input's largest exponent: [row][q] of
 // {hi, hi, lo, lo}, w = 1: [row] of (hi, lo); also clears the three tickets
 __global__ void pair_gather_kernel(const double *__restrict__ x, int ldx, const int *__restrict__ perm, int n, int c0, int w, int mu_src, const int *__restrict__ xexp, float *__restrict__ X,
                                    int *__restrict__ tickets) {
+    pdl_next();
+    pdl_wait();
     if (blockIdx.x == 0 && threadIdx.x < 3)
         tickets[threadIdx.x] = 0;
     const int shift = 1023 - max(*xexp, 1);
@@ -336,10 +466,13 @@ __global__ void pair_gather_kernel(const double *__restrict__ x, int ldx, const 
 // the tiles' sums of every multi-tile leaf into the first tile's slots
 __global__ void pair_reduce_kernel(const LrLeaf *__restrict__ lr, const int *__restrict__ multi, int w, float *__restrict__ A) {
     const LrLeaf L = lr[multi[blockIdx.x]];
+    pdl_next();
+    pdl_wait();
     if (w == 1) {
         float2 *base = reinterpret_cast<float2 *>(A) + L.a_off;
         for (int e = threadIdx.x; e < L.r; e += blockDim.x) {
             DF a{base[e].x, base[e].y};
+#pragma unroll 8
             for (int ch = 1; ch < L.nch; ch++) {
                 const float2 v = base[(long long)ch * L.r + e];
                 a              = df_add(a, DF{v.x, v.y});
@@ -354,6 +487,7 @@ __global__ void pair_reduce_kernel(const LrLeaf *__restrict__ lr, const int *__r
     for (int e = threadIdx.x; e < L.r * Q; e += blockDim.x) {
         const float4 v = base[e];
         DF2 a{fx(v.x, v.y), fx(v.z, v.w)};
+#pragma unroll 8
         for (int ch = 1; ch < L.nch; ch++) {
             const float4 u = base[(long long)ch * L.r * Q + e];
             a              = df2_add(a, DF2{fx(u.x, u.y), fx(u.z, u.w)});
@@ -367,6 +501,8 @@ __global__ void pair_reduce_kernel(const LrLeaf *__restrict__ lr, const int *__r
 // native complex layout: i times the sums (re, im) of every slot pair
 __global__ void pair_rotate_kernel(const int2 *__restrict__ rows, long long nrows, int Q, float4 *__restrict__ A) {
     const long long total = nrows * Q;
+    pdl_next();
+    pdl_wait();
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
         const int2 p               = rows[e / Q];
         const int q                = (int)(e % Q);
@@ -381,22 +517,34 @@ __global__ void pair_zsum_kernel(const ZItem *__restrict__ items, int nitems, co
                                  const int *__restrict__ xexp, double *__restrict__ y, int ldy, int shift) {
     const int w    = blockIdx.x * 8 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
+    pdl_next();
     if (w >= nitems)
         return;
     const ZItem it = items[w];
-    const int xs   = max(*xexp, 1) - 1023;
-    const int n    = it.h * mu;
-    for (int e = lane; e < n; e += 32) {
-        const int c = e / it.h, i = it.row0 + e - c * it.h;
+    // the atom's z bases, one per lane (more than 32 covering clusters: read again)
+    const int nl = it.lend - it.lbeg, base = lane < nl ? zl[it.lbeg + lane] : 0;
+    pdl_wait();
+    const int xs = max(*xexp, 1) - 1023;
+    const int n  = it.h * mu;
+    for (int e0 = 0; e0 < n; e0 += 32) {
+        const int e = min(e0 + lane, n - 1), c = e / it.h, i = it.row0 + e - c * it.h;
+        const float2 *zc = z + (long long)c * zlen + i;
         DF a{0.f, 0.f};
-        for (int l = it.lbeg; l < it.lend; l++) {
-            const float2 v = z[(long long)c * zlen + i + zl[l]];
+#pragma unroll 8
+        for (int l = 0; l < min(nl, 32); l++) {
+            const float2 v = zc[__shfl_sync(0xffffffffu, base, l)];
+            a              = df_add(a, DF{v.x, v.y});
+            df_renorm(a);
+        }
+        for (int l = it.lbeg + 32; l < it.lend; l++) {
+            const float2 v = zc[zl[l]];
             a              = df_add(a, DF{v.x, v.y});
             df_renorm(a);
         }
         const double v = df_to_double(a);
         // NaN stays NaN through the scaling (an exponent field of 0x7FF has no room)
-        y[(long long)c * ldy + (perm ? perm[i] : i - shift)] = v == v ? scale_pow2_safe(v, xs) : v;
+        if (e0 + lane < n)
+            y[(long long)c * ldy + (perm ? perm[i] : i - shift)] = v == v ? scale_pow2_safe(v, xs) : v;
     }
 }
 
@@ -405,8 +553,9 @@ __global__ void pair_zsum_kernel(const ZItem *__restrict__ items, int nitems, co
 // target cluster's row-chunk panels (pan0 .. of m rows in all)
 __global__ void pair_pack2_kernel(const PairPanel *__restrict__ panels, const PairSource *__restrict__ srcs, int npanels, const PanelItem *__restrict__ pan, const double *__restrict__ fac,
                                   unsigned char *__restrict__ mirror) {
-    const int lane = threadIdx.x & 31, nw = gridDim.x * (blockDim.x >> 5);
-    for (int p = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); p < npanels; p += nw) {
+    // a CTA per panel, its warps on slabs of 32 inputs
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    for (int p = blockIdx.x; p < npanels; p += gridDim.x) {
         const PairPanel d  = panels[p];
         const PairSource s = srcs[p];
         const int hp       = (d.h + 1) >> 1;
@@ -418,12 +567,13 @@ __global__ void pair_pack2_kernel(const PairPanel *__restrict__ panels, const Pa
         const PanelItem pi = pan[s.pan0 + q];
         const double *row  = fac + pi.off + (i - (long long)s.m * q / nchunk);
         float *dst         = reinterpret_cast<float *>(mirror + d.src) + 4 * (lane >> 1) + (lane & 1);
-#pragma unroll 4
-        for (int k = 0; k < d.ncol; k++) {
-            const F2 f            = split64_near(live ? row[(long long)pi.h * k] : 0.);
-            dst[4LL * hp * k]     = f.hi;
-            dst[4LL * hp * k + 2] = f.lo;
-        }
+        for (int k0 = 32 * (threadIdx.x >> 5); k0 < d.ncol; k0 += 32 * nw)
+#pragma unroll 8
+            for (int k = k0; k < min(k0 + 32, d.ncol); k++) {
+                const F2 f            = split64_near(live ? row[(long long)pi.h * k] : 0.);
+                dst[4LL * hp * k]     = f.hi;
+                dst[4LL * hp * k + 2] = f.lo;
+            }
     }
 }
 
@@ -432,12 +582,12 @@ __global__ void pair_pack2_kernel(const PairPanel *__restrict__ panels, const Pa
 __global__ void __launch_bounds__(128) pair_pack1_kernel(const PairPanel *__restrict__ panels, int npanels, const long long *__restrict__ osrc, const double *__restrict__ fac,
                                                          unsigned char *__restrict__ mirror) {
     __shared__ float2 tile[4][32][33];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = gridDim.x * 4;
-    for (int p = blockIdx.x * 4 + wid; p < npanels; p += nw) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (int p = blockIdx.x; p < npanels; p += gridDim.x) {
         const PairPanel d       = panels[p];
         const int hp            = (d.h + 1) >> 1;
         const long long my_src = lane < d.h ? osrc[d.out + lane] : 0;
-        for (int k0 = 0; k0 < d.ncol; k0 += 32) {
+        for (int k0 = 32 * wid; k0 < d.ncol; k0 += 128) {
             const int nk = min(32, d.ncol - k0);
             __syncwarp();
 #pragma unroll 8
@@ -477,9 +627,23 @@ void launch_pair_q(const PairPanel *panels, int npanels, int *ticket, const unsi
         if (dev < 64)
             done |= 1ull << dev;
     }
-    const int nctas = std::min(PairCfg<Q>::kCtas * pair_sms(), (npanels + kPairWarps - 1) / kPairWarps);
-    pair_kernel<Q, P1><<<nctas, 32 * kPairWarps, PairCfg<Q>::kSmem, st>>>(panels, npanels, ticket, mirror, cidx, oslot, X, A, z, zlen, nrhs, status);
-    HTGPU_CUDA(cudaGetLastError());
+    const int resident = PairCfg<Q>::kCtas * pair_sms();
+    // one right-hand side and fewer than two panels a CTA: four warps to a
+    // panel (4 000 points 0.055 -> 0.046 ms a product; no gain from 10 000 points
+    // or with more right-hand sides, whose panels take the warps longer)
+    if constexpr (Q == 0)
+        if (npanels < 2 * resident) {
+            static unsigned long long donec = 0;
+            if (dev >= 64 || !(donec >> dev & 1)) {
+                HTGPU_CUDA(cudaFuncSetAttribute(pair_coop_kernel<P1>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<0>::kSmem));
+                if (dev < 64)
+                    donec |= 1ull << dev;
+            }
+            pdl_launch(pair_coop_kernel<P1>, std::min(resident, npanels), 32 * kPairWarps, PairCfg<0>::kSmem, st, panels, npanels, mirror, cidx, oslot, X, A, z, zlen, nrhs, status);
+            return;
+        }
+    const int nctas = std::min(resident, (npanels + kPairWarps - 1) / kPairWarps);
+    pdl_launch(pair_kernel<Q, P1>, nctas, 32 * kPairWarps, PairCfg<Q>::kSmem, st, panels, npanels, ticket, mirror, cidx, oslot, X, A, z, zlen, nrhs, status);
 }
 
 template <bool P1>
@@ -510,8 +674,7 @@ int pair_pass_width(int left, bool exact) {
 void launch_pair_gather(const double *x, int ldx, const int *perm, int n, int c0, int w, int mu_src, const int *xexp, float *X, int *tickets, cudaStream_t st) {
     const long long total = (long long)n * (w == 1 ? 1 : w >> 1);
     const int blocks      = (int)std::max<long long>(1, std::min<long long>((total + 255) / 256, 16LL * pair_sms()));
-    pair_gather_kernel<<<blocks, 256, 0, st>>>(x, ldx, perm, n, c0, w, mu_src, xexp, X, tickets);
-    HTGPU_CUDA(cudaGetLastError());
+    pdl_launch(pair_gather_kernel, blocks, 256, 0, st, x, ldx, perm, n, c0, w, mu_src, xexp, X, tickets);
 }
 
 void launch_pair_phase1(const PairPanel *panels, int npanels, int *tickets, const unsigned char *mirror, const int *oslot, const float *X, float *A, int w, int *status, cudaStream_t st) {
@@ -526,8 +689,7 @@ void launch_pair_phase2(const PairPanel *panels, int npanels, int *tickets, cons
 void launch_pair_reduce(const LrLeaf *lr, const int *multi, int nmulti, int w, float *A, cudaStream_t st) {
     if (nmulti <= 0)
         return;
-    pair_reduce_kernel<<<nmulti, 128, 0, st>>>(lr, multi, w, A);
-    HTGPU_CUDA(cudaGetLastError());
+    pdl_launch(pair_reduce_kernel, nmulti, 128, 0, st, lr, multi, w, A);
 }
 
 void launch_pair_rotate(const int2 *rows, long long nrows, int w, float *A, cudaStream_t st) {
@@ -535,24 +697,22 @@ void launch_pair_rotate(const int2 *rows, long long nrows, int w, float *A, cuda
     const long long total = nrows * (w >> 1);
     if (total <= 0)
         return;
-    pair_rotate_kernel<<<(int)std::min<long long>((total + 255) / 256, 4096), 256, 0, st>>>(rows, nrows, w >> 1, reinterpret_cast<float4 *>(A));
-    HTGPU_CUDA(cudaGetLastError());
+    pdl_launch(pair_rotate_kernel, (int)std::min<long long>((total + 255) / 256, 4096), 256, 0, st, rows, nrows, w >> 1, reinterpret_cast<float4 *>(A));
 }
 
 void launch_pair_zsum(const ZItem *items, int nitems, const int *zl, const float2 *z, int zlen, int mu, const int *perm, const int *xexp, double *y, int ldy, cudaStream_t st, int shift) {
     if (nitems <= 0)
         return;
-    pair_zsum_kernel<<<(nitems + 7) / 8, 256, 0, st>>>(items, nitems, zl, z, zlen, mu, perm, xexp, y, ldy, shift);
-    HTGPU_CUDA(cudaGetLastError());
+    pdl_launch(pair_zsum_kernel, (nitems + 7) / 8, 256, 0, st, items, nitems, zl, z, zlen, mu, perm, xexp, y, ldy, shift);
 }
 
 void launch_pair_pack(const PairPanel *p1, int np1, const long long *osrc, const PairPanel *p2, const PairSource *s2, int np2, const PanelItem *pan, const double *fac, unsigned char *mirror,
                       cudaStream_t st) {
     const int most = 16 * pair_sms();
     if (np1 > 0)
-        pair_pack1_kernel<<<std::min(most, (np1 + 3) / 4), 128, 0, st>>>(p1, np1, osrc, fac, mirror);
+        pair_pack1_kernel<<<std::min(most, np1), 128, 0, st>>>(p1, np1, osrc, fac, mirror);
     if (np2 > 0)
-        pair_pack2_kernel<<<std::min(most, (np2 + 7) / 8), 256, 0, st>>>(p2, s2, np2, pan, fac, mirror);
+        pair_pack2_kernel<<<std::min(most, np2), 128, 0, st>>>(p2, s2, np2, pan, fac, mirror);
     HTGPU_CUDA(cudaGetLastError());
 }
 

@@ -119,11 +119,12 @@ __global__ void __launch_bounds__(32 * kRedWarps, Red1Cfg<W>::kCtas)
     RedPanel cur{}, nxt{};
     if (icur < npanels)
         cur = panels[icur];
-    if (inxt < npanels) {
+    if (inxt < npanels)
         nxt = panels[inxt];
-        if (lane == 0)
-            tk = 2 * nwarps + atomicAdd(ticket, 1);
-    }
+    pdl_next();
+    pdl_wait(); // X and the ticket are the previous kernels'
+    if (inxt < npanels && lane == 0)
+        tk = 2 * nwarps + atomicAdd(ticket, 1);
     int jc = 0, issued = 0;
     auto issue = [&]() {
         if (icur < npanels) {
@@ -290,9 +291,11 @@ __global__ void __launch_bounds__(32 * kRedWarps, Red2Cfg<W>::kCtas)
     if (inxt < nranges) {
         nk = rbeg[inxt];
         ne = rbeg[inxt + 1];
-        if (lane == 0)
-            tk = 2 * nwarps + atomicAdd(ticket, 1);
     }
+    pdl_next();
+    pdl_wait(); // A, z and the ticket are the previous kernels'
+    if (inxt < nranges && lane == 0)
+        tk = 2 * nwarps + atomicAdd(ticket, 1);
     auto step = [&]() { // (k, e) to the chunk after k; false at the end
         if (++k < e)
             return true;
@@ -509,7 +512,9 @@ __global__ void __launch_bounds__(32 * kRedWarps, Red2Cfg<W>::kCtas)
 __global__ void red_gather_kernel(const double *__restrict__ x, int ldx, const int *__restrict__ perm, int n, int c0, int w, int mu_src, const int *__restrict__ xexp, int hi_only,
                                   float *__restrict__ out) {
     const long long total = (long long)n * w;
-    const int shift       = 1023 - max(*xexp, 1);
+    pdl_next();
+    pdl_wait();
+    const int shift = 1023 - max(*xexp, 1);
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
         const int j = (int)(e / w), c = c0 + (int)(e - (long long)j * w);
         const double v = c < mu_src ? x[(long long)c * ldx + (perm ? perm[j] : j)] : 0.;
@@ -586,8 +591,7 @@ void launch_red1_w(const RedPanel *panels, int npanels, int *ticket, const unsig
     static unsigned long long done = 0; // devices whose shared-memory limit was raised
     red_smem(red1_kernel<W>, Red1Cfg<W>::kSmem, done);
     const int nctas = std::min(Red1Cfg<W>::kCtas * red_sms(), (npanels + kRedWarps - 1) / kRedWarps);
-    red1_kernel<W><<<nctas, 32 * kRedWarps, Red1Cfg<W>::kSmem, st>>>(panels, npanels, ticket, mirror, outs, scale, X, A, status);
-    HTGPU_CUDA(cudaGetLastError());
+    pdl_launch(red1_kernel<W>, nctas, 32 * kRedWarps, Red1Cfg<W>::kSmem, st, panels, npanels, ticket, mirror, outs, scale, X, A, status);
 }
 
 template <int W>
@@ -596,8 +600,7 @@ void launch_red2_w(const StreamChunk *chunks, const int *rbeg, int nranges, int 
     static unsigned long long done = 0;
     red_smem(red2_kernel<W>, Red2Cfg<W>::kSmem, done);
     const int nctas = std::min(Red2Cfg<W>::kCtas * red_sms(), (nranges + kRedWarps - 1) / kRedWarps);
-    red2_kernel<W><<<nctas, 32 * kRedWarps, Red2Cfg<W>::kSmem, st>>>(chunks, rbeg, nranges, ticket, mix, cidx, A, z, zlen, nrhs, status);
-    HTGPU_CUDA(cudaGetLastError());
+    pdl_launch(red2_kernel<W>, nctas, 32 * kRedWarps, Red2Cfg<W>::kSmem, st, chunks, rbeg, nranges, ticket, mix, cidx, A, z, zlen, nrhs, status);
 }
 
 } // namespace
@@ -605,8 +608,7 @@ void launch_red2_w(const StreamChunk *chunks, const int *rbeg, int nranges, int 
 void launch_red_gather(const double *x, int ldx, const int *perm, int n, int c0, int w, int mu_src, const int *xexp, bool hi_only, float *out, cudaStream_t st) {
     const long long total = (long long)n * w;
     const int blocks      = (int)std::max<long long>(1, std::min<long long>((total + 255) / 256, 16LL * red_sms()));
-    red_gather_kernel<<<blocks, 256, 0, st>>>(x, ldx, perm, n, c0, w, mu_src, xexp, hi_only, out);
-    HTGPU_CUDA(cudaGetLastError());
+    pdl_launch(red_gather_kernel, blocks, 256, 0, st, x, ldx, perm, n, c0, w, mu_src, xexp, hi_only, out);
 }
 
 void launch_red_phase1(const RedPanel *panels, int npanels, int *ticket, const unsigned char *mirror, const int2 *outs, const float *scale, const float *X, float *A, int w, int *status, cudaStream_t st) {

@@ -99,10 +99,11 @@ def test_choices_of_the_caller_leave_the_panels_and_autotune_returns():
     assert np.array_equal(hm.mvprod_global_to_global(x, 2), y)
 
 
-def test_a_wait_that_runs_out_is_reported():
+# 1500: four warps to a panel; 12000: a warp each
+@pytest.mark.parametrize("n", [1500, 12000])
+def test_a_wait_that_runs_out_is_reported(n):
     """a panel whose first copy never comes: the status reports it, a
     host-pointer product fails, and the next product is the one before"""
-    n = 6000
     pts = G.sphere(n, seed=11)
     t = H.Cluster().build(n, pts)
     hm = H.HMatrix(t, t, 1e-6, 10.0).build(H.LAPLACE, pts)
