@@ -118,20 +118,96 @@ struct BlockReduce {
 constexpr int kAcaThreads = 128;
 constexpr int kDotChunk   = 32; // estimator dot products reduced per pass
 
-// One CTA per block.  Scratch columns: U_s[:, k] (length M) and Vt_s[:, k]
-// (length N) hold the k-th cross c_k and r_k of partialACA.
-__global__ void __launch_bounds__(kAcaThreads) partial_aca_kernel(const AcaBlock *__restrict__ blocks, const double *__restrict__ xt, const double *__restrict__ xs, const int *__restrict__ perm_t,
-                                                                   const int *__restrict__ perm_s, KernelDesc kd, double eps, double *__restrict__ scratch, unsigned char *__restrict__ flags,
-                                                                   int *__restrict__ rank_out) {
-    constexpr int NT = kAcaThreads;
-    __shared__ double sv[NT / 32];
-    __shared__ int si[NT / 32];
-    __shared__ double sdot[NT / 32][kDotChunk];
-    __shared__ double sres[kDotChunk];
-    __shared__ double sacc[3]; // |c.c||r.r|, sum_p (vv_p.r)(uu_p.c), pending (vv_p.r)
+// The pivot searches as integers: the magnitude's bits order like the numbers
+// (comparing doubles runs on the FP64 pipe). -1 no candidate, 0 a NaN (it
+// loses to any number), else the bits of |v| plus one; ties go to the larger
+// index, the "last maximum" of htool's sequential loops.
+__device__ __forceinline__ long long pivot_key(double v) {
+    const long long b = __double_as_longlong(v) & 0x7fffffffffffffffll;
+    return b > 0x7ff0000000000000ll ? 0 : b + 1;
+}
 
-    const AcaBlock B = blocks[blockIdx.x];
-    const int M = B.M, N = B.N, tid = threadIdx.x;
+// partialACA of one block by a group of NT threads (a warp, or a CTA).
+// Scratch columns: U_s[:, k] (length M) and Vt_s[:, k] (length N) hold the
+// k-th cross c_k and r_k.
+//
+// FP64 work is bound by its pipe (two lanes a clock and SM), where a warp
+// instruction costs as much for one active lane as for 32: so small blocks go
+// one warp each, the sums of the Frobenius estimator are reduce-scattered eight
+// at a time (9 warp additions instead of 40), with multiply-adds, and only
+// the first warp turns them into the stopping test; the pivots are compared
+// as integers.  Laplace sphere, 50 000 points: the 82 442 blocks 32.3 -> 15.5
+// ms of kernels (CTAs of 128 threads for every block before).
+template <int NT>
+struct AcaShared {
+    long long key[2][NT / 32];
+    int idx[2][NT / 32];
+    double dot[NT / 32][104]; // dots of one cross: 8 per group of four earlier crosses, then c.c and r.r
+    double aux, frob;
+    int go;
+};
+
+template <int NT>
+__device__ __forceinline__ void aca_sync() {
+    if constexpr (NT == 32)
+        __syncwarp();
+    else
+        __syncthreads();
+}
+
+// the group's largest key and its index, to every thread
+template <int NT>
+__device__ __forceinline__ void aca_argmax(long long &key, int &idx, int buf, AcaShared<NT> &sm) {
+    auto take = [&](long long k, int i) {
+        if (k > key || (k == key && i > idx)) {
+            key = k;
+            idx = i;
+        }
+    };
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const long long k = __shfl_xor_sync(0xffffffffu, key, o);
+        const int i       = __shfl_xor_sync(0xffffffffu, idx, o);
+        take(k, i);
+    }
+    if constexpr (NT == 32) {
+        __syncwarp();
+    } else {
+        if ((threadIdx.x & 31) == 0) {
+            sm.key[buf][threadIdx.x >> 5] = key;
+            sm.idx[buf][threadIdx.x >> 5] = idx;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < NT / 32; w++)
+            take(sm.key[buf][w], sm.idx[buf][w]);
+    }
+}
+
+// eight per-lane values summed over the warp: lane l ends with the sum of
+// value 4 (l >> 4 & 1) + 2 (l >> 3 & 1) + (l >> 2 & 1); fixed order
+__device__ __forceinline__ double reduce_scatter8(double (&v)[8], int lane) {
+    double w[4], x[2];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const double keep = lane & 16 ? v[i + 4] : v[i], send = lane & 16 ? v[i] : v[i + 4];
+        w[i]              = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const double keep = lane & 8 ? w[i + 2] : w[i], send = lane & 8 ? w[i] : w[i + 2];
+        x[i]              = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+    }
+    const double keep = lane & 4 ? x[1] : x[0], send = lane & 4 ? x[0] : x[1];
+    double y          = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+    y                 = y + __shfl_xor_sync(0xffffffffu, y, 2);
+    return y + __shfl_xor_sync(0xffffffffu, y, 1);
+}
+
+template <int NT>
+__device__ int aca_block(const AcaBlock &B, int tid, AcaShared<NT> &sm, const double *__restrict__ xt, const double *__restrict__ xs, const int *__restrict__ perm_t,
+                         const int *__restrict__ perm_s, const KernelDesc &kd, double eps, double *__restrict__ scratch, unsigned char *__restrict__ flags) {
+    const int M = B.M, N = B.N, lane = tid & 31, warp = tid >> 5;
     const int *rows = perm_t + B.row_off;
     const int *cols = perm_s + B.col_off;
     double *U       = scratch + B.u_off;
@@ -142,166 +218,197 @@ __global__ void __launch_bounds__(kAcaThreads) partial_aca_kernel(const AcaBlock
     for (int i = tid; i < M + N; i += NT)
         vrow[i] = 0;
 
-    // first pivot row: the point closest to the target centre (first minimum)
-    double best = 1e300;
-    int I       = 0x7fffffff;
+    // first pivot row: the point closest to the target centre (first minimum:
+    // the largest key of the distances' complements, ties to the smaller index)
+    long long key = -1;
+    int I         = -1;
     for (int i = tid; i < M; i += NT) {
         const double *p = xt + 3 * (size_t)rows[i];
         double s        = 0.;
         for (int d = 0; d < 3; d++)
             s = s + (p[d] - B.ctr[d]) * (p[d] - B.ctr[d]);
-        double ad = sqrt(s);
-        if (ad < best) {
-            best = ad;
-            I    = i;
+        const double ad = sqrt(s);
+        if (!(ad < 1e30)) // htool starts from dist = 1e30 and row 0
+            continue;
+        const long long k = 0x7fffffffffffffffll - __double_as_longlong(ad);
+        if (k > key) {
+            key = k;
+            I   = -1 - i;
         }
     }
-    BlockReduce<NT>::argmin(best, I, sv, si);
-    if (!(best < 1e30))
-        I = 0; // htool starts from dist = 1e30 and row 0
+    aca_argmax<NT>(key, I, 0, sm);
+    I = key < 0 ? 0 : -1 - I;
 
     // q * (M + N) > M * N evaluated with 32-bit int products, as upstream
     const int MN32 = (int)((unsigned)M * (unsigned)N);
     int q          = 0;
-    double frob = 0., aux = 0.;
+    double frob    = 0.; // the first warp's
     while (true) {
-        if (!(q == 0 || sqrt(aux / frob) > eps))
-            break;
         q += 1;
-        if ((int)((unsigned)q * (unsigned)(M + N)) > MN32) {
-            q = -1;
-            break;
-        }
-        if (q > B.cap) {
-            q = -2;
-            break;
-        }
+        if ((int)((unsigned)q * (unsigned)(M + N)) > MN32)
+            return -1;
+        if (q > B.cap)
+            return -2;
         const int k = q - 1;
+        if (tid == 0)
+            vrow[I] = 1;
         // ---- row I of the residual -> Vt_s[:, k]
         const double *pI = xt + 3 * (size_t)rows[I];
-        double piv       = -1.;
+        long long piv    = -1;
         int J            = -1;
         for (int j = tid; j < N; j += NT) {
             double v = kernel_entry(kd, pI, xs + 3 * (size_t)cols[j]);
+#pragma unroll 4
             for (int p = 0; p < k; p++)
                 v = fma(-U[I + (size_t)M * p], Vt[j + (size_t)N * p], v);
             Vt[j + (size_t)N * k] = v;
             if (!vcol[j]) {
-                double a = fabs(v);
-                if (!(a < piv)) {
+                const long long a = pivot_key(v);
+                if (a >= piv) {
                     piv = a;
                     J   = j;
                 }
             }
         }
-        BlockReduce<NT>::argmax(piv, J, sv, si);
-        if (J < 0) { // no admissible pivot column (only with non-finite entries)
-            q = q - 1 == 0 ? -1 : q - 1;
-            break;
-        }
-        if (tid == 0)
-            vrow[I] = 1;
-        __syncthreads();
+        aca_argmax<NT>(piv, J, 1, sm);
+        if (J < 0) // no admissible pivot column (only with non-finite entries)
+            return q - 1 == 0 ? -1 : q - 1;
         const double rJ = Vt[J + (size_t)N * k];
-        if (fabs(rJ) > 1e-15) {
-            const double gamma = 1. / rJ;
-            // ---- column J of the residual, scaled -> U_s[:, k]
-            const double *pJ = xs + 3 * (size_t)cols[J];
-            double piv2      = -1.;
-            int I2           = -1;
-            for (int i = tid; i < M; i += NT) {
-                double v = kernel_entry(kd, xt + 3 * (size_t)rows[i], pJ);
-                for (int p = 0; p < k; p++)
-                    v = fma(-Vt[J + (size_t)N * p], U[i + (size_t)M * p], v);
-                v                    = v * gamma;
-                U[i + (size_t)M * k] = v;
-                if (!vrow[i]) {
-                    double a = fabs(v);
-                    if (!(a < piv2)) {
-                        piv2 = a;
-                        I2   = i;
-                    }
+        if (!(fabs(rJ) > 1e-15))
+            return q - 1 == 0 ? -1 : q - 1;
+        if (tid == 0)
+            vcol[J] = 1;
+        const double gamma = 1. / rJ;
+        // ---- column J of the residual, scaled -> U_s[:, k]
+        const double *pJ = xs + 3 * (size_t)cols[J];
+        long long piv2   = -1;
+        int I2           = -1;
+        for (int i = tid; i < M; i += NT) {
+            double v = kernel_entry(kd, xt + 3 * (size_t)rows[i], pJ);
+#pragma unroll 4
+            for (int p = 0; p < k; p++)
+                v = fma(-Vt[J + (size_t)N * p], U[i + (size_t)M * p], v);
+            v                    = v * gamma;
+            U[i + (size_t)M * k] = v;
+            if (!vrow[i]) {
+                const long long a = pivot_key(v);
+                if (a >= piv2) {
+                    piv2 = a;
+                    I2   = i;
                 }
             }
-            BlockReduce<NT>::argmax(piv2, I2, sv, si);
-            if (I2 < 0) { // no pivot row left (only with non-finite entries)
-                break;
-            }
-            if (tid == 0)
-                vcol[J] = 1;
-            // ---- Frobenius estimator (partialACA.hpp:127-141), in chunks of
-            // 32 dot products: c.c, r.r, then (vv_p . r), (uu_p . c) for p < k
-            const int nd = 2 + 2 * k;
-            const int lane = tid & 31, warp = tid >> 5;
-            if (tid == 0)
-                sacc[1] = 0.;
-            for (int d0 = 0; d0 < nd; d0 += kDotChunk) {
-                const int dn = min(kDotChunk, nd - d0);
-                for (int dd = 0; dd < dn; dd++) {
-                    const int d = d0 + dd;
-                    double s    = 0.;
-                    if (d == 0) {
-                        for (int i = tid; i < M; i += NT) {
-                            double c = U[i + (size_t)M * k];
-                            s        = s + c * c;
-                        }
-                    } else if (d == 1) {
-                        for (int j = tid; j < N; j += NT) {
-                            double r = Vt[j + (size_t)N * k];
-                            s        = s + r * r;
-                        }
-                    } else if (d & 1) { // (vv_p . r), p = (d - 3) / 2
-                        int p = (d - 2) >> 1;
-                        for (int j = tid; j < N; j += NT)
-                            s = s + Vt[j + (size_t)N * p] * Vt[j + (size_t)N * k];
-                    } else { // (uu_p . c), p = (d - 2) / 2
-                        int p = (d - 2) >> 1;
-                        for (int i = tid; i < M; i += NT)
-                            s = s + U[i + (size_t)M * p] * U[i + (size_t)M * k];
-                    }
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1)
-                        s = s + __shfl_down_sync(0xffffffffu, s, o);
-                    if (lane == 0)
-                        sdot[warp][dd] = s;
-                }
-                __syncthreads();
-                if (tid < dn) {
-                    double s = 0.;
-                    for (int w = 0; w < NT / 32; w++)
-                        s = s + sdot[w][tid];
-                    sres[tid] = s;
-                }
-                __syncthreads();
-                if (tid == 0) {
-                    for (int dd = 0; dd < dn; dd++) {
-                        const int d = d0 + dd;
-                        if (d == 0)
-                            sacc[0] = fabs(sres[dd]);
-                        else if (d == 1)
-                            sacc[0] = sacc[0] * fabs(sres[dd]);
-                        else if (d & 1) // (vv_p . r) times the pending (uu_p . c)
-                            sacc[1] = sacc[1] + sres[dd] * sacc[2];
-                        else
-                            sacc[2] = sres[dd];
-                    }
-                }
-                __syncthreads();
-            }
-            aux       = sacc[0];
-            double fa = sacc[1];
-            frob = frob + (aux + 2 * fa);
-            I    = I2;
-            __syncthreads();
-        } else {
-            q -= 1;
-            if (q == 0)
-                q = -1;
-            break;
         }
+        aca_argmax<NT>(piv2, I2, 0, sm);
+        if (I2 < 0) // no pivot row left (only with non-finite entries)
+            return q;
+        // ---- Frobenius estimator (partialACA.hpp:127-141): (uu_p . c) and
+        // (vv_p . r) of four earlier crosses p at a time, c.c and r.r with the last
+        double fa = 0., cc = 0., rr = 0.;
+        for (int p0 = 0; p0 < k || p0 == 0; p0 += 4) {
+            double v[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+                v[u] = 0.;
+            const int np = min(4, k - p0);
+            for (int i = tid; i < M; i += NT) {
+                const double c = U[i + (size_t)M * k];
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (u < np)
+                        v[u] = fma(U[i + (size_t)M * (p0 + u)], c, v[u]);
+                if (p0 == 0)
+                    cc = fma(c, c, cc);
+            }
+            for (int j = tid; j < N; j += NT) {
+                const double r = Vt[j + (size_t)N * k];
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (u < np)
+                        v[4 + u] = fma(Vt[j + (size_t)N * (p0 + u)], r, v[4 + u]);
+                if (p0 == 0)
+                    rr = fma(r, r, rr);
+            }
+            if (k > 0) {
+                const double y = reduce_scatter8(v, lane);
+                if constexpr (NT == 32) {
+                    // lanes of one p: (uu_p . c) below lane 16, (vv_p . r) above
+                    fa = fa + y * __shfl_xor_sync(0xffffffffu, y, 16);
+                } else if ((lane & 3) == 0) {
+                    sm.dot[warp][8 * (p0 >> 2) % 96 + (lane >> 2)] = y;
+                }
+            }
+            if (NT != 32 && (p0 >> 2) % 12 == 11 && p0 + 4 < k) { // the table is full: added up before it goes on
+                __syncthreads();
+                if (warp == 0)
+                    for (int g = 0; g < 12; g++) {
+                        double y = sm.dot[0][8 * g + (lane >> 2)];
+                        for (int w = 1; w < NT / 32; w++)
+                            y = y + sm.dot[w][8 * g + (lane >> 2)];
+                        fa = fa + y * __shfl_xor_sync(0xffffffffu, y, 16);
+                    }
+                __syncthreads();
+            }
+        }
+        {
+            double v[8] = {cc, rr, 0., 0., 0., 0., 0., 0.};
+            // two sums: c.c in the lanes of value 0 and r.r in those of value 1
+            double y = reduce_scatter8(v, lane);
+            if constexpr (NT == 32) {
+                cc = __shfl_sync(0xffffffffu, y, 0);
+                rr = __shfl_sync(0xffffffffu, y, 4);
+            } else {
+                if (lane == 0 || lane == 4)
+                    sm.dot[warp][96 + (lane >> 2)] = y;
+                __syncthreads();
+            }
+        }
+        bool go = true;
+        if (NT == 32 || warp == 0) {
+            if constexpr (NT != 32) {
+                cc = sm.dot[0][96];
+                rr = sm.dot[0][97];
+                for (int w = 1; w < NT / 32; w++) {
+                    cc = cc + sm.dot[w][96];
+                    rr = rr + sm.dot[w][97];
+                }
+                const int ngr = (k + 3) >> 2, g0 = ngr > 0 ? (ngr - 1) / 12 * 12 : 0;
+                for (int g = g0; g < ngr; g++) {
+                    double y = sm.dot[0][8 * (g - g0) + (lane >> 2)];
+                    for (int w = 1; w < NT / 32; w++)
+                        y = y + sm.dot[w][8 * (g - g0) + (lane >> 2)];
+                    fa = fa + y * __shfl_xor_sync(0xffffffffu, y, 16);
+                }
+            }
+            fa = fa + __shfl_xor_sync(0xffffffffu, fa, 8);
+            fa = fa + __shfl_xor_sync(0xffffffffu, fa, 4);
+            const double aux = cc * rr;
+            frob             = frob + (aux + 2 * fa);
+            go               = sqrt(aux / frob) > eps;
+            if (NT != 32 && tid == 0)
+                sm.go = go;
+        }
+        I = I2;
+        aca_sync<NT>();
+        if constexpr (NT != 32)
+            go = sm.go != 0;
+        if (!go)
+            return q;
     }
+}
+
+template <int NT>
+__global__ void __launch_bounds__(NT == 32 ? 128 : NT) partial_aca_kernel(const AcaBlock *__restrict__ blocks, const int *__restrict__ list, int nlist, const double *__restrict__ xt, const double *__restrict__ xs,
+                                                                         const int *__restrict__ perm_t, const int *__restrict__ perm_s, KernelDesc kd, double eps, double *__restrict__ scratch,
+                                                                         unsigned char *__restrict__ flags, int *__restrict__ rank_out) {
+    __shared__ AcaShared<NT> sm;
+    const int l = NT == 32 ? blockIdx.x * 4 + (threadIdx.x >> 5) : blockIdx.x, tid = NT == 32 ? threadIdx.x & 31 : threadIdx.x;
+    if (l >= nlist)
+        return;
+    const int b      = list[l];
+    const AcaBlock B = blocks[b];
+    const int q      = aca_block<NT>(B, tid, sm, xt, xs, perm_t, perm_s, kd, eps, scratch, flags);
     if (tid == 0)
-        rank_out[blockIdx.x] = q;
+        rank_out[b] = q;
 }
 
 // ---------------------------------------------------------------------------
@@ -813,11 +920,24 @@ __global__ void dense_fill_z_kernel(const DenseChunk *__restrict__ chunks, const
 
 } // namespace
 
-void launch_partial_aca(const AcaBlock *blocks, int nblocks, const double *xt, const double *xs, const int *perm_t, const int *perm_s, KernelDesc kd, double eps, double *scratch, unsigned char *flags,
-                        int *rank_out, cudaStream_t st) {
-    if (nblocks <= 0)
-        return;
-    partial_aca_kernel<<<nblocks, kAcaThreads, 0, st>>>(blocks, xt, xs, perm_t, perm_s, kd, eps, scratch, flags, rank_out);
+int aca_class(int M, int N) { return M + N > kAcaLarge ? 0 : M + N > kAcaSmall ? 1 : 2; }
+
+void launch_partial_aca(const AcaBlock *blocks, const int *list, const int *n, const double *xt, const double *xs, const int *perm_t, const int *perm_s, KernelDesc kd, double eps, double *scratch,
+                        unsigned char *flags, int *rank_out, cudaStream_t st, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join) {
+    const int *l1 = list + n[0], *l2 = l1 + n[1];
+    if (n[2] > 0) { // the small blocks run beside the others
+        HTGPU_CUDA(cudaEventRecord(fork, st));
+        HTGPU_CUDA(cudaStreamWaitEvent(side, fork, 0));
+    }
+    if (n[0] > 0)
+        partial_aca_kernel<256><<<n[0], 256, 0, st>>>(blocks, list, n[0], xt, xs, perm_t, perm_s, kd, eps, scratch, flags, rank_out);
+    if (n[1] > 0)
+        partial_aca_kernel<128><<<n[1], 128, 0, st>>>(blocks, l1, n[1], xt, xs, perm_t, perm_s, kd, eps, scratch, flags, rank_out);
+    if (n[2] > 0) {
+        partial_aca_kernel<32><<<(n[2] + 3) / 4, 128, 0, side>>>(blocks, l2, n[2], xt, xs, perm_t, perm_s, kd, eps, scratch, flags, rank_out);
+        HTGPU_CUDA(cudaEventRecord(join, side));
+        HTGPU_CUDA(cudaStreamWaitEvent(st, join, 0));
+    }
     HTGPU_CUDA(cudaGetLastError());
 }
 

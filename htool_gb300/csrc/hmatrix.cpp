@@ -478,7 +478,7 @@ void HMatrix::build_impl(const KernelDesc *kdp, const HostGen *hg, const double 
             DevBuf<AcaBlock> dblocks;
             DevBuf<double> scratch;
             DevBuf<unsigned char> flags;
-            DevBuf<int> dranks;
+            DevBuf<int> dranks, dlist;
             dblocks.upload(blocks, stream_);
             scratch.alloc(sc);
             st_.aca_scratch_bytes += 8 * sc;
@@ -503,10 +503,22 @@ void HMatrix::build_impl(const KernelDesc *kdp, const HostGen *hg, const double 
                     if ((int)blocks.size() > n_direct)
                         launch_partial_aca_z(dblocks.p + n_direct, (int)blocks.size() - n_direct, dxs.p, dxt.p, aca_ps, aca_pt, kd, eps_, scratch.p, flags.p, dranks.p + n_direct, stream_);
                 } else {
+                    // the blocks by size class, those of the mirrors after the others
+                    std::vector<int> list;
+                    int count[6] = {0, 0, 0, 0, 0, 0};
+                    for (int c = 0; c < 6; c++) {
+                        const std::size_t lo = c < 3 ? 0 : (std::size_t)n_direct, hi = c < 3 ? (std::size_t)n_direct : blocks.size();
+                        for (std::size_t b = lo; b < hi; b++)
+                            if (aca_class(blocks[b].M, blocks[b].N) == c % 3) {
+                                list.push_back((int)b);
+                                count[c]++;
+                            }
+                    }
+                    dlist.upload(list, stream_);
                     if (n_direct > 0)
-                        launch_partial_aca(dblocks.p, n_direct, dxt.p, dxs.p, aca_pt, aca_ps, kd, eps_, scratch.p, flags.p, dranks.p, stream_);
+                        launch_partial_aca(dblocks.p, dlist.p, count, dxt.p, dxs.p, aca_pt, aca_ps, kd, eps_, scratch.p, flags.p, dranks.p, stream_, aux_, fork_, join_);
                     if ((int)blocks.size() > n_direct)
-                        launch_partial_aca(dblocks.p + n_direct, (int)blocks.size() - n_direct, dxs.p, dxt.p, aca_ps, aca_pt, kd, eps_, scratch.p, flags.p, dranks.p + n_direct, stream_);
+                        launch_partial_aca(dblocks.p, dlist.p + n_direct, count + 3, dxs.p, dxt.p, aca_ps, aca_pt, kd, eps_, scratch.p, flags.p, dranks.p, stream_, aux_, fork_, join_);
                 }
                 HTGPU_CUDA(cudaMemcpyAsync(ranks.data(), dranks.p, sizeof(int) * ranks.size(), cudaMemcpyDeviceToHost, stream_));
                 HTGPU_CUDA(cudaStreamSynchronize(stream_));

@@ -18,10 +18,17 @@ struct AcaBlock {
     double ctr[3];        // centre of the target cluster (first pivot row)
 };
 
-// Batched partialACA: one CTA per block.  rank_out[b] = rank, -1 when htool
-// would reject the block, -2 when `cap` columns were not enough.
-void launch_partial_aca(const AcaBlock *blocks, int nblocks, const double *xt, const double *xs, const int *perm_t, const int *perm_s, KernelDesc kd, double eps, double *scratch, unsigned char *flags,
-                        int *rank_out, cudaStream_t st);
+// Batched partialACA of the blocks list[0 .. n[0] + n[1] + n[2]), by size: a
+// CTA of 256 threads for blocks of M + N above kAcaLarge, of 128 above
+// kAcaSmall, a warp for the rest (on `side`, joined to st).  A warp's
+// instruction on the FP64 pipe costs the same for any number of its lanes, and
+// a CTA's sums and barriers are its small blocks' time.
+// rank_out[b] = rank, -1 when htool would reject the block, -2 when `cap`
+// columns were not enough.
+constexpr int kAcaLarge = 2048, kAcaSmall = 192;
+int aca_class(int M, int N); // 0, 1, 2: the kernel a block's size takes
+void launch_partial_aca(const AcaBlock *blocks, const int *list, const int *n, const double *xt, const double *xs, const int *perm_t, const int *perm_s, KernelDesc kd, double eps, double *scratch,
+                        unsigned char *flags, int *rank_out, cudaStream_t st, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join);
 
 // partialACA fed by a host generator (htool's VirtualGenerator::copy_submatrix,
 // include/htool/types/virtual_generator.hpp:22): the steps of the
