@@ -352,6 +352,8 @@ void HMatrix::build_impl(const KernelDesc *kdp, const HostGen *hg, const double 
         }
     };
 
+    reqs.reserve(tasks.size());
+    pending.reserve(tasks.size());
     for (auto &tk : tasks) {
         if (!tk.adm) {
             dense_ts.push_back({tk.t, tk.s});
@@ -409,15 +411,20 @@ void HMatrix::build_impl(const KernelDesc *kdp, const HostGen *hg, const double 
                     fresh.push_back(id);
             predict_caps(fresh);
         }
-        std::sort(pending.begin(), pending.end(), [&](int a, int b) {
-            long long ca = (long long)Ta.nodes[reqs[a].t].size + Sa.nodes[reqs[a].s].size;
-            long long cb = (long long)Ta.nodes[reqs[b].t].size + Sa.nodes[reqs[b].s].size;
-            if (predictor_) {
-                ca *= reqs[a].cap;
-                cb *= reqs[b].cap;
+        if (!std::is_sorted(pending.begin(), pending.end()))
+            std::sort(pending.begin(), pending.end());
+        {
+            std::vector<unsigned long long> key(pending.size());
+            for (std::size_t i = 0; i < pending.size(); i++) {
+                const Req &r      = reqs[pending[i]];
+                const long long c = (long long)Ta.nodes[r.t].size + Sa.nodes[r.s].size;
+                key[i]            = ~(unsigned long long)(predictor_ ? c * r.cap : c);
             }
-            return ca != cb ? ca > cb : a < b;
-        });
+            std::vector<int> by = key_order(key);
+            for (int &i : by)
+                i = pending[i];
+            pending.swap(by);
+        }
         std::size_t free_b = 0, total_b = 0;
         HTGPU_CUDA(cudaMemGetInfo(&free_b, &total_b));
         const long long budget = (aca_budget_ > 0 ? aca_budget_ : (long long)(0.6 * (double)free_b)) / 9; // 8 B factors + 1 B flags per slot
@@ -441,6 +448,8 @@ void HMatrix::build_impl(const KernelDesc *kdp, const HostGen *hg, const double 
             // and run as a second launch on swapped point arrays
             std::vector<AcaBlock> blocks, mirrored;
             std::vector<int> ids, ids_m;
+            blocks.reserve(pending.size() - pos);
+            ids.reserve(pending.size() - pos);
             long long sc = 0, fl = 0;
             while (pos < pending.size()) {
                 Req &r = reqs[pending[pos]];
@@ -486,7 +495,25 @@ void HMatrix::build_impl(const KernelDesc *kdp, const HostGen *hg, const double 
             flags.alloc(fl);
             dranks.alloc(blocks.size());
             std::vector<int> ranks(blocks.size());
+            // on the host while the kernels run: the blocks' features (a sample
+            // for the rank predictor where the block is decided), and the
+            // lists filled below at their largest sizes, their pages touched
+            const std::size_t nb = blocks.size(), acc0 = acc.size(), smp0 = samples_y_.size();
+            std::vector<PackItem> items;
+            auto meanwhile = [&] {
+                samples_x_.resize((smp0 + nb) * kMlpIn);
+                host_parallel_chunks((long long)nb, 4096, [&](long long lo, long long hi) {
+                    for (long long b = lo; b < hi; b++) {
+                        const ClusterNode &tn = Ta.nodes[reqs[ids[b]].t], &sn = Sa.nodes[reqs[ids[b]].s];
+                        block_features(tn.size, sn.size, tn.rad, sn.rad, tn.ctr, sn.ctr, eps_, kd.id, &samples_x_[(smp0 + b) * kMlpIn]);
+                    }
+                });
+                samples_y_.resize(smp0 + nb);
+                items.resize(nb);
+                acc.resize(acc0 + nb);
+            };
             if (hg) {
+                meanwhile();
                 // rows and columns in user numbering; a mirrored block reads
                 // the generator with the roles of the two trees exchanged
                 std::vector<const int *> ru(blocks.size()), cu(blocks.size());
@@ -520,28 +547,27 @@ void HMatrix::build_impl(const KernelDesc *kdp, const HostGen *hg, const double 
                     if ((int)blocks.size() > n_direct)
                         launch_partial_aca(dblocks.p, dlist.p + n_direct, count + 3, dxs.p, dxt.p, aca_ps, aca_pt, kd, eps_, scratch.p, flags.p, dranks.p, stream_, aux_, fork_, join_);
                 }
+                meanwhile();
                 HTGPU_CUDA(cudaMemcpyAsync(ranks.data(), dranks.p, sizeof(int) * ranks.size(), cudaMemcpyDeviceToHost, stream_));
                 HTGPU_CUDA(cudaStreamSynchronize(stream_));
             }
             st_.aca_rounds++;
             st_.aca_blocks += (long long)blocks.size();
             // pack the accepted crosses of this slice
-            std::vector<PackItem> items;
             long long packed = 0;
             const int round  = (int)round_bufs.size();
-            for (std::size_t b = 0; b < blocks.size(); b++) {
+            std::size_t nacc = 0, nsmp = smp0;
+            for (std::size_t b = 0; b < nb; b++) {
                 const int id = ids[b];
                 const int r  = ranks[b];
                 if (r > 0 || r == -1) { // a decided block: a training sample for the rank predictor
-                    const ClusterNode &tn = Ta.nodes[reqs[id].t], &sn = Sa.nodes[reqs[id].s];
-                    const std::size_t at  = samples_x_.size();
-                    samples_x_.resize(at + kMlpIn);
-                    block_features(tn.size, sn.size, tn.rad, sn.rad, tn.ctr, sn.ctr, eps_, kd.id, &samples_x_[at]);
-                    samples_y_.push_back((float)(r > 0 ? r : max_profitable_rank(tn.size, sn.size)));
+                    if (nsmp != smp0 + b)
+                        std::copy_n(samples_x_.begin() + (smp0 + b) * kMlpIn, kMlpIn, samples_x_.begin() + nsmp * kMlpIn);
+                    samples_y_[nsmp++] = (float)(r > 0 ? r : max_profitable_rank(Ta.nodes[reqs[id].t].size, Sa.nodes[reqs[id].s].size));
                 }
                 if (r > 0) {
                     reqs[id].state = 1;
-                    PackItem it;
+                    PackItem &it = items[nacc];
                     it.src_u = blocks[b].u_off;
                     it.src_v = blocks[b].v_off;
                     it.M     = blocks[b].M;
@@ -551,13 +577,13 @@ void HMatrix::build_impl(const KernelDesc *kdp, const HostGen *hg, const double 
                     it.dst_u = packed; // real form: f M x f r and f N x f r; native: 2 M x r and 2 N x r
                     it.dst_v = packed + fu * it.M * r;
                     packed += fu * r * (it.M + it.N);
-                    items.push_back(it);
                     if ((int)b < n_direct)
-                        acc.push_back({id, round, r, it.dst_u, it.dst_v, 0});
+                        acc[acc0 + nacc] = {id, round, r, it.dst_u, it.dst_v, 0};
                     else // mirrored: U of the block is V^T of the mirror and V^T its U; in
                          // real form R(X^T) = J R(X)^T J (J = diag(1, -1, ..)), so both
                          // stored factors are copied as J X J
-                        acc.push_back({id, round, r, it.dst_v, it.dst_u, complex_ ? 1 : 0});
+                        acc[acc0 + nacc] = {id, round, r, it.dst_v, it.dst_u, complex_ ? 1 : 0};
+                    nacc++;
                 } else if (r == -1) {
                     st_.false_positive++;
                     split(id);
@@ -570,6 +596,10 @@ void HMatrix::build_impl(const KernelDesc *kdp, const HostGen *hg, const double 
                     throw Error(5, "[Htool error] device partialACA returned rank " + std::to_string(r));
                 }
             }
+            samples_x_.resize(nsmp * kMlpIn);
+            samples_y_.resize(nsmp);
+            items.resize(nacc);
+            acc.resize(acc0 + nacc);
             auto buf = std::unique_ptr<DevBuf<double>>(new DevBuf<double>());
             buf->alloc(packed);
             if (!items.empty()) {
@@ -619,15 +649,17 @@ void HMatrix::build_impl(const KernelDesc *kdp, const HostGen *hg, const double 
             dense_ts.push_back({reqs[id].t, reqs[id].s});
 
     // ---- final layout: low-rank leaves sorted by (offset_i, offset_j)
-    std::sort(acc.begin(), acc.end(), [&](const Accepted &a, const Accepted &b) {
-        int ia = Ta.nodes[reqs[a.req].t].offset, ib = Ta.nodes[reqs[b.req].t].offset;
-        if (ia != ib)
-            return ia < ib;
-        return Sa.nodes[reqs[a.req].s].offset < Sa.nodes[reqs[b.req].s].offset;
-    });
+    std::vector<unsigned long long> key(acc.size());
+    for (std::size_t i = 0; i < acc.size(); i++) {
+        const Req &r = reqs[acc[i].req];
+        key[i]       = (unsigned long long)Ta.nodes[r.t].offset << 32 | (unsigned)Sa.nodes[r.s].offset;
+    }
     lr_h.clear();
+    lr_h.reserve(acc.size());
     std::vector<LeafSrc> lr_src;
-    for (auto &a : acc) {
+    lr_src.reserve(acc.size());
+    for (int i : key_order(key)) {
+        const Accepted &a     = acc[i];
         const ClusterNode &tn = Ta.nodes[reqs[a.req].t], &sn = Sa.nodes[reqs[a.req].s];
         LrLeaf L;
         L.oi    = ft * tn.offset;
@@ -640,15 +672,15 @@ void HMatrix::build_impl(const KernelDesc *kdp, const HostGen *hg, const double 
         lr_h.push_back(L);
         lr_src.push_back({a.round, a.u, a.v, a.neg});
     }
-    std::sort(dense_ts.begin(), dense_ts.end(), [&](const std::pair<int, int> &a, const std::pair<int, int> &b) {
-        int ia = Ta.nodes[a.first].offset, ib = Ta.nodes[b.first].offset;
-        if (ia != ib)
-            return ia < ib;
-        return Sa.nodes[a.second].offset < Sa.nodes[b.second].offset;
-    });
+    key.resize(dense_ts.size());
+    for (std::size_t i = 0; i < dense_ts.size(); i++)
+        key[i] = (unsigned long long)Ta.nodes[dense_ts[i].first].offset << 32 | (unsigned)Sa.nodes[dense_ts[i].second].offset;
     dn_h.clear();
-    for (auto &d : dense_ts)
-        dn_h.push_back({ft * Ta.nodes[d.first].offset, f * Sa.nodes[d.second].offset, ft * Ta.nodes[d.first].size, f * Sa.nodes[d.second].size});
+    dn_h.reserve(dense_ts.size());
+    for (int i : key_order(key)) {
+        const ClusterNode &tn = Ta.nodes[dense_ts[i].first], &sn = Sa.nodes[dense_ts[i].second];
+        dn_h.push_back({ft * tn.offset, f * sn.offset, ft * tn.size, f * sn.size});
+    }
     if (symmetry_ != 'N')
         add_symmetric_twins(lr_src);
     std::vector<const double *> bufs;
@@ -894,30 +926,43 @@ void HMatrix::finalize(const std::vector<const double *> &bufs, const std::vecto
     // into balanced chunks of <= kRowChunk rows, one phase-2 item each,
     // listing the group's leaves (dense, then low-rank, each by offset_j)
     std::vector<std::pair<int, int>> groups; // (offset_i, m)
-    std::vector<std::vector<int>> members;   // ~d for dense leaf d, l for low-rank leaf l
+    std::vector<int> members, mbeg;          // ~d for dense leaf d, l for low-rank leaf l; first member of every group
     {
         // leaves sorted by (offset_i, m), dense first, each kind in its own
         // order: the groups and their members without a map lookup per leaf
-        std::vector<std::pair<std::pair<int, int>, long long>> keyed; // ((oi, m), order)
-        keyed.reserve(dn_h.size() + lr_h.size());
-        for (int d = 0; d < (int)dn_h.size(); d++)
-            keyed.push_back({{dn_h[d].oi, dn_h[d].m}, (long long)d});
-        for (int l = 0; l < (int)lr_h.size(); l++)
-            if (lr_h[l].r > 0)
-                keyed.push_back({{lr_h[l].oi, lr_h[l].m}, (long long)dn_h.size() + l});
-        std::stable_sort(keyed.begin(), keyed.end(), [](const std::pair<std::pair<int, int>, long long> &a, const std::pair<std::pair<int, int>, long long> &b) { return a.first < b.first; });
-        for (std::size_t k = 0; k < keyed.size(); k++) {
-            if (k == 0 || keyed[k].first != keyed[k - 1].first) {
-                groups.push_back(keyed[k].first);
-                members.emplace_back();
-            }
-            const long long o = keyed[k].second;
-            members.back().push_back(o < (long long)dn_h.size() ? ~(int)o : (int)(o - (long long)dn_h.size()));
+        std::vector<unsigned long long> key;
+        std::vector<int> leaf;
+        key.reserve(dn_h.size() + lr_h.size());
+        leaf.reserve(dn_h.size() + lr_h.size());
+        for (int d = 0; d < (int)dn_h.size(); d++) {
+            key.push_back((unsigned long long)dn_h[d].oi << 32 | (unsigned)dn_h[d].m);
+            leaf.push_back(~d);
         }
+        for (int l = 0; l < (int)lr_h.size(); l++)
+            if (lr_h[l].r > 0) {
+                key.push_back((unsigned long long)lr_h[l].oi << 32 | (unsigned)lr_h[l].m);
+                leaf.push_back(l);
+            }
+        members = key_order(key);
+        for (std::size_t k = 0; k < members.size(); k++) {
+            const unsigned long long kk = key[members[k]];
+            const std::pair<int, int> gk((int)(kk >> 32), (int)(kk & 0xffffffffu));
+            if (groups.empty() || gk != groups.back()) {
+                groups.push_back(gk);
+                mbeg.push_back((int)k);
+            }
+            members[k] = leaf[members[k]];
+        }
+        mbeg.push_back((int)members.size());
     }
+    // the groups by offset_i, the larger first (they are sorted by (offset_i, m))
     std::vector<int> gorder(groups.size());
     std::iota(gorder.begin(), gorder.end(), 0);
-    std::sort(gorder.begin(), gorder.end(), [&](int a, int b) { return groups[a].first != groups[b].first ? groups[a].first < groups[b].first : groups[a].second > groups[b].second; });
+    for (std::size_t a = 0, b = 0; a < gorder.size(); a = b) {
+        while (b < gorder.size() && groups[b].first == groups[a].first)
+            b++;
+        std::reverse(gorder.begin() + a, gorder.begin() + b);
+    }
     std::vector<long long> zbase(groups.size());
     zlen_ = 0;
     for (int g : gorder) {
@@ -934,7 +979,8 @@ void HMatrix::finalize(const std::vector<const double *> &bufs, const std::vecto
         const int g = gorder[gi], m = groups[g].second;
         const int nchunk = (m + kRowChunk - 1) / kRowChunk;
         long long width = 0, ncontrib = 0;
-        for (int leaf : members[g]) {
+        for (int k = mbeg[g]; k < mbeg[g + 1]; k++) {
+            const int leaf = members[k];
             width += leaf >= 0 ? lr_parts * lr_h[leaf].r : dn_h[~leaf].n;
             ncontrib += leaf >= 0 ? lr_parts : 1;
         }
@@ -984,7 +1030,8 @@ void HMatrix::finalize(const std::vector<const double *> &bufs, const std::vecto
                 pi.h    = it.h;
                 pi.q0   = (int)qpos;
                 long long col = 0;
-                for (int leaf : members[g]) { // dense leaves come first in members
+                for (int k = mbeg[g]; k < mbeg[g + 1]; k++) { // dense leaves come first in members
+                    const int leaf = members[k];
                     P2Contrib pc;
                     pc.off = poff + (long long)it.h * col;
                     if (leaf >= 0) {
@@ -1034,6 +1081,12 @@ void HMatrix::finalize(const std::vector<const double *> &bufs, const std::vecto
         }
     });
     off = off_p2 + g_off[ng];
+    for (std::size_t b = 0; b < bufs.size(); b++) {
+        std::size_t n = copies[b].size();
+        for (auto &rc : rcopies)
+            n += rc[b].size();
+        copies[b].reserve(n);
+    }
     for (long long rg = 0; rg < nranges; rg++) {
         for (std::size_t b = 0; b < bufs.size(); b++)
             copies[b].insert(copies[b].end(), rcopies[(std::size_t)rg][b].begin(), rcopies[(std::size_t)rg][b].end());
@@ -1048,30 +1101,41 @@ void HMatrix::finalize(const std::vector<const double *> &bufs, const std::vecto
             cuts.push_back(gk.first);
             cuts.push_back(gk.first + gk.second);
         }
-        std::sort(cuts.begin(), cuts.end());
-        cuts.erase(std::unique(cuts.begin(), cuts.end()), cuts.end());
+        std::vector<int> atom_of((std::size_t)nr + 1, 0); // 1 at the cuts, then the number of cuts before a row
+        for (int c : cuts)
+            atom_of[c] = 1;
+        cuts.clear();
+        for (int row = 0; row <= nr; row++) {
+            const bool cut = atom_of[row] != 0;
+            atom_of[row]   = (int)cuts.size();
+            if (cut)
+                cuts.push_back(row);
+        }
         const int natoms = (int)cuts.size() - 1;
-        auto atom_of     = [&](int row) { return (int)(std::lower_bound(cuts.begin(), cuts.end(), row) - cuts.begin()); };
-        std::vector<std::vector<int>> cover(natoms);
-        std::vector<int> by_size(groups.size());
-        std::iota(by_size.begin(), by_size.end(), 0);
-        std::sort(by_size.begin(), by_size.end(), [&](int a, int b) { return groups[a].second != groups[b].second ? groups[a].second > groups[b].second : groups[a].first < groups[b].first; });
-        for (int g : by_size)
-            for (int a = atom_of(groups[g].first); a < atom_of(groups[g].first + groups[g].second); a++)
-                cover[a].push_back((int)zbase[g]);
+        std::vector<unsigned long long> key(groups.size());
+        for (std::size_t g = 0; g < groups.size(); g++)
+            key[g] = (unsigned long long)~(unsigned)groups[g].second << 32 | (unsigned)groups[g].first;
+        std::vector<int> at((std::size_t)natoms + 1, 0);
+        for (auto &gk : groups)
+            for (int a = atom_of[gk.first]; a < atom_of[gk.first + gk.second]; a++)
+                at[a + 1]++;
+        for (int a = 0; a < natoms; a++)
+            at[a + 1] += at[a];
         zi_h.clear();
-        zl_h.clear();
         zsum_reads_ = 0;
         for (int a = 0; a < natoms; a++) {
             ZItem zi;
             zi.row0 = cuts[a];
             zi.h    = cuts[a + 1] - cuts[a];
-            zi.lbeg = (int)zl_h.size();
-            zl_h.insert(zl_h.end(), cover[a].begin(), cover[a].end());
-            zi.lend = (int)zl_h.size();
+            zi.lbeg = at[a];
+            zi.lend = at[a + 1];
             zsum_reads_ += (long long)zi.h * (zi.lend - zi.lbeg);
             zi_h.push_back(zi);
         }
+        zl_h.resize((std::size_t)at[natoms]);
+        for (int g : key_order(key))
+            for (int a = atom_of[groups[g].first]; a < atom_of[groups[g].first + groups[g].second]; a++)
+                zl_h[at[a]++] = (int)zbase[g];
         // the atoms of the local rows (global-to-local products write only these)
         zloc0_ = zloc1_ = 0;
         while (zloc0_ < natoms && cuts[zloc0_] < loff)

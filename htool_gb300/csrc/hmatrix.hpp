@@ -22,10 +22,6 @@ constexpr int kHostKernelId = 3; // kernel id of a host generator in the rank pr
 // numbering of a product's input and output
 constexpr int kUserNumbering = 0, kClusterNumbering = 1, kGlobalToLocal = 2;
 
-int host_threads();
-void host_parallel_for(long long n, const std::function<void(long long)> &body);
-// the same over ranges [lo, hi) of at most `grain` indices (few atomics for fine-grained loops)
-void host_parallel_chunks(long long n, long long grain, const std::function<void(long long, long long)> &body);
 void call_generator(const HostGen &g, int M, int N, const int *rows, const int *cols, double *ptr);
 
 // partialACA of a batch of blocks fed by a host generator (hostgen.cpp):

@@ -6,6 +6,7 @@
 #include <cstdint>
 #include <stdexcept>
 #include <string>
+#include <functional>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -90,6 +91,12 @@ struct BlockTreeParams {
 
 bool admissible(const ClusterNode &t, const ClusterNode &s, double eta);
 std::vector<BlockTask> build_local_tasks(const ClusterTree &T, const ClusterTree &S, const BlockTreeParams &p);
+int host_threads();
+void host_parallel_for(long long n, const std::function<void(long long)> &body);
+// the same over ranges [lo, hi) of at most `grain` indices (few atomics for fine-grained loops)
+void host_parallel_chunks(long long n, long long grain, const std::function<void(long long, long long)> &body);
+// the stable order of integer keys: counting passes over the digits that differ
+std::vector<int> key_order(const std::vector<unsigned long long> &key);
 
 // ---------------------------------------------------------------------------
 // device-side descriptors (plain structs, identical layout on host/device)
