@@ -2385,7 +2385,7 @@ void HMatrix::launch_product_with(const double *x, double *y, int mu_out, int nu
                 launch_phase2_tc(scm_d.p, p2rcm_d.p, n_p2rc_m_, tc2slab_d.p, tc2g_d.p, n_tc2_groups_, mix_.p, cidxm_d.p, reinterpret_cast<const float *>(w_A), w_xexp, mu, w_z, (int)zlen_,
                                  status_d.p, st);
             else
-                launch_phase2_mma(scm_d.p, p2rcm_d.p, n_p2rc_m_, mix_.p, cidxm_d.p, w_A, w_xexp, mu, w_z, (int)zlen_, st);
+                launches_ += launch_phase2_mma(scm_d.p, p2rcm_d.p, n_p2rc_m_, mix_.p, cidxm_d.p, w_A, w_xexp, mu, w_z, (int)zlen_, st) - 1;
             launches_ += 1;
             if (n_chunks_md_ > 0) {
                 dense_mrhs(w_xp, w_xs, w_xexp, w_A, w_z, mu, w_oz, st);

@@ -302,7 +302,7 @@ void tc_selftest(const float *a, const float *b, float *d, int *status, cudaStre
 // BF16 chunks of every row chunk (rc: first chunk of row chunk i, nrc + 1
 // entries) on the tensor cores; writes the row chunk's z rows (the dense
 // chunks are added afterwards: launch_phase2_df_mrhs)
-void launch_phase2_mma(const StreamChunk *chunks, const int *rc, int nrc, const unsigned char *mix, const int *cidx, const double *A, const int *xexp, int mu, double *z, int zlen, cudaStream_t st);
+int launch_phase2_mma(const StreamChunk *chunks, const int *rc, int nrc, const unsigned char *mix, const int *cidx, const double *A, const int *xexp, int mu, double *z, int zlen, cudaStream_t st);
 // ---- many right-hand sides in double-float arithmetic (mrhs.cu) -----------
 // phase 1 of an FP64 product with mu >= kDfMinRhs: every tile (DFMA or
 // emulated alike) for 16 right-hand sides per pass, A slots written as in

@@ -11,7 +11,9 @@
 // phase 2 (stream.cu) folds its FP32 partial sums into double-float
 // accumulators and uses DFMA on the dense leaves' FP64 blocks.
 #include "df64.cuh"
+#include "f32x2.cuh"
 #include "kernels.hpp"
+#include <atomic>
 
 #include <cuda_bf16.h>
 
@@ -578,156 +580,344 @@ void launch_phase1_mma(const P1Item *items, int nitems, const LrLeaf *lr, const 
 // slice q mod S = 32 / h, element ((g Ln + slice h + row) V + v) for
 // j = q / S = g V + v) and C their coefficients, the float phase-1 sums
 // gathered through the column indices.  mma.sync m16n8k8 TF32 with three
-// products per step as in phase 1, FP32 accumulation over the row chunk;
-// one warp per row chunk, right-hand sides in blocks of 64.  The row
-// chunk's z rows are written (FP64, x's exponent shift undone); its dense
-// FP64 chunks are added afterwards by phase2_df_mrhs_kernel (mrhs.cu).  Each chunk's bytes
-// and the coefficients of 32 of its columns are staged in the warp's shared
-// memory (every load issued before the first use), the fragments read there.
-// per warp: the chunk's bytes and the coefficients of up to 32 of its
-// columns for 64 right-hand sides (row stride 72 floats: the B fragments of
-// a step hit 32 distinct banks)
-constexpr int kP2Slab = 32, kP2CoefLd = 72;
-constexpr int kP2MmaSmem = kMmaWarps * (kStreamStage + 4 * kP2Slab * kP2CoefLd);
-
-__global__ void __launch_bounds__(32 * kMmaWarps) phase2_mma_kernel(const StreamChunk *__restrict__ chunks, const int *__restrict__ rc, int nrc, const unsigned char *__restrict__ mix,
-                                                                     const int *__restrict__ cidx, const double *__restrict__ A, const int *__restrict__ xexp, int mu,
-                                                                     double *__restrict__ z, int zlen) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-    const int W      = gridDim.x * kMmaWarps;
-    unsigned char *sd = smem + (size_t)wid * (kStreamStage + 4 * kP2Slab * kP2CoefLd); // the chunk's bytes
-    float *scf        = reinterpret_cast<float *>(sd + kStreamStage);                   // coefficients [column][rhs]
-    const float *Af   = reinterpret_cast<const float *>(A);                             // float phase-1 sums
-    const int shift   = max(*xexp, 1) - 1023;
-    for (int w = blockIdx.x * kMmaWarps + wid; w < nrc; w += W) {
-        const int kb = rc[w], ke = rc[w + 1];
-        const StreamChunk head = chunks[kb];
-        const int h = head.h, zrow = head.b, nmt = h > 16 ? 2 : 1;
-        for (int cb = 0; cb < mu; cb += 64) {
-            const int nn = min(64, mu - cb), nnt = (nn + 7) >> 3; // right-hand sides of this block, 8-column tiles
-            float acc[2][8][4];
-#pragma unroll
-            for (int a = 0; a < 2; a++)
-#pragma unroll
-                for (int b = 0; b < 8; b++)
-#pragma unroll
-                    for (int q = 0; q < 4; q++)
-                        acc[a][b][q] = 0.f;
-            for (int k = kb; k < ke; k++) {
-                const StreamChunk c = chunks[k];
-                if (c.kind != kStreamF32 && c.kind != kStreamBf16) // dense FP64: the streamed kernel
-                    continue;
-                // the chunk's bytes into shared memory: every load issued before the first store
-                {
-                    const uint4 *src = reinterpret_cast<const uint4 *>(mix + c.src);
-                    uint4 *dst       = reinterpret_cast<uint4 *>(sd);
-                    const int nw     = c.bytes >> 4; // <= 256
-                    uint4 r[kStreamStage / 512];
-                    __syncwarp(); // the previous chunk is read out
-#pragma unroll
-                    for (int i = 0; i < kStreamStage / 512; i++)
-                        r[i] = lane + 32 * i < nw ? __ldg(src + lane + 32 * i) : make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-                    for (int i = 0; i < kStreamStage / 512; i++)
-                        if (lane + 32 * i < nw)
-                            dst[lane + 32 * i] = r[i];
-                }
-                const int S = 32 / h, Ln = S * h, lv = c.kind == kStreamF32 ? 2 : 3;
-                auto uload = [&](int row, int q) -> float { // U[row][q], zero outside the chunk
-                    if (row >= h || q >= c.ncol)
-                        return 0.f;
-                    const int j = q / S, sl = q - j * S;
-                    const int e = (((j >> lv) * Ln + sl * h + row) << lv) + (j & ((1 << lv) - 1));
-                    return lv == 2 ? reinterpret_cast<const float *>(sd)[e] : bf16_to_f32(reinterpret_cast<const unsigned short *>(sd)[e]);
-                };
-                for (int qs = 0; qs < c.ncol; qs += kP2Slab) {
-                    const int ns = min(kP2Slab, c.ncol - qs);
-                    // coefficients of columns qs .. qs + ns (zero past them and past nn)
-                    const int kxl = lane < ns ? cidx[c.a + qs + lane] : -1;
-                    if (qs > 0)
-                        __syncwarp(); // the previous slab is read out
-                    if ((mu & 3) == 0) {
-                        float4 r[kP2Slab * 16 / 32];
-#pragma unroll
-                        for (int i = 0; i < kP2Slab * 16 / 32; i++) {
-                            const int e = lane + 32 * i, j = e >> 4, c4 = e & 15;
-                            const int kx = __shfl_sync(0xffffffffu, kxl, j);
-                            r[i]         = (kx >= 0 && 4 * c4 < nn) ? __ldg(reinterpret_cast<const float4 *>(Af + (long long)kx * mu + cb) + c4) : make_float4(0.f, 0.f, 0.f, 0.f);
-                        }
-#pragma unroll
-                        for (int i = 0; i < kP2Slab * 16 / 32; i++) {
-                            const int e = lane + 32 * i, j = e >> 4, c4 = e & 15;
-                            *reinterpret_cast<float4 *>(scf + j * kP2CoefLd + 4 * c4) = r[i];
-                        }
-                    } else {
-                        for (int j = 0; j < kP2Slab; j++) {
-                            const int kx = __shfl_sync(0xffffffffu, kxl, j);
-                            for (int cc = lane; cc < 64; cc += 32)
-                                scf[j * kP2CoefLd + cc] = (kx >= 0 && cc < nn) ? __ldg(Af + (long long)kx * mu + cb + cc) : 0.f;
-                        }
-                    }
-                    __syncwarp();
-                    for (int q0 = 0; q0 < ns; q0 += 8) {
-                        unsigned ah[2][4], al[2][4];
-#pragma unroll
-                        for (int mt = 0; mt < 2; mt++) {
-                            const int r0 = 16 * mt + g;
-                            split_tf32(uload(r0, qs + q0 + t), ah[mt][0], al[mt][0]);
-                            split_tf32(uload(r0 + 8, qs + q0 + t), ah[mt][1], al[mt][1]);
-                            split_tf32(uload(r0, qs + q0 + t + 4), ah[mt][2], al[mt][2]);
-                            split_tf32(uload(r0 + 8, qs + q0 + t + 4), ah[mt][3], al[mt][3]);
-                        }
-#pragma unroll
-                        for (int nt = 0; nt < 8; nt++) {
-                            if (nt >= nnt) // warp-uniform
-                                break;
-                            // zero past the slab's columns (those rows of scf are zero or stale: masked)
-                            const float b0 = q0 + t < ns ? scf[(q0 + t) * kP2CoefLd + 8 * nt + g] : 0.f;
-                            const float b1 = q0 + t + 4 < ns ? scf[(q0 + t + 4) * kP2CoefLd + 8 * nt + g] : 0.f;
-                            unsigned bh0, bl0, bh1, bl1;
-                            split_tf32(b0, bh0, bl0);
-                            split_tf32(b1, bh1, bl1);
-#pragma unroll
-                            for (int mt = 0; mt < 2; mt++) {
-                                if (mt >= nmt) // warp-uniform
-                                    break;
-                                mma_tf32(acc[mt][nt], al[mt], bh0, bh1);
-                                mma_tf32(acc[mt][nt], ah[mt], bl0, bl1);
-                                mma_tf32(acc[mt][nt], ah[mt], bh0, bh1);
-                            }
-                        }
-                    }
-                }
-            }
-#pragma unroll
-            for (int mt = 0; mt < 2; mt++)
-#pragma unroll
-                for (int nt = 0; nt < 8; nt++)
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        const int row = 16 * mt + g + 8 * (q >> 1), col = cb + 8 * nt + 2 * t + (q & 1);
-                        if (mt < nmt && nt < nnt && row < h && col < mu)
-                            z[(long long)col * zlen + zrow + row] = scale_pow2_safe((double)acc[mt][nt][q], shift);
-                    }
-        }
-    }
+// products per step as in phase 1 (two for BF16 columns, which TF32 holds
+// exactly), FP32 accumulation over the row chunk; one warp per row chunk, NT
+// blocks of 8 right-hand sides per launch.  The row chunk's z rows are
+// written (FP64, x's exponent shift undone); its dense FP64 chunks are added
+// afterwards by phase2_df_mrhs_kernel (mrhs.cu).
+//
+// Bound by instruction issue beside the tensor pipe (a step of 8 columns is 8
+// + 16 fragment words split and 48 MMAs, 8.25 cycles of the pipe each).  A
+// warp copies the next two slabs of 16 columns and their coefficients
+// asynchronously while it multiplies the present one; fragments are split
+// before the step's MMAs, which run over the tiles so that no two in a row
+// share an accumulator.  The block's right-hand side g NT + nt is column g of
+// tile nt, so a lane reads its words of a coefficient row in 16-byte loads;
+// rows' 16-byte units are exchanged (unit ^ row bits) against bank conflicts.
+// Helmholtz cube, 30 000 points in real form, FP32 / BF16 storage, 64
+// right-hand sides (16 420 row chunks, 747 000 steps): loads, divisions and
+// conversions of a step in one chain 1750 us, now 567 us at 6 CTAs of 2 warps
+// an SM (tensor pipe 36% busy, a warp issues an MMA every 12 cycles at most).
+// 32 right-hand sides a warp and twice the warps: 840 us (every column split
+// and read twice); 128 registers and 8 CTAs: 688 us (spills).
+constexpr int kP2Warps = 2, kP2Slab = 16, kP2Stages = 3; // warps of a CTA, columns of a slab, slabs in shared memory
+constexpr int kP2SlabBytes = 2048;        // a slab's columns: at most four groups of 32 lanes' 16 bytes
+template <int NT>
+constexpr int kP2CoefLd = NT == 2 ? 24 : 8 * NT; // floats of a coefficient row
+template <int NT>
+constexpr int kP2MmaWarp = kP2Stages * (kP2SlabBytes + 4 * kP2Slab * kP2CoefLd<NT>);
+// what unit numbers of coefficient row j are exchanged by: with it the 8
+// lanes (2 of g, 4 of t) of a 16-byte access phase are in distinct banks
+template <int NT>
+__device__ __forceinline__ int p2_swizzle(int j) {
+    return NT == 8 ? (j & 1) | (j & 2) << 1 : NT == 4 ? 2 * (j & 3) : 0;
 }
 
-void launch_phase2_mma(const StreamChunk *chunks, const int *rc, int nrc, const unsigned char *mix, const int *cidx, const double *A, const int *xexp, int mu, double *z, int zlen, cudaStream_t st) {
-    if (nrc <= 0)
-        return;
-    static unsigned long long done = 0; // devices whose shared-memory limit was raised
+template <int B>
+__device__ __forceinline__ void copy_async_or_zero(void *dst, const void *src, bool ok) {
+    if constexpr (B == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sa(dst)), "l"(src), "r"(ok ? 16 : 0) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %3, %2;" ::"r"(sa(dst)), "l"(src), "r"(ok ? B : 0), "n"(B) : "memory");
+}
+
+// split_tf32 of a finite v in integer arithmetic (4 instructions, the two
+// conversions take 8): the tensor core reads the upper 19 bits of lo
+__device__ __forceinline__ void split_tf32_finite(float v, unsigned &hi, unsigned &lo) {
+    hi = (__float_as_uint(v) + 0x1000u) & 0xffffe000u;
+    lo = __float_as_uint(v - __uint_as_float(hi)) + 0x1000u;
+}
+
+__device__ __forceinline__ void ldmatrix4(unsigned (&r)[4], unsigned addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+
+// one row chunk's sums; false (nothing written) where EXACT is off and a word
+// read is not finite
+template <int NT, bool EXACT>
+__device__ __forceinline__ bool phase2_mma_rows(int w, unsigned char *sd, const StreamChunk *__restrict__ chunks, const int *__restrict__ rc, const unsigned char *__restrict__ mix,
+                                                const int *__restrict__ cidx, const float *__restrict__ Af, const int *__restrict__ xexp, int mu, int cb, double *__restrict__ z, int zlen) {
+    constexpr int LD = kP2CoefLd<NT>, kUnits = 2 * NT; // 16-byte units of a coefficient row
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    float *scf     = reinterpret_cast<float *>(sd + kP2Stages * kP2SlabBytes); // the slabs' coefficients [column][rhs], after their columns
+    const int kb = rc[w], ke = rc[w + 1];
+    const int h = chunks[kb].h, zrow = chunks[kb].b, S = 32 / h, Ln = S * h;
+    const int inv  = (1 << 20) / S + (S > 1); // q / S = q inv >> 20 for the columns q < 2^11 of a chunk
+    const bool two = h > 16;
+    const int nn   = min(8 * NT, mu - cb);
+    const bool whole = nn == 8 * NT && (mu & 3) == 0; // rows of whole 16-byte units
+    int rowoff[4];                                    // rows of the A fragments; past h: the last row (sums not stored)
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        rowoff[i] = 16 * min(g + 8 * i, h - 1);
+    // rows of the lane's ldmatrix addresses (two tiles), and its half of a step's columns
+    const int mrow[2] = {16 * min(lane & 15, h - 1), 16 * min(16 + (lane & 15), h - 1)}, mcol = lane >> 4;
+
+    // the copies' position: a batch of 32 chunk descriptors, one per lane
+    struct Slab {
+        int qs, ncol;
+        bool f32;
+    };
+    int b0 = kb - 32, d_a = 0, d_n = 0, p_a = 0;
+    long long d_src = 0, p_src = 0;
+    unsigned left = 0;
+    Slab p{0, 0, false};
+    bool valid      = true;
+    auto next_chunk = [&] {
+        while (left == 0 && b0 + 32 < ke) {
+            b0 += 32;
+            bool lowrank = false;
+            if (b0 + lane < ke) {
+                const StreamChunk c = chunks[b0 + lane];
+                lowrank             = c.kind == kStreamF32 || c.kind == kStreamBf16; // dense FP64: another kernel
+                d_a                 = c.a;
+                d_src               = c.src;
+                d_n                 = c.ncol << 1 | (c.kind == kStreamF32 ? 1 : 0);
+            }
+            left = __ballot_sync(0xffffffffu, lowrank);
+        }
+        valid = left != 0;
+        if (!valid)
+            return;
+        const int j = __ffs(left) - 1;
+        left &= left - 1;
+        p_a         = __shfl_sync(0xffffffffu, d_a, j);
+        p_src       = __shfl_sync(0xffffffffu, d_src, j);
+        const int n = __shfl_sync(0xffffffffu, d_n, j);
+        p.qs        = 0;
+        p.ncol      = n >> 1;
+        p.f32       = n & 1;
+    };
+    // group of V columns of every slice (Ln 16-byte units) that holds column q
+    auto group = [&](const Slab &s, int q) { return (q * inv >> 20) >> (s.f32 ? 2 : 3); };
+    int kx           = -1;
+    auto index_ahead = [&] { kx = valid && lane < kP2Slab && p.qs + lane < p.ncol ? cidx[p_a + p.qs + lane] : -1; };
+    // the lane's first 16-byte unit of a slab: row j0, and every 32 / kUnits rows from there
+    const int j0 = lane / kUnits, u0 = (j0 * LD + ((lane % kUnits) ^ p2_swizzle<NT>(j0)) * 4) * 4;
+    const float *a0  = Af + cb + lane % kUnits * 4;
+    auto issue       = [&](int par) {
+        {
+            const int g0 = group(p, p.qs), n = (group(p, min(p.qs + kP2Slab, p.ncol) - 1) - g0 + 1) * Ln;
+            const unsigned char *src = mix + p_src + 16 * (g0 * Ln + lane);
+            unsigned char *dst       = sd + par * kP2SlabBytes + 16 * lane;
+#pragma unroll
+            for (int i = 0; i < kP2SlabBytes / 512; i++)
+                if (lane + 32 * i < n)
+                    copy_async<16>(dst + 512 * i, src + 512 * i);
+        }
+        unsigned char *c = reinterpret_cast<unsigned char *>(scf + par * (kP2Slab * LD));
+        if (whole && p.qs + kP2Slab <= p.ncol) {
+#pragma unroll
+            for (int i = 0; i < NT; i++) {
+                // two rows on, the exchange of NT = 8 flips bit 2 of the unit
+                const int u = (NT == 8 && (i & 1) ? u0 ^ 64 : u0) + i * (32 / kUnits) * LD * 4;
+                copy_async<16>(c + u, a0 + (long long)__shfl_sync(0xffffffffu, kx, j0 + i * (32 / kUnits)) * mu);
+            }
+            return;
+        }
+        auto fill = [&](auto width) {
+            constexpr int V = decltype(width)::value, per = 8 * NT / V; // floats a copy, copies a row
+#pragma unroll 1
+            for (int e = lane; e < kP2Slab * per; e += 32) {
+                const int j = e / per, q = e % per * V;
+                const int k  = __shfl_sync(0xffffffffu, kx, j);
+                const bool o = k >= 0 && q < nn;
+                copy_async_or_zero<4 * V>(c + (j * LD + ((q >> 2) ^ p2_swizzle<NT>(j)) * 4 + (q & 3)) * 4, o ? Af + (long long)k * mu + cb + q : Af, o);
+            }
+        };
+        if ((mu & 3) == 0)
+            fill(std::integral_constant<int, 4>());
+        else if ((mu & 1) == 0)
+            fill(std::integral_constant<int, 2>());
+        else
+            fill(std::integral_constant<int, 1>());
+    };
+    auto advance = [&] {
+        p.qs += kP2Slab;
+        if (p.qs >= p.ncol)
+            next_chunk();
+        index_ahead();
+    };
+
+    float acc[2][NT][4];
+#pragma unroll
+    for (int a = 0; a < 2; a++)
+#pragma unroll
+        for (int b = 0; b < NT; b++)
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                acc[a][b][q] = 0.f;
+    f2x fin = fx(0.f, 0.f); // NaN once a word read is not finite
+    Slab in[kP2Stages]; // the present slab and those on their way (no columns: past the last)
+    next_chunk();
+    index_ahead();
+    auto fetch = [&](int stage) {
+        Slab s{0, 0, false};
+        if (valid) {
+            s = p;
+            issue(stage);
+            advance();
+        }
+        copies_commit();
+        return s;
+    };
+#pragma unroll
+    for (int i = 0; i + 1 < kP2Stages; i++)
+        in[i] = fetch(i);
+    for (int par = 0; in[0].ncol > 0; par = par + 1 == kP2Stages ? 0 : par + 1) {
+        in[kP2Stages - 1] = fetch(par == 0 ? kP2Stages - 1 : par - 1);
+        copies_wait<kP2Stages - 1>();
+        __syncwarp();
+        const Slab cur = in[0];
+        const float *c = scf + par * (kP2Slab * LD) + t * LD;
+        const int lv = cur.f32 ? 2 : 3, ns = min(kP2Slab, cur.ncol - cur.qs);
+        const unsigned char *u = sd + par * kP2SlabBytes - group(cur, cur.qs) * Ln * 16;
+        for (int q0 = 0; q0 < ns; q0 += 8) {
+            unsigned ah[2][4], al[2][4];
+            const int qc = cur.qs + q0;
+            if (cur.f32 && S == 1 && qc + 8 <= cur.ncol) { // 16 bytes are 4 columns of a row: as the fragments want them
+#pragma unroll
+                for (int mt = 0; mt < 2; mt++)
+                    ldmatrix4(ah[mt], sa(u + ((qc >> 2) + mcol) * h * 16 + mrow[mt]));
+            } else {
+                // columns past the chunk's end: the last column, against zero coefficients
+                int at[2];
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    const int q = min(qc + t + 4 * k, cur.ncol - 1), j = q * inv >> 20, sl = q - j * S;
+                    at[k] = ((j >> lv) * Ln + sl * h) * 16 + ((j & ((1 << lv) - 1)) << (4 - lv));
+                }
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int k = 0; k < 2; k++) {
+                        const unsigned char *x = u + at[k] + rowoff[i];
+                        ah[i >> 1][2 * k + (i & 1)] = cur.f32 ? *reinterpret_cast<const unsigned *>(x) : (unsigned)*reinterpret_cast<const unsigned short *>(x) << 16;
+                    }
+            }
+            // four tiles of right-hand sides at a time
+#pragma unroll
+            for (int n0 = 0; n0 < NT; n0 += 4) {
+                constexpr int N = NT < 4 ? NT : 4;
+                unsigned bh[N][2], bl[N][2];
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    const float *row = c + (q0 + 4 * k) * LD;
+                    if constexpr (NT >= 4) {
+                        const float4 v = *reinterpret_cast<const float4 *>(row + ((g * (NT / 4) + n0 / 4) ^ p2_swizzle<NT>(t)) * 4);
+                        bh[0][k]       = __float_as_uint(v.x);
+                        bh[1][k]       = __float_as_uint(v.y);
+                        bh[2][k]       = __float_as_uint(v.z);
+                        bh[3][k]       = __float_as_uint(v.w);
+                        if (!EXACT)
+                            fin = fx_fma(fx(v.x, v.y), fx(0.f, 0.f), fin);
+                        fin = fx_fma(fx(v.z, v.w), fx(0.f, 0.f), fin);
+                    } else {
+#pragma unroll
+                        for (int nt = 0; nt < N; nt++) {
+                            const float v = row[g * NT + nt];
+                            bh[nt][k]     = __float_as_uint(v);
+                            fin           = fx_fma(fx(v, v), fx(0.f, 0.f), fin);
+                        }
+                    }
+                }
+                if (n0 == 0 && cur.f32)
+#pragma unroll
+                    for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+                        for (int i = 0; i < 4; i += 2)
+                            fin = fx_fma(fx(__uint_as_float(ah[mt][i]), __uint_as_float(ah[mt][i + 1])), fx(0.f, 0.f), fin);
+                auto split = [](unsigned &hi, unsigned &lo) {
+                    const float v = __uint_as_float(hi);
+                    if (EXACT)
+                        split_tf32(v, hi, lo);
+                    else
+                        split_tf32_finite(v, hi, lo);
+                };
+                if (n0 == 0 && cur.f32)
+#pragma unroll
+                    for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+                        for (int i = 0; i < 4; i++)
+                            split(ah[mt][i], al[mt][i]);
+#pragma unroll
+                for (int nt = 0; nt < N; nt++)
+#pragma unroll
+                    for (int k = 0; k < 2; k++)
+                        split(bh[nt][k], bl[nt][k]);
+                auto tiles = [&](const unsigned(&a)[2][4], const unsigned(&b)[N][2]) {
+#pragma unroll
+                    for (int nt = 0; nt < N; nt++)
+                        mma_tf32(acc[0][n0 + nt], a[0], b[nt][0], b[nt][1]);
+                    if (two)
+#pragma unroll
+                        for (int nt = 0; nt < N; nt++)
+                            mma_tf32(acc[1][n0 + nt], a[1], b[nt][0], b[nt][1]);
+                };
+                if (cur.f32)
+                    tiles(al, bh);
+                tiles(ah, bl);
+                tiles(ah, bh);
+            }
+        }
+        __syncwarp(); // read out before the next copies
+#pragma unroll
+        for (int i = 0; i + 1 < kP2Stages; i++)
+            in[i] = in[i + 1];
+    }
+    const float2 f = fx2(fin);
+    if (!EXACT && __any_sync(0xffffffffu, !(f.x + f.y == 0.f)))
+        return false;
+    const int shift = max(*xexp, 1) - 1023;
+#pragma unroll
+    for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+        for (int nt = 0; nt < NT; nt++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int row = 16 * mt + g + 8 * (q >> 1), col = (2 * t + (q & 1)) * NT + nt;
+                if (row < h && col < nn)
+                    z[(long long)(cb + col) * zlen + zrow + row] = scale_pow2_safe((double)acc[mt][nt][q], shift);
+            }
+    return true;
+}
+
+template <int NT>
+__global__ void __launch_bounds__(32 * kP2Warps, 6) phase2_mma_kernel(const StreamChunk *__restrict__ chunks, const int *__restrict__ rc, int nrc, const unsigned char *__restrict__ mix,
+                                                                       const int *__restrict__ cidx, const float *__restrict__ Af, const int *__restrict__ xexp, int mu, int cb,
+                                                                       double *__restrict__ z, int zlen) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int wid = threadIdx.x >> 5, w = blockIdx.x * kP2Warps + wid;
+    unsigned char *sd = smem + (size_t)wid * kP2MmaWarp<NT>;
+    if (w < nrc && !phase2_mma_rows<NT, false>(w, sd, chunks, rc, mix, cidx, Af, xexp, mu, cb, z, zlen))
+        phase2_mma_rows<NT, true>(w, sd, chunks, rc, mix, cidx, Af, xexp, mu, cb, z, zlen);
+}
+
+namespace {
+template <int NT>
+void phase2_mma(const StreamChunk *chunks, const int *rc, int nrc, const unsigned char *mix, const int *cidx, const float *A, const int *xexp, int mu, int cb, double *z, int zlen, cudaStream_t st) {
+    constexpr int smem = kP2Warps * kP2MmaWarp<NT>;
+    static std::atomic<unsigned long long> done{0}; // devices whose shared-memory limit was raised
     int dev = 0;
     HTGPU_CUDA(cudaGetDevice(&dev));
-    if (dev >= 64 || !(done >> dev & 1)) {
-        HTGPU_CUDA(cudaFuncSetAttribute(phase2_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kP2MmaSmem));
+    if (dev >= 64 || !(done.load() >> dev & 1)) {
+        HTGPU_CUDA(cudaFuncSetAttribute(phase2_mma_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         if (dev < 64)
             done |= 1ull << dev;
     }
-    const int blocks = (nrc + kMmaWarps - 1) / kMmaWarps; // one warp per row chunk
-    phase2_mma_kernel<<<blocks, 32 * kMmaWarps, kP2MmaSmem, st>>>(chunks, rc, nrc, mix, cidx, A, xexp, mu, z, zlen);
+    phase2_mma_kernel<NT><<<(nrc + kP2Warps - 1) / kP2Warps, 32 * kP2Warps, smem, st>>>(chunks, rc, nrc, mix, cidx, A, xexp, mu, cb, z, zlen); // one warp per row chunk
     HTGPU_CUDA(cudaGetLastError());
+}
+} // namespace
+
+int launch_phase2_mma(const StreamChunk *chunks, const int *rc, int nrc, const unsigned char *mix, const int *cidx, const double *A, const int *xexp, int mu, double *z, int zlen, cudaStream_t st) {
+    if (nrc <= 0)
+        return 0;
+    using Launch = void (*)(const StreamChunk *, const int *, int, const unsigned char *, const int *, const float *, const int *, int, int, double *, int, cudaStream_t);
+    static const Launch by_tiles[8] = {phase2_mma<1>, phase2_mma<2>, phase2_mma<4>, phase2_mma<4>, phase2_mma<8>, phase2_mma<8>, phase2_mma<8>, phase2_mma<8>};
+    for (int cb = 0; cb < mu; cb += 64)
+        by_tiles[(std::min(64, mu - cb) + 7) / 8 - 1](chunks, rc, nrc, mix, cidx, reinterpret_cast<const float *>(A), xexp, mu, cb, z, zlen, st);
+    return (mu + 63) / 64;
 }
 
 void launch_phase1_mixed(const P1Item *items, int nitems, const LrLeaf *lr, const unsigned char *mix, const double *scale, const F2 *xs, const int *xexp, int mu, double *A, cudaStream_t st) {
