@@ -1800,7 +1800,7 @@ void HMatrix::upload_mixed_phase2() {
         scr_d.upload(red, stream_);
         if (red.empty())
             scr_d.alloc(1);
-        { // the same where the dense chunks' sums come first only in the row chunks that have any
+        { // the same, the first chunk of a row chunk that has dense chunks starting from their sums
             std::vector<StreamChunk> redp = red;
             std::size_t k                 = 0;
             for (int w = 0; w < n_p2rc_m_; w++) {
@@ -1808,11 +1808,20 @@ void HMatrix::upload_mixed_phase2() {
                 int n            = 0;
                 for (int c = rc[w]; c < rc[w + 1]; c++)
                     n += ch2[c].kind == kStreamF32 || ch2[c].kind == kStreamBf16;
+                if (n > 0) {
+                    redp[k + n - 1].flags &= (unsigned char)~kStreamAdd;
+                    redp[k].flags |= dense ? kStreamAdd : 0;
+                }
                 k += n;
-                if (n > 0 && !dense)
-                    redp[k - 1].flags &= (unsigned char)~kStreamAdd;
             }
             redp_d.upload(redp, stream_);
+            // four times the ranges of the chunk kernels: a warp's last one is
+            // the kernel's tail (200 000 points, ms of phase 2 at 1, 2, 4, 8
+            // times: 2 right-hand sides 0.350, 0.340, 0.334, 0.332, 8: 0.576,
+            // 0.569, 0.565, 0.566)
+            const std::vector<int> rp = stream_ranges(red, 4 * n_sctas_);
+            n_ranges_p_               = (int)rp.size() - 1;
+            srp_d.upload(rp, stream_);
         }
         const std::vector<int> rr = stream_ranges(red, n_sctas_);
         n_ranges_r_               = (int)rr.size() - 1;
@@ -2549,8 +2558,8 @@ void HMatrix::launch_red_product(const double *x, double *y, int mu, int numberi
         if (marks && c0 + n == mu)
             HTGPU_CUDA(cudaEventRecord(marks[1], st));
         launch_pair_phase2(pair2_d.p, n_pair2_, tickets, pair_d.p, cidx_d.p, X, nullptr, w, n, zf + (long long)c0 * zlen_, (int)zlen_, status_d.p, st);
-        launch_red_phase2(redp_d.p, srr_d.p, n_ranges_r_, tickets + 2, mix_.p, cidxm_d.p, Af, w, n, zf + (long long)c0 * zlen_, (int)zlen_, status_d.p, st);
-        launches_ += 2 + (n_p1m_ > 0) + !multi_h.empty() + !rot_h.empty() + (n_pair2_ > 0) + (n_ranges_r_ > 0);
+        launch_red_phase2(redp_d.p, srp_d.p, n_ranges_p_, tickets + 2, mix_.p, cidxm_d.p, Af, w, n, zf + (long long)c0 * zlen_, (int)zlen_, status_d.p, st);
+        launches_ += 2 + (n_p1m_ > 0) + !multi_h.empty() + !rot_h.empty() + (n_pair2_ > 0) + (n_ranges_p_ > 0);
         c0 += n;
     }
     if (marks)

@@ -351,7 +351,9 @@ class HMatrix {
     DevBuf<unsigned char> red_d;
     DevBuf<RedPanel> red1_d;
     DevBuf<int2> redo_d;
-    DevBuf<StreamChunk> redp_d; // the reduced chunks, adding onto z where the row chunk has dense columns
+    DevBuf<StreamChunk> redp_d; // the reduced chunks, starting from z where the row chunk has dense columns
+    DevBuf<int> srp_d;          // their ranges
+    int n_ranges_p_ = 0;
     int n_red1_ = 0;
     void build_red(const std::vector<P1Item> &p1m);
     void release_red();

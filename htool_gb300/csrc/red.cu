@@ -18,11 +18,13 @@
 // and their order are those of phase1_stack_kernel and of the chunk kernels in
 // stream.cu, which a caller's choice of mode keeps.
 //
-// Bound by the shared-memory reads of the coefficients (every lane reads its
-// column's right-hand sides for each element).  Measured against those kernels,
-// Laplace sphere, FP32/BF16 factors, ms a product: 100 000 points 2 right-hand
-// sides 0.365 -> 0.342, 4: 0.726 -> 0.390, 8: 1.835 -> 0.562; 200 000 points
-// 8: 3.68 -> 1.05.  Every wait is bounded (status 2).
+// Bound by latency (12 to 16 warps an SM, the memory 60% busy with 8 right-hand
+// sides; reading half the coefficients, two rows a lane, gained 1%), so
+// descriptors and indices are loaded ahead and a row chunk starts from its
+// dense part.  Measured against those kernels, Laplace sphere, FP32/BF16
+// factors, ms a product: 100 000 points 2 right-hand sides 0.365 -> 0.309, 4:
+// 0.726 -> 0.348, 8: 1.835 -> 0.475; 200 000 points 8: 3.68 -> 0.922.  Every
+// wait is bounded (status 2).
 #include "f32x2.cuh"
 #include "kernels.hpp"
 
@@ -256,7 +258,7 @@ struct Red2Cfg {
     static constexpr int kBar   = kRedStages * kStage;
     static constexpr int kWarp  = (kBar + 8 * kRedStages + 127) & ~127;
     static constexpr int kSmem  = kRedWarps * kWarp;
-    static constexpr int kCtas  = W >= 6 ? 3 : 4;
+    static constexpr int kCtas  = W >= 4 ? 3 : 4; // what the shared memory holds
 };
 
 template <int W>
@@ -278,9 +280,11 @@ __global__ void __launch_bounds__(32 * kRedWarps, Red2Cfg<W>::kCtas)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncwarp();
     const unsigned long long pol = stream_policy();
-    // ranges of whole row chunks: the current one's chunks [k, e), the next
-    // one's bounds, the ticket after that; the chunk issued next and its
-    // column indices, the descriptor of the one after it
+    // ranges of whole row chunks: what is left of the one being taken [k, e),
+    // the next one's bounds, the ticket after that.  Their descriptors come 32
+    // at a time, one to a lane, a window ahead of their use, and a chunk's
+    // column indices two chunks ahead (loaded chunk by chunk, a descriptor and
+    // then its indices, they held a warp up for memory latencies)
     const int nwarps = gridDim.x * kRedWarps;
     int icur = blockIdx.x * kRedWarps + wid, inxt = icur + nwarps, tk = 0;
     int k = 0, e = 0, nk = 0, ne = 0;
@@ -292,84 +296,102 @@ __global__ void __launch_bounds__(32 * kRedWarps, Red2Cfg<W>::kCtas)
         nk = rbeg[inxt];
         ne = rbeg[inxt + 1];
     }
+    struct Win { // h, columns, kind, flags in the bytes of m
+        long long src;
+        int a, b, m, bytes, n;
+    };
+    auto load_window = [&](Win &w) {
+        w.n = min(32, e - k);
+        if (lane < w.n) {
+            const StreamChunk c = chunks[k + lane];
+            w.src               = c.src;
+            w.a                 = c.a;
+            w.b                 = c.b;
+            w.bytes             = c.bytes;
+            w.m                 = c.h | c.ncol << 8 | (int)c.kind << 16 | (int)c.flags << 24;
+        }
+        k += w.n;
+    };
+    Win w0{}, w1{};
+    load_window(w0);
     pdl_next();
     pdl_wait(); // A, z and the ticket are the previous kernels'
     if (inxt < nranges && lane == 0)
         tk = 2 * nwarps + atomicAdd(ticket, 1);
-    auto step = [&]() { // (k, e) to the chunk after k; false at the end
-        if (++k < e)
-            return true;
-        k = nk;
-        e = ne;
-        if (inxt >= nranges) {
-            k = e = 0;
-            return false;
+    auto next_window = [&]() {
+        if (k >= e && inxt < nranges) {
+            k    = nk;
+            e    = ne;
+            inxt = __shfl_sync(0xffffffffu, tk, 0);
+            if (inxt < nranges) {
+                nk = rbeg[inxt];
+                ne = rbeg[inxt + 1];
+                if (lane == 0)
+                    tk = 2 * nwarps + atomicAdd(ticket, 1);
+            }
         }
-        inxt = __shfl_sync(0xffffffffu, tk, 0);
-        if (inxt < nranges) {
-            nk = rbeg[inxt];
-            ne = rbeg[inxt + 1];
-            if (lane == 0)
-                tk = 2 * nwarps + atomicAdd(ticket, 1);
+        load_window(w1); // empty past the last range
+    };
+    next_window();
+    struct Chunk {
+        long long src;
+        int b, m, bytes, ix0, ix1;
+    };
+    int at          = 0;
+    auto next_chunk = [&]() { // m = 0: no more
+        Chunk c{};
+        if (at == w0.n) {
+            w0 = w1;
+            at = 0;
+            if (w0.n > 0)
+                next_window();
         }
-        return true;
+        if (w0.n > 0) {
+            c.src       = __shfl_sync(0xffffffffu, w0.src, at);
+            c.b         = __shfl_sync(0xffffffffu, w0.b, at);
+            c.m         = __shfl_sync(0xffffffffu, w0.m, at);
+            c.bytes     = __shfl_sync(0xffffffffu, w0.bytes, at);
+            const int a = __shfl_sync(0xffffffffu, w0.a, at), n = (c.m >> 8) & 255;
+            c.ix0 = lane < n ? __ldg(cidx + a + lane) : 0;
+            c.ix1 = lane + 32 < n ? __ldg(cidx + a + lane + 32) : 0;
+            at++;
+        }
+        return c;
     };
-    StreamChunk d0{}, d1{};
-    bool has0 = icur < nranges, has1 = false;
-    int ix0 = 0, ix1 = 0;
-    auto indices = [&]() { // of d0
-        ix0 = lane < d0.ncol ? __ldg(cidx + d0.a + lane) : 0;
-        ix1 = lane + 32 < d0.ncol ? __ldg(cidx + d0.a + lane + 32) : 0;
-    };
-    if (has0) {
-        d0   = chunks[k];
-        has1 = step();
-        if (has1)
-            d1 = chunks[k];
-        indices();
-    }
+    Chunk d0 = next_chunk(), d1 = next_chunk();
     int issued = 0;
     auto issue = [&]() {
-        if (has0) {
-            const int s       = issued % kRedStages;
+        if (d0.m != 0) {
+            const int s = issued % kRedStages, ncol = (d0.m >> 8) & 255;
             unsigned char *st = wbase + (size_t)s * C::kStage;
             float *cf         = reinterpret_cast<float *>(st + C::kCoef);
             if (lane == 0) {
-                *reinterpret_cast<int4 *>(st + C::kDesc) = make_int4(d0.h | d0.kind << 8 | d0.flags << 16, d0.ncol, d0.b, 0);
+                *reinterpret_cast<int2 *>(st + C::kDesc) = make_int2(d0.m, d0.b);
                 ring_copy(st, mix + d0.src, (unsigned)d0.bytes, &bar[s], pol);
             }
             if constexpr (W == 1) {
-                const int S = red_div(32, d0.h), lv = d0.kind == kStreamF32 ? 2 : 3;
+                const int S = red_div(32, d0.m & 255), lv = ((d0.m >> 16) & 255) == kStreamF32 ? 2 : 3;
 #pragma unroll
                 for (int r = 0; r < 2; r++) {
                     const int t = lane + 32 * r;
-                    if (t < d0.ncol) {
+                    if (t < ncol) {
                         const int jj = red_div(t, S), sl = t - jj * S;
-                        copy_async<4>(cf + ((((jj >> lv) * S + sl) << lv) | (jj & ((1 << lv) - 1))), A + (r ? ix1 : ix0));
+                        copy_async<4>(cf + ((((jj >> lv) * S + sl) << lv) | (jj & ((1 << lv) - 1))), A + (r ? d0.ix1 : d0.ix0));
                     }
                 }
             } else {
-                if (lane < d0.ncol)
-                    copy_row<W>(cf + W * lane, A + (long long)W * ix0);
-                if (lane + 32 < d0.ncol)
-                    copy_row<W>(cf + W * (lane + 32), A + (long long)W * ix1);
+                if (lane < ncol)
+                    copy_row<W>(cf + W * lane, A + (long long)W * d0.ix0);
+                if (lane + 32 < ncol)
+                    copy_row<W>(cf + W * (lane + 32), A + (long long)W * d0.ix1);
             }
             issued++;
-            d0   = d1;
-            has0 = has1;
-            if (has0) {
-                has1 = step();
-                if (has1)
-                    d1 = chunks[k];
-                indices();
-            }
+            d0 = d1;
+            d1 = next_chunk();
         }
         copies_commit();
     };
     DF2 acc[Q]; // W = 1: the low half
-#pragma unroll
-    for (int q = 0; q < Q; q++)
-        acc[q].s = acc[q].c = 0ull;
 #pragma unroll
     for (int s = 0; s < kRedStages - 1; s++)
         issue();
@@ -385,11 +407,21 @@ __global__ void __launch_bounds__(32 * kRedWarps, Red2Cfg<W>::kCtas)
         }
         __syncwarp();
         const unsigned char *st = wbase + (size_t)s * C::kStage;
-        const int4 d            = *reinterpret_cast<const int4 *>(st + C::kDesc);
-        const int h = d.x & 255, kind = (d.x >> 8) & 255, flags = d.x >> 16, ncol = d.y;
+        const int2 d            = *reinterpret_cast<const int2 *>(st + C::kDesc);
+        const int h = d.x & 255, kind = (d.x >> 16) & 255, flags = (d.x >> 24) & 255, ncol = (d.x >> 8) & 255;
         const int S = red_div(32, h), slice = red_div(lane, h), row = lane - slice * h, Ln = S * h;
         const float *cf = reinterpret_cast<const float *>(st + C::kCoef);
         const uint4 *D  = reinterpret_cast<const uint4 *>(st) + lane;
+        if (flags & kStreamFirst) { // from the dense part where there is one, its loads in flight over the chunk's sums
+            const bool add   = (flags & kStreamAdd) && lane < h;
+            const float2 *zr = z + d.y + row;
+#pragma unroll
+            for (int q = 0; q < Q; q++) {
+                const float2 a = add && 2 * q < nrhs ? zr[(long long)(2 * q) * zlen] : make_float2(0.f, 0.f);
+                const float2 b = add && W > 1 && 2 * q + 1 < nrhs ? zr[(long long)(2 * q + 1) * zlen] : make_float2(0.f, 0.f);
+                acc[q]         = DF2{fx(a.x, b.x), fx(a.y, b.y)};
+            }
+        }
         f2x part[Q], part2[Q]; // sums over even and odd columns (W = 1: the halves of part[0])
 #pragma unroll
         for (int q = 0; q < Q; q++)
@@ -471,16 +503,11 @@ __global__ void __launch_bounds__(32 * kRedWarps, Red2Cfg<W>::kCtas)
                         acc[q] = df2_add(acc[q], o);
                 }
             if (slice == 0) {
-                float2 *zr = z + d.z + row;
+                float2 *zr = z + d.y + row;
 #pragma unroll
                 for (int q = 0; q < Q; q++) {
                     df2_renorm(acc[q]);
                     const bool two = W > 1 && 2 * q + 1 < nrhs, one = 2 * q < nrhs;
-                    if (flags & kStreamAdd) { // the dense part is there
-                        const float2 a = one ? zr[(long long)(2 * q) * zlen] : make_float2(0.f, 0.f), b = two ? zr[(long long)(2 * q + 1) * zlen] : make_float2(0.f, 0.f);
-                        acc[q]         = df2_add(acc[q], DF2{fx(a.x, b.x), fx(a.y, b.y)});
-                        df2_renorm(acc[q]);
-                    }
                     const float2 vs = fx2(acc[q].s), vc = fx2(acc[q].c);
                     if (one)
                         zr[(long long)(2 * q) * zlen] = make_float2(vs.x, vc.x);
@@ -488,9 +515,6 @@ __global__ void __launch_bounds__(32 * kRedWarps, Red2Cfg<W>::kCtas)
                         zr[(long long)(2 * q + 1) * zlen] = make_float2(vs.y, vc.y);
                 }
             }
-#pragma unroll
-            for (int q = 0; q < Q; q++)
-                acc[q].s = acc[q].c = 0ull;
         }
         __syncwarp();
         done++;

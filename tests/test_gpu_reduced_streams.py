@@ -59,3 +59,21 @@ def test_rows_without_dense_leaves_and_rectangles():
     y = hm.mvprod_global_to_global(x, 4)
     hm.set_phase2_mode("warp")
     assert rel(y, hm.mvprod_global_to_global(x, 4)) < TOL
+
+
+@pytest.mark.parametrize("mu", [2, 8])
+def test_rows_of_more_than_a_window_of_chunks(mu):
+    """row chunks of more than 32 chunks: a second window of descriptors"""
+    n = 3000
+    rng = np.random.default_rng(7)
+    pts = G.sphere(n, seed=4)
+    t = H.Cluster().build(n, pts)
+    lr = np.array([[0, j, 40, 50, 40] for j in range(0, n, 50)] + [[40, 0, n - 40, n, 3]], np.int32)  # offsets, sizes, rank
+    uv = rng.standard_normal(int((lr[:, 4].astype(np.int64) * (lr[:, 2] + lr[:, 3])).sum()))
+    assert 60 * 40 > 33 * 64  # columns of the first 40 rows, at most 64 a chunk
+    hm = H.HMatrix(t, t, 1e-6, 10.0).set_leaves(lr, uv, np.empty((0, 4), np.int32), np.empty(0)).set_precision("mixed", 1.0)
+    x = G.rhs(n, mu, seed=3)
+    y = hm.mvprod_global_to_global(x, mu)
+    hm.set_phase2_mode("warp")
+    assert rel(y, hm.mvprod_global_to_global(x, mu)) < TOL
+    assert hm.device_status() == 0
