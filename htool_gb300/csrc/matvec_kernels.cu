@@ -318,14 +318,17 @@ __global__ void block_copy_kernel(const BlockCopy *__restrict__ items, const dou
 }
 
 // y[c * ldy + perm[i]] (no perm: i - shift) = sum over the covering
-// clusters (largest first) of z.  A warp takes an atom (up to 32 rows at a
-// time) for G right-hand sides (grid.y): the sums are bound by the latency of
-// loads from z, and G of them times the unrolled clusters are in flight.
-// 60 000 rows, 64 right-hand sides: one atom and all of them a warp 250 us,
-// now 92 us.
-template <int G>
-__global__ void zsum_kernel(const ZItem *__restrict__ items, int nitems, const int *__restrict__ zl, const double *__restrict__ z, int zlen, int mu, const int *__restrict__ perm,
-                            double *__restrict__ y, int ldy, int shift) {
+// clusters (largest first) of z.  A warp takes an atom for up to kZsumRhs
+// right-hand sides (grid.y), its lanes side by side over rows and right-hand
+// sides, K values each: the sums are bound by the latency of loads from z, and
+// K values times the unrolled clusters are in flight.
+// 64 right-hand sides, a row a lane and four of them a warp against this: sphere
+// of 60 000 points (atoms of 12 rows) 148 -> 107 us, Helmholtz cube of 30 000 in
+// real form (30 rows) 92 -> 98 us; with 8 a warp 116 and 96 us.
+constexpr int kZsumRhs = 16;
+template <int K>
+__global__ void __launch_bounds__(256) zsum_kernel(const ZItem *__restrict__ items, int nitems, const int *__restrict__ zl, const double *__restrict__ z, int zlen, int mu,
+                                                   const int *__restrict__ perm, double *__restrict__ y, int ldy, int shift) {
     const int w    = blockIdx.x * 8 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (w >= nitems)
@@ -333,36 +336,38 @@ __global__ void zsum_kernel(const ZItem *__restrict__ items, int nitems, const i
     const ZItem it = items[w];
     const int nl   = it.lend - it.lbeg;
     const int base = lane < nl ? zl[it.lbeg + lane] : 0; // the atom's z bases, one per lane (more than 32: read again)
-    for (int c0 = blockIdx.y * G; c0 < mu; c0 += gridDim.y * G) {
-        const int nc = min(G, mu - c0);
-        for (int r0 = 0; r0 < it.h; r0 += 32) {
-            const int i      = it.row0 + min(r0 + lane, it.h - 1);
-            const double *zc = z + (long long)c0 * zlen + i;
-            double s[G];
+    for (int c0 = blockIdx.y * kZsumRhs; c0 < mu; c0 += gridDim.y * kZsumRhs) {
+        const long long n = (long long)it.h * min(kZsumRhs, mu - c0);
+        for (long long e0 = 0; e0 < n; e0 += 32 * K) {
+            const double *zc[K];
+            int row[K], col[K];
+            double s[K];
 #pragma unroll
-            for (int c = 0; c < G; c++)
-                s[c] = 0.;
+            for (int k = 0; k < K; k++) {
+                const int e = (int)min(e0 + 32 * k + lane, n - 1), c = e / it.h;
+                row[k]      = it.row0 + e - c * it.h;
+                col[k]      = c0 + c;
+                zc[k]       = z + (long long)col[k] * zlen + row[k];
+                s[k]        = 0.;
+            }
             auto add = [&](int b) {
-                double v[G];
+                double v[K];
 #pragma unroll
-                for (int c = 0; c < G; c++)
-                    v[c] = zc[(long long)min(c, nc - 1) * zlen + b];
+                for (int k = 0; k < K; k++)
+                    v[k] = zc[k][b];
 #pragma unroll
-                for (int c = 0; c < G; c++)
-                    s[c] += v[c];
+                for (int k = 0; k < K; k++)
+                    s[k] += v[k];
             };
-#pragma unroll 4
+#pragma unroll (K == 1 ? 8 : 4)
             for (int l = 0; l < min(nl, 32); l++)
                 add(__shfl_sync(0xffffffffu, base, l));
             for (int l = it.lbeg + 32; l < it.lend; l++)
                 add(zl[l]);
-            if (r0 + lane < it.h) {
-                const int dst = perm ? perm[i] : i - shift;
 #pragma unroll
-                for (int c = 0; c < G; c++)
-                    if (c < nc)
-                        y[(long long)(c0 + c) * ldy + dst] = s[c];
-            }
+            for (int k = 0; k < K; k++)
+                if (e0 + 32 * k + lane < n)
+                    y[(long long)col[k] * ldy + (perm ? perm[row[k]] : row[k] - shift)] = s[k];
         }
     }
 }
@@ -573,10 +578,11 @@ void launch_zsum(const ZItem *items, int nitems, const int *zl, const double *z,
     if (nitems <= 0)
         return;
     const int blocks = (nitems + 7) / 8;
-    if (mu >= 3)
-        zsum_kernel<4><<<dim3(blocks, std::min((mu + 3) / 4, 65535)), 256, 0, st>>>(items, nitems, zl, z, zlen, mu, perm, y, ldy, shift);
+    const dim3 grid(blocks, std::min((mu + kZsumRhs - 1) / kZsumRhs, 65535));
+    if (mu >= 4)
+        zsum_kernel<4><<<grid, 256, 0, st>>>(items, nitems, zl, z, zlen, mu, perm, y, ldy, shift);
     else
-        zsum_kernel<1><<<dim3(blocks, mu), 256, 0, st>>>(items, nitems, zl, z, zlen, mu, perm, y, ldy, shift);
+        zsum_kernel<1><<<grid, 256, 0, st>>>(items, nitems, zl, z, zlen, mu, perm, y, ldy, shift);
     HTGPU_CUDA(cudaGetLastError());
 }
 
