@@ -1226,6 +1226,15 @@ void HMatrix::ensure_work(int mu) {
     ensure_oz_work(mu);
 }
 
+// The end of a product on host arrays: the output's copy lands, and the status
+// with it (the kernel that writes the output left it in pinned host memory; a
+// copy of its own took 8 us, a tenth of a product of 4 000 points)
+void HMatrix::finish_host_product(cudaStream_t st) {
+    HTGPU_CUDA(cudaStreamSynchronize(st));
+    const int status = *static_cast<volatile int *>(note_.get());
+    require(status == 0, "a device wait of the product ran out (status " + std::to_string(status) + ")", 3);
+}
+
 void HMatrix::mvprod(const double *in, double *out, int mu, bool host_ptrs, int numbering, cudaStream_t st) {
     require(mu >= 1, "number of right-hand sides must be positive");
     require(in != nullptr && out != nullptr, "null input or output");
@@ -1233,6 +1242,12 @@ void HMatrix::mvprod(const double *in, double *out, int mu, bool host_ptrs, int 
     HTGPU_CUDA(cudaSetDevice(device_));
     if (!st)
         st = stream_;
+    if (host_ptrs && !note_) {
+        int *p = nullptr;
+        HTGPU_CUDA(cudaMallocHost((void **)&p, sizeof(int)));
+        *p = 0;
+        note_.reset(p);
+    }
     if (znative_) {
         // complex x (nc / 2 points) -> its real form w, the real product with
         // 2 mu right-hand sides, its output -> complex y (nr points, or the
@@ -1253,10 +1268,7 @@ void HMatrix::mvprod(const double *in, double *out, int mu, bool host_ptrs, int 
         launches_ += 2;
         if (host_ptrs) {
             HTGPU_CUDA(cudaMemcpyAsync(out, ystage.p, sizeof(double) * 2 * (std::size_t)mout * mu, cudaMemcpyDeviceToHost, st));
-            HTGPU_CUDA(cudaStreamSynchronize(st));
-            int status = 0;
-            HTGPU_CUDA(cudaMemcpy(&status, status_d.p, sizeof(int), cudaMemcpyDeviceToHost));
-            require(status == 0, "a device wait of the product ran out (status " + std::to_string(status) + ")", 3);
+            finish_host_product(st);
         }
         return;
     }
@@ -1272,10 +1284,7 @@ void HMatrix::mvprod(const double *in, double *out, int mu, bool host_ptrs, int 
     launch_product(x, y, mu, numbering, st);
     if (host_ptrs) {
         HTGPU_CUDA(cudaMemcpyAsync(out, ystage.p, sizeof(double) * nout, cudaMemcpyDeviceToHost, st));
-        HTGPU_CUDA(cudaStreamSynchronize(st));
-        int status = 0;
-        HTGPU_CUDA(cudaMemcpy(&status, status_d.p, sizeof(int), cudaMemcpyDeviceToHost));
-        require(status == 0, "a device wait of the product ran out (status " + std::to_string(status) + ")", 3);
+        finish_host_product(st);
     }
 }
 
@@ -2523,9 +2532,9 @@ void HMatrix::launch_pair_product(const double *x, double *y, int mu, int number
 void HMatrix::launch_pair_sums(double *y, int mu, int numbering, const double *w_z, const int *w_xexp, cudaStream_t st) {
     const float2 *zf = reinterpret_cast<const float2 *>(w_z);
     if (numbering == kGlobalToLocal)
-        launch_pair_zsum(zi_d.p + zloc0_, zloc1_ - zloc0_, zl_d.p, zf, (int)zlen_, mu, nullptr, w_xexp, y, local_row_count(), st, local_row_offset());
+        launch_pair_zsum(zi_d.p + zloc0_, zloc1_ - zloc0_, zl_d.p, zf, (int)zlen_, mu, nullptr, w_xexp, y, local_row_count(), st, local_row_offset(), status_note());
     else
-        launch_pair_zsum(zi_d.p, (int)zi_h.size(), zl_d.p, zf, (int)zlen_, mu, numbering == kUserNumbering ? perm_t.p : nullptr, w_xexp, y, nr, st);
+        launch_pair_zsum(zi_d.p, (int)zi_h.size(), zl_d.p, zf, (int)zlen_, mu, numbering == kUserNumbering ? perm_t.p : nullptr, w_xexp, y, nr, st, 0, status_note());
 }
 
 // A reduced-precision product on the warp-fed streams: per pass the split
@@ -2591,9 +2600,9 @@ void HMatrix::phase1_tc(const F2 *w_xs, int mu, double *w_A, cudaStream_t st) {
 
 void HMatrix::launch_sums(double *y, int mu, int numbering, const double *w_z, cudaStream_t st) {
     if (numbering == kGlobalToLocal)
-        launch_zsum(zi_d.p + zloc0_, zloc1_ - zloc0_, zl_d.p, w_z, (int)zlen_, mu, nullptr, y, local_row_count(), st, local_row_offset());
+        launch_zsum(zi_d.p + zloc0_, zloc1_ - zloc0_, zl_d.p, w_z, (int)zlen_, mu, nullptr, y, local_row_count(), st, local_row_offset(), status_note());
     else
-        launch_zsum(zi_d.p, (int)zi_h.size(), zl_d.p, w_z, (int)zlen_, mu, numbering == kUserNumbering ? perm_t.p : nullptr, y, nr, st);
+        launch_zsum(zi_d.p, (int)zi_h.size(), zl_d.p, w_z, (int)zlen_, mu, numbering == kUserNumbering ? perm_t.p : nullptr, y, nr, st, 0, status_note());
 }
 
 void HMatrix::set_tensor_core_mode(int mode) {

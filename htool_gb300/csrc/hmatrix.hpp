@@ -359,6 +359,12 @@ class HMatrix {
     void release_red();
     void leave_red();
     void launch_red_product(const double *x, double *y, int mu, int numbering, cudaStream_t st, double *w_xp, F2 *w_xs, int *w_xexp, double *w_A, double *w_z, cudaEvent_t *marks, bool exact);
+    struct HostFree {
+        void operator()(int *p) const { cudaFreeHost(p); }
+    };
+    std::unique_ptr<int, HostFree> note_; // the status of the last product on host arrays (from the first of them on)
+    StatusNote status_note() const { return {status_d.p, note_.get()}; }
+    void finish_host_product(cudaStream_t st);
     void launch_pair_sums(double *y, int mu, int numbering, const double *w_z, const int *w_xexp, cudaStream_t st);
     void leave_pair();
     void upload_fp64_lists();

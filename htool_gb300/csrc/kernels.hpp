@@ -113,7 +113,13 @@ void launch_reduce_tiles_f(const LrLeaf *lr, const int *multi, int nmulti, int m
 void launch_block_copy(const BlockCopy *items, int nitems, const double *src, double *dst, cudaStream_t st);
 // y[c * ldy + perm[i]] = sum of the partial sums z of the clusters covering
 // row i; without perm, y[c * ldy + i - shift]
-void launch_zsum(const ZItem *items, int nitems, const int *zl, const double *z, int zlen, int mu, const int *perm, double *y, int ldy, cudaStream_t st, int shift = 0);
+// where the last kernel of a product on host arrays leaves the product's
+// status (a word of pinned host memory; none: nowhere)
+struct StatusNote {
+    const int *status = nullptr;
+    int *host         = nullptr;
+};
+void launch_zsum(const ZItem *items, int nitems, const int *zl, const double *z, int zlen, int mu, const int *perm, double *y, int ldy, cudaStream_t st, int shift = 0, StatusNote note = {});
 
 // ---- streamed phase 2 (stream.cu) ------------------------------------------
 // warps claim the chunk ranges rbeg[r] .. rbeg[r+1] (r < nranges) through
@@ -349,7 +355,7 @@ void launch_pair_reduce(const LrLeaf *lr, const int *multi, int nmulti, int w, f
 void launch_pair_rotate(const int2 *rows, long long nrows, int w, float *A, cudaStream_t st);
 void launch_pair_phase2(const PairPanel *panels, int npanels, int *tickets, const unsigned char *mirror, const int *cidx, const float *X, float *A, int w, int nrhs, float2 *z, int zlen, int *status,
                         cudaStream_t st);
-void launch_pair_zsum(const ZItem *items, int nitems, const int *zl, const float2 *z, int zlen, int mu, const int *perm, const int *xexp, double *y, int ldy, cudaStream_t st, int shift = 0);
+void launch_pair_zsum(const ZItem *items, int nitems, const int *zl, const float2 *z, int zlen, int mu, const int *perm, const int *xexp, double *y, int ldy, cudaStream_t st, int shift = 0, StatusNote note = {});
 // the limit of its waits and a panel whose first copy is left out (set_debug_waits)
 void set_pair_waits(long long cycles, long long skip);
 // ---- reduced-precision products off the tensor cores (red.cu) --------------

@@ -328,9 +328,11 @@ __global__ void block_copy_kernel(const BlockCopy *__restrict__ items, const dou
 constexpr int kZsumRhs = 16;
 template <int K>
 __global__ void __launch_bounds__(256) zsum_kernel(const ZItem *__restrict__ items, int nitems, const int *__restrict__ zl, const double *__restrict__ z, int zlen, int mu,
-                                                   const int *__restrict__ perm, double *__restrict__ y, int ldy, int shift) {
+                                                   const int *__restrict__ perm, double *__restrict__ y, int ldy, int shift, StatusNote note) {
     const int w    = blockIdx.x * 8 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
+    if (note.host && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
+        *note.host = *note.status;
     if (w >= nitems)
         return;
     const ZItem it = items[w];
@@ -574,15 +576,15 @@ void launch_reduce_tiles_f(const LrLeaf *lr, const int *multi, int nmulti, int m
     reduce_tiles(lr, multi, nmulti, mu, A, st);
 }
 
-void launch_zsum(const ZItem *items, int nitems, const int *zl, const double *z, int zlen, int mu, const int *perm, double *y, int ldy, cudaStream_t st, int shift) {
+void launch_zsum(const ZItem *items, int nitems, const int *zl, const double *z, int zlen, int mu, const int *perm, double *y, int ldy, cudaStream_t st, int shift, StatusNote note) {
     if (nitems <= 0)
         return;
     const int blocks = (nitems + 7) / 8;
     const dim3 grid(blocks, std::min((mu + kZsumRhs - 1) / kZsumRhs, 65535));
     if (mu >= 4)
-        zsum_kernel<4><<<grid, 256, 0, st>>>(items, nitems, zl, z, zlen, mu, perm, y, ldy, shift);
+        zsum_kernel<4><<<grid, 256, 0, st>>>(items, nitems, zl, z, zlen, mu, perm, y, ldy, shift, note);
     else
-        zsum_kernel<1><<<grid, 256, 0, st>>>(items, nitems, zl, z, zlen, mu, perm, y, ldy, shift);
+        zsum_kernel<1><<<grid, 256, 0, st>>>(items, nitems, zl, z, zlen, mu, perm, y, ldy, shift, note);
     HTGPU_CUDA(cudaGetLastError());
 }
 

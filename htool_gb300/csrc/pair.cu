@@ -514,7 +514,7 @@ __global__ void pair_rotate_kernel(const int2 *__restrict__ rows, long long nrow
 // y[c * ldy + perm[i]] (no perm: i - shift) = sum over the covering clusters
 // (largest first) of z, brought back to the input's scale
 __global__ void pair_zsum_kernel(const ZItem *__restrict__ items, int nitems, const int *__restrict__ zl, const float2 *__restrict__ z, int zlen, int mu, const int *__restrict__ perm,
-                                 const int *__restrict__ xexp, double *__restrict__ y, int ldy, int shift) {
+                                 const int *__restrict__ xexp, double *__restrict__ y, int ldy, int shift, StatusNote note) {
     const int w    = blockIdx.x * 8 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     pdl_next();
@@ -524,6 +524,8 @@ __global__ void pair_zsum_kernel(const ZItem *__restrict__ items, int nitems, co
     // the atom's z bases, one per lane (more than 32 covering clusters: read again)
     const int nl = it.lend - it.lbeg, base = lane < nl ? zl[it.lbeg + lane] : 0;
     pdl_wait();
+    if (note.host && blockIdx.x == 0 && threadIdx.x == 0)
+        *note.host = *note.status;
     const int xs = max(*xexp, 1) - 1023;
     const int n  = it.h * mu;
     for (int e0 = 0; e0 < n; e0 += 32) {
@@ -700,10 +702,10 @@ void launch_pair_rotate(const int2 *rows, long long nrows, int w, float *A, cuda
     pdl_launch(pair_rotate_kernel, (int)std::min<long long>((total + 255) / 256, 4096), 256, 0, st, rows, nrows, w >> 1, reinterpret_cast<float4 *>(A));
 }
 
-void launch_pair_zsum(const ZItem *items, int nitems, const int *zl, const float2 *z, int zlen, int mu, const int *perm, const int *xexp, double *y, int ldy, cudaStream_t st, int shift) {
+void launch_pair_zsum(const ZItem *items, int nitems, const int *zl, const float2 *z, int zlen, int mu, const int *perm, const int *xexp, double *y, int ldy, cudaStream_t st, int shift, StatusNote note) {
     if (nitems <= 0)
         return;
-    pdl_launch(pair_zsum_kernel, (nitems + 7) / 8, 256, 0, st, items, nitems, zl, z, zlen, mu, perm, xexp, y, ldy, shift);
+    pdl_launch(pair_zsum_kernel, (nitems + 7) / 8, 256, 0, st, items, nitems, zl, z, zlen, mu, perm, xexp, y, ldy, shift, note);
 }
 
 void launch_pair_pack(const PairPanel *p1, int np1, const long long *osrc, const PairPanel *p2, const PairSource *s2, int np2, const PanelItem *pan, const double *fac, unsigned char *mirror,
