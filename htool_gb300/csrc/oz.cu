@@ -253,7 +253,16 @@ __device__ __forceinline__ void oz_put8_fast(unsigned char *planes, int plane_by
 struct OzQuad {
     int c[4]; // diagonals 2p, 2p + 1
 };
-__device__ __forceinline__ int oz_duo(unsigned hi, unsigned lo) { return __float2int_rn(__uint_as_float(hi)) * 128 + __float2int_rn(__uint_as_float(lo)); }
+// 128 hi + lo of two neighbouring diagonals.  Conversions to integers run at
+// 16 a clock and SM, and the accumulators are held until they are done; at most
+// four sums of 256 digit products (2^12 each) stay below 2^22, where adding
+// 1.5 2^23 leaves the integer in the low bits instead.  wide: up to 2^23.
+__device__ __forceinline__ int oz_duo(unsigned hi, unsigned lo, bool wide) {
+    if (wide)
+        return __float2int_rn(__uint_as_float(hi)) * 128 + __float2int_rn(__uint_as_float(lo));
+    constexpr float kMagic = 12582912.f;
+    return (int)(__float_as_uint(__fadd_rn(__uint_as_float(hi), kMagic)) * 128u + __float_as_uint(__fadd_rn(__uint_as_float(lo), kMagic)) - 129u * 0x4B400000u);
+}
 __device__ __forceinline__ long long oz_high(const OzQuad &q) { return (long long)q.c[0] * 16384 + q.c[1]; }
 __device__ __forceinline__ long long oz_low(const OzQuad &q) { return (long long)q.c[2] * 16384 + q.c[3]; }
 
@@ -512,10 +521,11 @@ __global__ void __launch_bounds__(128) oz_xplanes_kernel(const double *__restric
 // after the last slab of each block and pass (tensor-memory lanes 32 (warp
 // mod 4) .., warps 1-4 the first 16 right-hand sides, 5-8 the next 16, ..),
 // while the next block's copies already fly.  Bound by the hand-over of the
-// one set of accumulators tensor memory holds (40% of the MMA warp's time it
-// waits for the read-out, 50% it issues); 64 right-hand sides of a 100 000-point
-// sphere 1.13 -> 0.98 ms with a warp that issues at compile-time shapes and
-// twice the read-out warps, which take 32-bit words out before they convert.
+// one set of accumulators tensor memory holds (of the MMA warp's time a third
+// is the read-out; the memory is 60% busy); 64 right-hand sides of a
+// 100 000-point sphere 1.13 -> 0.98 ms with a warp that issues at compile-time
+// shapes and twice the read-out warps, which take 32-bit words out before they
+// convert, 0.90 ms with half the conversions to integers as FP32 additions.
 constexpr int kOzFastThreads = 576;
 
 template <int S, bool OUT64>
@@ -667,7 +677,7 @@ __global__ void __launch_bounds__(kOzFastThreads, 1) phase1_ozb_kernel(const TcB
                     tmem_ld16(tacc + (unsigned)((2 * d + 1) * kOzN), r1);
 #pragma unroll
                     for (int q = 0; q < 16; q++)
-                        x[q][d] = oz_duo(r0[q], r1[q]);
+                        x[q][d] = oz_duo(r0[q], r1[q], d >= 2); // diagonal i sums i + 1 plane products
                 }
                 fence_before();
                 __syncwarp();
@@ -1049,7 +1059,8 @@ __device__ __forceinline__ void oz2_slab_mmas(unsigned tmem, unsigned a0, unsign
 // instructions a slab and SM, the ALU pipe 66% busy; DRAM 24%).  64 right-hand
 // sides of a 100 000-point sphere: 2.70 -> 2.04 ms, most of it from the MMA
 // warp, whose single issuing thread had bound the kernel, then from the cutting
-// in 16-byte stores and the second set of accumulators.
+// in 16-byte stores and the second set of accumulators; 1.88 ms with the
+// read-out's conversions to integers as FP32 additions.
 constexpr int kOz2Threads = 832;
 
 __global__ void __launch_bounds__(kOz2Threads, 1) phase2_oz_kernel(const OzPanel *__restrict__ panels, int npanels, const unsigned char *__restrict__ parena, const int *__restrict__ prexp,
@@ -1274,7 +1285,7 @@ __global__ void __launch_bounds__(kOz2Threads, 1) phase2_oz_kernel(const OzPanel
                         tmem_ld8x2(tacc + (unsigned)(max(s0, 0) * N + 8 * h8), tacc + (unsigned)((s0 + 1) * N + 8 * h8), r0, r1);
 #pragma unroll
                         for (int q = 0; q < 8; q++)
-                            x[q].c[d] = oz_duo(d == 0 && odd ? 0u : r0[q], r1[q]);
+                            x[q].c[d] = oz_duo(d == 0 && odd ? 0u : r0[q], r1[q], false); // at most four plane products a slot
                     }
                     long long *hs = sacc + 8 * 32 * h8 + lane, *hd = hs, *ld = hs + 16 * 32;
                     if (pass_end && h8 != odd) {

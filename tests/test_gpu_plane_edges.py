@@ -31,3 +31,24 @@ def test_passes_and_panels(n, mu):
     for c in sorted({0, 1, mu // 2, mu - 1}):
         r = hm.mvprod_global_to_global(x[c].copy(), 1)
         assert np.linalg.norm(y[c] - r) < 2e-13 * np.linalg.norm(r), c
+
+
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+def test_largest_digit_sums(sign):
+    """entries and inputs whose middle digits are all -64: the plane products
+    of 256 rows sum to 2^20 each, the most an accumulator can hold"""
+    n, mu = 512, 64
+    v = -float(32 * 128**7 + 64 * sum(128**k for k in range(2, 7))) * 2.0**-54
+    pts = G.sphere(n, seed=2)
+    t = H.Cluster().build(n, pts)
+    lr = np.array([[0, 0, 256, 256, 1]], np.int32)
+    uv = np.concatenate([np.ones(256), np.full(256, sign * v)])
+    dn = np.array([[256 + 32 * k, 256 * (k % 2), 32, 256] for k in range(8)], np.int32)
+    dd = np.full(8 * 32 * 256, sign * v)
+    hm = H.HMatrix(t, t, 1e-6, 10.0).set_leaves(lr, uv, dn, dd)
+    x = np.full(n * mu, v)
+    want = sign * 256 * v * v
+    hm.set_digit_planes(True)
+    y = hm.mvprod_global_to_global(x, mu)
+    assert np.abs(y - want).max() <= 1e-13 * abs(want)
+    assert hm.device_status() == 0
