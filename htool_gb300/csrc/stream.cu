@@ -1085,6 +1085,104 @@ __device__ __forceinline__ void tile_cols(const StreamChunk &c, const unsigned c
     }
 }
 
+// n columns of one kind (FP32: 4 rows a 16-byte word, BF16: 8) of a tile of few
+// rows, W <= L words a column: lanes in groups of L, one column each, so a
+// tile of 12 rows keeps 24 or 32 lanes at work instead of two or three.  A
+// column's sums are those of tile_mixed's full width: the words' chains, then
+// the lanes' in pairs 16, 8, .. 1 apart (pairs beyond the group add zeros
+// there).  first: the kind's first column of the chunk.  FP32 / BF16 storage,
+// Laplace sphere, phase 1: 100 000 points 1 right-hand side 0.101 -> 0.095 ms, 2:
+// 0.133 -> 0.117; 200 000 points 0.201 -> 0.191 and 0.267 -> 0.242 (tiles of more
+// than 64 rows fill the warp; what is left is latency: a claim, a descriptor and
+// the x rows for every tile).
+template <int MU, int L, bool F32>
+__device__ __forceinline__ void tile_narrow(const StreamChunk &c, const uint4 *V, int W, int first, int n, int lane, const float *xsm, double *__restrict__ A, const float *__restrict__ scale, int mu,
+                                            int c0) {
+    constexpr int NG = 32 / L, R = F32 ? 4 : 8;
+    const int j = lane & (L - 1), grp = lane / L;
+    const bool live = j < W;
+    float x[R][MU];
+#pragma unroll
+    for (int cc = 0; cc < MU; cc++)
+#pragma unroll
+        for (int i = 0; i < R; i += 4) {
+            const float4 f = *reinterpret_cast<const float4 *>(xsm + cc * 256 + R * j + i);
+            x[i][cc] = f.x, x[i + 1][cc] = f.y, x[i + 2][cc] = f.z, x[i + 3][cc] = f.w;
+        }
+    auto batch = [&](int g, auto count) {
+        constexpr int P = decltype(count)::value, NV = P * MU;
+        static_assert(NV <= L, "a lane ends with one value at most");
+        // the value this lane ends with: one bit per halving of the values
+        int mine = 0, off = L / 2;
+#pragma unroll
+        for (int h = NV / 2; h > 0; h /= 2, off /= 2)
+            mine += lane & off ? h : 0;
+        const int col = g + mine / MU * NG + grp;
+        const bool out = (lane & (L / NV - 1)) == 0 && col < n;
+        const float sc = out ? __ldg(scale + c.c + first + col) : 0.f; // requested before the sums
+        float v[NV];
+#pragma unroll
+        for (int p = 0; p < P; p++) {
+            const int k   = g + p * NG + grp;
+            const uint4 w = live && k < n ? V[W * k + j] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+            for (int cc = 0; cc < MU; cc++) {
+                float a;
+                if constexpr (F32) {
+                    a = __uint_as_float(w.x) * x[0][cc];
+                    a = fmaf(__uint_as_float(w.y), x[1][cc], a);
+                    a = fmaf(__uint_as_float(w.z), x[2][cc], a);
+                    a = fmaf(__uint_as_float(w.w), x[3][cc], a);
+                } else {
+                    a = __uint_as_float(w.x << 16) * x[0][cc];
+                    a = fmaf(__uint_as_float(w.x & 0xffff0000u), x[1][cc], a);
+                    a = fmaf(__uint_as_float(w.y << 16), x[2][cc], a);
+                    a = fmaf(__uint_as_float(w.y & 0xffff0000u), x[3][cc], a);
+                    a = fmaf(__uint_as_float(w.z << 16), x[4 % R][cc], a);
+                    a = fmaf(__uint_as_float(w.z & 0xffff0000u), x[5 % R][cc], a);
+                    a = fmaf(__uint_as_float(w.w << 16), x[6 % R][cc], a);
+                    a = fmaf(__uint_as_float(w.w & 0xffff0000u), x[7 % R][cc], a);
+                }
+                v[p * MU + cc] = a;
+            }
+        }
+        int h = NV;
+#pragma unroll
+        for (int o = L / 2; o > 0; o /= 2) {
+            if (h > 1) {
+                h /= 2;
+#pragma unroll
+                for (int i = 0; i < NV / 2; i++)
+                    if (i < h) {
+                        const bool up    = lane & o;
+                        const float give = up ? v[i] : v[i + h], keep = up ? v[i + h] : v[i];
+                        v[i]             = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                    }
+            } else
+                v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        }
+        if (out)
+            reinterpret_cast<float *>(A)[(long long)(c.a + first + col) * mu + c0 + mine % MU] = v[0] * sc;
+    };
+    for (int g = 0; g < n;) {
+        const int left = (n - g + NG - 1) / NG;
+        if constexpr (4 * MU <= L)
+            if (left > 2) {
+                batch(g, std::integral_constant<int, 4>{});
+                g += 4 * NG;
+                continue;
+            }
+        if constexpr (2 * MU <= L)
+            if (left > 1) {
+                batch(g, std::integral_constant<int, 2>{});
+                g += 2 * NG;
+                continue;
+            }
+        batch(g, std::integral_constant<int, 1>{});
+        g += NG;
+    }
+}
+
 // The reduced-precision part of one phase-1 tile as one chunk: n32 FP32
 // columns (stride ld_f32(jlen) rows) followed by the BF16 columns (stride
 // ld_bf16(jlen)), both in whole 16-byte words with zero rows past the tile.
@@ -1106,6 +1204,8 @@ __device__ __forceinline__ void tile_mixed(const StreamChunk &c, const unsigned 
 #pragma unroll
         for (int q = 0; q < 8; q++) {
             const int row = lane + 32 * q;
+            if (jlen <= 64 && 32 * q >= jlen) // not read there
+                break;
 #pragma unroll
             for (int cc = 0; cc < MU; cc++)
                 xsm[cc * 256 + row] = row < jlen ? X[(long long)row * mu + cc].hi : 0.f;
@@ -1113,6 +1213,20 @@ __device__ __forceinline__ void tile_mixed(const StreamChunk &c, const unsigned 
         __syncwarp();
         xrow = c.b;
         xlen = jlen;
+    }
+    if (jlen <= 64) {
+        const uint4 *V32 = reinterpret_cast<const uint4 *>(buf), *V16 = V32 + W32 * n32;
+        if (jlen <= 16) {
+            tile_narrow<MU, 4, true>(c, V32, W32, 0, n32, lane, xsm, A, scale, mu, c0);
+            tile_narrow<MU, 2, false>(c, V16, W16, n32, ncol - n32, lane, xsm, A, scale, mu, c0);
+        } else if (jlen <= 32) {
+            tile_narrow<MU, 8, true>(c, V32, W32, 0, n32, lane, xsm, A, scale, mu, c0);
+            tile_narrow<MU, 4, false>(c, V16, W16, n32, ncol - n32, lane, xsm, A, scale, mu, c0);
+        } else {
+            tile_narrow<MU, 16, true>(c, V32, W32, 0, n32, lane, xsm, A, scale, mu, c0);
+            tile_narrow<MU, 8, false>(c, V16, W16, n32, ncol - n32, lane, xsm, A, scale, mu, c0);
+        }
+        return;
     }
     float xf[8][MU], xb[8][MU];
 #pragma unroll

@@ -77,3 +77,27 @@ def test_rows_of_more_than_a_window_of_chunks(mu):
     hm.set_phase2_mode("warp")
     assert rel(y, hm.mvprod_global_to_global(x, mu)) < TOL
     assert hm.device_status() == 0
+
+
+@pytest.mark.parametrize("policy", ["fp32", "mixed", "bf16"])
+def test_narrow_tiles_exact(policy):
+    """low-rank leaves of 1 to 66 columns: tiles whose columns share a warp.
+    Factors of +-1 and inputs of small integers make every sum exact in FP32, in
+    any order and storage"""
+    n = 4096
+    rng = np.random.default_rng(3)
+    t = H.Cluster().build(n, G.sphere(n, seed=8))
+    sizes = [(j, r) for j in (1, 3, 4, 5, 12, 16, 17, 24, 31, 32, 33, 48, 63, 64, 65, 66) for r in (1, 4, 9, 33)]
+    lr = np.array([[8 * k, (67 * k) % 4000, 8, j, r] for k, (j, r) in enumerate(sizes)], np.int32)
+    sign = lambda *s: rng.choice([-1.0, 1.0], s)
+    uvs = [(sign(8, r), sign(r, j)) for j, r in sizes]
+    uv = np.concatenate([np.concatenate([u.ravel(order="F"), v.ravel(order="F")]) for u, v in uvs])
+    hm = H.HMatrix(t, t, 1e-6, 10.0).set_leaves(lr, uv, np.empty((0, 4), np.int32), np.empty(0)).set_precision(policy, 1.0)
+    perm = t.get_perm()
+    for mu in (1, 2):
+        x = rng.integers(-8, 9, (mu, n)).astype(np.float64)
+        want = np.zeros((mu, n))
+        for (oi, oj, m, j, r), (u, v) in zip(lr, uvs):
+            want[:, perm[oi:oi + m]] += (u @ (v @ x[:, perm[oj:oj + j]].T)).T
+        y = np.asarray(hm.mvprod_global_to_global(x.ravel(), mu)).reshape(mu, n)
+        assert np.array_equal(y, want), mu
