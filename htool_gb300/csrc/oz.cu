@@ -932,8 +932,8 @@ __global__ void __launch_bounds__(kOzThreads, S <= 4 ? 2 : 1) phase1_oz_kernel(c
 //
 //     z^T (mu x h) = C^T (mu x ncol) P^T (ncol x h),
 //
-// M = 128 right-hand-side rows (64 used per pass, the rest zero), N = h
-// rounded up to 16 or 32, K = 16 columns a slab.  The panel's planes (B,
+// M = 128 rows (two coefficient planes of 64 right-hand sides), N = h rounded
+// up to 16 or 32, K = 16 columns a slab.  The panel's planes (B,
 // N x 16 a slab) are laid out once (oz_panel_pack_kernel); the threads cut
 // the coefficients into planes (A) relative to a bound on the panel's
 // largest coefficient for each right-hand side (the maxima of the 32-row
