@@ -337,6 +337,8 @@ def run_gpu(args):
             p2 = "phase2_warp_kernel" if hm.get_phase2_mode() == 0 else "phase2_ws_kernel"
         if precision == "fp64" and int(hm.get_infos()["GPU_paired_panels"]) > 0 and not (run >= 8 and hm.get_digit_planes()[0]):
             p1 = p2 = "pair_kernel"
+        if precision != "fp64" and int(hm.get_infos()["GPU_reduced_streams"]) > 0 and not (run >= 8 and (hm.get_digit_planes()[0] or WORKLOAD["epsilon"] >= 1e-5)):
+            p1, p2 = ("red1_kernel" if run >= 3 else "phase1_cta_kernel"), "red2_kernel"
         names = ["gather_split_kernel", p1, p2, "zsum_kernel"]
         k = max(range(4), key=lambda i: ph[i])
         achieved = pb[k] / (ph[k] / 1e3) / 1e9

@@ -66,13 +66,15 @@ void stack_tiles(const std::vector<P1Item> &items, const std::vector<LrLeaf> &lr
 // (20 000 points 0.105 -> 0.093 ms, 50 000 with 8 right-hand sides 0.53 ->
 // 0.48).  More: as they lie, so that long panels, bound by HBM, run beside short
 // ones, bound by their set-up (400 000 points: 1.58 ms, the short ones last
-// 1.63).  A stable counting sort.
-std::vector<int> claim_order(const std::vector<PairPanel> &pan) {
+// 1.63).  Panels of dense columns alone are of much the same length and always
+// sorted (400 000 points, reduced precision: phase 2 0.580 -> 0.570 ms).  A
+// stable counting sort.
+std::vector<int> claim_order(const std::vector<PairPanel> &pan, bool dense_only = false) {
     constexpr int kKeys        = 4096;
     constexpr std::size_t kFew = 24576;
     std::vector<int> by(pan.size());
     std::iota(by.begin(), by.end(), 0);
-    if (pan.size() >= kFew)
+    if (pan.size() >= kFew && !dense_only)
         return by;
     auto key = [&](const PairPanel &p) { return kKeys - 1 - std::min<long long>(kKeys - 1, (long long)p.ncol * ((p.h + 1) / 2) / 64); };
     std::vector<int> at(kKeys + 1, 0);
@@ -1534,7 +1536,7 @@ bool HMatrix::build_pair(bool dense_only) {
             off += 16LL * ncol * ((h + 1) / 2);
         }
     }
-    const std::vector<int> by1 = claim_order(pan1), by2 = claim_order(pan2);
+    const std::vector<int> by1 = claim_order(pan1), by2 = claim_order(pan2, dense_only);
     permute(pan1, by1);
     permute(pan2, by2);
     permute(src2, by2);
@@ -2348,9 +2350,7 @@ void HMatrix::launch_product_with(const double *x, double *y, int mu_out, int nu
     launches_        = 0;
     // many right-hand sides on the tensor cores when epsilon leaves room for their FP32 sums
     const bool mma = mu >= kMmaMinRhs && eps_ >= kMmaMinEps;
-    // (one right-hand side stays on the producer-fed chunks: their bookkeeping
-    // runs on a warp of its own; 100 000 points 0.265 ms against 0.252 ms, 200 000 0.505 against 0.526)
-    if (red_ready_ && precision_ != 0 && mu >= 2 && !mma && !(mu >= kMmaMinRhs && oz_S_ == 4 && w_oz && n_tcblk_ > 0)) {
+    if (red_ready_ && precision_ != 0 && !mma && !(mu >= kMmaMinRhs && oz_S_ == 4 && w_oz && n_tcblk_ > 0)) {
         launch_red_product(x, y, mu_out, numbering, st, w_xp, w_xs, w_xexp, w_A, w_z, marks, w_A != A.p);
         return;
     }
@@ -2685,11 +2685,11 @@ void HMatrix::autotune(int mu, int reps, float *best_ms) {
         else
             set_digit_planes(was);
     };
-    if (precision_ != 0 && !red_ready_ && emu_ok_ && presplit_on_ && mu >= 2 && !(mu >= kMmaMinRhs && eps_ >= kMmaMinEps)) {
+    if (precision_ != 0 && !red_ready_ && emu_ok_ && presplit_on_ && !(mu >= kMmaMinRhs && eps_ >= kMmaMinEps)) {
         red_auto_ = true; // back from a caller's choice
         set_precision(precision_, tau_);
     }
-    if (red_ready_ && precision_ != 0 && mu >= 2 && !(mu >= kMmaMinRhs && eps_ >= kMmaMinEps)) {
+    if (red_ready_ && precision_ != 0 && !(mu >= kMmaMinRhs && eps_ >= kMmaMinEps)) {
         // the warp-fed streams, with many right-hand sides against the digit planes
         best = timed();
         if (mu >= kMmaMinRhs && n_tcblk_ > 0)
@@ -3300,6 +3300,7 @@ std::map<std::string, std::string> HMatrix::infos() const {
     m["GPU_phase1_mode"]               = inum(p1_mode_);
     m["GPU_presplit_bytes"]            = inum(presplit_bytes());
     m["GPU_paired_panels"]             = inum(pair_ready_ ? n_pair1_ + n_pair2_ : 0);
+    m["GPU_reduced_streams"]           = inum(red_ready_ ? n_red1_ : 0);
     return m;
 }
 

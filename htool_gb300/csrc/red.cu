@@ -18,13 +18,13 @@
 // and their order are those of phase1_stack_kernel and of the chunk kernels in
 // stream.cu, which a caller's choice of mode keeps.
 //
-// Bound by latency (12 to 16 warps an SM, the memory 60% busy with 8 right-hand
-// sides; reading half the coefficients, two rows a lane, gained 1%), so
-// descriptors and indices are loaded ahead and a row chunk starts from its
-// dense part.  Measured against those kernels, Laplace sphere, FP32/BF16
-// factors, ms a product: 100 000 points 2 right-hand sides 0.365 -> 0.309, 4:
-// 0.726 -> 0.348, 8: 1.835 -> 0.475; 200 000 points 8: 3.68 -> 0.922.  Every
-// wait is bounded (status 2).
+// Bound by latency (20 warps an SM, in phase 2 with 6 and 8 right-hand sides 12;
+// reading half the coefficients, two rows a lane, gained 1%), so descriptors and
+// indices are loaded ahead and a row chunk starts from its dense part.  Measured
+// against those kernels, Laplace sphere, FP32/BF16 factors, ms a product:
+// 100 000 points 1 right-hand side 0.258 -> 0.232, 2: 0.365 -> 0.276, 4: 0.726 ->
+// 0.304, 8: 1.835 -> 0.435; 200 000 points 1: 0.499 -> 0.467, 8: 3.68 -> 0.813.
+// Every wait is bounded (status 2).
 #include "f32x2.cuh"
 #include "kernels.hpp"
 
@@ -35,7 +35,12 @@ namespace htgpu {
 namespace {
 
 constexpr int kRedWarps  = 4; // warps per CTA, each with its own ring
-constexpr int kRedStages = 3;
+// Stages per warp.  Twenty warps an SM with one stage on its way each beat
+// twelve or sixteen with two (ms of 200 000 points, 3 stages and what then fits
+// against this: 1 right-hand side 0.508 -> 0.469, 2: 0.601 -> 0.533, 4: 0.636 ->
+// 0.55, 8: 0.904 -> 0.81); 6 and 8 right-hand sides keep 12 warps in phase 2,
+// where 16 or 20 leave too few registers (0.52 and more against 0.50 ms).
+constexpr int kRedStages = 2;
 
 // floor(t / d) for 0 <= t < 128, 1 <= d <= 32 (exact: the product overshoots
 // t / d by less than 128 / 65536, below the 1 / d gap to the next integer)
@@ -98,7 +103,7 @@ struct Red1Cfg {
     static constexpr int kBar   = kRedStages * kStage;
     static constexpr int kWarp  = (kBar + 8 * kRedStages + 127) & ~127;
     static constexpr int kSmem  = kRedWarps * kWarp;
-    static constexpr int kCtas  = 3;
+    static constexpr int kCtas  = 5;
 };
 
 template <int W>
@@ -258,7 +263,7 @@ struct Red2Cfg {
     static constexpr int kBar   = kRedStages * kStage;
     static constexpr int kWarp  = (kBar + 8 * kRedStages + 127) & ~127;
     static constexpr int kSmem  = kRedWarps * kWarp;
-    static constexpr int kCtas  = W >= 4 ? 3 : 4; // what the shared memory holds
+    static constexpr int kCtas  = W <= 4 ? 5 : 3;
 };
 
 template <int W>
