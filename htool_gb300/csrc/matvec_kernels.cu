@@ -34,18 +34,32 @@ namespace {
 
 constexpr int kWarpsPerBlock = 8; // phase 1: warps per CTA
 
-// biased exponent of max |x| over the input (atomicMax on the exponent field)
-__global__ void xexp_kernel(const double *__restrict__ x, long long total, int *__restrict__ xexp) {
-    int m = 0;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-        const int ex = (int)(((unsigned)__double2hiint(x[e]) >> 20) & 0x7FFu);
-        m            = max(m, ex == 0x7FF ? 0 : ex);
-    }
+// biased exponent of max |x| over the input (atomicMax on the exponent field).
+// One atomic a CTA: one a warp met at the one address, 9 700 of them for 400 000
+// entries (9.0 -> 3.5 us).  Eight loads a thread in flight.
+constexpr int kXexpThreads = 256;
+__global__ void __launch_bounds__(kXexpThreads) xexp_kernel(const double *__restrict__ x, long long total, int *__restrict__ xexp) {
+    __shared__ int sm[kXexpThreads / 32];
+    const long long step = (long long)gridDim.x * blockDim.x;
+    int m                = 0;
+    for (long long e0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; e0 < total; e0 += 8 * step) {
+        int ex[8];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-        m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0 && m > 0)
-        atomicMax(xexp, m);
+        for (int k = 0; k < 8; k++)
+            ex[k] = (int)(((unsigned)__double2hiint(x[min(e0 + k * step, total - 1)]) >> 20) & 0x7FFu);
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            m = max(m, ex[k] == 0x7FF ? 0 : ex[k]);
+    }
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0)
+        sm[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        m = __reduce_max_sync(0xffffffffu, threadIdx.x < kXexpThreads / 32 ? sm[threadIdx.x] : 0);
+        if (threadIdx.x == 0 && m > 0)
+            atomicMax(xexp, m);
+    }
 }
 
 // xp[j*mu + c] = x[c*ldx + perm[j]] and xs = split(xp * 2^(1023 - xexp));
@@ -410,8 +424,9 @@ void launch_xexp(const double *x, long long total, int *xexp, cudaStream_t st) {
     HTGPU_CUDA(cudaMemsetAsync(xexp, 0, sizeof(int), st));
     if (total <= 0)
         return;
-    int blocks = (int)std::min<long long>((total + 255) / 256, (long long)sm_count() * 8);
-    xexp_kernel<<<blocks, 256, 0, st>>>(x, total, xexp);
+    // two entries a thread at least: fewer atomics, and small inputs stay spread over the SMs
+    const int blocks = (int)std::max<long long>(1, std::min<long long>((total + 2 * kXexpThreads - 1) / (2 * kXexpThreads), (long long)sm_count() * 4));
+    xexp_kernel<<<blocks, kXexpThreads, 0, st>>>(x, total, xexp);
     HTGPU_CUDA(cudaGetLastError());
 }
 
