@@ -2506,11 +2506,17 @@ void HMatrix::launch_pair_product(const double *x, double *y, int mu, int number
     float *X = reinterpret_cast<float *>(w_xs), *Af = reinterpret_cast<float *>(w_A);
     float2 *zf   = reinterpret_cast<float2 *>(w_z);
     int *tickets = tickets_d.p + 10;
-    launch_xexp(x, (long long)nc * mu, w_xexp, st);
-    launches_ = 1;
+    const int *perm  = numbering == kUserNumbering ? perm_s.p : nullptr;
+    const bool small = (long long)nc * mu <= kPairPrepMax && pair_pass_width(mu, exact) >= mu;
+    if (!small)
+        launch_xexp(x, (long long)nc * mu, w_xexp, st);
+    launches_ = small ? 0 : 1;
     for (int c0 = 0; c0 < mu;) {
         const int w = pair_pass_width(mu - c0, exact), n = std::min(w, mu - c0);
-        launch_pair_gather(x, nc, numbering == kUserNumbering ? perm_s.p : nullptr, nc, c0, w, mu, w_xexp, X, tickets, st);
+        if (small)
+            launch_pair_prep(x, perm, nc, w, mu, w_xexp, X, tickets, st);
+        else
+            launch_pair_gather(x, nc, perm, nc, c0, w, mu, w_xexp, X, tickets, st);
         if (marks && c0 == 0)
             HTGPU_CUDA(cudaEventRecord(marks[0], st));
         launch_pair_phase1(pair1_d.p, n_pair1_, tickets, pair_d.p, pairo_d.p, X, Af, w, status_d.p, st);

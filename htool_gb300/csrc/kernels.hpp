@@ -349,6 +349,9 @@ void launch_pair_pack(const PairPanel *p1, int np1, const long long *osrc, const
 // (slots x w), the sums of multi-tile leaves, i times the sums (native complex
 // layout), the partial sums z of the first nrhs of them (zlen apart), and
 // the final sums over all mu
+// both the exponent and the gathered input of an input of one pass and at most kPairPrepMax entries
+constexpr int kPairPrepMax = 3072;
+void launch_pair_prep(const double *x, const int *perm, int n, int w, int mu_src, int *xexp, float *X, int *tickets, cudaStream_t st);
 void launch_pair_gather(const double *x, int ldx, const int *perm, int n, int c0, int w, int mu_src, const int *xexp, float *X, int *tickets, cudaStream_t st);
 void launch_pair_phase1(const PairPanel *panels, int npanels, int *tickets, const unsigned char *mirror, const int *oslot, const float *X, float *A, int w, int *status, cudaStream_t st);
 void launch_pair_reduce(const LrLeaf *lr, const int *multi, int nmulti, int w, float *A, cudaStream_t st);

@@ -429,16 +429,11 @@ __global__ void __launch_bounds__(32 * kPairWarps, PairCfg<0>::kCtas)
 }
 
 // the gathered input of right-hand sides c0 .. c0 + w (those past mu_src
-// zero), split relative to the input's largest exponent: [row][q] of
-// {hi, hi, lo, lo}, w = 1: [row] of (hi, lo); also clears the three tickets
-__global__ void pair_gather_kernel(const double *__restrict__ x, int ldx, const int *__restrict__ perm, int n, int c0, int w, int mu_src, const int *__restrict__ xexp, float *__restrict__ X,
-                                   int *__restrict__ tickets) {
-    pdl_next();
-    pdl_wait();
-    if (blockIdx.x == 0 && threadIdx.x < 3)
-        tickets[threadIdx.x] = 0;
-    const int shift = 1023 - max(*xexp, 1);
-    auto value      = [&](int src, int c) {
+// zero), split relative to the input's largest exponent (shift = 1023 - it):
+// [row][q] of {hi, hi, lo, lo}, w = 1: [row] of (hi, lo); entries e, e + step, ..
+__device__ __forceinline__ void pair_gather_rows(const double *__restrict__ x, int ldx, const int *__restrict__ perm, int n, int c0, int w, int mu_src, int shift, float *__restrict__ X, long long e,
+                                                 long long step) {
+    auto value = [&](int src, int c) {
         F2 r{0.f, 0.f};
         if (c >= mu_src)
             return r;
@@ -450,7 +445,7 @@ __global__ void pair_gather_kernel(const double *__restrict__ x, int ldx, const 
     };
     const int Q           = w == 1 ? 1 : w >> 1;
     const long long total = (long long)n * Q;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
+    for (; e < total; e += step) {
         const int j = (int)(e / Q), q = (int)(e - (long long)j * Q);
         const int src = perm ? perm[j] : j;
         if (w == 1) {
@@ -461,6 +456,48 @@ __global__ void pair_gather_kernel(const double *__restrict__ x, int ldx, const 
             reinterpret_cast<float4 *>(X)[e] = make_float4(a.hi, b.hi, a.lo, b.lo);
         }
     }
+}
+// clears the three tickets too
+__global__ void pair_gather_kernel(const double *__restrict__ x, int ldx, const int *__restrict__ perm, int n, int c0, int w, int mu_src, const int *__restrict__ xexp, float *__restrict__ X,
+                                   int *__restrict__ tickets) {
+    pdl_next();
+    pdl_wait();
+    if (blockIdx.x == 0 && threadIdx.x < 3)
+        tickets[threadIdx.x] = 0;
+    pair_gather_rows(x, ldx, perm, n, c0, w, mu_src, 1023 - max(*xexp, 1), X, blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
+}
+
+// A small input (of one pass) in one kernel of one CTA: its largest exponent,
+// the tickets and the gathered input.  A small product is a chain of kernels of
+// 2 to 8 us, and this takes one out: 1 000 points 19.2 -> 16.4 us a product, 3 000
+// 26.1 -> 24.6.  Beyond that one CTA takes longer than the launch it saves (4 000
+// points with eight loads a thread 26.6 us, with two kernels 25.9).
+constexpr int kPrepThreads = 1024, kPrepLoads = 3;
+static_assert(kPrepThreads * kPrepLoads == kPairPrepMax, "an input read in one step");
+__global__ void __launch_bounds__(kPrepThreads) pair_prep_kernel(const double *__restrict__ x, const int *__restrict__ perm, int n, int w, int mu_src, int *__restrict__ xexp, float *__restrict__ X,
+                                                                 int *__restrict__ tickets) {
+    __shared__ int sm[kPrepThreads / 32];
+    pdl_next();
+    if (threadIdx.x < 3)
+        tickets[threadIdx.x] = 0;
+    const int total = n * mu_src;
+    int ex[kPrepLoads], m = 0;
+#pragma unroll
+    for (int k = 0; k < kPrepLoads; k++) {
+        const int e = (int)threadIdx.x + kPrepThreads * k;
+        ex[k]       = e < total ? (int)(((unsigned)__double2hiint(x[e]) >> 20) & 0x7FFu) : 0;
+    }
+#pragma unroll
+    for (int k = 0; k < kPrepLoads; k++)
+        m = max(m, ex[k] == 0x7FF ? 0 : ex[k]);
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0)
+        sm[threadIdx.x >> 5] = m;
+    __syncthreads();
+    m = __reduce_max_sync(0xffffffffu, sm[threadIdx.x & 31]);
+    if (threadIdx.x == 0)
+        *xexp = m;
+    pair_gather_rows(x, n, perm, n, 0, w, mu_src, 1023 - max(m, 1), X, threadIdx.x, kPrepThreads);
 }
 
 // the tiles' sums of every multi-tile leaf into the first tile's slots
@@ -677,6 +714,11 @@ void launch_pair_gather(const double *x, int ldx, const int *perm, int n, int c0
     const long long total = (long long)n * (w == 1 ? 1 : w >> 1);
     const int blocks      = (int)std::max<long long>(1, std::min<long long>((total + 255) / 256, 16LL * pair_sms()));
     pdl_launch(pair_gather_kernel, blocks, 256, 0, st, x, ldx, perm, n, c0, w, mu_src, xexp, X, tickets);
+}
+
+void launch_pair_prep(const double *x, const int *perm, int n, int w, int mu_src, int *xexp, float *X, int *tickets, cudaStream_t st) {
+    pair_prep_kernel<<<1, kPrepThreads, 0, st>>>(x, perm, n, w, mu_src, xexp, X, tickets);
+    HTGPU_CUDA(cudaGetLastError());
 }
 
 void launch_pair_phase1(const PairPanel *panels, int npanels, int *tickets, const unsigned char *mirror, const int *oslot, const float *X, float *A, int w, int *status, cudaStream_t st) {

@@ -119,3 +119,21 @@ def test_a_wait_that_runs_out_is_reported(n):
     hm.reset_status()
     assert np.array_equal(hm.mvprod_global_to_global(x), y)
     assert hm.device_status() == 0
+
+
+# inputs of 3 072 entries are gathered by one CTA with their exponent, of
+# 16 384 have the exponent from one CTA
+@pytest.mark.parametrize("n,mu", [(3072, 1), (3073, 1), (1536, 2), (1537, 2), (1024, 3), (384, 8), (385, 8), (341, 9), (16384, 1), (16385, 1)])
+def test_small_inputs(n, mu):
+    pts = G.sphere(n, seed=n)
+    t = H.Cluster().build(n, pts)
+    hm = H.HMatrix(t, t, 1e-6, 10.0).build(H.LAPLACE, pts)
+    x = G.rhs(n, mu, seed=mu) * 1e30
+    x[:n] *= 2.0**-40  # the largest entries lie behind the first right-hand side
+    if mu == 1:
+        x[n - 1] = 3e33
+    y = np.asarray(hm.mvprod_global_to_global(x, mu)).reshape(mu, n)
+    hm.set_fp64_split(1000, 1000)
+    r = np.asarray(hm.mvprod_global_to_global(x, mu)).reshape(mu, n)
+    assert rel(y, r) < PIPE_TOL
+    assert hm.device_status() == 0
