@@ -360,7 +360,9 @@ int htgpu_hmatrix_phase_bytes(htgpu_hmatrix h, int mu, long long *bytes);
  * until a call of this function, htgpu_hmatrix_set_phase1_mode,
  * htgpu_hmatrix_set_phase2_mode or htgpu_hmatrix_set_presplit chooses the
  * kernels these functions configure; htgpu_hmatrix_autotune brings the
- * panels back.  Where the panels do not fit in three quarters of the free
+ * panels back.  Reduced-precision products off the tensor cores likewise run
+ * on streams of their own, their dense blocks on paired panels, until one of
+ * these calls.  Where the panels do not fit in three quarters of the free
  * memory, or a stored entry is too large for the emulation, those kernels
  * run with the defaults. */
 int htgpu_hmatrix_set_fp64_split(htgpu_hmatrix h, int phase1_dfma_permille, int phase2_dfma_permille);
