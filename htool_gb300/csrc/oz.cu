@@ -213,7 +213,8 @@ __device__ __forceinline__ void oz_put8(unsigned char *planes, int plane_bytes, 
 __device__ __forceinline__ unsigned long long oz_fields2x(double v, int emax) { // 2 (q + bias), rounded in its lowest bit
     constexpr unsigned long long kBias = 64ull * ((1ull << 56) - 1) / 127; // 64 at each of the eight positions
     const unsigned vh = (unsigned)__double2hiint(v), vl = (unsigned)__double2loint(v);
-    const int r       = min(emax - (int)((vh >> 20) & 0x7FFu), 63); // a zero or subnormal shifts out
+    const int e       = (int)((vh >> 20) & 0x7FFu);
+    const int r       = e ? min(emax - e, 63) : 63; // a zero or subnormal shifts out whatever the bound is
     const unsigned mh = (vh & 0xFFFFFu) | 0x100000u;
     unsigned h = __funnelshift_l(vl, mh, 2), l = vl << 2;
     if (r >= 32) {
