@@ -278,10 +278,6 @@ __global__ void __launch_bounds__(32 * kRedWarps, Red2Cfg<W>::kCtas)
     unsigned long long *bar = reinterpret_cast<unsigned long long *>(wbase + C::kBar);
     if (lane == 0)
         ring_init(bar, kRedStages);
-    // coefficients past a chunk's columns meet zero data: they only must be numbers
-    for (int s = 0; s < kRedStages; s++)
-        for (int i = lane; i < (C::kDesc - C::kCoef) / 4; i += 32)
-            reinterpret_cast<float *>(wbase + (size_t)s * C::kStage + C::kCoef)[i] = 0.f;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncwarp();
     const unsigned long long pol = stream_policy();
@@ -374,21 +370,35 @@ __global__ void __launch_bounds__(32 * kRedWarps, Red2Cfg<W>::kCtas)
                 *reinterpret_cast<int2 *>(st + C::kDesc) = make_int2(d0.m, d0.b);
                 ring_copy(st, mix + d0.src, (unsigned)d0.bytes, &bar[s], pol);
             }
+            // past the chunk's columns, up to the last group's end, the data are
+            // zero; the coefficients there must be numbers of this chunk's own
+            // (the stage's last chunk may have left a NaN): zero
+            const int S = red_div(32, d0.m & 255), lv = ((d0.m >> 16) & 255) == kStreamF32 ? 2 : 3;
+            const int end = ((red_div(ncol + S - 1, S) + (1 << lv) - 1) >> lv) * (S << lv);
             if constexpr (W == 1) {
-                const int S = red_div(32, d0.m & 255), lv = ((d0.m >> 16) & 255) == kStreamF32 ? 2 : 3;
 #pragma unroll
-                for (int r = 0; r < 2; r++) {
+                for (int r = 0; r < 4; r++) {
                     const int t = lane + 32 * r;
-                    if (t < ncol) {
+                    if (t < end) {
                         const int jj = red_div(t, S), sl = t - jj * S;
-                        copy_async<4>(cf + ((((jj >> lv) * S + sl) << lv) | (jj & ((1 << lv) - 1))), A + (r ? d0.ix1 : d0.ix0));
+                        float *c     = cf + ((((jj >> lv) * S + sl) << lv) | (jj & ((1 << lv) - 1)));
+                        if (t < ncol)
+                            copy_async<4>(c, A + (r ? d0.ix1 : d0.ix0));
+                        else
+                            *c = 0.f;
                     }
                 }
             } else {
-                if (lane < ncol)
-                    copy_row<W>(cf + W * lane, A + (long long)W * d0.ix0);
-                if (lane + 32 < ncol)
-                    copy_row<W>(cf + W * (lane + 32), A + (long long)W * d0.ix1);
+#pragma unroll
+                for (int r = 0; r < 2; r++) {
+                    const int t = lane + 32 * r;
+                    if (t < ncol)
+                        copy_row<W>(cf + W * t, A + (long long)W * (r ? d0.ix1 : d0.ix0));
+                    else if (t < end)
+#pragma unroll
+                        for (int i = 0; i < W; i += 2)
+                            *reinterpret_cast<float2 *>(cf + W * t + i) = make_float2(0.f, 0.f);
+                }
             }
             issued++;
             d0 = d1;
