@@ -1185,6 +1185,7 @@ void HMatrix::finalize(const std::vector<const double *> &bufs, const std::vecto
     assign_phase1_modes();
     emu_fresh_ = false; // fac was rewritten
     precision_ = 0;
+    release_red(); // the streams of the factors before
     upload_fp64_lists();
     lr_d.upload(lr_h, stream_);
     rot_d.upload(rot_h, stream_);
