@@ -108,6 +108,12 @@ int max_profitable_rank(int M, int N) {
 constexpr int kPhase1Chunk = 256;  // source rows per phase-1 warp (tile)
 constexpr int kRowChunk    = 32;   // target rows per phase-2 warp
 constexpr int kDefaultCap  = 48;   // initial ACA scratch columns per block
+// Target rows of an atom of the final sums, which a warp takes: without a limit
+// a cluster in one leaf's rows is one atom, and one warp sums it.  Two spheres of
+// 60 000 points far apart, us a product, without / 128 / 64 / 32 rows: 1 right-
+// hand side 1402 / 31.4 / 29.6 / 29.3, 64: 92 400 / 875 / 716 / 649; leaves of 100
+// rows (50 000 points), 8: 668 / 635 / 599 / 575; of 10 rows the same.
+constexpr int kAtomRows = 32;
 
 std::string num(double v) {
     std::ostringstream os;
@@ -1094,8 +1100,9 @@ void HMatrix::finalize(const std::vector<const double *> &bufs, const std::vecto
             copies[b].insert(copies[b].end(), rcopies[(std::size_t)rg][b].begin(), rcopies[(std::size_t)rg][b].end());
         fills.insert(fills.end(), rfills[(std::size_t)rg].begin(), rfills[(std::size_t)rg].end());
     }
-    // z sums: target rows cut at every group boundary into atoms; every atom
-    // lists the z bases of the groups covering it, largest group first
+    // z sums: target rows cut at every group boundary into atoms of at most
+    // kAtomRows rows; every atom lists the z bases of the groups covering it,
+    // largest group first
     {
         const int loff = local_row_offset(), lend = loff + local_row_count();
         std::vector<int> cuts{0, nr, loff, lend}; // the local rows are whole atoms
@@ -1108,7 +1115,7 @@ void HMatrix::finalize(const std::vector<const double *> &bufs, const std::vecto
             atom_of[c] = 1;
         cuts.clear();
         for (int row = 0; row <= nr; row++) {
-            const bool cut = atom_of[row] != 0;
+            const bool cut = atom_of[row] != 0 || row - cuts.back() == kAtomRows;
             atom_of[row]   = (int)cuts.size();
             if (cut)
                 cuts.push_back(row);
