@@ -586,8 +586,9 @@ class HMatrix:
         multiply-adds run on the FP64 pipe; the rest uses the FP32-pipe
         double-float emulation.  Under a reduced precision, the phase-2 share
         applies to that product's dense blocks (each precision keeps its own
-        split).  FP64 products run on paired panels until this, a phase mode
-        or set_presplit chooses other kernels; autotune brings them back."""
+        split).  FP64 products run on paired panels until this, or a change
+        of a phase mode or of set_presplit, chooses other kernels; autotune
+        brings them back."""
         _check(lib.htgpu_hmatrix_set_fp64_split(self.h, int(phase1_dfma_permille), int(phase2_dfma_permille)))
 
     def get_fp64_split(self):

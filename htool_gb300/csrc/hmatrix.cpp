@@ -2628,6 +2628,8 @@ void HMatrix::set_tensor_core_mode(int mode) {
 void HMatrix::set_phase2_mode(int mode) {
     layout_gen_++; // captured products are stale
     require(mode == 0 || mode == 1, "phase-2 mode must be 0 (per-warp streams) or 1 (producer-fed)");
+    if (mode == p2_mode_) // no choice made
+        return;
     p2_mode_ = mode;
     leave_red();
     leave_pair();
@@ -2636,12 +2638,26 @@ void HMatrix::set_phase2_mode(int mode) {
 void HMatrix::set_phase1_mode(int mode) {
     layout_gen_++; // buffers or launch lists change: captured products are stale
     require(mode >= 0 && mode <= 2, "phase-1 mode must be 0 (tile kernels), 1 (streamed chunks) or 2 (tensor cores for reduced-precision products with 8 or more right-hand sides)");
+    if (mode == p1_mode_) // no choice made
+        return;
     p1_mode_ = mode;
     leave_red();
     leave_pair();
 }
 
+void HMatrix::set_phase2_dense_split(bool on) {
+    layout_gen_++; // captured products are stale
+    if (on == split_dense_) // no choice made
+        return;
+    split_dense_ = on;
+    leave_red();
+}
+
 void HMatrix::set_presplit(bool on) {
+    if (on == presplit_on_) { // no choice made
+        layout_gen_++;
+        return;
+    }
     HTGPU_CUDA(cudaSetDevice(device_));
     leave_red();
     presplit_on_ = on;

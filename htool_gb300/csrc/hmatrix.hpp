@@ -228,11 +228,7 @@ class HMatrix {
     // tensor cores: the dense FP64 chunks in the streamed phase-2 kernel
     // (false) or first in the double-float many-right-hand-side kernel, the
     // streamed one then adding the FP32 / BF16 chunks (true); autotuned
-    void set_phase2_dense_split(bool on) {
-        split_dense_ = on;
-        layout_gen_++;
-        leave_red();
-    }
+    void set_phase2_dense_split(bool on);
     bool phase2_dense_split() const { return split_dense_; }
     bool emulation_allowed() const { return emu_ok_; }
     // time every candidate split on the current H-matrix and keep the fastest

@@ -357,10 +357,10 @@ int htgpu_hmatrix_phase_bytes(htgpu_hmatrix h, int mu, long long *bytes);
  * reference (its BLAS calls decide this, include/htool/types/matrix.hpp:320-383).
  * FP64 products run on paired panels (every factor pre-split into (hi, lo)
  * float pairs, both phases in double-float arithmetic, no FP64-pipe share)
- * until a call of this function, htgpu_hmatrix_set_phase1_mode,
- * htgpu_hmatrix_set_phase2_mode or htgpu_hmatrix_set_presplit chooses the
- * kernels these functions configure; htgpu_hmatrix_autotune brings the
- * panels back.  Reduced-precision products off the tensor cores likewise run
+ * until a call of this function, or one of htgpu_hmatrix_set_phase1_mode,
+ * htgpu_hmatrix_set_phase2_mode or htgpu_hmatrix_set_presplit that changes
+ * what it sets, chooses the kernels these functions configure;
+ * htgpu_hmatrix_autotune brings the panels back.  Reduced-precision products off the tensor cores likewise run
  * on streams of their own, their dense blocks on paired panels, until one of
  * these calls.  Where the panels do not fit in three quarters of the free
  * memory, or a stored entry is too large for the emulation, those kernels
