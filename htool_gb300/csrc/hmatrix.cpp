@@ -2730,6 +2730,10 @@ void HMatrix::autotune(int mu, int reps, float *best_ms) {
             *best_ms = best;
         return;
     }
+    if (precision_ == 0 && !pair_ready_ && presplit_on_ && emu_ok_) { // the panels again, where they fit now
+        pair_auto_ = true;
+        upload_fp64_lists();
+    }
     if (precision_ != 0) {
         // phase-1 modes with the dense blocks' DFMA / emulation split
         int arg_mode = p1_mode_, arg_split = p2m_n64_;
@@ -2777,8 +2781,9 @@ void HMatrix::autotune(int mu, int reps, float *best_ms) {
         }
         if (run >= kMmaMinRhs && n_tcblk_ > 0)
             try_digit_planes();
-    } else if (presplit_on_ && emu_ok_ && (pair_auto_ = true, upload_fp64_lists(), pair_ready_)) {
+    } else if (pair_ready_) {
         // paired panels, with many right-hand sides against the digit planes
+        layout_gen_++;
         best = timed();
         if (mu >= kDfMinRhs)
             try_digit_planes();
@@ -2788,7 +2793,10 @@ void HMatrix::autotune(int mu, int reps, float *best_ms) {
             *best_ms = best;
         return;
     } else {
-        // every phase-1 mode with every DFMA/emulation split
+        // every phase-1 mode with every DFMA/emulation split, without the
+        // panels (memory that a point frees would let them in midway)
+        if (emu_ok_)
+            pair_auto_ = false;
         std::vector<std::pair<int, int>> splits;
         if (!emu_ok_)
             splits.push_back({1000, 1000});

@@ -1,0 +1,71 @@
+"""Products where device memory is short: the copies of the factors that make
+products faster (paired panels, reduced-precision streams, pre-split pairs) are
+left out or given up, and the products stay.  The rest of the memory is held by
+torch meanwhile.  No counterpart in the reference (host memory).
+
+Tolerance: two FP64-grade products of the same sums, below 4e-13."""
+import numpy as np
+import pytest
+
+import htool_gb300 as H
+from htool_gb300 import geometry as G
+
+pytestmark = pytest.mark.gpu
+
+TOL = 4e-13
+MB = 1 << 20
+
+
+def rel(a, b):
+    return np.linalg.norm(a - b) / np.linalg.norm(b)
+
+
+class Held:
+    """all device memory but `leave` bytes, for the time of a with block"""
+
+    def __init__(self, leave):
+        self.leave = leave
+
+    def __enter__(self):
+        torch = pytest.importorskip("torch")
+        torch.cuda.empty_cache()
+        self.blocks = []
+        for unit in (16 << 30, 1 << 30, 64 * MB, 4 * MB):
+            while torch.cuda.mem_get_info()[0] >= self.leave + unit:
+                self.blocks.append(torch.empty(unit, dtype=torch.uint8, device="cuda"))
+        return self
+
+    def __exit__(self, *a):
+        import torch
+
+        self.blocks.clear()
+        torch.cuda.empty_cache()
+
+
+def matrix(n=40000):
+    pts = G.sphere(n, seed=3)
+    t = H.Cluster().build(n, pts)
+    return H.HMatrix(t, t, 1e-6, 10.0).build(H.LAPLACE, pts)
+
+
+def panels(hm):
+    return int(hm.get_infos()["GPU_paired_panels"])
+
+
+def test_autotune_without_room_for_the_panels():
+    """the sweep over the other kernels stays with them, also past the splits
+    that hold no copies and leave more memory free than at its start"""
+    hm = matrix()
+    n = hm.sizes()[1]
+    x = G.rhs(n, 2, seed=1)
+    y = hm.mvprod_global_to_global(x, 2)
+    nbytes = hm.get_presplit()[1]
+    hm.set_fp64_split(0, 350)
+    with Held(int(0.9 * nbytes)):
+        assert hm.autotune(2, 1) > 0
+        assert panels(hm) == 0
+        assert rel(hm.mvprod_global_to_global(x, 2), y) < TOL
+    assert hm.autotune(2, 1) > 0
+    assert panels(hm) > 0
+    assert np.array_equal(hm.mvprod_global_to_global(x, 2), y)
+    assert hm.device_status() == 0
