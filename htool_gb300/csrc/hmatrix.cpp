@@ -1657,8 +1657,10 @@ void HMatrix::build_red(const std::vector<P1Item> &p1m) {
     }
     std::size_t fr = 0, tot = 0;
     HTGPU_CUDA(cudaMemGetInfo(&fr, &tot));
-    if (outs.size() >= (1ULL << 31) || (std::size_t)off > fr / 4 * 3)
+    if (outs.size() >= (1ULL << 31) || (std::size_t)off > fr / 4 * 3) {
+        release_pair(); // nothing reads the dense blocks' panels alone
         return;
+    }
     red_d.alloc((std::size_t)std::max<long long>(off, 16));
     red1_d.upload(pan, stream_);
     redo_d.upload(outs, stream_);

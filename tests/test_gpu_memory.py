@@ -69,3 +69,27 @@ def test_autotune_without_room_for_the_panels():
     assert panels(hm) > 0
     assert np.array_equal(hm.mvprod_global_to_global(x, 2), y)
     assert hm.device_status() == 0
+
+
+def test_streams_without_room():
+    """one leaf whose reduced columns leave no room for the streams' copy of
+    them: the panels of the small dense leaf beside it are not kept either"""
+    n, r, m = 1000000, 40, 64
+    rng = np.random.default_rng(2)
+    t = H.Cluster().build(n, rng.random((n, 3)))
+    lr, dn = np.array([[0, 0, n, n, r]], np.int32), np.array([[0, 0, m, m]], np.int32)
+    hm = H.HMatrix(t, t, 1e-6, 10.0).set_leaves(lr, rng.choice([-1.0, 1.0], 2 * n * r), dn, rng.choice([-1.0, 1.0], m * m))
+    x = rng.integers(-2, 3, n).astype(np.float64)
+    y = hm.mvprod_global_to_global(x)
+    hm.set_fp64_split(1000, 1000)  # no panels, no pre-split pairs
+    reduced, copy = 4 * r * 2 * n, 4 * r * n
+    with Held(reduced + 110 * MB):
+        hm.set_precision("fp32", 1.0)
+        assert 110 * MB * 3 // 4 < copy
+        assert int(hm.get_infos()["GPU_reduced_streams"]) == 0
+        assert hm.get_presplit()[1] < 1.5 * 8 * m * m
+        assert rel(hm.mvprod_global_to_global(x), y) < 1e-6
+    hm.set_precision("fp32", 1.0)
+    assert int(hm.get_infos()["GPU_reduced_streams"]) > 0
+    assert rel(hm.mvprod_global_to_global(x), y) < 1e-6
+    assert hm.device_status() == 0
