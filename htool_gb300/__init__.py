@@ -623,12 +623,13 @@ class HMatrix:
 
     def set_presplit(self, on):
         """Keep the data of the emulated FP64 chunks pre-split into (hi, lo)
-        float pairs (more device memory, bitwise the same products)."""
+        float pairs (more device memory; off the panels bitwise the same
+        products).  Off: no panels and no reduced-precision streams either."""
         _check(lib.htgpu_hmatrix_set_presplit(self.h, 1 if on else 0))
         return self
 
     def get_presplit(self):
-        """(on, device bytes the pre-split copy holds now)."""
+        """(on, device bytes the pre-split copies, panels and streams hold now)."""
         v, b = C.c_int(), C.c_longlong()
         _check(lib.htgpu_hmatrix_get_presplit(self.h, C.byref(v), C.byref(b)))
         return bool(v.value), b.value

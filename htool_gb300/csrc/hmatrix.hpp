@@ -194,7 +194,7 @@ class HMatrix {
     int phase1_mode() const { return p1_mode_; }
     void set_presplit(bool on);
     bool presplit() const { return presplit_on_; }
-    long long presplit_bytes() const { return (long long)(((emu_fresh_ ? emu_.n : 0) + emu2_.n + emu3_.n) * sizeof(F2) + pair_d.n); } // and the paired panels
+    long long presplit_bytes() const { return (long long)(((emu_fresh_ ? emu_.n : 0) + emu2_.n + emu3_.n) * sizeof(F2) + pair_d.n + red_d.n); } // and the paired panels, and the streams' reduced columns
     void set_phase2_mode(int mode);
     int phase2_mode() const { return p2_mode_; }
     // tensor-core kernels of reduced-precision products with many

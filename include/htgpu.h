@@ -395,9 +395,11 @@ int htgpu_hmatrix_get_phase1_mode(htgpu_hmatrix h, int *mode);
  * (hi, lo) float pairs, so the kernels read the pairs instead of splitting
  * every double again -- the V-side factors when every phase-1 tile is
  * emulated (streamed phase 1), and the emulated phase-2 chunks.  Costs those
- * bytes once more in device memory while the FP64 policy is set (bytes:
- * the current size); results are bitwise the same either way.  No
- * counterpart in the reference. */
+ * bytes once more in device memory while the FP64 policy is set; these
+ * kernels' results are bitwise the same either way.  The paired panels and
+ * the reduced-precision streams are such copies too and go when this is
+ * switched off.  bytes: what all of them hold now.  No counterpart in the
+ * reference. */
 int htgpu_hmatrix_set_presplit(htgpu_hmatrix h, int on);
 int htgpu_hmatrix_get_presplit(htgpu_hmatrix h, int *on, long long *bytes);
 

@@ -91,5 +91,6 @@ def test_streams_without_room():
         assert rel(hm.mvprod_global_to_global(x), y) < 1e-6
     hm.set_precision("fp32", 1.0)
     assert int(hm.get_infos()["GPU_reduced_streams"]) > 0
+    assert hm.get_presplit()[1] >= copy + 8 * m * m
     assert rel(hm.mvprod_global_to_global(x), y) < 1e-6
     assert hm.device_status() == 0
