@@ -1672,8 +1672,13 @@ void HMatrix::build_red(const std::vector<P1Item> &p1m) {
     red_ready_ = true;
 }
 
+// whether reduced-precision products of some number of right-hand sides run
+// off the warp-fed streams, on the chunk lists: without streams all do, else
+// those of kMmaMinRhs and more on the tensor cores or the digit planes
+bool HMatrix::chunk_products() const { return !red_ready_ || oz_on_ || eps_ >= kMmaMinEps; }
+
 // the caller chose a kernel or a split: reduced-precision products leave the
-// warp-fed streams
+// warp-fed streams, for the chunk lists and their pre-split dense blocks
 void HMatrix::leave_red() {
     if (!red_auto_)
         return;
@@ -1685,6 +1690,7 @@ void HMatrix::leave_red() {
     HTGPU_CUDA(cudaStreamSynchronize(stream_));
     release_red();
     release_pair();
+    upload_mixed_phase2();
 }
 
 // the FP64 products' launch lists: paired panels, or the chunk lists and
@@ -1775,7 +1781,7 @@ void HMatrix::upload_mixed_phase2() {
     // emulated dense chunks read pre-split pairs (ch2_h_ keeps the fac offsets)
     std::vector<StreamChunk> ch2 = ch2_h_;
     emu3_.release();
-    if (presplit_on_)
+    if (presplit_on_ && chunk_products())
         presplit_chunks(ch2, emu3_);
     n_chunks_m_ = (long long)ch2.size();
     scm_d.upload(ch2, stream_);
@@ -1937,10 +1943,10 @@ void HMatrix::set_precision(int policy, double tau) {
     HTGPU_CUDA(cudaSetDevice(device_));
     precision_ = policy;
     tau_       = tau;
+    release_red(); // an earlier reduced precision's streams, with their dense blocks' panels
+    if (!pair_ready_)
+        release_pair();
     if (policy == 0) {
-        release_red();
-        if (!pair_ready_)
-            release_pair();
         emu3_.release(); // the reduced-precision products' mirror
         tca_d.release();  // and the tensor cores' copy of the factors
         tcoff_d.release();
@@ -2144,7 +2150,6 @@ void HMatrix::set_precision(int policy, double tau) {
         tcblk_h_ = std::move(blks);
     }
     ch2_h_ = std::move(ch2);
-    upload_mixed_phase2();
     cim.resize(cim.size() + 4, 0); // bulk copies read whole 16-byte words
     cidxm_d.upload(cim, stream_);
     if (p1m.empty())
@@ -2163,6 +2168,7 @@ void HMatrix::set_precision(int policy, double tau) {
         HTGPU_CUDA(cudaStreamSynchronize(stream_));
     }
     build_red(p1m);
+    upload_mixed_phase2();
     build_tc_arena();
     build_oz_arena();
 }
@@ -2308,6 +2314,8 @@ void HMatrix::set_digit_planes(bool on) {
     HTGPU_CUDA(cudaSetDevice(device_));
     layout_gen_++; // captured products are stale
     oz_on_ = on;
+    if (on && red_ready_ && presplit_on_ && n_chunks_md_ > 0 && !emu3_.p)
+        upload_mixed_phase2(); // products on the planes read the dense blocks' pre-split pairs
     build_oz_arena();
     ensure_oz_work(mu_cap);
 }

@@ -354,6 +354,7 @@ class HMatrix {
     void build_red(const std::vector<P1Item> &p1m);
     void release_red();
     void leave_red();
+    bool chunk_products() const;
     void launch_red_product(const double *x, double *y, int mu, int numbering, cudaStream_t st, double *w_xp, F2 *w_xs, int *w_xexp, double *w_A, double *w_z, cudaEvent_t *marks, bool exact);
     struct HostFree {
         void operator()(int *p) const { cudaFreeHost(p); }

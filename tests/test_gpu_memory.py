@@ -94,3 +94,36 @@ def test_streams_without_room():
     assert hm.get_presplit()[1] >= copy + 8 * m * m
     assert rel(hm.mvprod_global_to_global(x), y) < 1e-6
     assert hm.device_status() == 0
+
+
+@pytest.mark.parametrize("eps", [1e-6, 1e-4])
+def test_dense_blocks_are_held_once_beside_the_factors(eps):
+    """reduced storage below epsilon 1e-5: the streams' panels are the only
+    other copy of the dense blocks, until products leave the streams (digit
+    planes; a choice of kernels); from 1e-5 on products with 8 or more right-hand
+    sides read the pre-split chunks.  The products are the same without them"""
+    n, r, m = 3000, 4, 600
+    rng = np.random.default_rng(3)
+    t = H.Cluster().build(n, rng.random((n, 3)))
+    lr, dn = np.array([[m, 0, n - m, n, r]], np.int32), np.array([[0, 0, m, m]], np.int32)
+    hm = H.HMatrix(t, t, eps, 10.0).set_leaves(lr, rng.standard_normal((2 * n - m) * r), dn, rng.standard_normal(m * m)).set_precision("fp32", 1.0)
+    pairs, columns = 8 * m * m, 4 * r * n
+    small = pairs // 2
+    chunks = eps >= 1e-5
+    assert abs(hm.get_presplit()[1] - (1 + chunks) * pairs - columns) < small
+    X = G.rhs(n, 9, seed=4)
+    hm.set_digit_planes(True)
+    assert abs(hm.get_presplit()[1] - 2 * pairs - columns) < small
+    y = hm.mvprod_global_to_global(X, 9)
+    hm.set_presplit(False)  # the chunks split in the kernels
+    assert hm.get_presplit()[1] == 0
+    assert np.array_equal(hm.mvprod_global_to_global(X, 9), y)
+    hm.set_presplit(True).set_digit_planes(False)
+    hm.autotune(3, 1)
+    assert int(hm.get_infos()["GPU_reduced_streams"]) > 0
+    y = hm.mvprod_global_to_global(X[:3 * n].copy(), 3)
+    hm.set_phase2_mode("warp")
+    assert abs(hm.get_presplit()[1] - pairs) < small
+    assert rel(hm.mvprod_global_to_global(X[:3 * n].copy(), 3), y) < TOL
+    hm.set_precision("fp64")
+    assert hm.device_status() == 0
