@@ -1215,9 +1215,41 @@ void HMatrix::finalize(const std::vector<const double *> &bufs, const std::vecto
     build_oz_arena(); // the digit planes follow new factors (none while off)
 }
 
+// Runs `body`, whose allocations a product cannot do without; where the memory
+// for them is short, the panels or streams go and it runs again.  They are
+// laid out at a build from what is free then, before the buffers of many right-
+// hand sides, digit planes or a transposed twin are asked for.
+void HMatrix::with_room(const std::function<void()> &body) {
+    try {
+        body();
+        return;
+    } catch (const NoMemory &) {
+        if (!pair_ready_ && !red_ready_)
+            throw;
+    }
+    HTGPU_CUDA(cudaStreamSynchronize(stream_));
+    if (red_ready_)
+        leave_red();
+    else {
+        pair_auto_ = false;
+        release_pair();
+        try {
+            upload_phase1_lists(true);
+        } catch (const NoMemory &) {
+            upload_phase1_lists(false);
+        }
+    }
+    body();
+}
+
 void HMatrix::ensure_work(int mu) {
     if (mu <= mu_cap)
         return;
+    with_room([&] { alloc_work(mu); });
+}
+
+void HMatrix::alloc_work(int mu) {
+    mu_cap = 0;
     layout_gen_++; // work buffers move: captured products are stale
     // paired panels run an odd number of right-hand sides padded by one
     const std::size_t even = mu > 1 ? (std::size_t)(mu + 1) & ~(std::size_t)1 : 1;
@@ -1351,7 +1383,7 @@ void HMatrix::presplit_chunks(std::vector<StreamChunk> &ch, DevBuf<F2> &mirror) 
     HTGPU_CUDA(cudaStreamSynchronize(stream_));
 }
 
-void HMatrix::upload_phase1_lists() {
+void HMatrix::upload_phase1_lists(bool copies) {
     layout_gen_++; // buffers or launch lists change: captured products are stale
     std::vector<P1Item> a, b;
     for (auto &it : p1_h)
@@ -1376,7 +1408,7 @@ void HMatrix::upload_phase1_lists() {
         p1r_d.upload(st, stream_);
         // all tiles emulated: the streamed phase 1 reads a pre-split copy
         // of the tile region (the same (hi, lo) pairs it would form itself)
-        if (p1_kinds_ == 4 && presplit_on_ && precision_ == 0) {
+        if (p1_kinds_ == 4 && presplit_on_ && copies && precision_ == 0) {
             long long len = 0;
             for (auto &it : p1_h)
                 len = std::max(len, it.off + (long long)it.jlen * lr_h[it.leaf].r);
@@ -1440,7 +1472,7 @@ void HMatrix::upload_phase1_lists() {
         n_cols_ += pi.ncol;
     }
     emu2_.release();
-    if (presplit_on_ && precision_ == 0)
+    if (presplit_on_ && copies && precision_ == 0)
         presplit_chunks(ch, emu2_);
     fp64_lists_stale_ = presplit_on_ && precision_ != 0; // mirrors wait for the FP64 policy
     n_sctas_  = stream_ctas() * kStreamWarpsPerCta * 8; // ranges: ~8 per warp
@@ -2190,7 +2222,7 @@ void HMatrix::set_tensor_core_arena(bool on) {
     HTGPU_CUDA(cudaSetDevice(device_));
     layout_gen_++; // captured products are stale
     tc_arena_ = on;
-    build_tc_arena();
+    with_room([&] { build_tc_arena(); });
 }
 
 long long HMatrix::oz_arena_need() {
@@ -2316,8 +2348,10 @@ void HMatrix::set_digit_planes(bool on) {
     oz_on_ = on;
     if (on && red_ready_ && presplit_on_ && n_chunks_md_ > 0 && !emu3_.p)
         upload_mixed_phase2(); // products on the planes read the dense blocks' pre-split pairs
-    build_oz_arena();
-    ensure_oz_work(mu_cap);
+    with_room([&] {
+        build_oz_arena();
+        ensure_oz_work(mu_cap);
+    });
 }
 
 // the per-product scratch of the digit-plane phase 1 for up to mu
@@ -2335,6 +2369,7 @@ void HMatrix::ensure_oz_work(int mu) {
     if (mu <= ozx_mu_)
         return;
     layout_gen_++; // scratch moves: captured products are stale
+    ozx_mu_ = 0;
     ozg.alloc((std::size_t)((nc + 31) / 32) * mu + 1);
     ozc.alloc((std::size_t)mu + 1);
     ozx.alloc((std::size_t)oz_xplanes_bytes(nc, mu, 8));
@@ -2994,12 +3029,14 @@ void HMatrix::mvprod_transp(const double *in, double *out, int mu, bool host_ptr
                 std::swap(dn[4 * b + 2], dn[4 * b + 3]);
                 o += (long long)m * n;
             }
-            auto t = std::unique_ptr<HMatrix>(new HMatrix(Sz_, Tz_, eps_, eta_, device_, true));
-            t->set_complex_layout(true);
-            t->set_leaves(nl, lr.data(), uvt.data(), nd, dn.data(), ddt.data());
-            if (!pair_auto_)
-                t->set_fp64_split(p1_permille_, p2_n64_);
-            transp_ = std::move(t);
+            with_room([&] {
+                auto t = std::unique_ptr<HMatrix>(new HMatrix(Sz_, Tz_, eps_, eta_, device_, true));
+                t->set_complex_layout(true);
+                t->set_leaves(nl, lr.data(), uvt.data(), nd, dn.data(), ddt.data());
+                if (!pair_auto_)
+                    t->set_fp64_split(p1_permille_, p2_n64_);
+                transp_ = std::move(t);
+            });
         }
         if (transp_->precision() != precision_ || (precision_ != 0 && transp_->tau_ != tau_))
             transp_->set_precision(precision_, tau_);
@@ -3067,11 +3104,13 @@ void HMatrix::mvprod_transp(const double *in, double *out, int mu, bool host_ptr
             std::swap(dn[4 * b + 2], dn[4 * b + 3]);
             o += (long long)D.m * D.n;
         }
-        auto t = std::unique_ptr<HMatrix>(new HMatrix(S, T, eps_, eta_, device_));
-        t->set_leaves((int)lr_h.size(), lr.data(), uvt.data(), (int)dn_h.size(), dn.data(), ddt.data());
-        if (!pair_auto_)
-            t->set_fp64_split(p1_permille_, p2_n64_);
-        transp_ = std::move(t);
+        with_room([&] {
+            auto t = std::unique_ptr<HMatrix>(new HMatrix(S, T, eps_, eta_, device_));
+            t->set_leaves((int)lr_h.size(), lr.data(), uvt.data(), (int)dn_h.size(), dn.data(), ddt.data());
+            if (!pair_auto_)
+                t->set_fp64_split(p1_permille_, p2_n64_);
+            transp_ = std::move(t);
+        });
     }
     if (transp_->precision() != precision_ || (precision_ != 0 && transp_->tau_ != tau_))
         transp_->set_precision(precision_, tau_);

@@ -276,6 +276,8 @@ class HMatrix {
     void finalize(const std::vector<const double *> &bufs, const std::vector<LeafSrc> &lr_src, const std::vector<LeafSrc> *dn_src, const KernelDesc *kd, const double *dxt, const double *dxs);
     void assign_phase1_modes();
     void ensure_work(int mu);
+    void alloc_work(int mu);
+    void with_room(const std::function<void()> &body);
 
     std::shared_ptr<const ClusterTree> T, S;
     double eps_, eta_;
@@ -320,7 +322,7 @@ class HMatrix {
                              int mu_run = 0, const OzScratch *w_oz = nullptr);
     const OzScratch *oz_scratch(int mu); // the H-matrix's own, when it holds mu right-hand sides
     void launch_sums(double *y, int mu, int numbering, const double *w_z, cudaStream_t st);
-    void upload_phase1_lists();
+    void upload_phase1_lists(bool copies = true); // with the pre-split copies, where those are on
     // FP64 products on paired panels (pair.cu): the way they run unless the
     // caller chose a DFMA split, a phase mode or no pre-split copies
     // (pair_auto_), where every stored entry may be emulated and the mirror

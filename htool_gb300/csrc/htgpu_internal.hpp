@@ -29,6 +29,11 @@ struct Error : std::runtime_error {
                                         " at " __FILE__ ":" + std::to_string(__LINE__));             \
     } while (0)
 
+// an allocation that did not fit
+struct NoMemory : Error {
+    using Error::Error;
+};
+
 inline void require(bool ok, const std::string &msg, int code = 1) {
     if (!ok)
         throw Error(code, "[Htool error] " + msg);
@@ -229,7 +234,13 @@ struct DevBuf {
     void alloc(std::size_t count) {
         release();
         if (count) {
-            HTGPU_CUDA(cudaMalloc((void **)&p, count * sizeof(T)));
+            const cudaError_t rc = cudaMalloc((void **)&p, count * sizeof(T));
+            if (rc == cudaErrorMemoryAllocation) {
+                cudaGetLastError(); // reported here, not by the next launch's check
+                p = nullptr;
+                throw NoMemory(3, std::string("[Htool error] CUDA: ") + cudaGetErrorString(rc) + " (" + std::to_string(count * sizeof(T)) + " bytes)");
+            }
+            HTGPU_CUDA(rc);
             n = count;
         }
     }

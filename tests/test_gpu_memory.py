@@ -127,3 +127,81 @@ def test_dense_blocks_are_held_once_beside_the_factors(eps):
     assert rel(hm.mvprod_global_to_global(X[:3 * n].copy(), 3), y) < TOL
     hm.set_precision("fp64")
     assert hm.device_status() == 0
+
+
+def device_bytes(before):
+    """what has been taken since `before` bytes were free"""
+    import torch
+
+    torch.cuda.synchronize()
+    return before - torch.cuda.mem_get_info()[0]
+
+
+def streams(hm):
+    return panels(hm) + int(hm.get_infos()["GPU_reduced_streams"])
+
+
+@pytest.mark.parametrize("policy", ["fp64", "mixed"])
+@pytest.mark.parametrize("what", ["right-hand sides", "planes"])
+def test_copies_give_way(policy, what):
+    """work buffers and digit planes are allocated after the panels or streams,
+    which go where the rest of the memory does not hold them"""
+    torch = pytest.importorskip("torch")
+    mu = 400 if what == "right-hand sides" else 8
+    hm, ref = matrix().set_precision(policy, 1.0), matrix().set_precision(policy, 1.0)
+    n = hm.sizes()[1]
+    X = G.rhs(n, mu, seed=5)
+    call = lambda h: (h.set_digit_planes(True) if what == "planes" else h).mvprod_global_to_global(X, mu)
+    copies = ref.get_presplit()[1]
+    for h in (hm, ref):
+        h.mvprod_global_to_global(X[:n].copy(), 1)
+        if what == "planes":
+            h.mvprod_global_to_global(X, mu)
+    free = torch.cuda.mem_get_info()[0]
+    y = call(ref)
+    need = device_bytes(free)
+    ref.set_digit_planes(False).set_phase2_mode("warp")  # the kernels without the copies hold pre-split pairs
+    freed = copies - ref.get_presplit()[1]
+    assert freed > 16 * MB and need > freed // 2
+    del ref
+    assert streams(hm) > 0
+    with Held(need - freed // 2):
+        z = call(hm)
+        assert streams(hm) == 0
+        assert rel(z, y) < TOL
+        assert rel(call(hm), y) < TOL
+    assert hm.device_status() == 0
+
+
+def test_transposed_twin():
+    """the twin of transposed products: the least memory it takes beside a handle
+    off the panels is enough beside one on them, with what its panels hold"""
+    n = 40000
+    x = G.rhs(n, 1, seed=6)
+
+    def works(hm, leave):
+        with Held(leave):
+            try:
+                hm.mvprod_transp_global_to_global(x)
+                return True
+            except RuntimeError as e:
+                assert "out of memory" in str(e)
+                return False
+
+    hm, ref = matrix(n), matrix(n)
+    copies = ref.get_presplit()[1]
+    y = ref.mvprod_transp_global_to_global(x)
+    ref.set_phase2_mode("warp")
+    freed = copies - ref.get_presplit()[1]
+    assert freed > 16 * MB
+    del ref
+    lo, hi = 0, 5 * copies
+    while hi - lo > freed // 8:
+        mid = (lo + hi) // 2
+        off = matrix(n).set_phase2_mode("warp")
+        lo, hi = (lo, mid) if works(off, mid) else (mid, hi)
+        del off
+    assert works(hm, hi - freed // 2)
+    assert streams(hm) == 0
+    assert rel(hm.mvprod_transp_global_to_global(x), y) < TOL
+    assert hm.device_status() == 0
