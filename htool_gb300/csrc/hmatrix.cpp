@@ -521,7 +521,6 @@ void HMatrix::build_impl(const KernelDesc *kdp, const HostGen *hg, const double 
                 acc.resize(acc0 + nb);
             };
             if (hg) {
-                meanwhile();
                 // rows and columns in user numbering; a mirrored block reads
                 // the generator with the roles of the two trees exchanged
                 std::vector<const int *> ru(blocks.size()), cu(blocks.size());
@@ -531,6 +530,7 @@ void HMatrix::build_impl(const KernelDesc *kdp, const HostGen *hg, const double 
                     cu[b]          = (mir ? Ta.perm.data() : Sa.perm.data()) + blocks[b].col_off;
                 }
                 aca_host_batch(*hg, blocks, ru, cu, dblocks.p, n_direct, dxt.p, dxs.p, aca_pt, aca_ps, nullptr, -1, eps_, scratch.p, flags.p, ranks, stream_);
+                meanwhile(); // after the generator's calls, which may throw
             } else {
                 if (complex_) {
                     if (n_direct > 0)
