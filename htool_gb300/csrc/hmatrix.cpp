@@ -2128,7 +2128,7 @@ void HMatrix::set_precision(int policy, double tau) {
                 k.ncol  = nc;
                 k.kind  = es == 4 ? kStreamF32 : kStreamBf16;
                 k.flags = 0;
-                k.pad   = 0;
+                k.pad   = (unsigned short)((nc + V * S - 1) / (V * S) * (V * S));
                 ch2.push_back(k);
                 swz.push_back({off, q0 + c0, nc, h, es});
                 off += k.bytes;

@@ -146,7 +146,8 @@ enum StreamKind : unsigned char { kStreamDfma = 0, kStreamEmu = 1, kStreamF32 = 
 // first / last chunk of a row chunk (phase 2) or tile (phase 1); data in the
 // second arena; an emulated chunk whose data are (hi, lo) float pairs
 // kStreamAdd (on a row chunk's last chunk): add the row chunk's sums onto z
-// instead of writing them (another kernel wrote the rest of the row first)
+// instead of writing them (another kernel wrote the rest of the row first); the
+// warp-fed streams (red.cu) have it on the first chunk, and start from z
 enum StreamFlag : unsigned char { kStreamFirst = 1, kStreamLast = 2, kStreamArena1 = 4, kStreamPre = 8, kStreamAdd = 16 };
 
 // one run of doubles copied as (hi, lo) float pairs: n values from double
@@ -165,7 +166,7 @@ struct StreamChunk {
     int c;           // phase 1: per-column scale index of the first column
     int h, ncol;     // rows (phase 2: <= 32, phase 1: <= 256), columns
     unsigned char kind, flags;
-    unsigned short pad;
+    unsigned short pad; // chunks in lane order: the columns of whole groups of every slice, at most 128
 };
 
 // Streamed phase 1: consecutive phase-1 chunks packed into one bulk copy of

@@ -56,6 +56,15 @@ constexpr RedRcp red_rcp() {
 __constant__ RedRcp kRedRcp = red_rcp();
 __device__ __forceinline__ int red_div(int t, int d) { return (int)(((unsigned)t * kRedRcp.v[d]) >> 16); }
 
+// a chunk's shape in one word: rows (6 bits), columns (7), FP32, flags (5), the
+// end of its last column group (8)
+__device__ __forceinline__ int red_pack(const StreamChunk &c) { return c.h | c.ncol << 6 | (c.kind == kStreamF32 ? 1 << 13 : 0) | (int)c.flags << 14 | (int)c.pad << 19; }
+__device__ __forceinline__ int red_h(int m) { return m & 63; }
+__device__ __forceinline__ int red_ncol(int m) { return (m >> 6) & 127; }
+__device__ __forceinline__ bool red_f32(int m) { return m >> 13 & 1; }
+__device__ __forceinline__ int red_flags(int m) { return (m >> 14) & 31; }
+__device__ __forceinline__ int red_end(int m) { return (m >> 19) & 255; }
+
 // W floats (one row or slot) global -> shared, W x 4-byte aligned
 template <int W>
 __device__ __forceinline__ void copy_row(float *dst, const float *src) {
@@ -297,7 +306,7 @@ __global__ void __launch_bounds__(32 * kRedWarps, Red2Cfg<W>::kCtas)
         nk = rbeg[inxt];
         ne = rbeg[inxt + 1];
     }
-    struct Win { // h, columns, kind, flags in the bytes of m
+    struct Win {
         long long src;
         int a, b, m, bytes, n;
     };
@@ -309,7 +318,7 @@ __global__ void __launch_bounds__(32 * kRedWarps, Red2Cfg<W>::kCtas)
             w.a                 = c.a;
             w.b                 = c.b;
             w.bytes             = c.bytes;
-            w.m                 = c.h | c.ncol << 8 | (int)c.kind << 16 | (int)c.flags << 24;
+            w.m                 = red_pack(c);
         }
         k += w.n;
     };
@@ -352,7 +361,7 @@ __global__ void __launch_bounds__(32 * kRedWarps, Red2Cfg<W>::kCtas)
             c.b         = __shfl_sync(0xffffffffu, w0.b, at);
             c.m         = __shfl_sync(0xffffffffu, w0.m, at);
             c.bytes     = __shfl_sync(0xffffffffu, w0.bytes, at);
-            const int a = __shfl_sync(0xffffffffu, w0.a, at), n = (c.m >> 8) & 255;
+            const int a = __shfl_sync(0xffffffffu, w0.a, at), n = red_ncol(c.m);
             c.ix0 = lane < n ? __ldg(cidx + a + lane) : 0;
             c.ix1 = lane + 32 < n ? __ldg(cidx + a + lane + 32) : 0;
             at++;
@@ -363,7 +372,7 @@ __global__ void __launch_bounds__(32 * kRedWarps, Red2Cfg<W>::kCtas)
     int issued = 0;
     auto issue = [&]() {
         if (d0.m != 0) {
-            const int s = issued % kRedStages, ncol = (d0.m >> 8) & 255;
+            const int s = issued % kRedStages, ncol = red_ncol(d0.m), end = red_end(d0.m);
             unsigned char *st = wbase + (size_t)s * C::kStage;
             float *cf         = reinterpret_cast<float *>(st + C::kCoef);
             if (lane == 0) {
@@ -371,24 +380,22 @@ __global__ void __launch_bounds__(32 * kRedWarps, Red2Cfg<W>::kCtas)
                 ring_copy(st, mix + d0.src, (unsigned)d0.bytes, &bar[s], pol);
             }
             // past the chunk's columns, up to the last group's end, the data are
-            // zero; the coefficients there must be numbers of this chunk's own
-            // (the stage's last chunk may have left a NaN): zero
-            const int S = red_div(32, d0.m & 255), lv = ((d0.m >> 16) & 255) == kStreamF32 ? 2 : 3;
-            const int end = ((red_div(ncol + S - 1, S) + (1 << lv) - 1) >> lv) * (S << lv);
+            // zero; the coefficients there must be numbers (the stage's last
+            // chunk may have left a NaN): zero
             if constexpr (W == 1) {
+                const int S = red_div(32, red_h(d0.m)), lv = red_f32(d0.m) ? 2 : 3;
+                auto at     = [&](int t) {
+                    const int jj = red_div(t, S), sl = t - jj * S;
+                    return cf + ((((jj >> lv) * S + sl) << lv) | (jj & ((1 << lv) - 1)));
+                };
 #pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    const int t = lane + 32 * r;
-                    if (t < end) {
-                        const int jj = red_div(t, S), sl = t - jj * S;
-                        float *c     = cf + ((((jj >> lv) * S + sl) << lv) | (jj & ((1 << lv) - 1)));
-                        if (t < ncol)
-                            copy_async<4>(c, A + (r ? d0.ix1 : d0.ix0));
-                        else
-                            *c = 0.f;
-                    }
-                }
+                for (int r = 0; r < 2; r++)
+                    if (lane + 32 * r < ncol)
+                        copy_async<4>(at(lane + 32 * r), A + (r ? d0.ix1 : d0.ix0));
+                for (int t = ncol + lane; t < end; t += 32)
+                    *at(t) = 0.f;
             } else {
+                using V = std::conditional_t<W % 4 == 0, float4, float2>;
 #pragma unroll
                 for (int r = 0; r < 2; r++) {
                     const int t = lane + 32 * r;
@@ -396,8 +403,8 @@ __global__ void __launch_bounds__(32 * kRedWarps, Red2Cfg<W>::kCtas)
                         copy_row<W>(cf + W * t, A + (long long)W * (r ? d0.ix1 : d0.ix0));
                     else if (t < end)
 #pragma unroll
-                        for (int i = 0; i < W; i += 2)
-                            *reinterpret_cast<float2 *>(cf + W * t + i) = make_float2(0.f, 0.f);
+                        for (int i = 0; i < 4 * W / (int)sizeof(V); i++)
+                            reinterpret_cast<V *>(cf + W * t)[i] = V{};
                 }
             }
             issued++;
@@ -423,7 +430,8 @@ __global__ void __launch_bounds__(32 * kRedWarps, Red2Cfg<W>::kCtas)
         __syncwarp();
         const unsigned char *st = wbase + (size_t)s * C::kStage;
         const int2 d            = *reinterpret_cast<const int2 *>(st + C::kDesc);
-        const int h = d.x & 255, kind = (d.x >> 16) & 255, flags = (d.x >> 24) & 255, ncol = (d.x >> 8) & 255;
+        const int h = red_h(d.x), flags = red_flags(d.x), ncol = red_ncol(d.x);
+        const bool f32 = red_f32(d.x);
         const int S = red_div(32, h), slice = red_div(lane, h), row = lane - slice * h, Ln = S * h;
         const float *cf = reinterpret_cast<const float *>(st + C::kCoef);
         const uint4 *D  = reinterpret_cast<const uint4 *>(st) + lane;
@@ -444,7 +452,7 @@ __global__ void __launch_bounds__(32 * kRedWarps, Red2Cfg<W>::kCtas)
         if (lane < Ln) {
             const int J = red_div(ncol + S - 1, S);
             if constexpr (W == 1) {
-                if (kind == kStreamF32) {
+                if (f32) {
                     const float4 *cv = reinterpret_cast<const float4 *>(cf) + slice;
 #pragma unroll 2
                     for (int g = 0; g < (J + 3) >> 2; g++) {
@@ -479,7 +487,7 @@ __global__ void __launch_bounds__(32 * kRedWarps, Red2Cfg<W>::kCtas)
                     for (int q = 0; q < Q; q++)
                         part2[q] = fx_fma(fx(e1, e1), x[q], part2[q]);
                 };
-                if (kind == kStreamF32) {
+                if (f32) {
 #pragma unroll 1
                     for (int g = 0; g < (J + 3) >> 2; g++) {
                         const uint4 w = D[g * Ln];
