@@ -54,7 +54,7 @@ UNIT = "H-matvec/s"
 # the same `config` in both arms
 WORKLOAD = dict(workload="laplace_sphere", n=1000000, kernel="1/(4 pi r), 0 on the diagonal", eta=10.0, epsilon=1e-6, minclustersize=10, compressor="partialACA", mu=1,
                 l2="inputs larger than L2: the stored H-matrix read by every product is tens of GB")
-DTYPE = "f64 (FP64 storage; DFMA and double-float FP32-pipe evaluation)"
+DTYPE = "f64 (FP64 storage; double-float evaluation on the FP32 pipe)"
 
 
 def parse():
@@ -356,7 +356,7 @@ def run_gpu(args):
     clocks = Clocks(local)
     clocks.start()
     time.sleep(0.5)  # let the sampler start before the timed regions
-    # plain FP64 (autotuned DFMA / FP32-pipe split): the headline
+    # plain FP64 (autotuned: paired panels where they fit): the headline
     hm.set_precision("fp64")
     if fixed:
         if args.fp64_split is not None:

@@ -111,14 +111,14 @@ void launch_zout(const double *y, int m, int mu, double *out, cudaStream_t st);
 // the same over float phase-1 sums (reduced-precision products)
 void launch_reduce_tiles_f(const LrLeaf *lr, const int *multi, int nmulti, int mu, float *A, cudaStream_t st);
 void launch_block_copy(const BlockCopy *items, int nitems, const double *src, double *dst, cudaStream_t st);
-// y[c * ldy + perm[i]] = sum of the partial sums z of the clusters covering
-// row i; without perm, y[c * ldy + i - shift]
 // where the last kernel of a product on host arrays leaves the product's
 // status (a word of pinned host memory; none: nowhere)
 struct StatusNote {
     const int *status = nullptr;
     int *host         = nullptr;
 };
+// y[c * ldy + perm[i]] = sum of the partial sums z of the clusters covering
+// row i; without perm, y[c * ldy + i - shift]
 void launch_zsum(const ZItem *items, int nitems, const int *zl, const double *z, int zlen, int mu, const int *perm, double *y, int ldy, cudaStream_t st, int shift = 0, StatusNote note = {});
 
 // ---- streamed phase 2 (stream.cu) ------------------------------------------
@@ -349,9 +349,6 @@ void launch_pair_pack(const PairPanel *p1, int np1, const long long *osrc, const
 // (slots x w), the sums of multi-tile leaves, i times the sums (native complex
 // layout), the partial sums z of the first nrhs of them (zlen apart), and
 // the final sums over all mu
-// both the exponent and the gathered input of an input of one pass and at most kPairPrepMax entries
-constexpr int kPairPrepMax = 3072;
-void launch_pair_prep(const double *x, const int *perm, int n, int w, int mu_src, int *xexp, float *X, int *tickets, cudaStream_t st);
 void launch_pair_gather(const double *x, int ldx, const int *perm, int n, int c0, int w, int mu_src, const int *xexp, float *X, int *tickets, cudaStream_t st);
 void launch_pair_phase1(const PairPanel *panels, int npanels, int *tickets, const unsigned char *mirror, const int *oslot, const float *X, float *A, int w, int *status, cudaStream_t st);
 void launch_pair_reduce(const LrLeaf *lr, const int *multi, int nmulti, int w, float *A, cudaStream_t st);
@@ -359,6 +356,10 @@ void launch_pair_rotate(const int2 *rows, long long nrows, int w, float *A, cuda
 void launch_pair_phase2(const PairPanel *panels, int npanels, int *tickets, const unsigned char *mirror, const int *cidx, const float *X, float *A, int w, int nrhs, float2 *z, int zlen, int *status,
                         cudaStream_t st);
 void launch_pair_zsum(const ZItem *items, int nitems, const int *zl, const float2 *z, int zlen, int mu, const int *perm, const int *xexp, double *y, int ldy, cudaStream_t st, int shift = 0, StatusNote note = {});
+// the input's exponent and the split input in one kernel, for an input of one
+// pass and at most kPairPrepMax entries
+constexpr int kPairPrepMax = 3072;
+void launch_pair_prep(const double *x, const int *perm, int n, int w, int mu_src, int *xexp, float *X, int *tickets, cudaStream_t st);
 // the limit of its waits and a panel whose first copy is left out (set_debug_waits)
 void set_pair_waits(long long cycles, long long skip);
 // ---- reduced-precision products off the tensor cores (red.cu) --------------
@@ -374,7 +375,7 @@ constexpr int kRedOuts = 64; // outputs of a phase-1 panel at most
 // one pass of w right-hand sides: the leading floats of the split input
 // (hi_only, n x w floats) or its (hi, lo) pairs; the float phase-1 sums (slots
 // x w); the chunks' sums into z (double-float rows; kStreamAdd on a row
-// chunk's last chunk: onto the dense part that is there)
+// chunk's first chunk: from the dense part that is there on)
 void launch_red_gather(const double *x, int ldx, const int *perm, int n, int c0, int w, int mu_src, const int *xexp, bool hi_only, float *out, cudaStream_t st);
 void launch_red_phase1(const RedPanel *panels, int npanels, int *ticket, const unsigned char *mirror, const int2 *outs, const float *scale, const float *X, float *A, int w, int *status, cudaStream_t st);
 void launch_red_phase2(const StreamChunk *chunks, const int *rbeg, int nranges, int *ticket, const unsigned char *mix, const int *cidx, const float *A, int w, int nrhs, float2 *z, int zlen, int *status,

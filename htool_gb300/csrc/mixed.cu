@@ -747,7 +747,7 @@ __device__ __forceinline__ bool phase2_mma_rows(int w, unsigned char *sd, const 
 #pragma unroll
             for (int q = 0; q < 4; q++)
                 acc[a][b][q] = 0.f;
-    f2x fin = fx(0.f, 0.f); // NaN once a word read is not finite
+    f2x fin = fx(0.f, 0.f); // EXACT off: NaN once a word read is not finite
     Slab in[kP2Stages]; // the present slab and those on their way (no columns: past the last)
     next_chunk();
     index_ahead();
@@ -809,19 +809,21 @@ __device__ __forceinline__ bool phase2_mma_rows(int w, unsigned char *sd, const 
                         bh[1][k]       = __float_as_uint(v.y);
                         bh[2][k]       = __float_as_uint(v.z);
                         bh[3][k]       = __float_as_uint(v.w);
-                        if (!EXACT)
+                        if constexpr (!EXACT) {
                             fin = fx_fma(fx(v.x, v.y), fx(0.f, 0.f), fin);
-                        fin = fx_fma(fx(v.z, v.w), fx(0.f, 0.f), fin);
+                            fin = fx_fma(fx(v.z, v.w), fx(0.f, 0.f), fin);
+                        }
                     } else {
 #pragma unroll
                         for (int nt = 0; nt < N; nt++) {
                             const float v = row[g * NT + nt];
                             bh[nt][k]     = __float_as_uint(v);
-                            fin           = fx_fma(fx(v, v), fx(0.f, 0.f), fin);
+                            if constexpr (!EXACT)
+                                fin = fx_fma(fx(v, v), fx(0.f, 0.f), fin);
                         }
                     }
                 }
-                if (n0 == 0 && cur.f32)
+                if (!EXACT && n0 == 0 && cur.f32)
 #pragma unroll
                     for (int mt = 0; mt < 2; mt++)
 #pragma unroll

@@ -46,8 +46,8 @@
 // cut into planes once (oz_xplanes_kernel: per 16-row group and 64
 // right-hand sides, S planes of 2 KB, relative to each right-hand side's
 // maximum) and phase1_ozb_kernel brings both operands of every slab in by
-// bulk copies, four stages deep, one thread issuing the MMAs (kind::f16,
-// M 128, N 64, K 16), eight warps reading the accumulators out.  An input
+// bulk copies, four stages deep, one warp issuing the MMAs (kind::f16,
+// M 128, N 64, K 16), sixteen warps reading the accumulators out.  An input
 // with a 32-row group more than kOzWide binades below its right-hand side's
 // maximum takes phase1_oz_kernel instead, whose threads cut the input per
 // block relative to the block's own maxima.  Every wait is bounded (status 4
@@ -257,7 +257,9 @@ struct OzQuad {
 // 128 hi + lo of two neighbouring diagonals.  Conversions to integers run at
 // 16 a clock and SM, and the accumulators are held until they are done; at most
 // four sums of 256 digit products (2^12 each) stay below 2^22, where adding
-// 1.5 2^23 leaves the integer in the low bits instead.  wide: up to 2^23.
+// 1.5 2^23 leaves the integer in the low bits instead (phase 1 sums whole
+// slabs, up to 272 rows, of which those outside its tile of 256 are zero in A;
+// a top digit is 33 at most, so no sum reaches 2^22).  wide: up to 2^23.
 __device__ __forceinline__ int oz_duo(unsigned hi, unsigned lo, bool wide) {
     if (wide)
         return __float2int_rn(__uint_as_float(hi)) * 128 + __float2int_rn(__uint_as_float(lo));

@@ -53,7 +53,7 @@ __device__ long long g_pair_skip = -1; // a panel whose first copy is left out (
 
 // a double as hi + lo, both rounded to nearest (|a - hi - lo| <= 2^-48 |a|; the
 // truncating split64 of the other kernels keeps 2^-46), by bit operations:
-// the conversions between double and float run on the FP64 pipe. |a| < 2^127;
+// the conversions between double and float run on the FP64 pipe. |a| < 2^126;
 // below 2^-103 (and zero) gives 0, a value that is not finite NaN, so that it
 // reaches the outputs
 __device__ __forceinline__ F2 split64_near(double a) {
