@@ -2740,19 +2740,18 @@ void HMatrix::autotune(int mu, int reps, float *best_ms) {
         return ms / reps;
     };
     float best = 1e30f;
-    // the digit-plane phase 1 (products with 8 or more right-hand sides),
-    // where its planes fit in half the free memory; `best` is the time of
-    // the current configuration
+    // whether the digit planes are there, or fit in half the free memory
+    auto room_for_planes = [&]() {
+        std::size_t fr = 0, tot = 0;
+        HTGPU_CUDA(cudaMemGetInfo(&fr, &tot));
+        return !znative_ && (oz_on_ || (std::size_t)oz_arena_need() < fr / 2);
+    };
+    // the digit-plane phase 1 (products with 8 or more right-hand sides);
+    // `best` is the time of the current configuration
     auto try_digit_planes = [&]() {
-        if (znative_)
+        if (!room_for_planes())
             return;
         const bool was = oz_on_;
-        if (!was) {
-            std::size_t fr = 0, tot = 0;
-            HTGPU_CUDA(cudaMemGetInfo(&fr, &tot));
-            if ((std::size_t)oz_arena_need() >= fr / 2)
-                return;
-        }
         set_digit_planes(!was);
         const float ms = timed();
         if (ms < best)
@@ -2760,15 +2759,70 @@ void HMatrix::autotune(int mu, int reps, float *best_ms) {
         else
             set_digit_planes(was);
     };
+    // the streamed phase 2 of 8 or more right-hand sides in passes of 8 or of
+    // 4, from 4 right-hand sides on with the dense chunks in the double-float
+    // kernel (on the planes where they are on) or in the streamed one, with
+    // either phase-2 kernel for the rest
+    auto try_passes = [&]() {
+        p2_gmax_       = 8;
+        const float t8 = timed();
+        p2_gmax_       = 4;
+        const float t4 = timed();
+        p2_gmax_       = t4 < t8 ? 4 : 8;
+        best           = std::min(t4, t8);
+        layout_gen_++;
+    };
+    auto try_dense_split = [&]() {
+        float tbest  = 1e30f;
+        bool arg_sp  = false;
+        int arg_mode = p2_mode_;
+        for (bool sp : {false, true})
+            for (int m : {0, 1}) {
+                split_dense_  = sp;
+                p2_mode_      = m;
+                const float t = timed();
+                if (t < tbest) {
+                    tbest    = t;
+                    arg_sp   = sp;
+                    arg_mode = m;
+                }
+            }
+        split_dense_ = arg_sp;
+        p2_mode_     = arg_mode;
+        best         = tbest;
+        layout_gen_++;
+    };
     if (precision_ != 0 && !red_ready_ && emu_ok_ && presplit_on_ && !(mu >= kMmaMinRhs && eps_ >= kMmaMinEps)) {
         red_auto_ = true; // back from a caller's choice
         set_precision(precision_, tau_);
     }
     if (red_ready_ && precision_ != 0 && !(mu >= kMmaMinRhs && eps_ >= kMmaMinEps)) {
-        // the warp-fed streams, with many right-hand sides against the digit planes
+        // the warp-fed streams, with many right-hand sides against the digit
+        // planes and the best phase 2 beside them: dense blocks in the
+        // streamed phase 2 leave the planes no case, dense blocks on the planes
+        // do (64 right-hand sides at epsilon 1e-6, streams / planes / both on
+        // the planes: 2 000 points 551 / 900 / 286 us, 30 000 points in leaves
+        // of up to 1 000 31.5 / 75.1 / 7.3 ms)
+        const bool many = mu >= kMmaMinRhs && n_tcblk_ > 0 && room_for_planes();
+        if (many && oz_on_)
+            set_digit_planes(false);
         best = timed();
-        if (mu >= kMmaMinRhs && n_tcblk_ > 0)
-            try_digit_planes();
+        if (many) {
+            const float streams = best;
+            const bool split = split_dense_;
+            const int mode = p2_mode_, gmax = p2_gmax_;
+            set_digit_planes(true);
+            p2_gmax_ = 8;
+            try_dense_split();
+            try_passes();
+            if (best >= streams && red_ready_) {
+                split_dense_ = split;
+                p2_mode_     = mode;
+                p2_gmax_     = gmax;
+                best         = streams;
+                set_digit_planes(false);
+            }
+        }
         HTGPU_CUDA(cudaEventDestroy(e0));
         HTGPU_CUDA(cudaEventDestroy(e1));
         if (best_ms)
@@ -2898,42 +2952,14 @@ void HMatrix::autotune(int mu, int reps, float *best_ms) {
         best                = std::min(t_split, t_pad);
         layout_gen_++;
     }
-    // the streamed phase 2 with 8 or more right-hand sides (reduced
-    // precision off the tensor cores): passes of 8, or of 4
+    // the streamed phase 2 of reduced precision off the tensor cores
     {
         const int run  = rhs_run(mu);
         const bool tcs = run >= kMmaMinRhs && eps_ >= kMmaMinEps;
-        if (precision_ != 0 && run >= 8 && !tcs) {
-            p2_gmax_         = 8;
-            const float t8   = timed();
-            p2_gmax_         = 4;
-            const float t4   = timed();
-            p2_gmax_         = t4 < t8 ? 4 : 8;
-            best             = std::min(t4, t8);
-            layout_gen_++;
-        }
-        // and, from 4 right-hand sides on, the dense chunks in the
-        // double-float kernel or in the streamed one, with either phase-2
-        // kernel for the rest
+        if (precision_ != 0 && run >= 8 && !tcs)
+            try_passes();
         if (precision_ != 0 && run >= 4 && !tcs) {
-            float tbest   = 1e30f;
-            bool arg_sp   = false;
-            int arg_mode  = p2_mode_;
-            for (bool sp : {false, true})
-                for (int m : {0, 1}) {
-                    split_dense_  = sp;
-                    p2_mode_      = m;
-                    const float t = timed();
-                    if (t < tbest) {
-                        tbest    = t;
-                        arg_sp   = sp;
-                        arg_mode = m;
-                    }
-                }
-            split_dense_ = arg_sp;
-            p2_mode_     = arg_mode;
-            best         = tbest;
-            layout_gen_++;
+            try_dense_split();
             // the digit planes again, now that the dense blocks may come
             // first (on the planes when they are on)
             if (run >= kMmaMinRhs && n_tcblk_ > 0)

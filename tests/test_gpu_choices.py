@@ -98,3 +98,29 @@ def test_waits_of_the_producer_kernel():
     hm.reset_status()
     assert np.array_equal(hm.mvprod_global_to_global(x), ref)
     assert hm.device_status() == 0
+
+
+@pytest.mark.parametrize("policy", ["fp32", "mixed"])
+def test_autotune_of_many_right_hand_sides(policy):
+    """leaves of up to 300 points: most of the work in dense blocks, which the
+    digit planes take at a fifth of the streams' time where they come first;
+    products with fewer right-hand sides stay on the streams.  Tolerance: FP32
+    sums of up to 256 terms either way, 256 x 2^-24 at most and far less at
+    random: below epsilon"""
+    n, mu = 12000, 64
+    pts = G.sphere(n, seed=12)
+    c = H.Cluster()
+    c.set_minclustersize(300)
+    t = c.build(n, pts)
+    hm = H.HMatrix(t, t, 1e-6, 10.0).build(H.LAPLACE, pts).set_precision(policy, 1.0)
+    x, x3 = G.rhs(n, mu, seed=13), G.rhs(n, 3, seed=14)
+    y, y3 = hm.mvprod_global_to_global(x, mu), hm.mvprod_global_to_global(x3, 3)
+    before = streams(hm)
+    for start in (False, True):
+        hm.set_digit_planes(start)
+        assert hm.autotune(mu, 3) > 0
+        assert hm.get_digit_planes()[0] and hm.get_phase2_dense_split()
+        assert streams(hm) == before
+        assert rel(hm.mvprod_global_to_global(x, mu), y) < 1e-6
+        assert np.array_equal(hm.mvprod_global_to_global(x3, 3), y3)
+    assert hm.device_status() == 0
