@@ -51,23 +51,29 @@ constexpr int kPairWarps = 4; // warps per CTA, each with its own panels and rin
 
 __device__ long long g_pair_skip = -1; // a panel whose first copy is left out (test support)
 
-// a double as hi + lo, both rounded to nearest (|a - hi - lo| <= 2^-48 |a|; the
-// truncating split64 of the other kernels keeps 2^-46), by bit operations:
-// the conversions between double and float run on the FP64 pipe. |a| < 2^126;
-// below 2^-103 (and zero) gives 0, a value that is not finite NaN, so that it
-// reaches the outputs
+// a double as hi + lo, both rounded to nearest (|a - hi - lo| <= 2^-48 |a|, and
+// 2^-149 below 2^-101, where the floats run into the subnormal ones; the
+// truncating split64 of the other kernels keeps 2^-46 and drops what is below
+// 2^-103), by bit operations: the conversions between double and float run on
+// the FP64 pipe. |a| < 2^126; zero gives 0, a value that is not finite NaN, so
+// that it reaches the outputs
 __device__ __forceinline__ F2 split64_near(double a) {
     const long long b  = __double_as_longlong(a);
     const int e        = (int)(b >> 52) & 0x7FF;
     const long long m  = b + (1LL << 28);           // hi: 29 bits rounded off
-    const unsigned mh  = (unsigned)(m >> 32);
-    const unsigned hb  = (((unsigned)(m >> 29)) - 0xC0000000u) | (mh & 0x80000000u); // exponent 1023 -> 127 (mod 512), 23 fraction bits
+    const unsigned sg  = (unsigned)((unsigned long long)b >> 32) & 0x80000000u;
+    const unsigned hb  = (((unsigned)(m >> 29)) - 0xC0000000u) | sg; // exponent 1023 -> 127 (mod 512), 23 fraction bits
     const int r        = (int)(b - (m & ~((1LL << 29) - 1))); // a - hi in units of 2^(e - 1075), |r| <= 2^28
     F2 f;
     const float lo = (__int2float_rn(r) * 9.31322574615478515625e-10f) * __int_as_float((e - 918) << 23); // 2^-30, 2^(e - 1045)
     const bool ok  = (unsigned)(e - 920) < 229u;
     f.hi           = ok ? __uint_as_float(hb) : e == 0x7FF ? __int_as_float(0x7fffffff) : 0.f;
-    f.lo           = ok ? __int_as_float(__float_as_int(lo) ^ (int)((unsigned)(b >> 32) & 0x80000000u)) : 0.f;
+    f.lo           = ok ? __int_as_float(__float_as_int(lo) ^ (int)sg) : 0.f;
+    if ((unsigned)(e - 873) < 47u) { // the same, each scaled down by two normal powers of two
+        const int eh = (int)(m >> 52) & 0x7FF;
+        f.hi = __int_as_float(__float_as_int((__uint_as_float((hb & 0x7FFFFFu) | 0x3F800000u) * 0x1p-64f) * __int_as_float((eh - 832) << 23)) ^ (int)sg);
+        f.lo = __int_as_float(__float_as_int((__int2float_rn(r) * 0x1p-94f) * __int_as_float((e - 854) << 23)) ^ (int)sg);
+    }
     return f;
 }
 
