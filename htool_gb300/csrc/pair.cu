@@ -587,9 +587,11 @@ __global__ void pair_zsum_kernel(const ZItem *__restrict__ items, int nitems, co
             df_renorm(a);
         }
         const double v = df_to_double(a);
-        // NaN stays NaN through the scaling (an exponent field of 0x7FF has no room)
+        // an infinity or NaN has no room in its exponent field, and what has none after the scaling is infinite
+        const int ex   = (int)(((unsigned)__double2hiint(v) >> 20) & 0x7FFu);
+        const double o = ex == 0x7FF ? v : ex + xs < 0x7FF ? scale_pow2_safe(v, xs) : copysign(__longlong_as_double(0x7FFll << 52), v);
         if (e0 + lane < n)
-            y[(long long)c * ldy + (perm ? perm[i] : i - shift)] = v == v ? scale_pow2_safe(v, xs) : v;
+            y[(long long)c * ldy + (perm ? perm[i] : i - shift)] = o;
     }
 }
 
