@@ -31,11 +31,14 @@
 // Measured against the tile and chunk kernels of stream.cu and
 // matvec_kernels.cu (which shuffle every coefficient, reduce every tile over
 // the warp and leave lanes idle on tiles of few rows), Laplace sphere, FP64:
-//   100 000 points  1 right-hand side 0.489 -> 0.356 ms, 2: 0.82 -> 0.40,
-//                   4: 1.79 -> 0.57, 8: 2.66 -> 1.01
-//   400 000 points  1: 2.11 -> 1.58 (6.7 TB/s in phase 1, 7.0 in phase 2, a
-//                   copy takes 6.8), 4: 7.94 -> 2.42
-// at no larger an error against the FP64 pipe (1.2e-14 .. 2.0e-14).
+//   100 000 points  1 right-hand side 0.485 -> 0.342 ms, 2: 0.82 -> 0.379,
+//                   4: 1.81 -> 0.551, 8: 2.66 -> 0.989
+//   400 000 points  1: 2.15 -> 1.57 (6.7 TB/s in phase 1, 7.0 in phase 2, a
+//                   copy takes 6.8), 4: 8.05 -> 2.42
+// at no larger an error against the FP64 pipe, though 35% of phase 2 ran on it
+// there (six inputs each; Laplace 1.9e-14 .. 2.3e-14 -> 1.0e-14 .. 1.8e-14,
+// Helmholtz 2.6e-14 .. 4.8e-14 -> 2.4e-14 .. 3.1e-14): both operands are rounded
+// to 2^-48 here and truncated at 2^-46 there.
 //
 // Every wait is bounded; a warp whose wait ran out records status 2, lets its
 // copies in flight land (again bounded) and ends.

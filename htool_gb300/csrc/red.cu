@@ -22,8 +22,8 @@
 // reading half the coefficients, two rows a lane, gained 1%), so descriptors and
 // indices are loaded ahead and a row chunk starts from its dense part.  Measured
 // against those kernels, Laplace sphere, FP32/BF16 factors, ms a product:
-// 100 000 points 1 right-hand side 0.258 -> 0.232, 2: 0.365 -> 0.276, 4: 0.726 ->
-// 0.304, 8: 1.835 -> 0.435; 200 000 points 1: 0.499 -> 0.467, 8: 3.68 -> 0.813.
+// 100 000 points 1 right-hand side 0.258 -> 0.221, 2: 0.362 -> 0.268, 4: 0.720 ->
+// 0.297, 8: 1.82 -> 0.418; 200 000 points 1: 0.505 -> 0.460, 8: 3.66 -> 0.799.
 // Every wait is bounded (status 2).
 #include "f32x2.cuh"
 #include "kernels.hpp"
