@@ -65,6 +65,11 @@ __device__ __forceinline__ bool red_f32(int m) { return m >> 13 & 1; }
 __device__ __forceinline__ int red_flags(int m) { return (m >> 14) & 31; }
 __device__ __forceinline__ int red_end(int m) { return (m >> 19) & 255; }
 
+// one float global -> shared, or zero (nothing is read)
+__device__ __forceinline__ void copy_or_zero(float *dst, const float *src, bool live) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(sa(dst)), "l"(src), "r"(live ? 4 : 0) : "memory");
+}
+
 // W floats (one row or slot) global -> shared, W x 4-byte aligned
 template <int W>
 __device__ __forceinline__ void copy_row(float *dst, const float *src) {
@@ -390,9 +395,9 @@ __global__ void __launch_bounds__(32 * kRedWarps, Red2Cfg<W>::kCtas)
                 };
 #pragma unroll
                 for (int r = 0; r < 2; r++)
-                    if (lane + 32 * r < ncol)
-                        copy_async<4>(at(lane + 32 * r), A + (r ? d0.ix1 : d0.ix0));
-                for (int t = ncol + lane; t < end; t += 32)
+                    if (lane + 32 * r < end)
+                        copy_or_zero(at(lane + 32 * r), A + (r ? d0.ix1 : d0.ix0), lane + 32 * r < ncol);
+                for (int t = 64 + lane; t < end; t += 32)
                     *at(t) = 0.f;
             } else {
                 using V = std::conditional_t<W % 4 == 0, float4, float2>;
